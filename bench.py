@@ -257,8 +257,13 @@ class Step:
         self.o = torch.empty_like(q)
         self.lse = torch.empty(self.B, self.H, self.T, dtype=torch.float32, device=q.device)
         self.dq, self.dk, self.dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        self.scratch = torch.empty(self.lib.nlfa_bwd_fused_scratch_bytes(self.B, self.T, self.H, self.D),
+        self.scratch = torch.empty(max(self.lib.nlfa_bwd_fused_scratch_bytes(self.B, self.T, self.H, self.D),
+                                       self.lib.nlfa_bwd_workspace_bytes(*self._mask_dims())),
                                    dtype=torch.uint8, device=q.device)
+
+    def _mask_dims(self):
+        return (self.B, self.T, self.H, self.Hkv, self.D, self.window, self.sinks, 0, self.L.DTYPE_BF16,
+                self.L.PATH_TENSOR)
 
     def _dims(self):
         return (self.B, self.T, self.H, self.Hkv, self.D, self.scale, self.window, self.sinks,
@@ -288,9 +293,9 @@ class Step:
     @property
     def launches_per_step(self):
         """Forward + what the backward launches for this shape: Delta, dK/dV, dQ -- or, for a large
-        problem at D = 64, the dQ pass that forms Delta itself and then dK/dV."""
-        return 1 + self.lib.nlfa_bwd_kernel_count(self.B, self.T, self.H, self.D, self.L.DTYPE_BF16,
-                                                  self.L.PATH_TENSOR, self.L.PASS_ALL)
+        problem at D = 64, the dQ pass that forms Delta itself and then dK/dV; at D = 128 dK/dV and dQ
+        once per part of the problem whose dS the scratch holds."""
+        return 1 + self.lib.nlfa_bwd_workspace_kernel_count(*self._mask_dims(), self.scratch.numel())
 
     def captured(self):
         """The same step as one CUDA graph (replayed, the host issues one launch per step)."""

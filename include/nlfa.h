@@ -100,6 +100,20 @@ int nlfa_fwd_masked(const void* q, const void* k, const void* v, void* o, float*
  * The reference allocates the same tensor itself (flash_attn_cuda.cu:1770-1773). */
 size_t nlfa_bwd_scratch_bytes(int B, int T, int H);
 
+/* Bytes of scratch with which the backward runs fastest: the tape, and behind it (rounded up to 256
+ * bytes) room for dS of as many (batch, KV head) pairs as fit 2 GiB -- 32 KB per query head, 128-row
+ * query tile and 128-key block the tile sees.  Given at least one pair's worth, the entry points below
+ * (every pass asked for, tensor-core path) let the dK/dV kernel leave dS there and form dQ as one product
+ * over it, that many pairs per launch; given less they recompute dS in the dQ kernel.  Same bits either way.
+ * Equals nlfa_bwd_scratch_bytes where there is nothing to gain (head dims below 128, fp32 path, a pair larger
+ * than 2 GiB). */
+size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
+                                int path);
+
+/* Kernels the whole backward launches with that much scratch (0: arguments it refuses). */
+int nlfa_bwd_workspace_kernel_count(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
+                                    int path, size_t scratch_bytes);
+
 /* Backward: Delta = rowsum(dO * O), then dQ, dK, dV with P recomputed from the
  * taped lse.  Replaces `flash_attn_bwd` (nanolab/csrc/flash_attn_cuda.cu:1744-1813)
  * and its launch sequence (:1518-1587): Delta kernel, dK/dV kernel, dQ kernel on

@@ -32,6 +32,8 @@ SIGNATURES = {
     "nlfa_bwd_masked": (_c_int, [_c_void_p] * 10 + [_c_size_t] + [_c_int] * 5 + [_c_float]
                         + [_c_int] * 6 + [_c_void_p]),
     "nlfa_bwd_scratch_bytes": (_c_size_t, [_c_int, _c_int, _c_int]),
+    "nlfa_bwd_workspace_bytes": (_c_size_t, [_c_int] * 10),
+    "nlfa_bwd_workspace_kernel_count": (_c_int, [_c_int] * 10 + [_c_size_t]),
     "nlfa_bwd": (_c_int, [_c_void_p] * 10 + [_c_size_t] + [_c_int] * 5 + [_c_float]
                  + [_c_int] * 4 + [_c_void_p]),
     "nlfa_bwd_passes": (_c_int, [_c_void_p] * 10 + [_c_size_t] + [_c_int] * 5 + [_c_float]

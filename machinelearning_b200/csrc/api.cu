@@ -111,6 +111,12 @@ int check_problem(const Problem& p) {
   return NLFA_OK;
 }
 
+// Masks that cut nothing become the plain causal one.
+void simplify_mask(Problem& p) {
+  if (p.window > 0 && p.window - p.sinks >= p.T) p.window = p.sinks = 0;      // the window never cuts anything
+  if (p.block == 1) p.block = 0;                                             // blocks of one position
+}
+
 float bits_to_float(uint16_t bits, int dtype) {
   if (dtype == NLFA_DTYPE_BF16) {
     uint32_t w = static_cast<uint32_t>(bits) << 16;
@@ -349,11 +355,7 @@ int nlfa_fwd_masked(const void* q, const void* k, const void* v, void* o, float*
   if (B == 0 || T == 0 || H == 0) return NLFA_OK;
   if (!q || !k || !v || !o || !lse) return NLFA_ERR_NULL_POINTER;
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return NLFA_ERR_MISALIGNED;
-  if (p.window > 0 && p.window - p.sinks >= p.T) {
-    p.window = 0;            // the window never cuts anything: plain causal
-    p.sinks = 0;
-  }
-  if (p.block == 1) p.block = 0;                            // blocks of one position: plain causal
+  simplify_mask(p);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (resolved == NLFA_PATH_SIMT) return launch_fwd_simt(p, q, k, v, o, lse, s);
   if (!nlfa_device_supported()) return NLFA_ERR_NOT_SM100;
@@ -378,7 +380,29 @@ int nlfa_bwd(const void* dout, const void* q, const void* k, const void* v, cons
 
 namespace {
 size_t round256(size_t n) { return (n + 255) / 256 * 256; }
+
+// Bytes of the dS tiles of one (batch, KV head) pair.
+size_t ds_pair_bytes(const Problem& p) {
+  const DsLayout l = ds_layout(p.T, p.window, p.sinks, p.block);
+  return static_cast<size_t>(ds_tile_offset(l, l.n_tiles)) * kDsTileBytes * (p.H / p.Hkv);
+}
+
+constexpr size_t kDsMostBytes = size_t{2} << 30;        // dS of as many pairs at a time as fit here
 }  // namespace
+
+size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
+                                int path) {
+  const size_t tape = nlfa_bwd_scratch_bytes(B, T, H);
+  Problem p{B, T, H, Hkv, D, window, sinks, 1.f, dtype, block};
+  if (tape == 0 || check_problem(p) != NLFA_OK || D != 128 ||
+      nlfa_resolve_path(dtype, D, path) != NLFA_PATH_TENSOR)
+    return tape;
+  simplify_mask(p);
+  const size_t pair = ds_pair_bytes(p), all = static_cast<size_t>(B) * Hkv;
+  const size_t most = kDsMostBytes / pair;
+  if (most == 0) return tape;
+  return round256(tape) + pair * (all < most ? all : most);
+}
 
 size_t nlfa_bwd_fused_scratch_bytes(int B, int T, int H, int D) {
   if (B <= 0 || T <= 0 || H <= 0) return 0;
@@ -416,6 +440,18 @@ int nlfa_bwd_kernel_count(int B, int T, int H, int D, int dtype, int path, int p
   return delta + two;
 }
 
+int nlfa_bwd_workspace_kernel_count(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
+                                    int path, size_t scratch_bytes) {
+  Problem p{B, T, H, Hkv, D, window, sinks, 1.f, dtype, block};
+  if (B <= 0 || T <= 0 || H <= 0 || check_problem(p) != NLFA_OK) return 0;
+  simplify_mask(p);
+  const size_t tape = round256(nlfa_bwd_scratch_bytes(B, T, H)), pair = ds_pair_bytes(p);
+  if (D != 128 || nlfa_resolve_path(dtype, D, path) != NLFA_PATH_TENSOR || scratch_bytes < tape + pair)
+    return nlfa_bwd_kernel_count(B, T, H, D, dtype, path, NLFA_PASS_ALL);
+  const size_t pairs = (scratch_bytes - tape) / pair, all = static_cast<size_t>(B) * Hkv;
+  return 1 + 2 * static_cast<int>((all + pairs - 1) / pairs);
+}
+
 int nlfa_bwd_passes(const void* dout, const void* q, const void* k, const void* v, const void* o,
                     const float* lse, void* dq, void* dk, void* dv, void* scratch,
                     size_t scratch_bytes, int B, int T, int H, int Hkv, int D, float scale,
@@ -446,11 +482,7 @@ int nlfa_bwd_masked(const void* dout, const void* q, const void* k, const void* 
   if (want_fused && !aligned16(scratch)) return NLFA_ERR_MISALIGNED;
   if (scratch_bytes < (want_fused ? nlfa_bwd_fused_scratch_bytes(B, T, H, D) : nlfa_bwd_scratch_bytes(B, T, H)))
     return NLFA_ERR_SCRATCH_TOO_SMALL;
-  if (p.window > 0 && p.window - p.sinks >= p.T) {
-    p.window = 0;
-    p.sinks = 0;
-  }
-  if (p.block == 1) p.block = 0;
+  simplify_mask(p);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* delta = static_cast<float*>(scratch);
   if (resolved == NLFA_PATH_SIMT)
@@ -466,8 +498,16 @@ int nlfa_bwd_masked(const void* dout, const void* q, const void* k, const void* 
     fs.dq_turn = reinterpret_cast<unsigned*>(ws);
     fs.dq_acc = reinterpret_cast<float*>(ws + round256(tiles * sizeof(unsigned)));
   }
+  // room for dS behind the tape (nlfa_bwd_workspace_bytes): the dK/dV pass leaves it there for the dQ pass
+  DsScratch ds{nullptr, 0};
+  const size_t tape = round256(nlfa_bwd_scratch_bytes(B, T, H)), pair = ds_pair_bytes(p);
+  if (passes == NLFA_PASS_ALL && D == 128 && aligned16(scratch) && scratch_bytes >= tape + pair) {
+    ds.tiles = static_cast<uint8_t*>(scratch) + tape;
+    const size_t n = (scratch_bytes - tape) / pair, all = static_cast<size_t>(B) * Hkv;
+    ds.pairs = static_cast<int>(n < all ? n : all);
+  }
   return launch_bwd_tc(p, dout, q, k, v, o, lse, dq, dk, dv, delta, passes, status, s,
-                       want_fused ? &fs : nullptr);
+                       want_fused ? &fs : nullptr, ds.pairs > 0 ? &ds : nullptr);
 }
 
 int nlfa_selftest_tiles(int dtype, int head_dim, const void* q, const void* k, const void* v,

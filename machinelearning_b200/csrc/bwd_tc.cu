@@ -40,7 +40,7 @@ namespace nlfa {
 
 namespace {
 
-enum { MODE_DQ = 0, MODE_DKV = 1, MODE_FUSED = 2 };
+enum { MODE_DQ = 0, MODE_DKV = 1, MODE_FUSED = 2, MODE_DKV_DS = 3 };
 
 struct BwdParams {
   int T, H, Hkv;
@@ -61,6 +61,11 @@ struct BwdParams {
   float* dq_acc;         // per (b, h, query tile): 128 x 64 fp32 partial sums, rows permuted (see drain)
   unsigned* dq_turn;     // per (b, h, query tile): how many key blocks have added their share
   int sched_group;       // (batch, KV head) pairs whose units are handed out together
+  // dK/dV pass that leaves dS behind (MODE_DKV_DS)
+  uint8_t* ds;           // tiles of the pairs of this launch, laid out as bwd_dq.cu reads them
+  DsLayout ds_layout;
+  int ds_per_head;       // tiles per query head
+  int first_pair;        // first (batch, KV head) pair of this launch
   float* delta_out;      // dQ pass, when it also forms Delta (see kDeltaIn): where the dK/dV pass will read it
   int delta_in_pass;     // 1: this dQ launch computes Delta = rowsum(dO * O) itself, tile by tile
   int dep_wait_first;    // 1: wait for the stream's previous kernel before the first global read; 0: the
@@ -68,14 +73,14 @@ struct BwdParams {
                          // read -- it is waited for on the way out instead
 };
 
-template <int D, int STAGES, int XBUF, int YR, bool FUSED = false, bool DELTA = false>
+template <int D, int STAGES, int XBUF, int YR, bool DS_TILE = false, bool DELTA = false>
 struct BwdSmem {
   static constexpr int kTileBytes = kTile * D * 2;              // stationary tile: 128 rows
   static constexpr int kYTileBytes = YR * D * 2;                // streamed tile: YR rows
   static constexpr int kX = 0;                                  // [XBUF] x (X0, X1)
   static constexpr int kY = kX + XBUF * 2 * kTileBytes;         // per stage: Y0, Y1
-  static constexpr int kDs = kY + STAGES * 2 * kYTileBytes;     // fused pass: dS^T [128 keys][128 queries] 16-bit
-  static constexpr int kO = kDs + (FUSED ? kTile * YR * 2 : 0);     // dQ pass forming Delta: the next unit's O tile
+  static constexpr int kDs = kY + STAGES * 2 * kYTileBytes;     // fused pass, dS-leaving pass: dS^T [128 keys][YR queries] 16-bit
+  static constexpr int kO = kDs + (DS_TILE ? kTile * YR * 2 : 0);     // dQ pass forming Delta: the next unit's O tile
   static constexpr int kVec = kO + (DELTA ? kTileBytes : 0);        // per stage: -lse2[YR], -delta[YR]
   static constexpr int kDeltaS = kVec + STAGES * 1024;              // dQ pass forming Delta: [XBUF][128] fp32
   static constexpr int kBar = kDeltaS + (DELTA ? XBUF * 512 : 0);
@@ -83,8 +88,8 @@ struct BwdSmem {
   //           sched_full[kRing], y_full[S], y_empty[S]
   static constexpr int kRing = 8;
   //           unit_done, out_drained, dq_ready, dq_drained, group, issued[4],
-  //           o_full, o_empty, delta_full[XBUF]
-  static constexpr int kNumBars = 2 * XBUF + 4 + kRing + 2 * STAGES + 9 + 2 + XBUF;
+  //           o_full, o_empty, delta_full[XBUF], ds_staged, ds_free
+  static constexpr int kNumBars = 2 * XBUF + 4 + kRing + 2 * STAGES + 9 + 2 + XBUF + 2;
   static constexpr int kSched = (kBar + 8 * kNumBars + 15) / 16 * 16;   // ring of unit descriptors (8 ints each)
   static constexpr int kTmemSlot = kSched + 32 * kRing;
   static constexpr int kAbort = kTmemSlot + 4;
@@ -145,11 +150,16 @@ __device__ __forceinline__ BwdUnit<MODE> make_bwd_unit(int u, const BwdParams& p
     w.n_iters = w.n_inner;
   } else {
     w.tile = rank;                              // early key blocks are seen by the most queries
+    if (MODE == MODE_DKV_DS) bh += p.first_pair;
     w.b = bh / p.Hkv;
     w.hk = bh - w.b * p.Hkv;
     w.h = w.hk * group;
     w.s_lo = first_query_of_key(w.tile * kTile, p.block) / YR;   // first query tile that reaches the block
-    const int s_hi = last_query_tile_of_block(w.tile, p.n_ytiles, YR, p.window, p.sinks);
+    int s_hi = last_query_tile_of_block(w.tile, p.n_ytiles, YR, p.window, p.sinks);
+    if (MODE == MODE_DKV_DS) {                  // dS tiles hold 128 queries: both halves of each are written
+      w.s_lo &= ~1;
+      s_hi = (s_hi | 1) < p.n_ytiles ? (s_hi | 1) : p.n_ytiles - 1;
+    }
     w.extra = 0;
     w.n_inner = s_hi - w.s_lo + 1;
     w.n_iters = w.n_inner * group;
@@ -199,8 +209,9 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
   // (a full pass over dO and O) from the backward.  Same arithmetic, same order of additions as
   // delta_vec_kernel, so the results are bit-identical to it.
   constexpr bool kDeltaIn = MODE == MODE_DQ && XBUF == 2 && D == 64;
-  using L = BwdSmem<D, STAGES, XBUF, YR, MODE == MODE_FUSED, kDeltaIn>;
+  using L = BwdSmem<D, STAGES, XBUF, YR, MODE == MODE_FUSED || MODE == MODE_DKV_DS, kDeltaIn>;
   static_assert(YR == 64 || YR == 128, "streamed tiles are 64 or 128 rows");
+  static_assert(MODE != MODE_DKV_DS || (D == 128 && YR == 64), "dS is left behind at head dim 128 only");
   static_assert(MODE != MODE_FUSED || (D == 64 && YR == 128), "the fused pass exists for 64-wide tiles");
   constexpr int kBoxes = D / 64;
   constexpr int kBoxBytes = kTile * 128;          // one 64-column box of a stationary tile
@@ -235,7 +246,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
                 UNIT_DONE = Y_EMPTY + STAGES, OUT_DRAINED = UNIT_DONE + 1,
                 DQ_READY = UNIT_DONE + 2, DQ_DRAINED = UNIT_DONE + 3, GROUP = UNIT_DONE + 4,
                 ISSUED = UNIT_DONE + 5,          // [4]: iteration g uses ISSUED + (g & 3)
-                O_FULL = ISSUED + 4, O_EMPTY = O_FULL + 1, DELTA_FULL = O_FULL + 2;   // DELTA_FULL[XBUF]
+                O_FULL = ISSUED + 4, O_EMPTY = O_FULL + 1, DELTA_FULL = O_FULL + 2,   // DELTA_FULL[XBUF]
+                DS_STAGED = DELTA_FULL + XBUF, DS_FREE = DS_STAGED + 1;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + L::kAbort);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L::kTmemSlot);
   volatile int* sched_ring = reinterpret_cast<volatile int*>(gen + L::kSched);
@@ -260,6 +272,8 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
     mbar_init(bar(O_FULL), 1);
     mbar_init(bar(O_EMPTY), 4);              // one arrival per epilogue warp
     for (int i = 0; i < XBUF; ++i) mbar_init(bar(DELTA_FULL + i), 4);
+    mbar_init(bar(DS_STAGED), 256);
+    mbar_init(bar(DS_FREE), 1);
     reinterpret_cast<volatile int*>(gen + L::kTurnOk)[0] = 0;      // iterations whose turn has come
     reinterpret_cast<volatile int*>(gen + L::kTurnOk)[1] = 0;      // iterations whose share has been released
     for (int i = 0; i < kRing; ++i) mbar_init(bar(SCHED_FULL + i), 1);
@@ -310,8 +324,39 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
   // warps that shrink must free at least what the eight that grow take.
   static_assert((kRegsLaunch - kRegsOther) * 8 >= (kRegsCompute - kRegsLaunch) * 8,
                 "register reallocation does not balance");
-  if (dead || ((warp == 10 || warp == 11) && (!kFused || lane != 0))) {
+  constexpr bool kLeaveDs = MODE == MODE_DKV_DS;
+  if (dead || ((warp == 10 || warp == 11) && (!(kFused || (kLeaveDs && warp == 10)) || lane != 0))) {
     // nothing to do (spare warps only complete the warpgroup)
+  } else if (kLeaveDs && warp == 10) {
+    // ============ dS for the dQ pass: one lane sends each staged tile to the scratch =================
+    bool ok = true;
+    int g = 0;
+    for (int uc = 0; ok; ++uc) {
+      BwdUnit<MODE> w;
+      const int u = next_unit(uc, ok, w);
+      if (!ok || u < 0) break;
+      const long long head = static_cast<long long>(w.b) * p.H + w.h - static_cast<long long>(p.first_pair) * (p.H / p.Hkv);
+      uint8_t* tiles = p.ds + head * p.ds_per_head * kDsTileBytes;
+      int inner = 0;
+      for (int it = 0; it < w.n_iters; ++it, ++g, ++inner) {
+        if (inner == w.n_inner) {
+          inner = 0;
+          tiles += static_cast<long long>(p.ds_per_head) * kDsTileBytes;
+        }
+        const int idx = w.s_lo + inner, qt = idx >> 1;             // 64-query tile; the 128-query tile it is half of
+        int n_blocks;
+        const int slot = ds_tile_offset(p.ds_layout, qt) +
+                         dq_turn_of_block(w.tile, qt, p.window, p.sinks, &n_blocks, p.block, p.ds_layout.n_tiles);
+        uint8_t* dst = tiles + static_cast<long long>(slot) * kDsTileBytes + (idx & 1) * (kDsTileBytes / 4);
+        if (!(ok = mbar_wait_idle(bar(DS_STAGED), g & 1, wctx, 50))) break;
+        bulk_store(dst, base + L::kDs, kDsTileBytes / 4);           // keys 0-63
+        bulk_store(dst + kDsTileBytes / 2, base + L::kDs + kDsTileBytes / 4, kDsTileBytes / 4);
+        tma_store_commit();
+        tma_store_wait_read();
+        mbar_arrive(bar(DS_FREE));
+      }
+    }
+    tma_store_wait_all();
   } else if (warp == 10 || warp == 11) {
     // ===================== fused pass: turn watcher (warp 10), releaser (warp 11) ==================
     // The dQ shares of a query tile are added to its fp32 sums in a fixed order -- ascending key
@@ -891,7 +936,9 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
       unsigned vw;
       // the causal edge as this row sees it: a query's last visible key, a key's first query
       // (block-causal masks move both to the ends of the row's block)
-      const int edge = MODE == MODE_DQ ? last_key_of_query(pos, p.block, p.T) : first_query_of_key(pos, p.block);
+      // (a key past the end of the sequence is seen by no query: its dS is multiplied with a zero row of K)
+      const int edge = MODE == MODE_DQ ? last_key_of_query(pos, p.block, p.T)
+                       : MODE == MODE_DKV_DS && pos >= p.T ? 1 << 30 : first_query_of_key(pos, p.block);
       if (MODE == MODE_DQ) {                           // row = query `pos`, columns = keys
         const int lo = p.window > 0 ? pos - (p.window - p.sinks) + 1 : 0;
         va = lo > 0 ? lo : 0;
@@ -1105,6 +1152,21 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
         tc_wait_st();
         tc_fence_before();
         mbar_arrive(bar(PD_FULL));
+        if constexpr (MODE == MODE_DKV_DS) {
+          // dS for the dQ pass, staged as bwd_dq.cu's matrix descriptor takes it: eight queries of one key
+          // are 16 bytes, 64 keys of them 1024 (a warp's store is 512 contiguous bytes).  Warp 10 sends it off.
+          if (g > 0) {
+            ok = mbar_wait(bar(DS_FREE), (g - 1) & 1, wctx, 51);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+          }
+          const uint32_t dst = base + L::kDs + (row >> 6) * (YR * 128) + (YR / 16) * half * 1024 + (row & 63) * 16;
+#pragma unroll
+          for (int c = 0; c < 4 * kCh; ++c)
+            st_shared_v4(dst + c * 1024, dd[4 * c], dd[4 * c + 1], dd[4 * c + 2], dd[4 * c + 3]);
+          fence_proxy_async_smem();
+          mbar_arrive(bar(DS_STAGED));
+        }
       }
       if (!ok) break;
 
@@ -1139,7 +1201,7 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
                 const float* lse, const float* delta, void* out0, void* out1, unsigned* status,
                 cudaStream_t stream, void* dq = nullptr, const FusedScratch* fused = nullptr,
                 bool beside_previous = false, const void* o_for_delta = nullptr, float* delta_out = nullptr,
-                bool plain_launch = false) {
+                bool plain_launch = false, void* ds = nullptr, int first_pair = 0, int pairs = 0) {
   // stationary tensors in boxes of 128 rows, streamed tensors in boxes of YR rows; output tiles
   // leave through TMA stores: dQ is [B,T,H,D], dK and dV are [B,T,Hkv,D]
   const void* x0 = MODE == MODE_DQ ? q : k;
@@ -1161,7 +1223,7 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
   if (mst != NLFA_OK) return mst;
   constexpr bool kDeltaIn = MODE == MODE_DQ && XBUF == 2 && D == 64;
   if (o_for_delta != nullptr && !kDeltaIn) return NLFA_ERR_UNSUPPORTED_PATH;
-  using L = BwdSmem<D, STAGES, XBUF, YR, MODE == MODE_FUSED, kDeltaIn>;
+  using L = BwdSmem<D, STAGES, XBUF, YR, MODE == MODE_FUSED || MODE == MODE_DKV_DS, kDeltaIn>;
   static_assert(L::kDynamic <= 232448, "over the shared memory a CTA can have");
   auto kern = bwd_tc_kernel<T, D, MODE, STAGES, XBUF, YR>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kDynamic) != NLFA_OK)
@@ -1176,6 +1238,13 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
   bp.n_tiles = (p.T + kTile - 1) / kTile;
   bp.n_ytiles = (p.T + YR - 1) / YR;
   bp.BH = p.B * (MODE == MODE_DQ ? p.H : p.Hkv);
+  if (MODE == MODE_DKV_DS) {
+    bp.BH = pairs;
+    bp.ds = static_cast<uint8_t*>(ds);
+    bp.ds_layout = ds_layout(p.T, p.window, p.sinks, p.block);
+    bp.ds_per_head = ds_tile_offset(bp.ds_layout, bp.n_tiles);
+    bp.first_pair = first_pair;
+  }
   bp.total_units = bp.n_tiles * bp.BH;
   bp.scale = p.scale;
   bp.scale_log2 = p.scale * kLog2e;
@@ -1238,8 +1307,27 @@ inline bool delta_in_dq_pass(const Problem& p, int passes) {
 template <typename T, int D, int STAGES, int XBUF, int YR>
 int launch_both(const Problem& p, const void* dout, const void* q, const void* k, const void* v, const void* o,
                 const float* lse, float* delta, void* dq, void* dk, void* dv, int passes,
-                unsigned* status, cudaStream_t stream, const FusedScratch* fused) {
+                unsigned* status, cudaStream_t stream, const FusedScratch* fused, const DsScratch* ds) {
   int st = NLFA_OK;
+  if constexpr (D == 128) if (ds != nullptr) {
+    // The dK/dV pass leaves dS in the scratch and the dQ pass is one product over it: five products and one
+    // exponent phase per tile pair instead of seven and two.  As many (batch, KV head) pairs at a time as
+    // the scratch holds, shared out evenly.  At D = 128 the dS traffic (32 KB written and read per pair of
+    // 128 x 128) hides behind the pass's products and the dQ pass runs at DRAM speed: B=1 H=16 T=16384
+    // backward 3.70 -> 3.08 ms, B=2 T=8192 1.82 -> 1.64 ms, B=4 H=12/4 T=2048 190 -> 172 us.  At D = 64 a
+    // tile pair has half the products for the same bytes and the staging tile costs a streamed stage
+    // (B=32 H=12 T=1024: 274 -> 300 us), so there the dQ pass recomputes dS.
+    const DsLayout layout = ds_layout(p.T, p.window, p.sinks, p.block);
+    const int all = p.B * p.Hkv, chunks = (all + ds->pairs - 1) / ds->pairs, per = (all + chunks - 1) / chunks;
+    for (int first = 0; first < all; first += per) {
+      const int pairs = all - first < per ? all - first : per;
+      st = launch_mode<T, D, MODE_DKV_DS, STAGES, XBUF, YR>(p, dout, q, k, v, lse, delta, dk, dv, status, stream, nullptr,
+                                                           nullptr, false, nullptr, nullptr, false, ds->tiles, first, pairs);
+      if (st == NLFA_OK) st = launch_dq_from_ds(p, k, ds->tiles, layout, first, pairs, dq, status, stream);
+      if (st != NLFA_OK) return st;
+    }
+    return NLFA_OK;
+  }
   if constexpr (D == 64 && YR == 128) {
     // one pass for all three gradients: three streamed stages (the dS tile takes the fourth's room)
     if (passes & NLFA_PASS_FUSED)
@@ -1273,7 +1361,8 @@ bool bwd_delta_in_dq(const Problem& p, int passes) { return delta_in_dq_pass(p, 
 
 int launch_bwd_tc(const Problem& p, const void* dout, const void* q, const void* k, const void* v,
                   const void* o, const float* lse, void* dq, void* dk, void* dv, float* delta,
-                  int passes, unsigned* status, cudaStream_t stream, const FusedScratch* fused) {
+                  int passes, unsigned* status, cudaStream_t stream, const FusedScratch* fused,
+                  const DsScratch* ds) {
   if (p.dtype != NLFA_DTYPE_F16 && p.dtype != NLFA_DTYPE_BF16) return NLFA_ERR_UNSUPPORTED_PATH;
   if (p.D != 32 && p.D != 64 && p.D != 128) return NLFA_ERR_UNSUPPORTED_PATH;
   if ((passes & NLFA_PASS_FUSED) && p.D > 64) return NLFA_ERR_UNSUPPORTED_PATH;
@@ -1281,19 +1370,19 @@ int launch_bwd_tc(const Problem& p, const void* dout, const void* q, const void*
   // TMA boxes are 64 wide, so loads fill columns 32-63 with zeros (which add nothing to any
   // product) and stores drop them.
   int st = NLFA_OK;
-  if ((passes & NLFA_PASS_DELTA) && !delta_in_dq_pass(p, passes)) st = launch_delta(p, dout, o, delta, stream);
+  if ((passes & NLFA_PASS_DELTA) && (ds != nullptr || !delta_in_dq_pass(p, passes))) st = launch_delta(p, dout, o, delta, stream);
   if (st != NLFA_OK) return st;
   const bool bf16 = p.dtype == NLFA_DTYPE_BF16;
   if (p.D <= 64) {
     // 128-row streamed tiles, four stages, two stationary buffers
-    return bf16 ? launch_both<__nv_bfloat16, 64, 4, 2, 128>(p, dout, q, k, v, o, lse, delta, dq, dk, dv, passes, status, stream, fused)
-                : launch_both<__half, 64, 4, 2, 128>(p, dout, q, k, v, o, lse, delta, dq, dk, dv, passes, status, stream, fused);
+    return bf16 ? launch_both<__nv_bfloat16, 64, 4, 2, 128>(p, dout, q, k, v, o, lse, delta, dq, dk, dv, passes, status, stream, fused, ds)
+                : launch_both<__half, 64, 4, 2, 128>(p, dout, q, k, v, o, lse, delta, dq, dk, dv, passes, status, stream, fused, ds);
   }
   // D = 128: shared memory holds one stationary pair (64 KB) and 128 KB of streamed tiles.
   // As 64-row tiles that is four stages in flight instead of two, and the narrower T tiles
   // leave TMEM columns for separate P / dS operands, i.e. for the one-iteration lookahead.
-  return bf16 ? launch_both<__nv_bfloat16, 128, 4, 1, 64>(p, dout, q, k, v, o, lse, delta, dq, dk, dv, passes, status, stream, fused)
-              : launch_both<__half, 128, 4, 1, 64>(p, dout, q, k, v, o, lse, delta, dq, dk, dv, passes, status, stream, fused);
+  return bf16 ? launch_both<__nv_bfloat16, 128, 4, 1, 64>(p, dout, q, k, v, o, lse, delta, dq, dk, dv, passes, status, stream, fused, ds)
+              : launch_both<__half, 128, 4, 1, 64>(p, dout, q, k, v, o, lse, delta, dq, dk, dv, passes, status, stream, fused, ds);
 }
 
 

@@ -135,6 +135,35 @@ __host__ __device__ inline int dq_turn_of_block(int block, int tile, int window,
   return block < extra ? block : extra + (block - r.lo);
 }
 
+// Where the dK/dV pass leaves dS for the dQ pass (bwd_dq.cu): one 32 KB tile of 16-bit values per
+// (query head, query tile, key block the tile sees), a query tile's blocks side by side in the order
+// of dq_turn_of_block.  Tile `i`'s blocks start at slot ds_tile_offset(i) of its head.
+constexpr int kDsTileBytes = kTile * kTile * 2;
+struct DsLayout {
+  int n_tiles;
+  int stride;            // > 0 (windows): every query tile has this many slots
+  int ahead;             // otherwise: tile i has min(n_tiles, i + 1 + ahead) of them (block-causal: ahead > 0)
+};
+__host__ __device__ inline int ds_tile_offset(const DsLayout& l, int i) {
+  if (l.stride > 0) return i * l.stride;
+  const int full = l.n_tiles - 1 - l.ahead > 0 ? l.n_tiles - 1 - l.ahead : 0;    // first tile that sees every block
+  return i <= full ? i * (i + 1) / 2 + i * l.ahead : full * (full + 1) / 2 + full * l.ahead + (i - full) * l.n_tiles;
+}
+inline DsLayout ds_layout(int T, int window, int sinks, int block) {
+  DsLayout l{(T + kTile - 1) / kTile, 0, 0};
+  if (window > 0) {
+    for (int t = 0; t < l.n_tiles; ++t) {
+      int count = 0;
+      (void)dq_turn_of_block(t, t, window, sinks, &count, block, l.n_tiles);
+      if (count > l.stride) l.stride = count;
+    }
+  } else if (block > 1) {
+    l.ahead = (block - 1 + kTile - 1) / kTile;      // blocks past the diagonal a tile's last row can reach
+    if (l.ahead > l.n_tiles - 1) l.ahead = l.n_tiles - 1;
+  }
+  return l;
+}
+
 __host__ __device__ inline bool key_visible(int q, int k, int window, int sinks, int block = 0,
                                             int t_len = 1 << 30) {
   if (k > last_key_of_query(q, block, t_len)) return false;
@@ -158,9 +187,18 @@ struct FusedScratch {
   float* dq_acc;
   unsigned* dq_turn;
 };
+// Room for dS behind the Delta tape in the caller's buffer, in whole (batch, KV head) pairs.
+struct DsScratch {
+  void* tiles;
+  int pairs;
+};
 int launch_bwd_tc(const Problem& p, const void* dout, const void* q, const void* k, const void* v,
                   const void* o, const float* lse, void* dq, void* dk, void* dv, float* delta,
-                  int passes, unsigned* status, cudaStream_t stream, const FusedScratch* fused);
+                  int passes, unsigned* status, cudaStream_t stream, const FusedScratch* fused,
+                  const DsScratch* ds);
+// dQ of the query heads of (batch, KV head) pairs [first_pair, first_pair + pairs) from their dS tiles.
+int launch_dq_from_ds(const Problem& p, const void* k, const void* ds, const DsLayout& layout, int first_pair, int pairs,
+                      void* dq, unsigned* status, cudaStream_t stream);
 int launch_selftest_tiles(int dtype, int head_dim, const void* q, const void* k, const void* v,
                           float* s_out, float* o_out, unsigned* status, cudaStream_t stream);
 

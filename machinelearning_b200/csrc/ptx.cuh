@@ -174,6 +174,13 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
+// Untiled copy of `bytes` contiguous bytes (a multiple of 16, both addresses 16-byte aligned).
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
 // 4-D tiled store from shared memory (same box and swizzle as the loads).  Rows that fall
 // outside the tensor are clipped by the hardware.
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1,
@@ -183,12 +190,21 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t sr
       ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
+// Untiled store of `bytes` contiguous bytes (a multiple of 16, both addresses 16-byte aligned).
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void tma_store_commit() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 // returns once the committed stores have finished READING shared memory
 __device__ __forceinline__ void tma_store_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+
+// returns once the committed stores have completed
+__device__ __forceinline__ void tma_store_wait_all() {
+  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // adds four fp32 values to four consecutive ones in global memory (16-byte aligned), no result
@@ -357,6 +373,15 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
   return static_cast<uint64_t>((smem_addr & 0x3ffffu) >> 4) |
          (static_cast<uint64_t>((lbo_bytes >> 4) & 0x3fffu) << 16) |
          (static_cast<uint64_t>((sbo_bytes >> 4) & 0x3fffu) << 32) | (1ull << 46) | (2ull << 61);
+}
+
+// Shared-memory matrix descriptor without swizzle, MN-major operand: core matrices of 8 rows (along
+// K) x 16 bytes (8 elements along M/N) are 128 contiguous bytes; `k_step` bytes lead to the next 8
+// rows along K, `mn_step` bytes to the next 8 elements along M/N.
+__device__ __forceinline__ uint64_t make_smem_desc_plain_mn(uint32_t smem_addr, uint32_t k_step, uint32_t mn_step) {
+  return static_cast<uint64_t>((smem_addr & 0x3ffffu) >> 4) |
+         (static_cast<uint64_t>((k_step >> 4) & 0x3fffu) << 16) |
+         (static_cast<uint64_t>((mn_step >> 4) & 0x3fffu) << 32) | (1ull << 46);
 }
 
 // TMEM address: lane in bits [16,32), column in bits [0,16).

@@ -295,7 +295,10 @@ def bwd(dout, q, k, v, o, lse, scale: float, use_mma: bool, window: int = 0, sin
     elif fused and not can_fuse:
         raise ValueError("the fused backward exists on the tensor-core path for head dims up to 64")
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    nbytes = lib.nlfa_bwd_fused_scratch_bytes(B, T, H, D) if fused else lib.nlfa_bwd_scratch_bytes(B, T, H)
+    path = _lib.PATH_TENSOR if use_mma else _lib.PATH_SIMT
+    nbytes = (lib.nlfa_bwd_fused_scratch_bytes(B, T, H, D) if fused else
+              lib.nlfa_bwd_workspace_bytes(B, T, H, Hkv, D, int(window), int(sinks), int(block),
+                                           _DTYPE_CODE[q.dtype], path))
     scratch = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
     passes = (_lib.PASS_DELTA | _lib.PASS_FUSED) if fused else _lib.PASS_ALL
     with _on_device(index):
@@ -303,8 +306,7 @@ def bwd(dout, q, k, v, o, lse, scale: float, use_mma: bool, window: int = 0, sin
                                  lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                                  scratch.data_ptr(), scratch.numel(), B, T, H, Hkv, D, float(scale),
                                  int(window), int(sinks), int(block), _DTYPE_CODE[q.dtype],
-                                 _lib.PATH_TENSOR if use_mma else _lib.PATH_SIMT, passes,
-                                 _stream_of(index))
+                                 path, passes, _stream_of(index))
     if st:
         _lib.check("nlfa_bwd_masked", st)
     return dq, dk, dv

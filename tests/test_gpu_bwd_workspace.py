@@ -1,0 +1,56 @@
+"""Backward at head dim 128 with room for dS (``nlfa_bwd_workspace_bytes``): the dK/dV pass leaves dS in the
+scratch and dQ is one product over it.  Held to the float64 oracle and, bit for bit, to the layout that
+recomputes dS (tape-only scratch), at lengths around the 64- and 128-row tile edges, under every mask, with the
+scratch poisoned and with room for one (batch, KV head) pair at a time."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import attention_f64 as orc
+
+pytestmark = pytest.mark.gpu
+
+#        B, T, H, Hkv, window, sinks, block, dtype
+CASES = [(1, 1, 1, 1, 0, 0, 0, torch.bfloat16), (2, 65, 2, 1, 0, 0, 0, torch.float16),
+         (1, 128, 2, 2, 0, 0, 0, torch.bfloat16), (1, 257, 4, 2, 0, 0, 0, torch.bfloat16),
+         (1, 513, 2, 2, 64, 0, 0, torch.bfloat16), (1, 700, 2, 1, 200, 4, 0, torch.float16),
+         (1, 640, 2, 2, 300, 130, 0, torch.bfloat16), (3, 333, 3, 1, 0, 0, 100, torch.bfloat16),
+         (1, 385, 2, 2, 0, 0, 385, torch.float16)]
+
+
+def _backward(lib, L, do, q, k, v, o, lse, scale, window, sinks, block, nbytes):
+    B, T, H, D = q.shape
+    code = L.DTYPE_BF16 if q.dtype == torch.bfloat16 else L.DTYPE_F16
+    scratch = torch.full((nbytes,), 0xff, dtype=torch.uint8, device="cuda")           # NaN in every type
+    dq, dk, dv = (torch.full_like(t, float("nan")) for t in (q, k, v))
+    L.check("nlfa_bwd_masked", lib.nlfa_bwd_masked(
+        *(t.data_ptr() for t in (do, q, k, v, o, lse, dq, dk, dv, scratch)), nbytes, B, T, H, k.shape[2], D, scale,
+        window, sinks, block, code, L.PATH_TENSOR, L.PASS_ALL, torch.cuda.current_stream().cuda_stream))
+    return dq, dk, dv
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,window,sinks,block,dtype", CASES)
+def test_backward_with_room_for_ds(B, T, H, Hkv, window, sinks, block, dtype):
+    from machinelearning_b200 import _lib as L, flash_cuda as fc
+    assert fc.is_available(), fc.unavailable_reason()
+    lib, D = fc._load(), 128
+    g = torch.Generator().manual_seed(T + H)
+    q, k, v, do = (torch.randn(B, T, h, D, generator=g).to(dtype).cuda() for h in (H, Hkv, Hkv, H))
+    scale = 1.0 / math.sqrt(D)
+    o, lse = fc.fwd(q, k, v, scale, True, window, sinks, block)
+    code = L.DTYPE_BF16 if dtype == torch.bfloat16 else L.DTYPE_F16
+    dims = (B, T, H, Hkv, D, window, sinks, block, code, L.PATH_TENSOR)
+    tape = lib.nlfa_bwd_scratch_bytes(B, T, H)
+    whole = lib.nlfa_bwd_workspace_bytes(*dims)
+    base = (tape + 255) // 256 * 256
+    one_pair = base + (whole - base) // (B * Hkv)
+    assert whole > tape and lib.nlfa_bwd_workspace_kernel_count(*dims, whole) == 3
+    assert lib.nlfa_bwd_workspace_kernel_count(*dims, one_pair) == 1 + 2 * B * Hkv
+    args = (lib, L, do, q, k, v, o, lse, scale, window, sinks, block)
+    recomputed, left, by_pair = (_backward(*args, n) for n in (tape, whole, one_pair))
+    want = orc.attention_bwd(do, q, k, v, scale, window, sinks, block)
+    for a, b, c, w in zip(recomputed, left, by_pair, want):
+        assert torch.equal(a, b) and torch.equal(b, c)
+        assert np.abs(b.double().cpu().numpy() - w).max() <= 2e-2 * max(np.abs(w).max(), 1e-2)
