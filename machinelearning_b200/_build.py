@@ -1,4 +1,5 @@
-"""Builds ``libnlfa.so`` (the C-ABI attention library) in-tree with nvcc.
+"""Builds ``libnlfa.so`` (the C-ABI attention library) in-tree with nvcc, and ``_host.so`` (its
+torch-facing call path, ``csrc/host.cpp``) with g++ against torch's headers.
 
     python -m machinelearning_b200._build [--force] [--verbose]
 
@@ -20,6 +21,7 @@ PKG = pathlib.Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "_obj"
 LIB = PKG / "libnlfa.so"
+HOST = PKG / "_host.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -79,7 +81,31 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_host(force)
     return LIB
+
+
+def build_host(force: bool = False) -> pathlib.Path:
+    """Compile ``csrc/host.cpp``; it finds ``libnlfa.so`` next to itself."""
+    src = CSRC / "host.cpp"
+    if not force and not _stale(HOST, [src, PKG.parent / "include" / "nlfa.h"]):
+        return HOST
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    cuda = pathlib.Path(_nvcc()).resolve().parent.parent
+    include = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda / "include")]
+    libs = pathlib.Path(torch.__file__).parent / "lib"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *(f"-isystem{p}" for p in include), str(src), "-o", str(HOST),
+           f"-L{libs}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
+           f"-L{PKG}", "-l:libnlfa.so", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on host.cpp:\n{r.stdout}\n{r.stderr}")
+    return HOST
 
 
 if __name__ == "__main__":

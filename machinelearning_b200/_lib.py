@@ -98,6 +98,16 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
     return lib
 
 
+def load_host():
+    """The extension module of ``csrc/host.cpp`` (torch-facing call path); built in-tree when it is absent."""
+    lib = load()
+    if not (PKG / "_host.so").exists():
+        from . import _build
+        _build.build_host()
+    from . import _host
+    return lib, _host
+
+
 def strerror(status: int) -> str:
     return load().nlfa_strerror(int(status)).decode()
 

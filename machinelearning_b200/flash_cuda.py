@@ -3,10 +3,11 @@
 Drop-in for ``nanolab/flash_cuda.py``: same public names, same call signatures,
 same exceptions.  What is different underneath:
 
-* the native side is a C-ABI shared library (``libnlfa.so``, ``include/nlfa.h``)
-  called through ctypes, not a pybind11 module built by ninja;
-* Python owns every buffer (outputs, the logsumexp tape, the backward's Delta
-  scratch) so torch's caching allocator and stream semantics apply;
+* the native side is a C-ABI shared library (``libnlfa.so``, ``include/nlfa.h``), not a pybind11
+  module built by ninja; a thin extension (``csrc/host.cpp``) makes a call -- checks, casts, output
+  allocation, autograd node, launch -- without Python in it;
+* every buffer (outputs, the logsumexp tape, the backward's scratch) comes from torch's caching
+  allocator, so its stream semantics apply;
 * ``use_mma`` still picks the kernel family (reference: ``flash_cuda.py:233-279``):
   ``False`` is the fp32 SIMT kernels, ``True`` demands the tensor-core kernels
   (TMA + tcgen05 + TMEM, sm_100a), ``None`` takes them whenever dtype and head dim
@@ -51,6 +52,7 @@ _DTYPE_CODE = {torch.float32: _lib.DTYPE_F32, torch.float16: _lib.DTYPE_F16,
                torch.bfloat16: _lib.DTYPE_BF16}
 
 _ext = None
+_host = None                                      # csrc/host.cpp, once the library is loaded
 _load_error: str | None = None
 _load_attempted = False
 _mma_ok = False
@@ -71,6 +73,7 @@ def _watch_device(lib, index: int) -> None:
     _lib.check("nlfa_set_status_mirror", st)
     word.view = ctypes.c_uint.from_address(word.data_ptr())      # read without going through torch
     _status_words[index] = word
+    _host.watch(index)
 
 
 def device_timed_out() -> bool:
@@ -121,7 +124,7 @@ def _probe_mma(lib) -> tuple[bool, str]:
 def _load():
     """Load the library once.  Never raises (reference: ``flash_cuda.py:91-135``);
     callers gate on ``is_available()``."""
-    global _ext, _load_error, _load_attempted, _mma_ok, _mma_error
+    global _ext, _host, _load_error, _load_attempted, _mma_ok, _mma_error
     if _load_attempted:
         return _ext
     _load_attempted = True
@@ -132,15 +135,16 @@ def _load():
         _load_error = "no CUDA device"
         return None
     try:
-        _ext = _lib.load()
+        _ext, _host = _lib.load_host()
     except Exception as e:                                    # noqa: BLE001
-        _ext = None
+        _ext = _host = None
         _load_error = f"{type(e).__name__}: {e}"
         log.warning("libnlfa did not load (%s)", _load_error)
         return None
     _mma_ok, _mma_error = _probe_mma(_ext)
     if not _mma_ok:
         log.warning("tensor-core path off (%s); using the SIMT kernels", _mma_error)
+    _host.configure(_lib.check, _mma_ok)
     try:
         _watch_device(_ext, torch.cuda.current_device())
     except Exception as e:                                    # noqa: BLE001
@@ -255,22 +259,9 @@ def fwd(q, k, v, scale: float, use_mma: bool, window: int = 0, sinks: int = 0, b
     lib = _load()
     if lib is None:
         raise RuntimeError(f"flash_cuda is unavailable ({unavailable_reason()})")
-    B, T, H, D = q.shape
-    Hkv = k.shape[2]
-    index = q.device.index
-    if index not in _status_words:
-        _watch_device(lib, index)
-    o = torch.empty_like(q)
-    lse = torch.empty((B, H, T), dtype=torch.float32, device=q.device)
-    with _on_device(index):
-        st = lib.nlfa_fwd_masked(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(),
-                                 B, T, H, Hkv, D, float(scale), int(window), int(sinks), int(block),
-                                 _DTYPE_CODE[q.dtype],
-                                 _lib.PATH_TENSOR if use_mma else _lib.PATH_SIMT,
-                                 _stream_of(index))
-    if st:
-        _lib.check("nlfa_fwd", st)
-    return o, lse
+    if q.device.index not in _status_words:
+        _watch_device(lib, q.device.index)
+    return _host.attn_fwd(q, k, v, scale, use_mma, window, sinks, block)
 
 
 def bwd(dout, q, k, v, o, lse, scale: float, use_mma: bool, window: int = 0, sinks: int = 0,
@@ -284,32 +275,17 @@ def bwd(dout, q, k, v, o, lse, scale: float, use_mma: bool, window: int = 0, sin
     lib = _load()
     if lib is None:
         raise RuntimeError(f"flash_cuda is unavailable ({unavailable_reason()})")
-    B, T, H, D = q.shape
-    Hkv = k.shape[2]
-    index = q.device.index
-    if index not in _status_words:
-        _watch_device(lib, index)
-    can_fuse = bool(use_mma) and D <= 64
+    if q.device.index not in _status_words:
+        _watch_device(lib, q.device.index)
+    can_fuse = bool(use_mma) and q.shape[-1] <= 64
     if fused is None:
         fused = can_fuse and FUSED_BACKWARD
     elif fused and not can_fuse:
         raise ValueError("the fused backward exists on the tensor-core path for head dims up to 64")
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    path = _lib.PATH_TENSOR if use_mma else _lib.PATH_SIMT
-    nbytes = (lib.nlfa_bwd_fused_scratch_bytes(B, T, H, D) if fused else
-              lib.nlfa_bwd_workspace_bytes(B, T, H, Hkv, D, int(window), int(sinks), int(block),
-                                           _DTYPE_CODE[q.dtype], path))
-    scratch = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=q.device)
-    passes = (_lib.PASS_DELTA | _lib.PASS_FUSED) if fused else _lib.PASS_ALL
-    with _on_device(index):
-        st = lib.nlfa_bwd_masked(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
-                                 lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                                 scratch.data_ptr(), scratch.numel(), B, T, H, Hkv, D, float(scale),
-                                 int(window), int(sinks), int(block), _DTYPE_CODE[q.dtype],
-                                 path, passes, _stream_of(index))
-    if st:
-        _lib.check("nlfa_bwd_masked", st)
-    return dq, dk, dv
+    return _host.attn_bwd(dout, q, k, v, o, lse, scale, use_mma, fused, window, sinks, block)
+
+
+_own_fwd, _own_bwd = fwd, bwd                     # flash_attn goes through these names when a caller replaces them
 
 
 class _FlashAttnFn(torch.autograd.Function):
@@ -388,6 +364,10 @@ def flash_attn(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     (``nanolab/mixers.py:78-93``: a query sees its own block of ``block`` positions and every
     earlier one; ``block >= T`` is fully bidirectional attention); it excludes a window.
     """
+    if _host is not None and not torch.compiler.is_compiling() and fwd is _own_fwd and bwd is _own_bwd and not FUSED_BACKWARD:
+        y = _host.attn(q, k, v, scale, use_mma, window, sinks, block)
+        if y is not None:
+            return y
     q, k, v, scale, use_mma = prepare(q, k, v, scale, use_mma, window, sinks, block)
     if torch.compiler.is_compiling():
         from . import compile_ops              # registered operators: one graph node instead of a graph break
@@ -414,6 +394,11 @@ def flash_attn_cached(q: torch.Tensor, k_full: torch.Tensor, v_full: torch.Tenso
     applies (16-bit inputs, a block of at least 16 rows per KV head over at least 256 keys) and the fp32
     kernel elsewhere; ``False`` / ``True`` force one (``True`` raises where it does not apply).
     """
+    if _load() is not None:
+        out = _host.attn_cached(q, k_full, v_full, scale, qpos, kpos, causal, window, sinks, return_lse, use_mma)
+        if out is not None:
+            return out
+    # what the call above declined: say why
     ok = (q.dim() == 4 and k_full.dim() == 4 and v_full.dim() == 4 and q.is_cuda and k_full.is_cuda and v_full.is_cuda
           and q.dtype == k_full.dtype == v_full.dtype and q.dtype in SUPPORTED_DTYPES
           and q.shape[-1] in SUPPORTED_HEAD_DIMS and k_full.shape == v_full.shape
@@ -426,33 +411,18 @@ def flash_attn_cached(q: torch.Tensor, k_full: torch.Tensor, v_full: torch.Tenso
     if window and not causal:
         raise ValueError("cached SWA decode requires causal=True")          # nanolab/mixers.py:410-414
     B, T, H, D = q.shape
-    Hkv, L = k_full.shape[1], k_full.shape[2]
+    L = k_full.shape[2]
     if qpos is None and T > L:
         raise ValueError("without positions the block must be the last T of the L keys")
-    lib = _load()
-    if lib is None:
+    if _load() is None:
         raise RuntimeError(f"flash_cuda is unavailable ({unavailable_reason()})")
-    if scale is None:
-        scale = 1.0 / math.sqrt(D)
+    # positions on another device or of another shape, tensors with a dispatch of their own
     pos = lambda t, n: None if t is None else t.detach().to(device=q.device, dtype=torch.int32).reshape(n).contiguous()
-    qp, kp = pos(qpos, T), pos(kpos, L)
-    q, k_full, v_full = q.detach().contiguous(), k_full.detach().contiguous(), v_full.detach().contiguous()
-    o = torch.empty_like(q)
-    lse = torch.empty((B, H, T), dtype=torch.float32, device=q.device) if return_lse else None
-    nbytes = lib.nlfa_fwd_cached_scratch_bytes(B, T, H, Hkv, L, D)      # > 0: the keys are split over CTAs
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=q.device) if nbytes else None
-    with _on_device(q.device.index):
-        path = _lib.PATH_AUTO if use_mma is None else (_lib.PATH_TENSOR if use_mma else _lib.PATH_SIMT)
-        st = lib.nlfa_fwd_cached_path(q.data_ptr(), k_full.data_ptr(), v_full.data_ptr(), o.data_ptr(),
-                                      None if lse is None else lse.data_ptr(),
-                                      None if qp is None else qp.data_ptr(), None if kp is None else kp.data_ptr(),
-                                      B, T, H, Hkv, L, D, float(scale), int(bool(causal)), int(window), int(sinks),
-                                      _DTYPE_CODE[q.dtype], path, None if scratch is None else scratch.data_ptr(),
-                                      nbytes, _stream_of(q.device.index))
-    if st == 7 and use_mma:
-        raise ValueError("flash_attn_cached: use_mma=True but the tensor-core kernel does not apply to these inputs")
-    _lib.check("nlfa_fwd_cached", st)
-    return (o, lse) if return_lse else o
+    out = _host.attn_cached(q.detach().contiguous(), k_full.detach().contiguous(), v_full.detach().contiguous(), scale,
+                            pos(qpos, T), pos(kpos, L), causal, window, sinks, return_lse, use_mma)
+    if out is None:
+        raise ValueError("flash_attn_cached: q, k and v must be plain tensors on one CUDA device")
+    return out
 
 
 def sdpa_reference(q, k, v, scale):

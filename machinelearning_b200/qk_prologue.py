@@ -117,6 +117,10 @@ def qk_prologue(x: torch.Tensor, weight=None, cos=None, sin=None, eps: float = E
     when CUDA autocast is on (``nanolab/flash_cuda.py:161-177``), else ``x.dtype``.
     Raises ``ValueError`` for inputs ``supports`` rejects.
     """
+    if flash_cuda._load() is not None and not torch.compiler.is_compiling():
+        y = flash_cuda._host.qk_prologue(x, weight, cos, sin, eps, out_dtype)
+        if y is not None:
+            return y
     if not supports(x, weight, cos, sin):
         raise ValueError(f"qk_prologue: unsupported inputs {tuple(x.shape)} {x.dtype} on {x.device}")
     if out_dtype is None:

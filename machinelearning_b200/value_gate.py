@@ -125,6 +125,10 @@ class _HeadGateFn(torch.autograd.Function):
 def value_blend(v: torch.Tensor, v0: torch.Tensor, lam: torch.Tensor, out_dtype=None) -> torch.Tensor:
     """``(1 - sigmoid(lam)) * v + sigmoid(lam) * v0`` in ``out_dtype`` (default: the autocast dtype
     under CUDA autocast -- what ``flash_attn`` would cast to -- else ``v.dtype``)."""
+    if flash_cuda._load() is not None and not torch.compiler.is_compiling():
+        out = flash_cuda._host.value_blend(v, v0, lam, out_dtype)
+        if out is not None:
+            return out
     if not supports_blend(v, v0, lam):
         raise ValueError(f"value_blend: unsupported inputs {tuple(v.shape)} {v.dtype} / {v0.dtype} on {v.device}")
     if out_dtype is None:
@@ -141,6 +145,10 @@ def value_blend(v: torch.Tensor, v0: torch.Tensor, lam: torch.Tensor, out_dtype=
 
 def head_gate(y: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
     """``y * sigmoid(gate)[..., None]`` for ``y [B,T,H,D]`` and gate logits ``[B,T,H]``."""
+    if flash_cuda._load() is not None and not torch.compiler.is_compiling():
+        out = flash_cuda._host.head_gate(y, gate)
+        if out is not None:
+            return out
     if not supports_gate(y, gate):
         raise ValueError(f"head_gate: unsupported inputs {tuple(y.shape)} {y.dtype}, gate {tuple(gate.shape)} "
                          f"{gate.dtype} on {y.device}")
