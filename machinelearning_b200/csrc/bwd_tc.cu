@@ -207,7 +207,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
   // already there, hand the row sums to the compute warps through shared memory and write them
   // out for the dK/dV pass, which then runs second.  That removes the separate Delta kernel
   // (a full pass over dO and O) from the backward.  Same arithmetic, same order of additions as
-  // delta_vec_kernel, so the results are bit-identical to it.
+  // delta_kernel, so the results are bit-identical to it.
   constexpr bool kDeltaIn = MODE == MODE_DQ && XBUF == 2 && D == 64;
   using L = BwdSmem<D, STAGES, XBUF, YR, MODE == MODE_FUSED || MODE == MODE_DKV_DS, kDeltaIn>;
   static_assert(YR == 64 || YR == 128, "streamed tiles are 64 or 128 rows");
@@ -457,7 +457,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
       ok = __all_sync(0xffffffffu, done && *abort_flag == 0);
     };
     // dQ pass forming Delta: row sums of dO * O for unit `duc` (descriptor `dw`), eight lanes per
-    // row and eight elements per lane, summed exactly as delta_vec_kernel does; handed to the
+    // row and eight elements per lane, summed exactly as delta_kernel does; handed to the
     // compute warps through shared memory and written out for the dK/dV pass.
     auto form_delta = [&](int duc, const BwdUnit<MODE>& dw) {
       const int xb = duc % XBUF;
@@ -1288,7 +1288,7 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
 
 // True when the backward does without the separate Delta kernel: Delta and the dQ pass both asked
 // for, real head dim 64 (two stationary buffers in the dQ pass; the sums then match
-// delta_vec_kernel's bit for bit) -- and a problem large enough for it to pay.  With fewer than
+// delta_kernel's bit for bit) -- and a problem large enough for it to pay.  With fewer than
 // sixteen query tiles per SM the backward is faster the other way round (measured at B = 4, 8, 16
 // of H = 12, T = 1024: the dQ pass can then start beside the dK/dV pass, and a short Delta kernel
 // costs less than the later start of the first unit).  NLFA_DELTA_IN_DQ=0 / 1 forces either.

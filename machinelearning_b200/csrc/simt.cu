@@ -1,8 +1,17 @@
-// fp32 SIMT attention kernels: the accuracy path (fp32 inputs need 1e-5) and the
-// path for head dims the tensor-core kernels do not cover.  One warp owns one
-// row (a query row in the forward and in dQ, a key row in dK/dV); lanes split the
-// head dimension; scores are reduced with shuffles.  No shared memory, no
-// atomics: results are bit-reproducible.
+// fp32 attention kernels on the FMA pipe: the accuracy path (fp32 inputs need 1e-5), for every dtype and head dim.
+//
+// Register-tiled: a CTA of 128 threads owns BM = 8 RM rows (queries in the forward and in dQ, keys in dK/dV) and
+// streams tiles of 64 rows of the other side past them through shared memory, everything held as fp32.  The threads
+// form 8 groups of 16: a group owns RM rows, a thread of it the columns c, c + 16, c + 32, c + 48 of a score tile
+// (so that its 16-byte reads along D fall on different banks) and D / 16 columns of an output.  A score product
+// takes RM + 4 vector loads for 16 RM multiply-adds: at RM = 8 the FMA pipe, not shared memory, is the bound.
+// The group's probabilities go through shared memory to become the other operand of the output product; only the
+// warp's own rows are involved, so that exchange needs no CTA-wide barrier.  No atomics: bit-reproducible.
+//
+// RM = 8 where there are enough row tiles to fill the GPU, RM = 4 (twice as many, half as long CTAs) otherwise.
+// Measured, a row per warp before -> tiles: B=4 H=4 T=256 D=64 forward 82 -> 19 us, backward 174 -> 53 us (one
+// CTA of four warps per SM there: latency); B=8 H=12/4 T=2048 D=64 forward 14.9 -> 1.41 ms (37 TFLOP/s, half of
+// what the FMA pipe can issue), backward 32.0 -> 4.98 ms.
 //
 // Algebra follows the reference's FMA kernels (nanolab/csrc/flash_attn_cuda.cu
 // :147-281 forward, :1234-1262 Delta, :1265-1366 dQ, :1371-1482 dK/dV): softmax
@@ -17,7 +26,9 @@
 namespace nlfa {
 namespace {
 
-constexpr int kWarpsPerBlock = 4;
+constexpr int kThreads = 128;
+constexpr int kBN = 64;                    // rows of a streamed tile
+constexpr int kPPitch = kBN + 16;          // row pitch of the probability tile: neighbouring rows 16 banks apart
 
 template <typename T>
 __device__ __forceinline__ float to_f32(T x);
@@ -37,308 +48,510 @@ __device__ __forceinline__ __half from_f32<__half>(float x) { return __float2hal
 template <>
 __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
 
-__device__ __forceinline__ float warp_sum(float x) {
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+
+// `rows` rows of D values, `stride` elements apart, into shared memory as fp32 at a pitch of D + 4; rows from
+// `valid` on become zeros.  fp32 goes by asynchronous copies (the caller commits and waits), 16-bit types are
+// converted on the way.
+template <typename T, int D>
+__device__ __forceinline__ void load_rows(float* dst, const T* src, long long stride, int rows, int valid) {
+  constexpr int kPitch = D + 4;
+  if constexpr (sizeof(T) == 4) {
+    constexpr int V = D / 4;
+    for (int i = threadIdx.x; i < rows * V; i += kThreads) {
+      const int r = i / V, c = 4 * (i % V);
+      const bool in = r < valid;
+      const T* s = in ? src + r * stride + c : src;
+      const int bytes = in ? 16 : 0;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                   ::"r"(smem_u32(dst + r * kPitch + c)), "l"(s), "r"(bytes) : "memory");
+    }
+  } else {
+    constexpr int V = D / 8;
+    for (int i = threadIdx.x; i < rows * V; i += kThreads) {
+      const int r = i / V, c = 8 * (i % V);
+      uint4 w = make_uint4(0u, 0u, 0u, 0u);
+      if (r < valid) w = *reinterpret_cast<const uint4*>(src + r * stride + c);
+      T x[8];
+      *reinterpret_cast<uint4*>(x) = w;
+      float* d = dst + r * kPitch + c;
+      *reinterpret_cast<float4*>(d) = make_float4(to_f32(x[0]), to_f32(x[1]), to_f32(x[2]), to_f32(x[3]));
+      *reinterpret_cast<float4*>(d + 4) = make_float4(to_f32(x[4]), to_f32(x[5]), to_f32(x[6]), to_f32(x[7]));
+    }
+  }
+}
+__device__ __forceinline__ void load_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void load_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// s[i][j] = row (grp + 8 i) of A . row (col + 16 j) of B
+template <int D, int RM>
+__device__ __forceinline__ void score_product(const float* a, const float* b, int grp, int col, float (&s)[RM][4]) {
+  constexpr int kPitch = D + 4;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+  const float* ap = a + grp * kPitch;
+  const float* bp = b + col * kPitch;
+#pragma unroll 2
+  for (int d = 0; d < D; d += 4) {
+    float4 bv[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) bv[j] = ld4(bp + 16 * j * kPitch + d);
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+      const float4 av = ld4(ap + 8 * i * kPitch + d);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        s[i][j] = fmaf(av.w, bv[j].w, fmaf(av.z, bv[j].z, fmaf(av.y, bv[j].y, fmaf(av.x, bv[j].x, s[i][j]))));
+    }
+  }
 }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-fwd_simt_kernel(Problem p, const T* __restrict__ q, const T* __restrict__ k,
-                const T* __restrict__ v, T* __restrict__ o, float* __restrict__ lse) {
-  constexpr int R = D / 32;
-  const int lane = threadIdx.x & 31;
-  const long long row = static_cast<long long>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
-  const long long rows = static_cast<long long>(p.B) * p.H * p.T;
-  if (row >= rows) return;
-  const int t = static_cast<int>(row % p.T);
-  const long long bh = row / p.T;
-  const int h = static_cast<int>(bh % p.H);
-  const int b = static_cast<int>(bh / p.H);
-  const int hk = h / (p.H / p.Hkv);
-  const float scale2 = p.scale * kLog2e;
-
-  const T* qrow = q + ((static_cast<long long>(b) * p.T + t) * p.H + h) * D;
-  float qr[R], acc[R];
+// acc[i][.] += row (grp + 8 i) of the [rows][kBN] tile w times B [kBN][D]; a thread's D / 16 columns are 4 col ..
+// (per 64 columns), or 2 col .. at D = 32
+template <int D, int RM>
+__device__ __forceinline__ void output_product(const float* w, const float* b, int grp, int col, float (&acc)[RM][D / 16]) {
+  constexpr int kPitch = D + 4;
+  const float* wp = w + grp * kPPitch;
+#pragma unroll 2
+  for (int k = 0; k < kBN; k += 4) {
+    float wv[RM][4];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    qr[r] = to_f32(qrow[lane + 32 * r]) * scale2;
-    acc[r] = 0.f;
+    for (int i = 0; i < RM; ++i) {
+      const float4 t = ld4(wp + 8 * i * kPPitch + k);
+      wv[i][0] = t.x; wv[i][1] = t.y; wv[i][2] = t.z; wv[i][3] = t.w;
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      float bv[D / 16];
+      const float* row = b + (k + x) * kPitch;
+      if constexpr (D == 32) {
+        const float2 t = *reinterpret_cast<const float2*>(row + 2 * col);
+        bv[0] = t.x; bv[1] = t.y;
+      } else {
+#pragma unroll
+        for (int h = 0; h < D / 64; ++h) {
+          const float4 t = ld4(row + 64 * h + 4 * col);
+          bv[4 * h] = t.x; bv[4 * h + 1] = t.y; bv[4 * h + 2] = t.z; bv[4 * h + 3] = t.w;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int n = 0; n < D / 16; ++n) acc[i][n] = fmaf(wv[i][x], bv[n], acc[i][n]);
+    }
   }
-  float m = -INFINITY, l = 0.f;
+}
 
-  int lo = 0, nsink = 0;
+// one thread's D / 16 columns of an output row, times `mul`
+template <typename T, int D>
+__device__ __forceinline__ void store_row(T* row, int col, const float (&acc)[D / 16], float mul) {
+  if constexpr (D == 32) {
+    T x[2] = {from_f32<T>(acc[0] * mul), from_f32<T>(acc[1] * mul)};
+    if constexpr (sizeof(T) == 4) *reinterpret_cast<float2*>(row + 2 * col) = make_float2(x[0], x[1]);
+    else *reinterpret_cast<uint32_t*>(row + 2 * col) = *reinterpret_cast<uint32_t*>(x);
+  } else {
+#pragma unroll
+    for (int h = 0; h < D / 64; ++h) {
+      T x[4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) x[n] = from_f32<T>(acc[4 * h + n] * mul);
+      if constexpr (sizeof(T) == 4) *reinterpret_cast<float4*>(row + 64 * h + 4 * col) = make_float4(x[0], x[1], x[2], x[3]);
+      else *reinterpret_cast<uint2*>(row + 64 * h + 4 * col) = *reinterpret_cast<uint2*>(x);
+    }
+  }
+}
+
+// The 64-key blocks query rows [q_lo, q_hi] can see: block `it` of `count`, sink blocks first.
+struct KeyBlocks {
+  int lo, extra, count;
+  __device__ __forceinline__ int at(int it) const { return it < extra ? it : lo + (it - extra); }
+};
+__device__ __forceinline__ KeyBlocks key_blocks(const Problem& p, int q_lo, int q_hi) {
+  KeyBlocks r;
+  int hi = last_key_of_query(q_hi < p.T ? q_hi : p.T - 1, p.block, p.T) / kBN;
+  int lo = 0, sinks = 0;
   if (p.window > 0) {
-    const int first = t - (p.window - p.sinks) + 1;
-    lo = first > 0 ? first : 0;
-    nsink = p.sinks < lo ? p.sinks : lo;          // sinks not already inside the window
+    const int first = q_lo - (p.window - p.sinks) + 1;
+    lo = first > 0 ? first / kBN : 0;
+    sinks = (p.sinks + kBN - 1) / kBN;
   }
-  const long long kv_stride = static_cast<long long>(p.Hkv) * D;
-  const T* kbase = k + (static_cast<long long>(b) * p.T * p.Hkv + hk) * D;
-  const T* vbase = v + (static_cast<long long>(b) * p.T * p.Hkv + hk) * D;
-
-  int t_last = last_key_of_query(t, p.block);            // block-causal: to the end of the row's block
-  t_last = t_last < p.T - 1 ? t_last : p.T - 1;
-  const int n = nsink + (t_last - lo + 1);
-  for (int idx = 0; idx < n; ++idx) {
-    const int j = idx < nsink ? idx : lo + (idx - nsink);
-    const T* krow = kbase + j * kv_stride;
-    const T* vrow = vbase + j * kv_stride;
-    float part = 0.f;
-#pragma unroll
-    for (int r = 0; r < R; ++r) part = fmaf(qr[r], to_f32(krow[lane + 32 * r]), part);
-    const float s = warp_sum(part);
-    const float m_new = fmaxf(m, s);
-    const float alpha = exp2f(m - m_new);
-    const float pj = exp2f(s - m_new);
-    l = fmaf(l, alpha, pj);
-#pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = fmaf(acc[r], alpha, pj * to_f32(vrow[lane + 32 * r]));
-    m = m_new;
-  }
-  const float inv = 1.f / l;
-  T* orow = o + ((static_cast<long long>(b) * p.T + t) * p.H + h) * D;
-#pragma unroll
-  for (int r = 0; r < R; ++r) orow[lane + 32 * r] = from_f32<T>(acc[r] * inv);
-  if (lane == 0) lse[bh * p.T + t] = (m + log2f(l)) * kLn2;
+  r.lo = lo;
+  r.extra = sinks < lo ? sinks : lo;
+  r.count = r.extra + hi - lo + 1;
+  return r;
 }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-delta_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ o,
-             float* __restrict__ delta) {
-  constexpr int R = D / 32;
-  const int lane = threadIdx.x & 31;
-  const long long row = static_cast<long long>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
-  const long long rows = static_cast<long long>(p.B) * p.T * p.H;
-  if (row >= rows) return;               // row indexes [B,T,H]
-  const int h = static_cast<int>(row % p.H);
-  const long long bt = row / p.H;
-  const int t = static_cast<int>(bt % p.T);
-  const int b = static_cast<int>(bt / p.T);
-  float part = 0.f;
+template <typename T, int D, int RM>
+__global__ void __launch_bounds__(kThreads)
+fwd_tile_kernel(Problem p, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
+                T* __restrict__ o, float* __restrict__ lse) {
+  constexpr int BM = 8 * RM, kPitch = D + 4;
+  extern __shared__ __align__(16) float smem[];
+  float* qs = smem;
+  float* ks = qs + BM * kPitch;
+  float* vs = ks + kBN * kPitch;
+  float* ps = vs + kBN * kPitch;
+  const int grp = threadIdx.x >> 4, col = threadIdx.x & 15;
+  const int BH = p.B * p.H, n_tiles = (p.T + BM - 1) / BM;
+  const int rank = blockIdx.x / BH, bh = blockIdx.x - rank * BH;      // late (heavy) query tiles first
+  const int b = bh / p.H, h = bh - b * p.H, hk = h / (p.H / p.Hkv);
+  const int q0 = (n_tiles - 1 - rank) * BM;
+  const long long q_stride = static_cast<long long>(p.H) * D, k_stride = static_cast<long long>(p.Hkv) * D;
+  const T* kb = k + (static_cast<long long>(b) * p.T * p.Hkv + hk) * D;
+  const T* vb = v + (static_cast<long long>(b) * p.T * p.Hkv + hk) * D;
+  const KeyBlocks blocks = key_blocks(p, q0, q0 + BM - 1);
+  auto load_kv = [&](float* dst, const T* src, int j) {
+    load_rows<T, D>(dst, src + j * kBN * k_stride, k_stride, kBN, p.T - j * kBN);
+    load_commit();
+  };
+
+  load_rows<T, D>(qs, q + ((static_cast<long long>(b) * p.T + q0) * p.H + h) * D, q_stride, BM, p.T - q0);
+  load_kv(ks, kb, blocks.at(0));
+  load_kv(vs, vb, blocks.at(0));
+
+  const float scale2 = p.scale * kLog2e;
+  float m[RM], l[RM], acc[RM][D / 16];
+  int qlim[RM];
 #pragma unroll
-  for (int r = 0; r < R; ++r)
-    part = fmaf(to_f32(dout[row * D + lane + 32 * r]), to_f32(o[row * D + lane + 32 * r]), part);
-  const float s = warp_sum(part);
-  if (lane == 0) delta[(static_cast<long long>(b) * p.H + h) * p.T + t] = s;
+  for (int i = 0; i < RM; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+    qlim[i] = last_key_of_query(q0 + grp + 8 * i, p.block, p.T);
+#pragma unroll
+    for (int n = 0; n < D / 16; ++n) acc[i][n] = 0.f;
+  }
+  for (int it = 0; it < blocks.count; ++it) {
+    const int k0 = blocks.at(it) * kBN;
+    load_wait<1>();
+    __syncthreads();                                   // K (and Q) are there; V may be on its way
+    float s[RM][4];
+    score_product<D, RM>(qs, ks, grp, col, s);
+    __syncthreads();
+    if (it + 1 < blocks.count) load_kv(ks, kb, blocks.at(it + 1));
+    else load_commit();
+    const bool full = rect_fully_visible(q0, q0 + BM - 1, k0, k0 + kBN - 1, p.window, p.sinks, p.block, p.T);
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+      const int qpos = q0 + grp + 8 * i;
+      float mx = m[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] *= scale2;
+        if (!full) {
+          const int kp = k0 + col + 16 * j;
+          const bool vis = kp <= qlim[i] && (p.window == 0 || kp > qpos - (p.window - p.sinks) || kp < p.sinks);
+          s[i][j] = vis ? s[i][j] : -INFINITY;
+        }
+        mx = fmaxf(mx, s[i][j]);
+      }
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      const float ref = mx == -INFINITY ? 0.f : mx;    // nothing seen yet
+      const float alpha = exp2f(m[i] - ref);
+      m[i] = mx;
+      l[i] *= alpha;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float e = exp2f(s[i][j] - ref);
+        l[i] += e;
+        ps[(grp + 8 * i) * kPPitch + col + 16 * j] = e;
+      }
+#pragma unroll
+      for (int n = 0; n < D / 16; ++n) acc[i][n] *= alpha;
+    }
+    load_wait<1>();
+    __syncthreads();                                   // V is there (and this warp's probabilities)
+    output_product<D, RM>(ps, vs, grp, col, acc);
+    __syncthreads();
+    if (it + 1 < blocks.count) load_kv(vs, vb, blocks.at(it + 1));
+    else load_commit();
+  }
+#pragma unroll
+  for (int i = 0; i < RM; ++i) {
+    float sum = l[i];
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    const int t = q0 + grp + 8 * i;
+    if (t >= p.T) continue;
+    store_row<T, D>(o + ((static_cast<long long>(b) * p.T + t) * p.H + h) * D, col, acc[i], 1.f / sum);
+    if (col == 0) lse[static_cast<long long>(bh) * p.T + t] = (m[i] + log2f(sum)) * kLn2;
+  }
 }
 
-// Delta for 16-bit tensors: pure streaming, so every thread moves 16 bytes of dO and of O
-// per load (8 elements); D / 8 consecutive lanes share a row and combine with shuffles.
+// dQ pass (DKV = false): stationary Q, dO, streamed K, V.  dK/dV pass: stationary K, V, streamed Q, dO of every
+// head of the group.  T0 = X0 Y0^T, T1 = X1 Y1^T; P from T0 and the taped logsumexp, dS = P (T1 - Delta) scale;
+// dV += P dO, dQ or dK += dS Y0.  NB: buffers of streamed tiles.
+template <typename T, int D, int RM, bool DKV, int NB>
+__global__ void __launch_bounds__(kThreads)
+bwd_tile_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q, const T* __restrict__ k,
+                const T* __restrict__ v, const float* __restrict__ lse, const float* __restrict__ delta,
+                T* __restrict__ out0, T* __restrict__ out1) {
+  constexpr int BM = 8 * RM, kPitch = D + 4;
+  extern __shared__ __align__(16) float smem[];
+  float* x0 = smem;
+  float* x1 = x0 + BM * kPitch;
+  float* ys = x1 + BM * kPitch;                                  // [NB][2][kBN * kPitch]
+  float* ws = ys + NB * 2 * kBN * kPitch;
+  float* vec = ws + BM * kPPitch;                                // [NB][2][kBN]: base-2 logsumexp, Delta of streamed queries
+  const int grp = threadIdx.x >> 4, col = threadIdx.x & 15;
+  const int group = p.H / p.Hkv;
+  const int heads = DKV ? p.Hkv : p.H;
+  const int BH = p.B * heads, n_tiles = (p.T + BM - 1) / BM;
+  const int rank = blockIdx.x / BH, bh = blockIdx.x - rank * BH;
+  const int b = bh / heads, xh = bh - b * heads, hk = DKV ? xh : xh / group;
+  const int r0 = (DKV ? rank : n_tiles - 1 - rank) * BM;          // heavy tiles first: early keys, late queries
+  const long long q_stride = static_cast<long long>(p.H) * D, k_stride = static_cast<long long>(p.Hkv) * D;
+  const T* qb = q + (static_cast<long long>(b) * p.T * p.H) * D;
+  const T* dob = dout + (static_cast<long long>(b) * p.T * p.H) * D;
+  const T* kb = k + (static_cast<long long>(b) * p.T * p.Hkv + hk) * D;
+  const T* vb = v + (static_cast<long long>(b) * p.T * p.Hkv + hk) * D;
+
+  // what is streamed: key blocks of a query tile, or the query blocks that see a key tile, per head of the group
+  KeyBlocks blocks{0, 0, 0};
+  int y_first = 0, n_inner = 0;
+  if (DKV) {
+    y_first = first_query_of_key(r0, p.block) / kBN;
+    int last = p.T - 1;
+    if (p.window > 0 && r0 >= p.sinks) {
+      const int w_last = r0 + BM - 1 + (p.window - p.sinks) - 1;
+      last = w_last < last ? w_last : last;
+    }
+    n_inner = last / kBN - y_first + 1;
+  } else {
+    blocks = key_blocks(p, r0, r0 + BM - 1);
+    n_inner = blocks.count;
+  }
+  const int n_iters = DKV ? n_inner * group : n_inner;
+  auto load_y = [&](int it) {
+    float* y = ys + (it % NB) * 2 * kBN * kPitch;
+    if (DKV) {
+      const int g = it / n_inner, y0 = (y_first + it - g * n_inner) * kBN, h = hk * group + g;
+      load_rows<T, D>(y, qb + h * D + y0 * q_stride, q_stride, kBN, p.T - y0);
+      load_rows<T, D>(y + kBN * kPitch, dob + h * D + y0 * q_stride, q_stride, kBN, p.T - y0);
+      if (threadIdx.x < kBN) {
+        const int t = y0 + threadIdx.x;
+        const long long row = (static_cast<long long>(b) * p.H + h) * p.T + t;
+        float* w = vec + (it % NB) * 2 * kBN + threadIdx.x;
+        w[0] = t < p.T ? lse[row] * kLog2e : 0.f;
+        w[kBN] = t < p.T ? delta[row] : 0.f;
+      }
+    } else {
+      const int y0 = blocks.at(it) * kBN;
+      load_rows<T, D>(y, kb + y0 * k_stride, k_stride, kBN, p.T - y0);
+      load_rows<T, D>(y + kBN * kPitch, vb + y0 * k_stride, k_stride, kBN, p.T - y0);
+    }
+    load_commit();
+  };
+
+  if (DKV) {
+    load_rows<T, D>(x0, kb + r0 * k_stride, k_stride, BM, p.T - r0);
+    load_rows<T, D>(x1, vb + r0 * k_stride, k_stride, BM, p.T - r0);
+  } else {
+    load_rows<T, D>(x0, qb + xh * D + r0 * q_stride, q_stride, BM, p.T - r0);
+    load_rows<T, D>(x1, dob + xh * D + r0 * q_stride, q_stride, BM, p.T - r0);
+  }
+  load_y(0);
+
+  const float scale2 = p.scale * kLog2e;
+  float acc0[RM][D / 16], acc1[DKV ? RM : 1][D / 16];
+  float l2[RM], dl[RM];
+  int edge[RM];                                                  // a query's last key, a key's first query
+#pragma unroll
+  for (int i = 0; i < RM; ++i) {
+    const int r = r0 + grp + 8 * i;
+    edge[i] = DKV ? first_query_of_key(r, p.block) : last_key_of_query(r, p.block, p.T);
+    l2[i] = dl[i] = 0.f;
+    if (!DKV && r < p.T) {
+      l2[i] = lse[static_cast<long long>(bh) * p.T + r] * kLog2e;
+      dl[i] = delta[static_cast<long long>(bh) * p.T + r];
+    }
+#pragma unroll
+    for (int n = 0; n < D / 16; ++n) {
+      acc0[i][n] = 0.f;
+      if (DKV) acc1[i][n] = 0.f;
+    }
+  }
+  for (int it = 0; it < n_iters; ++it) {
+    if (NB == 1 && it > 0) {
+      __syncthreads();
+      load_y(it);
+    }
+    load_wait<0>();
+    __syncthreads();
+    if (NB == 2 && it + 1 < n_iters) load_y(it + 1);             // its buffer was last read before the barrier
+    const float* y0s = ys + (it % NB) * 2 * kBN * kPitch;
+    const float* y1s = y0s + kBN * kPitch;
+    const float* w = vec + (it % NB) * 2 * kBN;
+    const int c0 = (DKV ? y_first + it % n_inner : blocks.at(it)) * kBN;
+    const bool full = DKV ? c0 + kBN <= p.T && rect_fully_visible(c0, c0 + kBN - 1, r0, r0 + BM - 1, p.window, p.sinks, p.block, p.T)
+                          : rect_fully_visible(r0, r0 + BM - 1, c0, c0 + kBN - 1, p.window, p.sinks, p.block, p.T);
+    float s[RM][4], ds[RM][4];
+    score_product<D, RM>(x0, y0s, grp, col, s);
+    score_product<D, RM>(x1, y1s, grp, col, ds);
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+      const int r = r0 + grp + 8 * i;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int c = c0 + col + 16 * j;
+        const float ref = DKV ? w[col + 16 * j] : l2[i], dlt = DKV ? w[kBN + col + 16 * j] : dl[i];
+        float e = exp2f(fmaf(s[i][j], scale2, -ref));
+        if (!full) {
+          const int qp = DKV ? c : r, kp = DKV ? r : c;
+          const bool vis = (DKV ? c >= edge[i] && c < p.T : c <= edge[i]) &&
+                           (p.window == 0 || kp > qp - (p.window - p.sinks) || kp < p.sinks);
+          e = vis ? e : 0.f;
+        }
+        s[i][j] = e;
+        ds[i][j] = e * (ds[i][j] - dlt) * p.scale;
+      }
+    }
+    auto hand_over = [&](const float (&x)[RM][4]) {              // within this warp's rows
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ws[(grp + 8 * i) * kPPitch + col + 16 * j] = x[i][j];
+      __syncwarp();
+    };
+    if constexpr (DKV) {
+      hand_over(s);
+      output_product<D, RM>(ws, y1s, grp, col, acc1);
+    }
+    hand_over(ds);
+    output_product<D, RM>(ws, y0s, grp, col, acc0);
+  }
+#pragma unroll
+  for (int i = 0; i < RM; ++i) {
+    const int t = r0 + grp + 8 * i;
+    if (t >= p.T) continue;
+    const long long at = ((static_cast<long long>(b) * p.T + t) * heads + xh) * D;
+    store_row<T, D>(out0 + at, col, acc0[i], 1.f);
+    if constexpr (DKV) store_row<T, D>(out1 + at, col, acc1[i], 1.f);
+  }
+}
+
+// Delta = rowsum(dO * O): pure streaming.  A lane moves 16 bytes of dO and of O per row and has two rows in flight;
+// D values are 16 bytes each of D sizeof(T) / 16 consecutive lanes, which combine with shuffles.
 template <typename T, int D>
 __global__ void __launch_bounds__(256)
-delta_vec_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ o,
-                 float* __restrict__ delta) {
-  constexpr int kLanesPerRow = D / 8;                      // 8 (D = 64) or 16 (D = 128)
+delta_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ o, float* __restrict__ delta) {
+  constexpr int kPer = 16 / sizeof(T);                     // values per lane and row
+  constexpr int kLanesPerRow = D / kPer;                   // 4 .. 32
   constexpr int kRowsPerWarp = 32 / kLanesPerRow;
+  constexpr int U = 2;
   grid_dep_wait();                                         // O comes from the stream's previous kernel
   grid_dep_release();
   const int lane = threadIdx.x & 31;
   const long long warp_id = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const long long rows = static_cast<long long>(p.B) * p.T * p.H;     // rows index [B,T,H]
-  const long long row = warp_id * kRowsPerWarp + lane / kLanesPerRow;
-  float part = 0.f;
-  if (row < rows) {
-    const uint4 a = *reinterpret_cast<const uint4*>(dout + row * D + 8 * (lane % kLanesPerRow));
-    const uint4 b = *reinterpret_cast<const uint4*>(o + row * D + 8 * (lane % kLanesPerRow));
-    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+  const long long row0 = warp_id * (kRowsPerWarp * U) + lane / kLanesPerRow;
+  uint4 a[U], c[U];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      T a2[2], b2[2];
-      *reinterpret_cast<uint32_t*>(a2) = aw[i];
-      *reinterpret_cast<uint32_t*>(b2) = bw[i];
-      part = fmaf(to_f32(a2[0]), to_f32(b2[0]), part);
-      part = fmaf(to_f32(a2[1]), to_f32(b2[1]), part);
+  for (int u = 0; u < U; ++u) {
+    const long long row = row0 + u * kRowsPerWarp;
+    a[u] = c[u] = make_uint4(0u, 0u, 0u, 0u);
+    if (row < rows) {
+      a[u] = *reinterpret_cast<const uint4*>(dout + row * D + kPer * (lane % kLanesPerRow));
+      c[u] = *reinterpret_cast<const uint4*>(o + row * D + kPer * (lane % kLanesPerRow));
     }
   }
 #pragma unroll
-  for (int off = kLanesPerRow / 2; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-  if (row < rows && (lane % kLanesPerRow) == 0) {
-    const int h = static_cast<int>(row % p.H);
-    const long long bt = row / p.H;
-    const int t = static_cast<int>(bt % p.T);
-    const int b = static_cast<int>(bt / p.T);
-    delta[(static_cast<long long>(b) * p.H + h) * p.T + t] = part;
-  }
-}
-
-template <typename T, int D>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-dq_simt_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q,
-               const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ lse,
-               const float* __restrict__ delta, T* __restrict__ dq) {
-  constexpr int R = D / 32;
-  const int lane = threadIdx.x & 31;
-  const long long row = static_cast<long long>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
-  const long long rows = static_cast<long long>(p.B) * p.H * p.T;
-  if (row >= rows) return;
-  const int t = static_cast<int>(row % p.T);
-  const long long bh = row / p.T;
-  const int h = static_cast<int>(bh % p.H);
-  const int b = static_cast<int>(bh / p.H);
-  const int hk = h / (p.H / p.Hkv);
-  const float scale2 = p.scale * kLog2e;
-
-  const long long qoff = ((static_cast<long long>(b) * p.T + t) * p.H + h) * D;
-  float qr[R], dor[R], acc[R];
+  for (int u = 0; u < U; ++u) {
+    T x[kPer], y[kPer];
+    *reinterpret_cast<uint4*>(x) = a[u];
+    *reinterpret_cast<uint4*>(y) = c[u];
+    float part = 0.f;
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    qr[r] = to_f32(q[qoff + lane + 32 * r]);
-    dor[r] = to_f32(dout[qoff + lane + 32 * r]);
-    acc[r] = 0.f;
-  }
-  const float l2 = lse[bh * p.T + t] * kLog2e;
-  const float dl = delta[bh * p.T + t];
-
-  int lo = 0, nsink = 0;
-  if (p.window > 0) {
-    const int first = t - (p.window - p.sinks) + 1;
-    lo = first > 0 ? first : 0;
-    nsink = p.sinks < lo ? p.sinks : lo;
-  }
-  const long long kv_stride = static_cast<long long>(p.Hkv) * D;
-  const T* kbase = k + (static_cast<long long>(b) * p.T * p.Hkv + hk) * D;
-  const T* vbase = v + (static_cast<long long>(b) * p.T * p.Hkv + hk) * D;
-  int t_last = last_key_of_query(t, p.block);            // block-causal: to the end of the row's block
-  t_last = t_last < p.T - 1 ? t_last : p.T - 1;
-  const int n = nsink + (t_last - lo + 1);
-  for (int idx = 0; idx < n; ++idx) {
-    const int j = idx < nsink ? idx : lo + (idx - nsink);
-    const T* krow = kbase + j * kv_stride;
-    const T* vrow = vbase + j * kv_stride;
-    float kr[R];
-    float ps = 0.f, pd = 0.f;
+    for (int i = 0; i < kPer; ++i) part = fmaf(to_f32(x[i]), to_f32(y[i]), part);
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      kr[r] = to_f32(krow[lane + 32 * r]);
-      ps = fmaf(qr[r], kr[r], ps);
-      pd = fmaf(dor[r], to_f32(vrow[lane + 32 * r]), pd);
-    }
-    const float s = warp_sum(ps);
-    const float dp = warp_sum(pd);
-    const float pj = exp2f(fmaf(s, scale2, -l2));
-    const float ds = pj * (dp - dl) * p.scale;
-#pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = fmaf(ds, kr[r], acc[r]);
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) dq[qoff + lane + 32 * r] = from_f32<T>(acc[r]);
-}
-
-template <typename T, int D>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-dkv_simt_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q,
-                const T* __restrict__ k, const T* __restrict__ v, const float* __restrict__ lse,
-                const float* __restrict__ delta, T* __restrict__ dk, T* __restrict__ dv) {
-  constexpr int R = D / 32;
-  const int lane = threadIdx.x & 31;
-  const long long row = static_cast<long long>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
-  const long long rows = static_cast<long long>(p.B) * p.Hkv * p.T;
-  if (row >= rows) return;
-  const int j = static_cast<int>(row % p.T);               // key position
-  const long long bhk = row / p.T;
-  const int hk = static_cast<int>(bhk % p.Hkv);
-  const int b = static_cast<int>(bhk / p.Hkv);
-  const int group = p.H / p.Hkv;
-  const float scale2 = p.scale * kLog2e;
-
-  const long long koff = ((static_cast<long long>(b) * p.T + j) * p.Hkv + hk) * D;
-  float kr[R], vr[R], acck[R], accv[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    kr[r] = to_f32(k[koff + lane + 32 * r]);
-    vr[r] = to_f32(v[koff + lane + 32 * r]);
-    acck[r] = 0.f;
-    accv[r] = 0.f;
-  }
-  // queries that see key j: i >= j, and inside the window unless j is a sink
-  int last = p.T - 1;
-  if (p.window > 0 && j >= p.sinks) {
-    const int w_last = j + (p.window - p.sinks) - 1;
-    last = w_last < last ? w_last : last;
-  }
-  for (int g = 0; g < group; ++g) {
-    const int h = hk * group + g;
-    const long long bh = static_cast<long long>(b) * p.H + h;
-    for (int i = first_query_of_key(j, p.block); i <= last; ++i) {
-      const long long qoff = ((static_cast<long long>(b) * p.T + i) * p.H + h) * D;
-      float qr[R], dor[R];
-      float ps = 0.f, pd = 0.f;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        qr[r] = to_f32(q[qoff + lane + 32 * r]);
-        dor[r] = to_f32(dout[qoff + lane + 32 * r]);
-        ps = fmaf(qr[r], kr[r], ps);
-        pd = fmaf(dor[r], vr[r], pd);
-      }
-      const float s = warp_sum(ps);
-      const float dp = warp_sum(pd);
-      const float pj = exp2f(fmaf(s, scale2, -lse[bh * p.T + i] * kLog2e));
-      const float ds = pj * (dp - delta[bh * p.T + i]) * p.scale;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        acck[r] = fmaf(ds, qr[r], acck[r]);
-        accv[r] = fmaf(pj, dor[r], accv[r]);
-      }
+    for (int off = kLanesPerRow / 2; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+    const long long row = row0 + u * kRowsPerWarp;
+    if (row < rows && (lane % kLanesPerRow) == 0) {
+      const int h = static_cast<int>(row % p.H);
+      const long long bt = row / p.H;
+      const int t = static_cast<int>(bt % p.T);
+      const int b = static_cast<int>(bt / p.T);
+      delta[(static_cast<long long>(b) * p.H + h) * p.T + t] = part;
     }
   }
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    dk[koff + lane + 32 * r] = from_f32<T>(acck[r]);
-    dv[koff + lane + 32 * r] = from_f32<T>(accv[r]);
-  }
 }
 
-inline unsigned blocks_for(long long rows) {
-  return static_cast<unsigned>((rows + kWarpsPerBlock - 1) / kWarpsPerBlock);
+// Row tiles of 64 (RM = 8) when there are two per SM, else of 32.  At D = 128 always 32: the accumulators of both
+// gradients and the tiles of 64 rows would leave one CTA of four warps per SM.
+inline bool tall_tiles(const Problem& p, int heads) {
+  return p.D <= 64 && static_cast<long long>(p.B) * heads * ((p.T + 63) / 64) >= 2ll * sm_count();
+}
+
+int launched() { return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA; }
+
+template <typename T, int D, int RM>
+int fwd_rm(const Problem& p, const T* q, const T* k, const T* v, T* o, float* lse, cudaStream_t s) {
+  constexpr int BM = 8 * RM;
+  constexpr int smem = ((BM + 2 * kBN) * (D + 4) + BM * kPPitch) * 4;
+  auto kern = fwd_tile_kernel<T, D, RM>;
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != NLFA_OK) return NLFA_ERR_CUDA;
+  const long long blocks = static_cast<long long>(p.B) * p.H * ((p.T + BM - 1) / BM);
+  kern<<<static_cast<unsigned>(blocks), kThreads, smem, s>>>(p, q, k, v, o, lse);
+  return launched();
 }
 
 template <typename T, int D>
-int fwd_t(const Problem& p, const void* q, const void* k, const void* v, void* o, float* lse,
-          cudaStream_t s) {
-  const long long rows = static_cast<long long>(p.B) * p.H * p.T;
-  fwd_simt_kernel<T, D><<<blocks_for(rows), kWarpsPerBlock * 32, 0, s>>>(
-      p, static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v),
-      static_cast<T*>(o), lse);
-  return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
+int fwd_t(const Problem& p, const void* q, const void* k, const void* v, void* o, float* lse, cudaStream_t s) {
+  const T *q_ = static_cast<const T*>(q), *k_ = static_cast<const T*>(k), *v_ = static_cast<const T*>(v);
+  if constexpr (D <= 64)
+    if (tall_tiles(p, p.H)) return fwd_rm<T, D, 8>(p, q_, k_, v_, static_cast<T*>(o), lse, s);
+  return fwd_rm<T, D, 4>(p, q_, k_, v_, static_cast<T*>(o), lse, s);
 }
 
 template <typename T, int D>
 int delta_t(const Problem& p, const void* dout, const void* o, float* delta, cudaStream_t s) {
   const long long rows = static_cast<long long>(p.B) * p.H * p.T;
-  if constexpr (sizeof(T) == 2 && (D == 64 || D == 128)) {
-    constexpr int kRowsPerBlock = 8 * (32 / (D / 8));           // 8 warps per block
-    const unsigned blocks = static_cast<unsigned>((rows + kRowsPerBlock - 1) / kRowsPerBlock);
-    if (launch_kernel(delta_vec_kernel<T, D>, dim3(blocks), dim3(256), 0, s, overlap_launches(kOverlapDelta), p,
-                      static_cast<const T*>(dout), static_cast<const T*>(o), delta) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return NLFA_ERR_CUDA;
-    }
-  } else {
-    delta_kernel<T, D><<<blocks_for(rows), kWarpsPerBlock * 32, 0, s>>>(
-        p, static_cast<const T*>(dout), static_cast<const T*>(o), delta);
+  constexpr int kRowsPerBlock = 8 * 2 * (32 / (D * static_cast<int>(sizeof(T)) / 16));
+  const unsigned blocks = static_cast<unsigned>((rows + kRowsPerBlock - 1) / kRowsPerBlock);
+  if (launch_kernel(delta_kernel<T, D>, dim3(blocks), dim3(256), 0, s, overlap_launches(kOverlapDelta), p,
+                    static_cast<const T*>(dout), static_cast<const T*>(o), delta) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return NLFA_ERR_CUDA;
   }
-  return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
+  return NLFA_OK;
+}
+
+template <typename T, int D, int RM, bool DKV>
+int bwd_rm(const Problem& p, const T* dout, const T* q, const T* k, const T* v, const float* lse, const float* delta,
+           void* out0, void* out1, cudaStream_t s) {
+  constexpr int BM = 8 * RM;
+  constexpr int NB = RM == 4 && D <= 64 ? 2 : 1;       // a second streamed buffer where two CTAs still fit an SM
+  constexpr int smem = ((2 * BM + NB * 2 * kBN) * (D + 4) + BM * kPPitch + NB * 2 * kBN) * 4;
+  auto kern = bwd_tile_kernel<T, D, RM, DKV, NB>;
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != NLFA_OK) return NLFA_ERR_CUDA;
+  const long long blocks = static_cast<long long>(p.B) * (DKV ? p.Hkv : p.H) * ((p.T + BM - 1) / BM);
+  kern<<<static_cast<unsigned>(blocks), kThreads, smem, s>>>(p, dout, q, k, v, lse, delta, static_cast<T*>(out0),
+                                                             static_cast<T*>(out1));
+  return launched();
+}
+
+template <typename T, int D, bool DKV>
+int bwd_pass(const Problem& p, const void* dout, const void* q, const void* k, const void* v, const float* lse,
+             const float* delta, void* out0, void* out1, cudaStream_t s) {
+  const T *g = static_cast<const T*>(dout), *q_ = static_cast<const T*>(q), *k_ = static_cast<const T*>(k),
+          *v_ = static_cast<const T*>(v);
+  if constexpr (D <= 64)
+    if (tall_tiles(p, DKV ? p.Hkv : p.H)) return bwd_rm<T, D, 8, DKV>(p, g, q_, k_, v_, lse, delta, out0, out1, s);
+  return bwd_rm<T, D, 4, DKV>(p, g, q_, k_, v_, lse, delta, out0, out1, s);
 }
 
 template <typename T, int D>
 int bwd_t(const Problem& p, const void* dout, const void* q, const void* k, const void* v,
           const float* lse, void* dq, void* dk, void* dv, const float* delta, int passes,
           cudaStream_t s) {
-  const long long qrows = static_cast<long long>(p.B) * p.H * p.T;
-  const long long krows = static_cast<long long>(p.B) * p.Hkv * p.T;
-  if (passes & NLFA_PASS_DQ)
-    dq_simt_kernel<T, D><<<blocks_for(qrows), kWarpsPerBlock * 32, 0, s>>>(
-        p, static_cast<const T*>(dout), static_cast<const T*>(q), static_cast<const T*>(k),
-        static_cast<const T*>(v), lse, delta, static_cast<T*>(dq));
-  if (cudaGetLastError() != cudaSuccess) return NLFA_ERR_CUDA;
-  if (passes & NLFA_PASS_DKV)
-    dkv_simt_kernel<T, D><<<blocks_for(krows), kWarpsPerBlock * 32, 0, s>>>(
-        p, static_cast<const T*>(dout), static_cast<const T*>(q), static_cast<const T*>(k),
-        static_cast<const T*>(v), lse, delta, static_cast<T*>(dk), static_cast<T*>(dv));
-  return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
+  int st = NLFA_OK;
+  if (passes & NLFA_PASS_DQ) st = bwd_pass<T, D, false>(p, dout, q, k, v, lse, delta, dq, nullptr, s);
+  if (st == NLFA_OK && (passes & NLFA_PASS_DKV)) st = bwd_pass<T, D, true>(p, dout, q, k, v, lse, delta, dk, dv, s);
+  return st;
 }
 
 #define NLFA_DISPATCH(p, CALL)                                                        \
