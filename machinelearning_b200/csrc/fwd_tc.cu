@@ -508,6 +508,12 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       ok = __all_sync(0xffffffffu, ok);
       if (!ok || u < 0) break;
       if (!w.valid[t]) {
+        // Q_FULL first: it says that the buffer's previous use is over.  A warpgroup without a tile would
+        // otherwise run through the published units ahead of the other one, and its arrival for a later unit
+        // would complete the phase of this one -- the buffer reloaded under the other tile's output.
+        ok = mbar_wait(bar(Q_FULL + uc % QBUF), (uc / QBUF) & 1, wctx, 15);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
         if (row == 0) {
           release_pending();
           mbar_arrive(bar(Q_EMPTY + (uc % QBUF)));                // nothing to store for this tile
