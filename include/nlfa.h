@@ -276,11 +276,10 @@ int nlfa_head_gate_bwd(const void* g, const void* y, int y_dtype, const void* ga
  * kpos < sinks) (mixers.py:417-432; positions stay correct after cache eviction);
  * causal: kpos <= qpos (:433-437); neither: every key.  A row that sees no key gives
  * zeros and lse = -inf.
- * `scratch` is optional: with nlfa_fwd_cached_scratch_bytes(...) bytes of device memory the
- * keys are split over several CTAs when there are few query rows (long caches, small
- * batches) and a second small kernel combines the partial rows in a fixed order; with
- * NULL (or too little) one CTA walks all keys of its rows.  Same results up to fp32
- * rounding. */
+ * With few query rows (long caches, small batches) the keys are split over the CTAs of a cluster, which
+ * combine their partial rows in a fixed order through distributed shared memory.  Nothing is kept in
+ * `scratch`, which may be NULL; it and nlfa_fwd_cached_scratch_bytes (what a split through global memory
+ * would take) remain for existing callers. */
 size_t nlfa_fwd_cached_scratch_bytes(int B, int Tq, int H, int Hkv, int L, int D);
 int nlfa_fwd_cached(const void* q, const void* k_cache, const void* v_cache, void* o, float* lse,
                     const int* qpos, const int* kpos, int B, int Tq, int H, int Hkv, int L, int D,
@@ -289,14 +288,21 @@ int nlfa_fwd_cached(const void* q, const void* k_cache, const void* v_cache, voi
 
 /* The same with the kernel family chosen by the caller (NLFA_PATH_*).  AUTO, which is what
  * nlfa_fwd_cached does, takes the tensor-core kernel (TMA + tcgen05, keys in blocks of 128, the
- * query rows of a KV head's whole group in one tile) for 16-bit inputs when the block has at
- * least 16 rows per KV head (Tq x group) and the cache at least 256 keys, on a compute-capability
- * 10.x device with 16-byte-aligned pointers and a positive scale; otherwise the fp32 kernel.
- * TENSOR returns NLFA_ERR_UNSUPPORTED_PATH when those conditions do not hold. */
+ * query rows of a KV head's whole group in one tile) for 16-bit inputs with up to 128 query heads per KV
+ * head, on a compute-capability 10.x device with 16-byte-aligned pointers and a positive scale;
+ * otherwise the fp32 kernel.  Below 16 rows per KV head (Tq x group) or 256 keys the probabilities
+ * enter the product as two 16-bit values each, so that such blocks get fp32-kernel precision.
+ * TENSOR returns NLFA_ERR_UNSUPPORTED_PATH below those sizes or when those conditions do not hold. */
 int nlfa_fwd_cached_path(const void* q, const void* k_cache, const void* v_cache, void* o, float* lse,
                          const int* qpos, const int* kpos, int B, int Tq, int H, int Hkv, int L, int D,
                          float scale, int causal, int window, int sinks, int dtype, int path,
                          void* scratch, size_t scratch_bytes, void* stream);
+
+/* The same with positions of `position_bytes` (4 or 8) bytes each, i.e. int32 or int64. */
+int nlfa_fwd_cached_positions(const void* q, const void* k_cache, const void* v_cache, void* o, float* lse,
+                              const void* qpos, const void* kpos, int position_bytes, int B, int Tq, int H, int Hkv,
+                              int L, int D, float scale, int causal, int window, int sinks, int dtype, int path,
+                              void* scratch, size_t scratch_bytes, void* stream);
 
 /* Bytes of device workspace `nlfa_selftest` needs. */
 size_t nlfa_selftest_workspace_bytes(void);

@@ -148,40 +148,42 @@ namespace {
 
 struct MapKey {
   const void* base;
-  int dtype, B, T, heads, D, rows;
-  bool operator==(const MapKey& o) const {
-    return base == o.base && dtype == o.dtype && B == o.B && T == o.T && heads == o.heads &&
-           D == o.D && rows == o.rows;
-  }
+  unsigned long long dims[4], strides[3];
+  unsigned box[4];
+  int dtype, pad;
+  bool operator==(const MapKey& o) const { return std::memcmp(this, &o, sizeof(MapKey)) == 0; }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     size_t h = reinterpret_cast<uintptr_t>(k.base) * 0x9e3779b97f4a7c15ull;
-    auto mix = [&h](int v) { h = (h ^ static_cast<size_t>(v)) * 0x100000001b3ull; };
-    mix(k.dtype); mix(k.B); mix(k.T); mix(k.heads); mix(k.D); mix(k.rows);
-    return h;
+    auto mix = [&h](unsigned long long v) { h = (h ^ v) * 0x100000001b3ull; };
+    for (unsigned long long v : k.dims) mix(v);
+    mix(k.box[1] | (static_cast<unsigned long long>(k.box[2]) << 32) | (static_cast<unsigned long long>(k.dtype) << 16));
+    return h ^ (h >> 29);
   }
 };
 std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;
 std::mutex g_maps_mutex;
 constexpr size_t kMaxCachedMaps = 4096;
 
-int encode_tile_map(CUtensorMap* map, const void* base, int dtype, int B, int T, int heads, int D,
-                    int rows) {
+int encode_map(CUtensorMap* map, const MapKey& k) {
   EncodeTiledFn fn = encode_tiled();
   if (fn == nullptr) return NLFA_ERR_CUDA;
-  const cuuint64_t dims[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(heads),
-                              static_cast<cuuint64_t>(T), static_cast<cuuint64_t>(B)};
-  const cuuint64_t strides[3] = {static_cast<cuuint64_t>(D) * 2,
-                                 static_cast<cuuint64_t>(heads) * D * 2,
-                                 static_cast<cuuint64_t>(T) * heads * D * 2};
-  const cuuint32_t box[4] = {64u, 1u, static_cast<cuuint32_t>(rows), 1u};
+  cuuint64_t dims[4], strides[3];
+  cuuint32_t box[4];
+  for (int i = 0; i < 4; ++i) {
+    dims[i] = k.dims[i];
+    box[i] = k.box[i];
+    if (i < 3) strides[i] = k.strides[i];
+  }
   const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
   const CUtensorMapDataType dt =
-      dtype == NLFA_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  CUresult r = fn(map, dt, 4, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      k.dtype == NLFA_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  auto encode = [&]() {
+    return fn(map, dt, 4, const_cast<void*>(k.base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
   if (r != CUDA_SUCCESS) {
     // The encoder is a driver entry point and wants a context current on the calling thread.  A
     // host thread that has made no runtime call yet (an autograd worker, say) has none: a
@@ -192,9 +194,7 @@ int encode_tile_map(CUtensorMap* map, const void* base, int dtype, int B, int T,
     (void)cudaDeviceGetAttribute(&attr, cudaDevAttrMultiProcessorCount, dev);
     size_t free_b = 0, total_b = 0;
     (void)cudaMemGetInfo(&free_b, &total_b);
-    r = fn(map, dt, 4, const_cast<void*>(base), dims, strides, box, estr,
-           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    r = encode();
   }
   return r == CUDA_SUCCESS ? NLFA_OK : NLFA_ERR_CUDA;
 }
@@ -203,10 +203,16 @@ int encode_tile_map(CUtensorMap* map, const void* base, int dtype, int B, int T,
 
 unsigned* status_block() { return status_word(); }
 
-int make_tile_map(CUtensorMap* map, const void* base, int dtype, int B, int T, int heads, int D,
-                  int rows) {
+int make_map(CUtensorMap* map, const void* base, int dtype, const unsigned long long dims[4],
+             const unsigned long long strides[3], const unsigned box[4]) {
   if (!aligned16(base)) return NLFA_ERR_MISALIGNED;
-  const MapKey key{base, dtype, B, T, heads, D, rows};
+  MapKey key;
+  std::memset(&key, 0, sizeof(key));
+  key.base = base;
+  std::memcpy(key.dims, dims, sizeof(key.dims));
+  std::memcpy(key.strides, strides, sizeof(key.strides));
+  std::memcpy(key.box, box, sizeof(key.box));
+  key.dtype = dtype;
   {
     std::lock_guard<std::mutex> lock(g_maps_mutex);
     auto it = g_maps.find(key);
@@ -215,12 +221,21 @@ int make_tile_map(CUtensorMap* map, const void* base, int dtype, int B, int T, i
       return NLFA_OK;
     }
   }
-  const int st = encode_tile_map(map, base, dtype, B, T, heads, D, rows);
+  const int st = encode_map(map, key);
   if (st != NLFA_OK) return st;
   std::lock_guard<std::mutex> lock(g_maps_mutex);
   if (g_maps.size() >= kMaxCachedMaps) g_maps.clear();
   g_maps.emplace(key, *map);
   return NLFA_OK;
+}
+
+int make_tile_map(CUtensorMap* map, const void* base, int dtype, int B, int T, int heads, int D,
+                  int rows) {
+  const unsigned long long d = D, h = heads, t = T;
+  const unsigned long long dims[4] = {d, h, t, static_cast<unsigned long long>(B)};
+  const unsigned long long strides[3] = {d * 2, h * d * 2, t * h * d * 2};
+  const unsigned box[4] = {64u, 1u, static_cast<unsigned>(rows), 1u};
+  return make_map(map, base, dtype, dims, strides, box);
 }
 
 int sched_counters(cudaStream_t stream, unsigned** out) {
@@ -260,6 +275,36 @@ int ensure_dynamic_smem(const void* kernel, int bytes) {
     return NLFA_ERR_CUDA;
   mask |= 1ull << dev;
   return NLFA_OK;
+}
+
+int resident_clusters(const void* kernel, int threads, int smem, int size) {
+  static std::mutex mutex;
+  static std::unordered_map<const void*, std::vector<int>> known[kMaxDevices];      // kernel -> clusters, by size
+  const int dev = current_device();
+  if (dev < 0 || size < 1 || size > kMostCluster) return 0;
+  std::lock_guard<std::mutex> lock(mutex);
+  std::vector<int>& v = known[dev][kernel];
+  if (v.empty()) {
+    v.assign(kMostCluster + 1, 0);
+    const bool big = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    for (int s = 1; s <= (big ? kMostCluster : 8); ++s) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(1, static_cast<unsigned>(s));
+      cfg.blockDim = dim3(static_cast<unsigned>(threads));
+      cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 1;
+      attr[0].val.clusterDim.y = static_cast<unsigned>(s);
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int n = 0;
+      v[s] = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess ? n : 0;
+    }
+    (void)cudaGetLastError();
+  }
+  return v[size];
 }
 
 bool overlap_launches(int kernel) {

@@ -10,283 +10,213 @@
 //     causal     : kpos <= qpos              (full to the cache, lower-triangular in the block)
 //     neither    : every key                 (block diffusion: a bidirectional block)
 //
-// Forward only (the cached path is inference).  A decode-sized problem: Tq is a block of a few
-// dozen tokens.  A CTA owns a few query rows of one (batch, KV head) -- the rows of every query head
-// of the group, so K and V are fetched once for all of them -- and walks the keys in tiles of 32
-// that the whole CTA copies into shared memory with coalesced 16-byte loads.  Inside a tile a
-// warp's lanes split the keys: a lane forms the whole dot product of its key (the query rows sit
-// in shared memory and are read as broadcasts) and keeps its own partial of the output row; the
-// running maximum of a row is shared through one warp reduction per tile and the lanes' partial
-// rows are added once at the end.  Tiles no row of the CTA can see are skipped without being
-// read.  fp32 arithmetic throughout, no atomics.
-#include "rowwise.cuh"
+// Forward only (the cached path is inference).  This file has the entry points and the fp32 kernel; 16-bit inputs
+// go to the tensor cores (cached_tc.cu).  The fp32 kernel: a CTA of 128 threads owns 8 RM query rows of one (batch, KV
+// head) -- the rows (t, g) of every query head of the group, so K and V are fetched once for all of them -- and
+// streams 64 keys at a time through shared memory, products in register tiles (tiles.cuh).  RM is the
+// largest of 4, 2, 1 that leaves two CTAs per SM: more rows per thread take fewer shared-memory reads per
+// multiply-add, but a block of a few rows needs CTAs.  Key blocks no row of the CTA can see (contiguous positions)
+// are skipped without being read; with few row tiles the key blocks are split over the CTAs of a cluster, which
+// combine the partial rows through distributed shared memory in a fixed order.  No atomics: bit-reproducible.
+// A warp of lanes over the keys of 8 rows before -> tiles: B=2 H=8 T=32 L=2048 D=64 in fp32 56 -> 28 us,
+// B=4 H=16/4 T=100 L=4096 848 -> 353 us.
+#include "cached.cuh"
+#include "tiles.cuh"
 
 namespace nlfa {
 namespace {
 
-using rowwise::Elem;
-constexpr int kWarps = 4;
+using namespace tiles;
+using cached::CachedParams;
+using cached::KeyRange;
 
-struct CachedParams {
-  int B, Tq, H, Hkv, L;
-  int causal, window, sinks;
-  float scale;
-  const int* qpos;   // nullptr: the block is the last Tq positions of a contiguous [0, L)
-  const int* kpos;   // nullptr: contiguous
-  int splits;        // > 1: blockIdx.y walks its share of the key tiles and leaves a partial result
-  int tiles_per_split;
-  float* part_o;     // [rows][splits][D]: each split's own normalised output row
-  float* part_l;     // [rows][splits]: its base-2 logsumexp (-inf: the split saw no key)
-};
-
-template <int D> __host__ __device__ constexpr int rows_per_warp() { return D <= 64 ? 2 : 1; }
-
-template <typename T, int D>
-__global__ void __launch_bounds__(kWarps * 32)
-fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
-                  T* __restrict__ o, float* __restrict__ lse) {
-  constexpr int RPW = rows_per_warp<D>();                  // query rows per warp
-  constexpr int RPC = kWarps * RPW;                        // ... per CTA
-  constexpr int kRowBytes = D * static_cast<int>(sizeof(T));
-  constexpr int kPitch = kRowBytes + 16;                   // padded: a lane's 16-byte reads of its own row do not collide
-  constexpr int kChunksPerRow = kRowBytes / 16, kChunks = 32 * kChunksPerRow;
-  __shared__ __align__(16) unsigned char ks[32 * kPitch];
-  __shared__ __align__(16) unsigned char vs[32 * kPitch];
-  __shared__ __align__(16) float qs[RPC][D];
-  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+template <typename T, int D, int RM>
+__global__ void __launch_bounds__(kThreads)
+fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v) {
+  constexpr int BM = 8 * RM, kPitch = D + 4;
+  extern __shared__ __align__(16) float smem[];
+  float* qs = smem;
+  float* ks = qs + BM * kPitch;
+  float* vs = ks + kBN * kPitch;
+  float* ps = vs + kBN * kPitch;
+  const int grp = threadIdx.x >> 4, col = threadIdx.x & 15;
   const int G = p.H / p.Hkv;
   const int head_rows = p.Tq * G;                          // query rows that share this KV head: (t, g)
-  const int chunks = (head_rows + RPC - 1) / RPC;
-  const int chunk = blockIdx.x % chunks;
-  const int bh = blockIdx.x / chunks;
+  const int chunks = (head_rows + BM - 1) / BM;
+  const int chunk = blockIdx.x % chunks, bh = blockIdx.x / chunks;
   const int hk = bh % p.Hkv, b = bh / p.Hkv;
-  const float scale2 = p.scale * kLog2e;
-  const int j_begin = static_cast<int>(blockIdx.y) * p.tiles_per_split * 32;        // this CTA's keys
-  const int j_stop = j_begin + p.tiles_per_split * 32;
-  const int j_end = j_stop < p.L ? j_stop : p.L;
+  const int r0 = chunk * BM, rows = head_rows - r0 < BM ? head_rows - r0 : BM;
+  const int t0 = r0 / G, t1 = (r0 + rows - 1) / G;
+  // row r of the tile in q / o [B,Tq,H]
+  auto out_row = [&](int r) -> long long {
+    const int t = (r0 + r) / G, g = (r0 + r) - t * G;
+    return (static_cast<long long>(b) * p.Tq + t) * p.H + hk * G + g;
+  };
+  const bool given = p.qpos != nullptr || p.kpos != nullptr;
+  const KeyRange range = cached::key_range(p.Tq, p.L, given, p.causal, p.window, p.sinks, t0, t1, kBN);
+  const int per = (range.count + p.splits - 1) / p.splits;
+  const int n_begin = static_cast<int>(blockIdx.y) * per;
+  const int n_stop = n_begin + per < range.count ? n_begin + per : range.count;
 
-  int qp[RPW], lo[RPW];
-  long long orow[RPW];                                     // row of q / o in [B,Tq,H]; -1: no such row
-#pragma unroll
-  for (int i = 0; i < RPW; ++i) {
-    const int r = chunk * RPC + wi * RPW + i;
-    orow[i] = -1;
-    qp[i] = lo[i] = 0;
-    if (r < head_rows) {
-      const int t = r / G, h = hk * G + r % G;
-      orow[i] = (static_cast<long long>(b) * p.Tq + t) * p.H + h;
-      qp[i] = p.qpos ? p.qpos[t] : p.L - p.Tq + t;
-      lo[i] = qp[i] - (p.window - p.sinks);                // window: keys above lo, or below sinks
-      for (int d = lane; d < D; d += 32) qs[wi * RPW + i][d] = static_cast<float>(q[orow[i] * D + d]) * scale2;
+  for (int i = threadIdx.x; i < BM * (D / 4); i += kThreads) {
+    const int r = i / (D / 4), c = 4 * (i % (D / 4));
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < rows) {
+      const T* src = q + out_row(r) * D + c;
+      if constexpr (sizeof(T) == 4) x = *reinterpret_cast<const float4*>(src);
+      else x = make_float4(to_f32(src[0]), to_f32(src[1]), to_f32(src[2]), to_f32(src[3]));
     }
+    *reinterpret_cast<float4*>(qs + r * kPitch + c) = x;
   }
-  __syncwarp();
-
-  const unsigned char* kb = reinterpret_cast<const unsigned char*>(k + (static_cast<long long>(b) * p.Hkv + hk) * p.L * D);
-  const unsigned char* vb = reinterpret_cast<const unsigned char*>(v + (static_cast<long long>(b) * p.Hkv + hk) * p.L * D);
-  float acc[RPW][D];
-  float m[RPW], l[RPW];                                    // m: shared by the warp; l: this lane's keys
+  const T* kb = k + (static_cast<long long>(b) * p.Hkv + hk) * p.L * D;
+  const T* vb = v + (static_cast<long long>(b) * p.Hkv + hk) * p.L * D;
+  auto load_kv = [&](float* dst, const T* src, int n) {
+    const long long j = range.at(n);
+    load_rows<T, D>(dst, src + j * kBN * D, D, kBN, p.L - static_cast<int>(j) * kBN);
+    load_commit();
+  };
+  float m[RM], l[RM], acc[RM][D / 16];
+  int qp[RM];
 #pragma unroll
-  for (int i = 0; i < RPW; ++i) {
+  for (int i = 0; i < RM; ++i) {
     m[i] = -INFINITY;
     l[i] = 0.f;
+    const int r = grp + 8 * i;
+    qp[i] = r < rows ? cached::query_position(p, (r0 + r) / G) : 0;
 #pragma unroll
-    for (int d = 0; d < D; ++d) acc[i][d] = 0.f;
+    for (int n = 0; n < D / 16; ++n) acc[i][n] = 0.f;
   }
-  // Which rows of this warp see key j0 + lane; `any`: some row does.
-  auto visible = [&](int j0, bool (&see)[RPW]) -> bool {
-    const int j = j0 + lane;
-    const int kp = j < j_end ? (p.kpos ? p.kpos[j] : j) : 0;
-    bool any = false;
+  if (n_begin < n_stop) {
+    load_kv(ks, kb, n_begin);
+    load_kv(vs, vb, n_begin);
+  }
+  for (int n = n_begin; n < n_stop; ++n) {
+    const int k0 = range.at(n) * kBN;
+    int kp[4];
+    bool in[4];
 #pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-      see[i] = j < j_end && orow[i] >= 0;
-      if (see[i]) {
-        if (p.window > 0) see[i] = kp <= qp[i] && (kp > lo[i] || kp < p.sinks);
-        else if (p.causal) see[i] = kp <= qp[i];
+    for (int j = 0; j < 4; ++j) {
+      const int key = k0 + col + 16 * j;
+      in[j] = key < p.L;
+      kp[j] = in[j] ? cached::key_position(p, key) : 0;
+    }
+    const bool full = !given && k0 + kBN <= p.L &&
+                      cached::all_visible(p, k0, k0 + kBN - 1, p.L - p.Tq + t0, p.L - p.Tq + t1);
+    load_wait<1>();
+    __syncthreads();                                       // K (and Q) are there; V may be on its way
+    float s[RM][4];
+    score_product<D, RM>(qs, ks, grp, col, s);
+    __syncthreads();
+    if (n + 1 < n_stop) load_kv(ks, kb, n + 1);
+    else load_commit();
+#pragma unroll
+    for (int i = 0; i < RM; ++i) {
+      float mx = m[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] *= p.scale_log2;
+        if (!full && !(in[j] && cached::position_visible(p, qp[i], kp[j]))) s[i][j] = -INFINITY;
+        mx = fmaxf(mx, s[i][j]);
       }
-      any |= see[i];
-    }
-    return any;
-  };
-  // A thread's share of a tile: kPer 16-byte chunks of K and of V, fetched into registers one tile
-  // ahead (while the current tile is being used) when that is few enough registers.
-  constexpr int kPer = kChunks / (kWarps * 32);
-  constexpr bool kAhead = kPer <= 4;
-  uint4 nk[kAhead ? kPer : 1], nv[kAhead ? kPer : 1];
-  auto fetch = [&](int j0) {
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int c = threadIdx.x + u * kWarps * 32;
-      const int r = c / kChunksPerRow, cc = c % kChunksPerRow;
-      if (j0 + r < j_end) {
-        const long long src = static_cast<long long>(j0 + r) * kRowBytes + cc * 16;
-        if constexpr (kAhead) {
-          nk[u] = *reinterpret_cast<const uint4*>(kb + src);
-          nv[u] = *reinterpret_cast<const uint4*>(vb + src);
-        } else {
-          *reinterpret_cast<uint4*>(ks + r * kPitch + cc * 16) = *reinterpret_cast<const uint4*>(kb + src);
-          *reinterpret_cast<uint4*>(vs + r * kPitch + cc * 16) = *reinterpret_cast<const uint4*>(vb + src);
-        }
+      for (int off = 8; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      const float ref = mx == -INFINITY ? 0.f : mx;        // nothing seen yet
+      const float alpha = exp2f(m[i] - ref);
+      m[i] = mx;
+      l[i] *= alpha;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float e = exp2f(s[i][j] - ref);
+        l[i] += e;
+        ps[(grp + 8 * i) * kPPitch + col + 16 * j] = e;
       }
-    }
-  };
-  auto stage = [&]() {                                     // registers -> shared memory (kAhead only)
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int c = threadIdx.x + u * kWarps * 32;
-      const int r = c / kChunksPerRow, cc = c % kChunksPerRow;
-      *reinterpret_cast<uint4*>(ks + r * kPitch + cc * 16) = nk[u];
-      *reinterpret_cast<uint4*>(vs + r * kPitch + cc * 16) = nv[u];
+      for (int x = 0; x < D / 16; ++x) acc[i][x] *= alpha;
     }
-  };
-  bool see[RPW];
-  bool cur = __syncthreads_or(visible(j_begin, see)) != 0;  // every thread of the CTA votes on every tile
-  if (kAhead && cur) fetch(j_begin);
-  for (int j0 = j_begin; j0 < j_end; j0 += 32) {
-    bool see_next[RPW];
-    const bool nxt = j0 + 32 < j_end && __syncthreads_or(visible(j0 + 32, see_next)) != 0;
-    if (cur) {
-      if constexpr (kAhead) stage(); else fetch(j0);
-      __syncthreads();
-    }
-    if (kAhead && nxt) fetch(j0 + 32);                     // in flight while this tile is used
-    if (!cur) {
-      cur = nxt;
+    load_wait<1>();
+    __syncthreads();                                       // V is there (and this warp's probabilities)
+    output_product<D, RM>(ps, vs, grp, col, acc);
+    __syncthreads();
+    if (n + 1 < n_stop) load_kv(vs, vb, n + 1);
+    else load_commit();
+  }
 #pragma unroll
-      for (int i = 0; i < RPW; ++i) see[i] = see_next[i];
+  for (int i = 0; i < RM; ++i) {
+    float sum = l[i];
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    const int r = grp + 8 * i;
+    if (r >= rows) continue;
+    if (p.splits > 1) {                                    // (K's and V's tiles are dead: the last product has read them)
+      store_row<float, D>(ks + r * kPitch, col, acc[i], 1.f);
+      if (col == 0) reinterpret_cast<float2*>(vs)[r] = make_float2(m[i], sum);
       continue;
     }
-    const T* kr = reinterpret_cast<const T*>(ks + lane * kPitch);
-    const T* vr = reinterpret_cast<const T*>(vs + lane * kPitch);
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) {
-      if (!__any_sync(0xffffffffu, see[i])) continue;
-      const float* qrow = qs[wi * RPW + i];
-      float s = -INFINITY;
-      if (see[i]) {
-        float dot[8];                                      // eight independent chains: the sum is latency bound otherwise
-#pragma unroll
-        for (int e = 0; e < 8; ++e) dot[e] = 0.f;
-#pragma unroll
-        for (int c = 0; c < D; c += 8) {
-          float x[8];
-          Elem<T>::load(kr + c, x);
-          const float4 qa = *reinterpret_cast<const float4*>(qrow + c), qb = *reinterpret_cast<const float4*>(qrow + c + 4);
-          dot[0] = fmaf(qa.x, x[0], dot[0]); dot[1] = fmaf(qa.y, x[1], dot[1]);
-          dot[2] = fmaf(qa.z, x[2], dot[2]); dot[3] = fmaf(qa.w, x[3], dot[3]);
-          dot[4] = fmaf(qb.x, x[4], dot[4]); dot[5] = fmaf(qb.y, x[5], dot[5]);
-          dot[6] = fmaf(qb.z, x[6], dot[6]); dot[7] = fmaf(qb.w, x[7], dot[7]);
-        }
-        s = ((dot[0] + dot[1]) + (dot[2] + dot[3])) + ((dot[4] + dot[5]) + (dot[6] + dot[7]));
-      }
-      float mx = s;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-      const float m_new = fmaxf(m[i], mx);                 // finite: some lane sees a key
-      const float alpha = exp2f(m[i] - m_new);             // first tile: exp2(-inf) = 0
-      const float pj = see[i] ? exp2f(s - m_new) : 0.f;
-      l[i] = fmaf(l[i], alpha, pj);
-      m[i] = m_new;
-      if (see[i]) {
-#pragma unroll
-        for (int c = 0; c < D; c += 8) {
-          float x[8];
-          Elem<T>::load(vr + c, x);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) acc[i][c + e] = fmaf(acc[i][c + e], alpha, pj * x[e]);
-        }
-      } else if (alpha != 1.f) {
-#pragma unroll
-        for (int d = 0; d < D; ++d) acc[i][d] *= alpha;
-      }
+    const long long row = out_row(r);
+    const float inv = sum > 0.f ? 1.f / sum : 0.f;         // a row that sees no key gives zeros
+    store_row<T, D>(static_cast<T*>(p.o) + row * D, col, acc[i], inv);
+    if (p.lse && col == 0) {
+      const long long t = (row / p.H) % p.Tq, h = row % p.H;
+      p.lse[(static_cast<long long>(b) * p.H + h) * p.Tq + t] = sum > 0.f ? (m[i] + log2f(sum)) * kLn2 : -INFINITY;
     }
-    __syncthreads();                                       // the tile may be overwritten
-    cur = nxt;
-#pragma unroll
-    for (int i = 0; i < RPW; ++i) see[i] = see_next[i];
   }
-#pragma unroll
-  for (int i = 0; i < RPW; ++i) {
-    float lsum = l[i];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
-    const float inv = lsum > 0.f ? 1.f / lsum : 0.f;       // a row that sees no key gives zeros
-    // add the lanes' partial rows: after the butterfly every lane holds every sum; lane d % 32 keeps d
-    float* out_row = qs[wi * RPW + i];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      float x = acc[i][d];
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-      if (lane == (d & 31)) out_row[d] = x * inv;
-    }
-    __syncwarp();
-    if (orow[i] >= 0 && p.splits > 1) {                    // partial result; merge_splits_kernel finishes the row
-      const long long slot = orow[i] * p.splits + blockIdx.y;
-      for (int d = lane; d < D; d += 32) p.part_o[slot * D + d] = out_row[d];
-      if (lane == 0) p.part_l[slot] = lsum > 0.f ? m[i] + log2f(lsum) : -INFINITY;
-    } else if (orow[i] >= 0) {
-      for (int d = lane; d < D; d += 32) o[orow[i] * D + d] = static_cast<T>(out_row[d]);
-      if (lse && lane == 0) {
-        const long long t = (orow[i] / p.H) % p.Tq, h = orow[i] % p.H;
-        lse[(static_cast<long long>(b) * p.H + h) * p.Tq + t] = lsum > 0.f ? (m[i] + log2f(lsum)) * kLn2 : -INFINITY;
-      }
-    }
+  if (p.splits > 1) {
+    cluster_arrive();
+    cluster_wait();
+    cached::merge_rows<T, D, 1>(p, rows, out_row, smem_u32(ks), 0, smem_u32(vs), ps, static_cast<int>(blockIdx.y),
+                                [] { __syncthreads(); return true; }, threadIdx.x, kThreads);
+    cluster_arrive();                                      // no CTA leaves while another reads its shared memory
+    cluster_wait();
   }
 }
 
-// One warp per query row: the splits' partial rows, each normalised by its own sum, are combined with the
-// weights 2^(lse_s - max lse), in a fixed order.
+template <typename T, int D, int RM>
+int launch_rm(CachedParams p, const void* q, const void* k, const void* v, int splits, cudaStream_t st) {
+  constexpr int BM = 8 * RM;
+  constexpr int smem = ((BM + 2 * kBN) * (D + 4) + BM * kPPitch) * 4;
+  auto kern = fwd_cached_kernel<T, D, RM>;
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != NLFA_OK) return NLFA_ERR_CUDA;
+  const long long head_rows = static_cast<long long>(p.Tq) * (p.H / p.Hkv);
+  const long long grid = static_cast<long long>(p.B) * p.Hkv * ((head_rows + BM - 1) / BM);
+  if (grid >= (1ll << 31)) return NLFA_ERR_BAD_SHAPE;
+  p.splits = splits > 1 ? cached::cluster_splits(reinterpret_cast<const void*>(kern), kThreads, smem, grid, splits) : 1;
+  if (launch_cluster(kern, dim3(static_cast<unsigned>(grid), static_cast<unsigned>(p.splits)), dim3(kThreads), smem, st, false,
+                     p.splits, p, static_cast<const T*>(q), static_cast<const T*>(k), static_cast<const T*>(v)) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return NLFA_ERR_CUDA;
+  }
+  return NLFA_OK;
+}
+
 template <typename T, int D>
-__global__ void __launch_bounds__(kWarps * 32)
-merge_splits_kernel(CachedParams p, T* __restrict__ o, float* __restrict__ lse) {
-  const int lane = threadIdx.x & 31;
-  const long long row = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5);    // over [B,Tq,H]
-  if (row >= static_cast<long long>(p.B) * p.Tq * p.H) return;
-  const float* pl = p.part_l + row * p.splits;
-  float mx = -INFINITY;
-  for (int s = 0; s < p.splits; ++s) mx = fmaxf(mx, pl[s]);
-  float wsum = 0.f;
-  for (int s = 0; s < p.splits; ++s) wsum += mx > -INFINITY ? exp2f(pl[s] - mx) : 0.f;
-  const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
-  for (int d = lane; d < D; d += 32) {
-    float acc = 0.f;
-    for (int s = 0; s < p.splits; ++s)
-      if (pl[s] > -INFINITY) acc = fmaf(exp2f(pl[s] - mx), p.part_o[(row * p.splits + s) * D + d], acc);
-    o[row * D + d] = static_cast<T>(acc * inv);
-  }
-  if (lse && lane == 0) {
-    const long long t = (row / p.H) % p.Tq, h = row % p.H, b = row / (static_cast<long long>(p.H) * p.Tq);
-    lse[(b * p.H + h) * p.Tq + t] = wsum > 0.f ? (mx + log2f(wsum)) * kLn2 : -INFINITY;
-  }
+int launch_dim(const CachedParams& p, const void* q, const void* k, const void* v, cudaStream_t st) {
+  const long long head_rows = static_cast<long long>(p.Tq) * (p.H / p.Hkv), heads = static_cast<long long>(p.B) * p.Hkv;
+  const long long want = 2ll * sm_count(), pairs = ((p.L + kBN - 1) / kBN + 1) / 2;      // two key blocks per CTA at least
+  // the taller tile first, its keys split as far as it takes to fill the GPU; only then shorter ones
+  auto splits = [&](int rm) {
+    const long long tiles = heads * ((head_rows + 8 * rm - 1) / (8 * rm));
+    long long s = (2 * want + tiles - 1) / tiles;
+    if (tiles >= want) s = 1;
+    if (s > kMostCluster) s = kMostCluster;
+    if (s > pairs) s = pairs;
+    return static_cast<int>(s < 1 ? 1 : s);
+  };
+  auto fills = [&](int rm) { return heads * ((head_rows + 8 * rm - 1) / (8 * rm)) * splits(rm) >= want; };
+  if (head_rows > 16 && fills(4)) return launch_rm<T, D, 4>(p, q, k, v, splits(4), st);
+  if (head_rows > 8 && fills(2)) return launch_rm<T, D, 2>(p, q, k, v, splits(2), st);
+  return launch_rm<T, D, 1>(p, q, k, v, splits(1), st);
 }
 
 template <typename T>
-int launch_for_dim(const CachedParams& p, int D, const void* q, const void* k, const void* v, void* o, float* lse,
-                   cudaStream_t st) {
-  const long long head_rows = static_cast<long long>(p.Tq) * (p.H / p.Hkv);
-#define NLFA_GO(DD)                                                                                      \
-  do {                                                                                                   \
-    constexpr int rpc = kWarps * rows_per_warp<DD>();                                                    \
-    const long long grid = static_cast<long long>(p.B) * p.Hkv * ((head_rows + rpc - 1) / rpc);          \
-    if (grid >= (1ll << 31)) return NLFA_ERR_BAD_SHAPE;                                                  \
-    fwd_cached_kernel<T, DD><<<dim3(static_cast<unsigned>(grid), p.splits), kWarps * 32, 0, st>>>(        \
-        p, (const T*)q, (const T*)k, (const T*)v, (T*)o, lse);                                           \
-    if (p.splits > 1) {                                                                                  \
-      const long long rows = static_cast<long long>(p.B) * p.Tq * p.H;                                   \
-      merge_splits_kernel<T, DD><<<static_cast<unsigned>((rows + kWarps - 1) / kWarps), kWarps * 32, 0, st>>>( \
-          p, (T*)o, lse);                                                                                \
-    }                                                                                                    \
-  } while (0)
-  if (D == 32) NLFA_GO(32); else if (D == 64) NLFA_GO(64); else NLFA_GO(128);
-#undef NLFA_GO
-  return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
+int launch_simt(const CachedParams& p, const void* q, const void* k, const void* v, cudaStream_t st) {
+  if (p.D == 32) return launch_dim<T, 32>(p, q, k, v, st);
+  if (p.D == 64) return launch_dim<T, 64>(p, q, k, v, st);
+  return launch_dim<T, 128>(p, q, k, v, st);
 }
 
-// How many ways the keys are split: only when the row chunks alone leave most SMs idle.
+// How many ways the keys would be split through global memory (nlfa_fwd_cached_scratch_bytes).
 int choose_splits(int B, int Tq, int H, int Hkv, int L, int D) {
-  const long long rpc = kWarps * (D <= 64 ? 2 : 1);
+  const long long rpc = D <= 64 ? 8 : 4;
   const long long base = static_cast<long long>(B) * Hkv * ((static_cast<long long>(Tq) * (H / Hkv) + rpc - 1) / rpc);
   const long long tiles = (L + 31) / 32;
   if (base <= 0 || base >= 296 || tiles < 8) return 1;
@@ -296,39 +226,21 @@ int choose_splits(int B, int Tq, int H, int Hkv, int L, int D) {
   return s < 1 ? 1 : static_cast<int>(s);
 }
 
-template <typename T>
-int merge_for_dim(const CachedParams& p, int D, void* o, float* lse, cudaStream_t st) {
-  const long long rows = static_cast<long long>(p.B) * p.Tq * p.H;
-  const unsigned grid = static_cast<unsigned>((rows + kWarps - 1) / kWarps);
-  if (D == 32) merge_splits_kernel<T, 32><<<grid, kWarps * 32, 0, st>>>(p, (T*)o, lse);
-  else if (D == 64) merge_splits_kernel<T, 64><<<grid, kWarps * 32, 0, st>>>(p, (T*)o, lse);
-  else merge_splits_kernel<T, 128><<<grid, kWarps * 32, 0, st>>>(p, (T*)o, lse);
-  return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
-}
-
-size_t split_scratch_bytes(int B, int Tq, int H, int D, int s) {
-  return s <= 1 ? 0 : static_cast<size_t>(B) * Tq * H * s * (static_cast<size_t>(D) + 1) * sizeof(float);
-}
-
 }  // namespace
 
 // tensor-core form (cached_tc.cu)
 bool cached_tc_applies(int Tq, int H, int Hkv, int L, int D, int dtype);
-int cached_tc_splits(int B, int Tq, int H, int Hkv, int L);
-int launch_fwd_cached_tc(const void* q, const void* k_cache, const void* v_cache, void* o, float* lse,
-                         const int* qpos, const int* kpos, int B, int Tq, int H, int Hkv, int L, int D,
-                         float scale, int causal, int window, int sinks, int dtype, float* part_o,
-                         float* part_l, int splits, unsigned* status, cudaStream_t stream);
+bool cached_tc_can(int H, int Hkv, int D, int dtype);
+int launch_fwd_cached_tc(CachedParams p, const void* q, const void* k_cache, const void* v_cache, int dtype, bool split_p,
+                         unsigned* status, cudaStream_t stream);
 unsigned* status_block();      // api.cu
 
 }  // namespace nlfa
 
 extern "C" size_t nlfa_fwd_cached_scratch_bytes(int B, int Tq, int H, int Hkv, int L, int D) {
   if (B <= 0 || Tq <= 0 || H <= 0 || Hkv <= 0 || L <= 0 || H % Hkv != 0) return 0;
-  // the larger of what the two kernel families would split into (the family is chosen per call)
-  const size_t simt = nlfa::split_scratch_bytes(B, Tq, H, D, nlfa::choose_splits(B, Tq, H, Hkv, L, D));
-  const size_t tc = H / Hkv <= 128 ? nlfa::split_scratch_bytes(B, Tq, H, D, nlfa::cached_tc_splits(B, Tq, H, Hkv, L)) : 0;
-  return simt > tc ? simt : tc;
+  const int s = nlfa::choose_splits(B, Tq, H, Hkv, L, D);
+  return s <= 1 ? 0 : static_cast<size_t>(B) * Tq * H * s * (static_cast<size_t>(D) + 1) * sizeof(float);
 }
 
 extern "C" int nlfa_fwd_cached(const void* q, const void* k_cache, const void* v_cache, void* o, float* lse,
@@ -343,8 +255,19 @@ extern "C" int nlfa_fwd_cached_path(const void* q, const void* k_cache, const vo
                                     const int* qpos, const int* kpos, int B, int Tq, int H, int Hkv, int L, int D,
                                     float scale, int causal, int window, int sinks, int dtype, int path,
                                     void* scratch, size_t scratch_bytes, void* stream) {
+  return nlfa_fwd_cached_positions(q, k_cache, v_cache, o, lse, qpos, kpos, 4, B, Tq, H, Hkv, L, D, scale, causal, window,
+                                   sinks, dtype, path, scratch, scratch_bytes, stream);
+}
+
+extern "C" int nlfa_fwd_cached_positions(const void* q, const void* k_cache, const void* v_cache, void* o, float* lse,
+                                         const void* qpos, const void* kpos, int position_bytes, int B, int Tq, int H,
+                                         int Hkv, int L, int D, float scale, int causal, int window, int sinks, int dtype,
+                                         int path, void* scratch, size_t scratch_bytes, void* stream) {
   using namespace nlfa;
+  (void)scratch;                 // the split's partial rows stay in shared memory
+  (void)scratch_bytes;
   if (path != NLFA_PATH_AUTO && path != NLFA_PATH_SIMT && path != NLFA_PATH_TENSOR) return NLFA_ERR_UNSUPPORTED_PATH;
+  if (position_bytes != 4 && position_bytes != 8) return NLFA_ERR_BAD_ARGUMENT;
   if (B < 0 || Tq < 0 || H < 0 || L < 0 || Hkv <= 0 || H % Hkv != 0 || !(scale == scale)) return NLFA_ERR_BAD_SHAPE;
   if (D != 32 && D != 64 && D != 128) return NLFA_ERR_BAD_HEAD_DIM;
   if (dtype != NLFA_DTYPE_F32 && dtype != NLFA_DTYPE_F16 && dtype != NLFA_DTYPE_BF16) return NLFA_ERR_BAD_DTYPE;
@@ -356,37 +279,24 @@ extern "C" int nlfa_fwd_cached_path(const void* q, const void* k_cache, const vo
   if (rows == 0) return NLFA_OK;
   if (rows / 4 >= (1ll << 31)) return NLFA_ERR_BAD_SHAPE;
   if (!q || !o || (L > 0 && (!k_cache || !v_cache))) return NLFA_ERR_NULL_POINTER;
-  CachedParams p{B, Tq, H, Hkv, L, causal ? 1 : 0, window, sinks, scale, qpos, kpos, 1, (L + 31) / 32, nullptr, nullptr};
+  const CachedParams p{B, Tq, H, Hkv, L, D, causal ? 1 : 0, window, sinks, scale * kLog2e, qpos, kpos, position_bytes == 8,
+                       1, o, lse};
   cudaStream_t st = (cudaStream_t)stream;
   const bool aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_cache) |
                          reinterpret_cast<uintptr_t>(v_cache) | reinterpret_cast<uintptr_t>(o)) & 15u) == 0;
-  if (path != NLFA_PATH_SIMT && aligned && scale > 0.f && nlfa_device_supported() &&
-      cached_tc_applies(Tq, H, Hkv, L, D, dtype)) {
-    // blocks of a few dozen rows and more over a long cache: the products run on the tensor cores
+  // 16-bit inputs: the products run on the tensor cores, whatever the block's size, because the cache's
+  // bandwidth is what counts.  Blocks a caller cannot force onto them (fewer than 16 rows per KV head, or under
+  // 256 keys) keep the fp32 kernel's precision there (SPLIT_P).
+  const bool applies = cached_tc_applies(Tq, H, Hkv, L, D, dtype);
+  if (aligned && L > 0 && scale > 0.f && nlfa_device_supported() &&
+      (path == NLFA_PATH_TENSOR ? applies : path == NLFA_PATH_AUTO && cached_tc_can(H, Hkv, D, dtype))) {
     if (nlfa_peek_status() != NLFA_OK) return NLFA_ERR_DEVICE_TIMEOUT;
     unsigned* status = status_block();
     if (!status) return NLFA_ERR_CUDA;
-    int splits = cached_tc_splits(B, Tq, H, Hkv, L);
-    if (split_scratch_bytes(B, Tq, H, D, splits) > (scratch ? scratch_bytes : 0)) splits = 1;
-    float* part_o = static_cast<float*>(scratch);
-    float* part_l = splits > 1 ? part_o + rows * splits * D : nullptr;
-    const int rc = launch_fwd_cached_tc(q, k_cache, v_cache, o, lse, qpos, kpos, B, Tq, H, Hkv, L, D, scale, causal,
-                                        window, sinks, dtype, splits > 1 ? part_o : nullptr, part_l, splits, status, st);
-    if (rc != NLFA_OK || splits == 1) return rc;
-    p.splits = splits;
-    p.part_o = part_o;
-    p.part_l = part_l;
-    return dtype == NLFA_DTYPE_BF16 ? merge_for_dim<__nv_bfloat16>(p, D, o, lse, st) : merge_for_dim<__half>(p, D, o, lse, st);
+    return launch_fwd_cached_tc(p, q, k_cache, v_cache, dtype, !applies, status, st);
   }
   if (path == NLFA_PATH_TENSOR) return NLFA_ERR_UNSUPPORTED_PATH;
-  const size_t need = split_scratch_bytes(B, Tq, H, D, choose_splits(B, Tq, H, Hkv, L, D));
-  if (need > 0 && scratch != nullptr && scratch_bytes >= need) {     // without scratch: one CTA walks all keys
-    p.splits = choose_splits(B, Tq, H, Hkv, L, D);
-    p.tiles_per_split = ((L + 31) / 32 + p.splits - 1) / p.splits;
-    p.part_o = static_cast<float*>(scratch);
-    p.part_l = p.part_o + rows * p.splits * D;
-  }
-  if (dtype == NLFA_DTYPE_BF16) return launch_for_dim<__nv_bfloat16>(p, D, q, k_cache, v_cache, o, lse, st);
-  if (dtype == NLFA_DTYPE_F16) return launch_for_dim<__half>(p, D, q, k_cache, v_cache, o, lse, st);
-  return launch_for_dim<float>(p, D, q, k_cache, v_cache, o, lse, st);
+  if (dtype == NLFA_DTYPE_BF16) return launch_simt<__nv_bfloat16>(p, q, k_cache, v_cache, st);
+  if (dtype == NLFA_DTYPE_F16) return launch_simt<__half>(p, q, k_cache, v_cache, st);
+  return launch_simt<float>(p, q, k_cache, v_cache, st);
 }

@@ -209,6 +209,9 @@ int launch_selftest_tiles(int dtype, int head_dim, const void* q, const void* k,
 // per map (ten maps per forward + backward).
 int make_tile_map(CUtensorMap* map, const void* base, int dtype, int B, int T, int heads, int D,
                   int rows);
+// The same for any 4-D tensor of 16-bit elements: extents, byte strides of dimensions 1-3, box.
+int make_map(CUtensorMap* map, const void* base, int dtype, const unsigned long long dims[4],
+             const unsigned long long strides[3], const unsigned box[4]);
 
 // Two work counters for one launch of a persistent kernel ([0] next unit, [1] CTAs finished;
 // the last CTA of a launch zeroes them again).  Launches on a capturing stream draw from a
@@ -222,6 +225,11 @@ int ensure_dynamic_smem(const void* kernel, int bytes);
 
 int sm_count();
 
+// How many clusters of `size` CTAs (up to kMostCluster, along y) of a kernel can be resident at once; asked of the
+// driver once per kernel and device.
+constexpr int kMostCluster = 16;
+int resident_clusters(const void* kernel, int threads, int smem, int size);
+
 // Which kernels are launched with programmatic stream serialization, so that their set-up
 // (barriers, TMEM, descriptors) overlaps the predecessor's last CTAs.  NLFA_PDL=<mask> overrides
 // the default (0: none).
@@ -233,22 +241,36 @@ bool overlap_launches(int kernel);
 bool bwd_delta_in_dq(const Problem& p, int passes);
 
 // One launch through cudaLaunchKernelEx, with the programmatic-serialization attribute when
-// `overlap` is set.  The kernel must then call grid_dep_wait() before it reads anything an earlier
+// `overlap` is set and, given `cluster_y` > 1, in clusters of that many CTAs along y.  The kernel must then call grid_dep_wait() before it reads anything an earlier
 // kernel of the stream wrote.
 template <typename... Params, typename... Args>
-cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                          bool overlap, Args&&... args) {
+cudaError_t launch_cluster(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                           bool overlap, int cluster_y, Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  unsigned n = 0;
+  if (overlap) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster_y > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = 1;
+    attr[n].val.clusterDim.y = static_cast<unsigned>(cluster_y);
+    attr[n++].val.clusterDim.z = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = overlap ? 1u : 0u;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <typename... Params, typename... Args>
+cudaError_t launch_kernel(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                          bool overlap, Args&&... args) {
+  return launch_cluster(kernel, grid, block, smem, stream, overlap, 1, static_cast<Args&&>(args)...);
 }
 
 }  // namespace nlfa

@@ -474,21 +474,19 @@ PyObject* py_attn_cached(PyObject*, PyObject* const* a, Py_ssize_t n) {
     q = detached(q);
     k = detached(k);
     v = detached(v);
+    const auto kind = [](const Tensor& t) { return t.defined() ? t.scalar_type() : at::kLong; };
+    const bool wide = kind(qpos) == at::kLong && kind(kpos) == at::kLong;        // read as they are
     auto positions = [&](const Tensor& t) {
-      return !t.defined() ? t : contiguous(t.device() == q.device() ? cast(t, at::kInt) : t.to(q.device(), at::kInt));
+      return !t.defined() ? t : contiguous((t.device() == q.device() ? t : t.to(q.device())).to(wide ? at::kLong : at::kInt));
     };
     qpos = positions(qpos);
     kpos = positions(kpos);
     o = empty_as(q);
     if (want_lse) lse = empty({B, H, T}, at::kFloat, q);
-    const size_t bytes = nlfa_fwd_cached_scratch_bytes(B, T, H, Hkv, L, D);      // > 0: the keys are split over CTAs
-    const Tensor scratch = bytes ? empty({static_cast<int64_t>(bytes)}, at::kByte, q) : Tensor();
-    const int st = nlfa_fwd_cached_path(
+    const int st = nlfa_fwd_cached_positions(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), want_lse ? static_cast<float*>(lse.data_ptr()) : nullptr,
-        qpos.defined() ? static_cast<int*>(qpos.data_ptr()) : nullptr,
-        kpos.defined() ? static_cast<int*>(kpos.data_ptr()) : nullptr, B, T, H, Hkv, L, D, static_cast<float>(scale),
-        causal ? 1 : 0, m.window, m.sinks, dtype_code(q.scalar_type()), path, bytes ? scratch.data_ptr() : nullptr, bytes,
-        stream_of(q));
+        qpos.defined() ? qpos.data_ptr() : nullptr, kpos.defined() ? kpos.data_ptr() : nullptr, wide ? 8 : 4, B, T, H, Hkv, L, D, static_cast<float>(scale),
+        causal ? 1 : 0, m.window, m.sinks, dtype_code(q.scalar_type()), path, nullptr, 0, stream_of(q));
     if (st == NLFA_ERR_UNSUPPORTED_PATH && path == NLFA_PATH_TENSOR)
       TORCH_CHECK_VALUE(false, "flash_attn_cached: use_mma=True but the tensor-core kernel does not apply to these inputs");
     check("nlfa_fwd_cached", st);
