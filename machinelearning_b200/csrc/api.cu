@@ -432,7 +432,7 @@ size_t ds_pair_bytes(const Problem& p) {
   return static_cast<size_t>(ds_tile_offset(l, l.n_tiles)) * kDsTileBytes * (p.H / p.Hkv);
 }
 
-constexpr size_t kDsMostBytes = size_t{2} << 30;        // dS of as many pairs at a time as fit here
+constexpr size_t kDsMostBytes = size_t{4} << 30;        // dS of as many pairs at a time as fit here
 }  // namespace
 
 size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
@@ -446,6 +446,14 @@ size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window,
   const size_t pair = ds_pair_bytes(p), all = static_cast<size_t>(B) * Hkv;
   const size_t most = kDsMostBytes / pair;
   if (most == 0) return tape;
+  // The dQ pass that recomputes dS starts beside the dK/dV pass and takes the SMs it leaves idle; one that reads
+  // dS cannot.  So every launch has to keep the GPU busy by itself: half as many units (key blocks) again as SMs,
+  // three per SM where the problem goes in parts.  Measured recomputing / reading: B=2 H=8/2 T=3000 (96 units)
+  // 200 / 264 us, B=4 H=12/4 T=2048 (256) 198 / 182, B=22 H=12 T=60 (264) 32 / 29, two parts of 218 units each
+  // (B=4 H=4/1 T=13866) 3.26 / 3.42 ms for the whole step.
+  const size_t parts = (all + most - 1) / most, per = (all + parts - 1) / parts;
+  const size_t units = per * ((T + kTile - 1) / kTile), sms = static_cast<size_t>(sm_count());
+  if (2 * units < 3 * sms || (parts > 1 && units < 3 * sms)) return tape;
   return round256(tape) + pair * (all < most ? all : most);
 }
 

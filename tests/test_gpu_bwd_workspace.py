@@ -1,4 +1,4 @@
-"""Backward at head dim 128 with room for dS (``nlfa_bwd_workspace_bytes``): the dK/dV pass leaves dS in the
+"""Backward at head dim 128 with room for dS behind the tape: the dK/dV pass leaves dS in the
 scratch and dQ is one product over it.  Held to the float64 oracle and, bit for bit, to the layout that
 recomputes dS (tape-only scratch), at lengths around the 64- and 128-row tile edges, under every mask, with the
 scratch poisoned and with room for one (batch, KV head) pair at a time."""
@@ -43,11 +43,16 @@ def test_backward_with_room_for_ds(B, T, H, Hkv, window, sinks, block, dtype):
     code = L.DTYPE_BF16 if dtype == torch.bfloat16 else L.DTYPE_F16
     dims = (B, T, H, Hkv, D, window, sinks, block, code, L.PATH_TENSOR)
     tape = lib.nlfa_bwd_scratch_bytes(B, T, H)
-    whole = lib.nlfa_bwd_workspace_bytes(*dims)
-    base = (tape + 255) // 256 * 256
-    one_pair = base + (whole - base) // (B * Hkv)
-    assert whole > tape and lib.nlfa_bwd_workspace_kernel_count(*dims, whole) == 3
-    assert lib.nlfa_bwd_workspace_kernel_count(*dims, one_pair) == 1 + 2 * B * Hkv
+    base, tiles, pairs = (tape + 255) // 256 * 256, (T + 127) // 128, B * Hkv
+    whole = base + B * H * tiles * tiles * 32768                     # every tile pair: enough for any mask
+    assert lib.nlfa_bwd_workspace_kernel_count(*dims, whole) == 3
+    # the least that holds one pair: its launches go pair by pair
+    count = lambda n: lib.nlfa_bwd_workspace_kernel_count(*dims, base + n * (H // Hkv) * 32768)
+    one_pair = whole
+    if pairs > 1:
+        n = next(n for n in range(1, tiles * tiles + 1) if count(n) > 3)
+        assert count(n) == 1 + 2 * pairs
+        one_pair = base + n * (H // Hkv) * 32768
     args = (lib, L, do, q, k, v, o, lse, scale, window, sinks, block)
     recomputed, left, by_pair = (_backward(*args, n) for n in (tape, whole, one_pair))
     want = orc.attention_bwd(do, q, k, v, scale, window, sinks, block)
