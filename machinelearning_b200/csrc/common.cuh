@@ -233,7 +233,7 @@ int resident_clusters(const void* kernel, int threads, int smem, int size);
 // Which kernels are launched with programmatic stream serialization, so that their set-up
 // (barriers, TMEM, descriptors) overlaps the predecessor's last CTAs.  NLFA_PDL=<mask> overrides
 // the default (0: none).
-enum { kOverlapFwd = 1, kOverlapDelta = 2, kOverlapDkv = 4, kOverlapDq = 8, kOverlapDefault = 15 };
+enum { kOverlapFwd = 1, kOverlapDelta = 2, kOverlapDkv = 4, kOverlapDq = 8, kOverlapRowwise = 16, kOverlapDefault = 31 };
 bool overlap_launches(int kernel);
 
 // Whether the tensor-core backward forms Delta inside its dQ pass for this problem and mask

@@ -8,8 +8,9 @@
 //
 // and their backward passes.  In torch each is several full passes over [B,T,H,D]
 // (multiplies, an add, a cast; the backward also a reduction).  Here: HBM-bound, every
-// operand read once, every result written once.  Reductions (the scalar's gradient, the
-// gate's gradient per row) run in a fixed order: bit-reproducible, no atomics.
+// operand read once, every result written once.  Reductions (the scalar's gradient -- partial sums per CTA,
+// added up by the CTA that finishes last -- and the gate's gradient per row) run in a fixed order: bit-reproducible.
+// Each kernel starts under its predecessor's tail (programmatic launch).
 #include "rowwise.cuh"
 
 namespace nlfa {
@@ -25,6 +26,8 @@ __global__ void __launch_bounds__(kThreads)
 value_blend_fwd_kernel(const TV* __restrict__ v, const TV* __restrict__ v0, const float* __restrict__ lambda,
                        TOut* __restrict__ out, unsigned nvec) {
   constexpr int U = Elem<TV>::kInFlight / 2;           // two operands per element
+  grid_dep_wait();
+  grid_dep_release();
   const float s = sigmoidf(*lambda), c = 1.f - s;
   const unsigned span = gridDim.x * kThreads;          // consecutive threads take consecutive 8-element vectors
   for (unsigned i0 = blockIdx.x * kThreads + threadIdx.x; i0 < nvec; i0 += span * U) {
@@ -56,8 +59,11 @@ template <typename TV, typename TG>
 __global__ void __launch_bounds__(kThreads)
 value_blend_bwd_kernel(const TG* __restrict__ g, const TV* __restrict__ v, const TV* __restrict__ v0,
                        const float* __restrict__ lambda, TV* __restrict__ dv, TV* __restrict__ dv0,
-                       float* __restrict__ partial, unsigned nvec) {
+                       float* __restrict__ partial, float* __restrict__ dlambda, unsigned* ticket, unsigned nvec) {
   __shared__ float red[kThreads / 32];
+  __shared__ int last;
+  grid_dep_wait();
+  grid_dep_release();
   const float s = sigmoidf(*lambda), c = 1.f - s;
   const unsigned stride = gridDim.x * kThreads;
   float acc = 0.f;
@@ -78,35 +84,26 @@ value_blend_bwd_kernel(const TG* __restrict__ g, const TV* __restrict__ v, const
     Elem<TV>::store(dv + (size_t)i * kVec, x);
     Elem<TV>::store(dv0 + (size_t)i * kVec, y);
   }
+  auto cta_sum = [&](float a) -> float {                // in thread 0
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+    for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
+    __syncthreads();
     float t = 0.f;
+    if (threadIdx.x == 0) {
 #pragma unroll
-    for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-    partial[blockIdx.x] = t;
-  }
-}
-
-__global__ void __launch_bounds__(1024)
-value_blend_scalar_grad_kernel(const float* __restrict__ partial, int n, const float* __restrict__ lambda,
-                               float* __restrict__ dlambda) {
-  __shared__ float red[32];
+      for (int w = 0; w < kThreads / 32; ++w) t += red[w];
+    }
+    return t;
+  };
+  const float mine = cta_sum(acc);
+  if (threadIdx.x == 0) partial[blockIdx.x] = mine;
+  if (!last_cta(ticket, gridDim.x, &last)) return;
   float a = 0.f;
-  for (int i = threadIdx.x; i < n; i += 1024) a += partial[i];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = a;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-#pragma unroll
-    for (int w = 0; w < 32; ++w) t += red[w];
-    const float s = sigmoidf(*lambda);
-    *dlambda = t * s * (1.f - s);
-  }
+#pragma unroll 4
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += kThreads) a += __ldcg(partial + i);
+  const float total = cta_sum(a);
+  if (threadIdx.x == 0) *dlambda = total * s * (1.f - s);
 }
 
 // ------------------------------------------------------------------ head gate
@@ -116,6 +113,8 @@ template <typename TY, typename TGate, int D>
 __global__ void __launch_bounds__(kThreads)
 head_gate_fwd_kernel(const TY* __restrict__ y, const TGate* __restrict__ gate, TY* __restrict__ out, unsigned rows) {
   constexpr int LPR = D / kVec, RPW = 32 / LPR, U = Elem<TY>::kInFlight;
+  grid_dep_wait();
+  grid_dep_release();
   const unsigned lane = threadIdx.x & 31, sub = lane % LPR;
   const unsigned warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   const unsigned stride = gridDim.x * (kThreads / 32) * (RPW * U);
@@ -152,6 +151,8 @@ __global__ void __launch_bounds__(kThreads)
 head_gate_bwd_kernel(const TY* __restrict__ g, const TY* __restrict__ y, const TGate* __restrict__ gate,
                      TY* __restrict__ dy, TGate* __restrict__ dgate, unsigned rows) {
   constexpr int LPR = D / kVec, RPW = 32 / LPR, U = 2;
+  grid_dep_wait();
+  grid_dep_release();
   const unsigned lane = threadIdx.x & 31, sub = lane % LPR;
   const unsigned warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   const unsigned stride = gridDim.x * (kThreads / 32) * (RPW * U);
@@ -199,51 +200,62 @@ int cta_count(long long units, int per_cta, int cap) {
   return (int)(need < cap ? need : cap);
 }
 
+int launched(cudaError_t e) {
+  if (e == cudaSuccess) return NLFA_OK;
+  (void)cudaGetLastError();
+  return NLFA_ERR_CUDA;
+}
+
+template <typename TV, typename TOut>
+int blend_fwd_go(const void* v, const void* v0, const float* lam, void* out, unsigned nvec, cudaStream_t st) {
+  const int grid = cta_count(nvec, kThreads * (Elem<TV>::kInFlight / 2), 148 * 8);
+  return launched(launch_kernel(value_blend_fwd_kernel<TV, TOut>, dim3(grid), dim3(kThreads), 0, st,
+                                overlap_launches(kOverlapRowwise), (const TV*)v, (const TV*)v0, lam, (TOut*)out, nvec));
+}
 template <typename TV>
 int blend_fwd_out(int out_dtype, const void* v, const void* v0, const float* lam, void* out, unsigned nvec,
                   cudaStream_t st) {
-  const int grid = cta_count(nvec, kThreads * (Elem<TV>::kInFlight / 2), 148 * 8);
-  if (out_dtype == NLFA_DTYPE_BF16)
-    value_blend_fwd_kernel<TV, __nv_bfloat16><<<grid, kThreads, 0, st>>>((const TV*)v, (const TV*)v0, lam,
-                                                                         (__nv_bfloat16*)out, nvec);
-  else if (out_dtype == NLFA_DTYPE_F16)
-    value_blend_fwd_kernel<TV, __half><<<grid, kThreads, 0, st>>>((const TV*)v, (const TV*)v0, lam, (__half*)out, nvec);
-  else
-    value_blend_fwd_kernel<TV, float><<<grid, kThreads, 0, st>>>((const TV*)v, (const TV*)v0, lam, (float*)out, nvec);
-  return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
+  if (out_dtype == NLFA_DTYPE_BF16) return blend_fwd_go<TV, __nv_bfloat16>(v, v0, lam, out, nvec, st);
+  if (out_dtype == NLFA_DTYPE_F16) return blend_fwd_go<TV, __half>(v, v0, lam, out, nvec, st);
+  return blend_fwd_go<TV, float>(v, v0, lam, out, nvec, st);
 }
 
+template <typename TV, typename TG>
+int blend_bwd_go(const void* g, const void* v, const void* v0, const float* lam, void* dv, void* dv0, float* partial,
+                 float* dlam, unsigned nvec, cudaStream_t st) {
+  const int grid = cta_count(nvec, kThreads, kMaxPartials);
+  unsigned* ticket = nullptr;
+  const int rc = sched_counters(st, &ticket);
+  if (rc != NLFA_OK) return rc;
+  return launched(launch_kernel(value_blend_bwd_kernel<TV, TG>, dim3(grid), dim3(kThreads), 0, st,
+                                overlap_launches(kOverlapRowwise), (const TG*)g, (const TV*)v, (const TV*)v0, lam, (TV*)dv,
+                                (TV*)dv0, partial, dlam, ticket, nvec));
+}
 template <typename TV>
 int blend_bwd_g(int g_dtype, const void* g, const void* v, const void* v0, const float* lam, void* dv, void* dv0,
                 float* partial, float* dlam, unsigned nvec, cudaStream_t st) {
-  const int grid = cta_count(nvec, kThreads, kMaxPartials);
-#define NLFA_GO(TG)                                                                                              \
-  value_blend_bwd_kernel<TV, TG><<<grid, kThreads, 0, st>>>((const TG*)g, (const TV*)v, (const TV*)v0, lam, (TV*)dv, \
-                                                            (TV*)dv0, partial, nvec)
-  if (g_dtype == NLFA_DTYPE_BF16) NLFA_GO(__nv_bfloat16);
-  else if (g_dtype == NLFA_DTYPE_F16) NLFA_GO(__half);
-  else NLFA_GO(float);
-#undef NLFA_GO
-  value_blend_scalar_grad_kernel<<<1, 1024, 0, st>>>(partial, grid, lam, dlam);
-  return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
+  if (g_dtype == NLFA_DTYPE_BF16) return blend_bwd_go<TV, __nv_bfloat16>(g, v, v0, lam, dv, dv0, partial, dlam, nvec, st);
+  if (g_dtype == NLFA_DTYPE_F16) return blend_bwd_go<TV, __half>(g, v, v0, lam, dv, dv0, partial, dlam, nvec, st);
+  return blend_bwd_go<TV, float>(g, v, v0, lam, dv, dv0, partial, dlam, nvec, st);
 }
 
+template <typename TY, typename TGate, int D>
+int gate_go(bool backward, const void* g, const void* y, const void* gate, void* out, void* dgate, unsigned rows,
+            cudaStream_t st) {
+  const int grid = cta_count(rows, (kThreads / 32) * (32 / (D / kVec)) * (backward ? 2 : Elem<TY>::kInFlight), 148 * 8);
+  const bool overlap = overlap_launches(kOverlapRowwise);
+  if (backward)
+    return launched(launch_kernel(head_gate_bwd_kernel<TY, TGate, D>, dim3(grid), dim3(kThreads), 0, st, overlap,
+                                  (const TY*)g, (const TY*)y, (const TGate*)gate, (TY*)out, (TGate*)dgate, rows));
+  return launched(launch_kernel(head_gate_fwd_kernel<TY, TGate, D>, dim3(grid), dim3(kThreads), 0, st, overlap,
+                                (const TY*)y, (const TGate*)gate, (TY*)out, rows));
+}
 template <typename TY, typename TGate>
 int gate_for_dim(bool backward, int D, const void* g, const void* y, const void* gate, void* out, void* dgate,
                  unsigned rows, cudaStream_t st) {
-  const int grid = cta_count(rows, (kThreads / 32) * (32 / (D / kVec)) * (backward ? 2 : Elem<TY>::kInFlight),
-                             148 * 8);
-#define NLFA_GO(DD)                                                                                               \
-  do {                                                                                                            \
-    if (backward)                                                                                                 \
-      head_gate_bwd_kernel<TY, TGate, DD><<<grid, kThreads, 0, st>>>((const TY*)g, (const TY*)y, (const TGate*)gate, \
-                                                                     (TY*)out, (TGate*)dgate, rows);             \
-    else                                                                                                          \
-      head_gate_fwd_kernel<TY, TGate, DD><<<grid, kThreads, 0, st>>>((const TY*)y, (const TGate*)gate, (TY*)out, rows); \
-  } while (0)
-  if (D == 32) NLFA_GO(32); else if (D == 64) NLFA_GO(64); else NLFA_GO(128);
-#undef NLFA_GO
-  return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
+  if (D == 32) return gate_go<TY, TGate, 32>(backward, g, y, gate, out, dgate, rows, st);
+  if (D == 64) return gate_go<TY, TGate, 64>(backward, g, y, gate, out, dgate, rows, st);
+  return gate_go<TY, TGate, 128>(backward, g, y, gate, out, dgate, rows, st);
 }
 
 template <typename TY>

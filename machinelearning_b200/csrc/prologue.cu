@@ -7,9 +7,16 @@
 // (nanolab/flash_cuda.py:263-266).  Here a row of D elements is read once and
 // written once: HBM-bound, 2 + 2 bytes per element for 16-bit in and out.
 //
-// Thread mapping: a lane owns 8 consecutive elements of a row (one 16-byte load for
-// 16-bit input), so a row is D/8 lanes and a warp holds 256/D rows.  The rotary
-// partner of element e is e +- D/2, i.e. the same slot of lane ^ (D/16).
+// Thread mapping: a lane owns elements 4 s .. 4 s + 3 of each half of a row, so a row is D/8 lanes, a warp
+// holds 256/D rows, and the rotary partner of an element (e +- D/2) is the lane's own: no exchange.  A lane's U rows
+// are consecutive, so its position (row / H) % T is divided out once and stepped from there, and the cos / sin entries
+// are fetched again only when the position changes (H heads share it).  Bound by HBM; with eight elements in a
+// row per lane, the partner by shuffle and two divisions per row, instruction issue was in the way:
+// [64,1024,12,64] bf16 forward 48.1 -> 36.5 us (5.5 TB/s), backward 77.7 -> 65.8 us (4.6 TB/s: half of the issue
+// slots and half of the DRAM bandwidth, waiting on loads; fetching an iteration ahead cost registers, 78 us).
+//
+// The weight's gradient: a row of partial sums per CTA; the CTA that finishes last adds them up in a fixed order, so
+// there is no second kernel.
 //
 // Rounding follows torch's path for 16-bit input under autocast: the normalised,
 // weighted row is rounded to the input type (rms_norm returns the input's type), the
@@ -24,6 +31,22 @@ using namespace rowwise;
 // Rows are indexed with 32 bits (the host refuses B*T*H >= 2^31): the position of a row, (row / H) % T,
 // would otherwise cost two 64-bit divisions per row group.
 
+// A lane's place in the sequence: position and head of its first row, stepped row by row.
+struct Place {
+  unsigned t, h;
+  __device__ Place(unsigned row, unsigned T, unsigned H) {
+    const unsigned q = row / H;
+    h = row - q * H;
+    t = q % T;
+  }
+  __device__ bool step(unsigned T, unsigned H) {           // true: another position
+    if (++h < H) return false;
+    h = 0;
+    if (++t == T) t = 0;
+    return true;
+  }
+};
+
 // x [rows, D] (rows = B*T*H, position t = (row / H) % T) -> y [rows, D]; rstd [rows] when weight != nullptr.
 template <typename TIn, typename TOut, int D>
 __global__ void __launch_bounds__(kThreads)
@@ -32,117 +55,120 @@ qk_prologue_fwd_kernel(const TIn* __restrict__ x, const float* __restrict__ weig
                        unsigned rows, unsigned T, unsigned H, float eps) {
   constexpr int LPR = D / kVec;              // lanes per row
   constexpr int RPW = 32 / LPR;              // rows per warp and group
-  constexpr int U = Elem<TIn>::kInFlight;    // row groups a warp has in flight per loop iteration
+  constexpr int U = Elem<TIn>::kInFlight;    // rows a lane has in flight
+  constexpr int kHalf = D / 2;
+  grid_dep_wait();
+  grid_dep_release();
   const unsigned lane = threadIdx.x & 31;
-  const unsigned sub = lane % LPR;           // which 8-element slot of the row
+  const unsigned e0 = 4 * (lane % LPR);      // first element in the low half
   const unsigned warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-  const unsigned stride = gridDim.x * (kThreads / 32) * (RPW * U);
-  const float sign = sub < LPR / 2 ? -1.f : 1.f;       // rot = (-hi, lo)
-  float w[kVec];
+  const unsigned r0 = warp * (RPW * U) + (lane / LPR) * U;
+  typename Elem<TIn>::Raw raw[U];
 #pragma unroll
-  for (int i = 0; i < kVec; ++i) w[i] = weight ? weight[sub * kVec + i] : 1.f;
-
-  for (unsigned r0 = warp * (RPW * U); r0 < rows; r0 += stride) {
-    typename Elem<TIn>::Raw raw[U];
+  for (int u = 0; u < U; ++u)                // every load first; the whole warp stays for the shuffles
+    raw[u] = r0 + u < rows ? Elem<TIn>::load_halves(x + (size_t)(r0 + u) * D + e0, kHalf) : Elem<TIn>::zero();
+  float w[kVec], c[kVec], s[kVec];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {            // every load first; the whole warp stays for the shuffles
-      const unsigned row = r0 + (lane / LPR) * U + u;
-      raw[u] = row < rows ? Elem<TIn>::load_raw(x + (size_t)row * D + sub * kVec) : Elem<TIn>::zero();
+  for (int i = 0; i < kVec; ++i) w[i] = weight ? weight[e0 + (i & 3) + (i >> 2) * kHalf] : 1.f;
+  Place at(r0 < rows ? r0 : 0u, T, H);
+  bool fresh = true;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const unsigned row = r0 + u;
+    const bool live = row < rows;
+    float v[kVec];
+    Elem<TIn>::unpack(raw[u], v);
+    if (weight) {
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) ss = fmaf(v[i], v[i], ss);
+      const float r = rsqrtf(row_sum<LPR>(ss) * (1.f / D) + eps);
+      if (live && e0 == 0) rstd[row] = r;
+#pragma unroll
+      for (int i = 0; i < kVec; ++i) v[i] = Elem<TIn>::round(v[i] * r * w[i]);
     }
-    // A lane's U rows are consecutive, so most of them share a position (H heads per position): the
-    // table entries are fetched again only when the position changes.  (Fetching them per row made the
-    // L1 the busiest unit: 64 bytes of table for every 16 bytes of x.)
-    float c[kVec], s[kVec];
-    unsigned t_have = 0xffffffffu;
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const unsigned row = r0 + (lane / LPR) * U + u;
-      const bool live = row < rows;
-      float v[kVec];
-      Elem<TIn>::unpack(raw[u], v);
-      if (weight) {
-        float ss = 0.f;
-#pragma unroll
-        for (int i = 0; i < kVec; ++i) ss = fmaf(v[i], v[i], ss);
-        const float r = rsqrtf(row_sum<LPR>(ss) * (1.f / D) + eps);
-        if (live && sub == 0) rstd[row] = r;
-#pragma unroll
-        for (int i = 0; i < kVec; ++i) v[i] = Elem<TIn>::round(v[i] * r * w[i]);
+    if (cosT) {
+      if (u > 0 && at.step(T, H)) fresh = true;
+      if (fresh) {
+        Elem<float>::unpack(Elem<float>::load_halves(cosT + (size_t)at.t * D + e0, kHalf), c);
+        Elem<float>::unpack(Elem<float>::load_halves(sinT + (size_t)at.t * D + e0, kHalf), s);
+        fresh = false;
       }
-      if (cosT) {
-        const unsigned t = live ? (row / H) % T : 0u;
-        if (t != t_have) {
-          Elem<float>::load(cosT + (size_t)t * D + sub * kVec, c);
-          Elem<float>::load(sinT + (size_t)t * D + sub * kVec, s);
-          t_have = t;
-        }
 #pragma unroll
-        for (int i = 0; i < kVec; ++i) {
-          const float partner = __shfl_xor_sync(0xffffffffu, v[i], LPR / 2);
-          v[i] = v[i] * c[i] + sign * partner * s[i];
-        }
+      for (int i = 0; i < 4; ++i) {          // rot = (-hi, lo)
+        const float lo = v[i], hi = v[i + 4];
+        v[i] = lo * c[i] - hi * s[i];
+        v[i + 4] = hi * c[i + 4] + lo * s[i + 4];
       }
-      if (live) Elem<TOut>::store(y + (size_t)row * D + sub * kVec, v);
     }
+    if (live) Elem<TOut>::store_halves(y + (size_t)row * D + e0, kHalf, v);
   }
 }
 
-// gy [rows, D] (gradient of the prologue's output), x and rstd from the forward -> gx [rows, D] and one
-// row of weight-gradient partial sums per CTA (partial [gridDim.x, D]).
+// gy [rows, D] (gradient of the prologue's output), x and rstd from the forward -> gx [rows, D]; gweight [D] by way of
+// one row of partial sums per CTA (partial [gridDim.x, D]).
 template <typename TIn, typename TG, int D>
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreads, 2)
 qk_prologue_bwd_kernel(const TG* __restrict__ gy, const TIn* __restrict__ x, const float* __restrict__ weight,
                        const float* __restrict__ cosT, const float* __restrict__ sinT,
                        const float* __restrict__ rstd, TIn* __restrict__ gx, float* __restrict__ partial,
-                       unsigned rows, unsigned T, unsigned H) {
+                       float* __restrict__ gweight, unsigned* ticket, unsigned rows, unsigned T, unsigned H) {
   constexpr int LPR = D / kVec;
   constexpr int RPW = 32 / LPR;
-  constexpr int U = 2;
-  __shared__ float red[kThreads / 32][D];
+  constexpr int U = Elem<TIn>::kInFlight;
+  constexpr int kHalf = D / 2;
+  __shared__ __align__(16) float red[kThreads * 4];        // [warp][D] sums, then [thread][4] for the last CTA
+  __shared__ int last;
+  grid_dep_wait();
+  grid_dep_release();
   const unsigned lane = threadIdx.x & 31;
-  const unsigned sub = lane % LPR;
+  const unsigned e0 = 4 * (lane % LPR);
   const unsigned warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   const unsigned stride = gridDim.x * (kThreads / 32) * (RPW * U);
-  const float sign = sub < LPR / 2 ? 1.f : -1.f;       // transpose of the rotation
   float w[kVec], dw[kVec];
 #pragma unroll
-  for (int i = 0; i < kVec; ++i) { w[i] = weight ? weight[sub * kVec + i] : 1.f; dw[i] = 0.f; }
+  for (int i = 0; i < kVec; ++i) {
+    w[i] = weight ? weight[e0 + (i & 3) + (i >> 2) * kHalf] : 1.f;
+    dw[i] = 0.f;
+  }
 
-  for (unsigned r0 = warp * (RPW * U); r0 < rows; r0 += stride) {
+  for (unsigned r1 = warp * (RPW * U); r1 < rows; r1 += stride) {
+    const unsigned r0 = r1 + (lane / LPR) * U;
     typename Elem<TG>::Raw graw[U];
     typename Elem<TIn>::Raw xraw[U];
     float r[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const unsigned row = r0 + (lane / LPR) * U + u;
+      const unsigned row = r0 + u;
       graw[u] = Elem<TG>::zero();
       xraw[u] = Elem<TIn>::zero();
       r[u] = 0.f;
       if (row < rows) {
-        graw[u] = Elem<TG>::load_raw(gy + (size_t)row * D + sub * kVec);
-        if (weight) { xraw[u] = Elem<TIn>::load_raw(x + (size_t)row * D + sub * kVec); r[u] = rstd[row]; }
+        graw[u] = Elem<TG>::load_halves(gy + (size_t)row * D + e0, kHalf);
+        if (weight) { xraw[u] = Elem<TIn>::load_halves(x + (size_t)row * D + e0, kHalf); r[u] = rstd[row]; }
       }
     }
     float c[kVec], s[kVec];                  // table entries, kept while the position stays the same
-    unsigned t_have = 0xffffffffu;
+    Place at(r0 < rows ? r0 : 0u, T, H);
+    bool fresh = true;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const unsigned row = r0 + (lane / LPR) * U + u;
-      const bool live = row < rows;
+      const unsigned row = r0 + u;
       float g[kVec], v[kVec];
       Elem<TG>::unpack(graw[u], g);
       Elem<TIn>::unpack(xraw[u], v);
       if (cosT) {
-        const unsigned t = live ? (row / H) % T : 0u;
-        if (t != t_have) {
-          Elem<float>::load(cosT + (size_t)t * D + sub * kVec, c);
-          Elem<float>::load(sinT + (size_t)t * D + sub * kVec, s);
-          t_have = t;
+        if (u > 0 && at.step(T, H)) fresh = true;
+        if (fresh) {
+          Elem<float>::unpack(Elem<float>::load_halves(cosT + (size_t)at.t * D + e0, kHalf), c);
+          Elem<float>::unpack(Elem<float>::load_halves(sinT + (size_t)at.t * D + e0, kHalf), s);
+          fresh = false;
         }
 #pragma unroll
-        for (int i = 0; i < kVec; ++i) {
-          const float partner = __shfl_xor_sync(0xffffffffu, g[i] * s[i], LPR / 2);
-          g[i] = g[i] * c[i] + sign * partner;
+        for (int i = 0; i < 4; ++i) {        // transpose of the rotation
+          const float lo = g[i], hi = g[i + 4];
+          g[i] = lo * c[i] + hi * s[i + 4];
+          g[i + 4] = hi * c[i + 4] - lo * s[i];
         }
       }
       if (weight) {
@@ -159,51 +185,49 @@ qk_prologue_bwd_kernel(const TG* __restrict__ gy, const TIn* __restrict__ x, con
 #pragma unroll
         for (int i = 0; i < kVec; ++i) g[i] = r[u] * (g[i] - v[i] * c);
       }
-      if (live) Elem<TIn>::store(gx + (size_t)row * D + sub * kVec, g);
+      if (row < rows) Elem<TIn>::store_halves(gx + (size_t)row * D + e0, kHalf, g);
     }
   }
 
-  if (weight) {                              // CTA-wide sum of dw, fixed order: reproducible
+  if (!weight) return;
+  // CTA-wide sum of dw, then the last CTA's sum over all CTAs: both in a fixed order
 #pragma unroll
-    for (int i = 0; i < kVec; ++i) {
+  for (int i = 0; i < kVec; ++i) {
 #pragma unroll
-      for (int off = LPR; off < 32; off <<= 1) dw[i] += __shfl_xor_sync(0xffffffffu, dw[i], off);
-    }
-    if (lane < LPR) {
-#pragma unroll
-      for (int i = 0; i < kVec; ++i) red[threadIdx.x >> 5][sub * kVec + i] = dw[i];
-    }
-    __syncthreads();
-    if (threadIdx.x < D) {
-      float s = 0.f;
-#pragma unroll
-      for (int wi = 0; wi < kThreads / 32; ++wi) s += red[wi][threadIdx.x];
-      partial[(size_t)blockIdx.x * D + threadIdx.x] = s;
-    }
+    for (int off = LPR; off < 32; off <<= 1) dw[i] += __shfl_xor_sync(0xffffffffu, dw[i], off);
   }
-}
-
-// gweight[e] = sum over the n per-CTA rows of partial[:, e].  One CTA of 1024 threads: thread (g, e) adds
-// rows g, g + G, ... (G = 1024 / D), then the G sums of a column are added in a fixed order.
-template <int D>
-__global__ void __launch_bounds__(1024)
-weight_grad_reduce_kernel(const float* __restrict__ partial, int n, float* __restrict__ gweight) {
-  constexpr int G = 1024 / D;
-  __shared__ float red[G][D];
-  const int e = threadIdx.x % D, g = threadIdx.x / D;
-  float s = 0.f;
-  for (int i = g; i < n; i += G) s += partial[(long long)i * D + e];
-  red[g][e] = s;
+  if (lane < LPR) {
+#pragma unroll
+    for (int i = 0; i < kVec; ++i) red[(threadIdx.x >> 5) * D + e0 + (i & 3) + (i >> 2) * kHalf] = dw[i];
+  }
   __syncthreads();
-  if (g == 0) {
+  if (threadIdx.x < D) {
+    float sum = 0.f;
+#pragma unroll
+    for (int wi = 0; wi < kThreads / 32; ++wi) sum += red[wi * D + threadIdx.x];
+    partial[(size_t)blockIdx.x * D + threadIdx.x] = sum;
+  }
+  if (!last_cta(ticket, gridDim.x, &last)) return;
+  // thread (g, e4): rows g, g + G, .. of four columns, past L1 (other SMs wrote them); then the G sums of a column
+  constexpr int E = D / 4, G = kThreads / E;
+  const int e4 = threadIdx.x % E, g = threadIdx.x / E, n = gridDim.x;
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (int i = g; i < n; i += G) {
+    const float4 p = __ldcg(reinterpret_cast<const float4*>(partial + (size_t)i * D) + e4);
+    sum = make_float4(sum.x + p.x, sum.y + p.y, sum.z + p.z, sum.w + p.w);
+  }
+  reinterpret_cast<float4*>(red)[threadIdx.x] = sum;
+  __syncthreads();
+  if (threadIdx.x < D) {
     float t = 0.f;
 #pragma unroll
-    for (int j = 0; j < G; ++j) t += red[j][e];
-    gweight[e] = t;
+    for (int j = 0; j < G; ++j) t += red[j * D + threadIdx.x];
+    gweight[threadIdx.x] = t;
   }
 }
 
-int grid_for(long long rows, int D, int cap, int in_flight) {
+int grid_for(long long rows, int D, long long cap, int in_flight) {
   const long long rows_per_cta = (long long)(kThreads / 32) * (32 / (D / kVec)) * in_flight;
   long long need = (rows + rows_per_cta - 1) / rows_per_cta;
   if (need < 1) need = 1;
@@ -213,30 +237,37 @@ int grid_for(long long rows, int D, int cap, int in_flight) {
 template <typename TIn, typename TOut>
 int fwd_for_dim(int D, const void* x, const float* w, const float* c, const float* s, void* y, float* rstd,
                 long long rows, int T, int H, float eps, cudaStream_t st) {
-  const int grid = grid_for(rows, D, 148 * 8, Elem<TIn>::kInFlight);
-#define NLFA_GO(DD)                                                                               \
-  qk_prologue_fwd_kernel<TIn, TOut, DD><<<grid, kThreads, 0, st>>>((const TIn*)x, w, c, s, (TOut*)y, rstd,       \
-                                                                   (unsigned)rows, (unsigned)T, (unsigned)H, eps)
+  const int grid = grid_for(rows, D, 1ll << 31, Elem<TIn>::kInFlight);          // one pass per warp
+  cudaError_t e;
+#define NLFA_GO(DD)                                                                                               \
+  e = launch_kernel(qk_prologue_fwd_kernel<TIn, TOut, DD>, dim3(grid), dim3(kThreads), 0, st,                     \
+                    overlap_launches(kOverlapRowwise), (const TIn*)x, w, c, s, (TOut*)y, rstd, (unsigned)rows,    \
+                    (unsigned)T, (unsigned)H, eps)
   if (D == 32) NLFA_GO(32); else if (D == 64) NLFA_GO(64); else NLFA_GO(128);
 #undef NLFA_GO
-  return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
 }
 
 template <typename TIn, typename TG>
 int bwd_for_dim(int D, const void* gy, const void* x, const float* w, const float* c, const float* s,
                 const float* rstd, void* gx, float* partial, float* gweight, long long rows, int T, int H,
                 cudaStream_t st) {
-  const int grid = grid_for(rows, D, kMaxPartials, 2);
-#define NLFA_GO(DD)                                                                                      \
-  do {                                                                                                   \
-    qk_prologue_bwd_kernel<TIn, TG, DD><<<grid, kThreads, 0, st>>>((const TG*)gy, (const TIn*)x, w, c, s, rstd, \
-                                                                   (TIn*)gx, partial, (unsigned)rows,    \
-                                                                   (unsigned)T, (unsigned)H);            \
-    if (w) weight_grad_reduce_kernel<DD><<<1, 1024, 0, st>>>(partial, grid, gweight);                     \
-  } while (0)
+  const int grid = grid_for(rows, D, 2 * sm_count() < kMaxPartials ? 2 * sm_count() : kMaxPartials, Elem<TIn>::kInFlight);
+  unsigned* ticket = nullptr;
+  if (w != nullptr) {
+    const int rc = sched_counters(st, &ticket);
+    if (rc != NLFA_OK) return rc;
+  }
+  cudaError_t e;
+#define NLFA_GO(DD)                                                                                               \
+  e = launch_kernel(qk_prologue_bwd_kernel<TIn, TG, DD>, dim3(grid), dim3(kThreads), 0, st,                       \
+                    overlap_launches(kOverlapRowwise), (const TG*)gy, (const TIn*)x, w, c, s, rstd, (TIn*)gx,     \
+                    partial, gweight, ticket, (unsigned)rows, (unsigned)T, (unsigned)H)
   if (D == 32) NLFA_GO(32); else if (D == 64) NLFA_GO(64); else NLFA_GO(128);
 #undef NLFA_GO
-  return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
 }
 
 
@@ -293,6 +324,8 @@ int nlfa_qk_prologue_bwd(const void* gy, int gy_dtype, const void* x, int x_dtyp
   if (weight && scratch_bytes < nlfa_qk_prologue_scratch_bytes(D)) return NLFA_ERR_SCRATCH_TOO_SMALL;
   if (!aligned16(gy) || !aligned16(gx) || !aligned16(x) || !aligned16(cos_table) || !aligned16(sin_table))
     return NLFA_ERR_MISALIGNED;
+  // (the kernel reads the partial sums 16 bytes at a time; the scratch has room to spare)
+  scratch = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(scratch) + 15u) & ~static_cast<uintptr_t>(15u));
 #define NLFA_G(TIn)                                                                                               \
   (gy_dtype == NLFA_DTYPE_BF16 ? bwd_for_dim<TIn, __nv_bfloat16>(D, gy, x, weight, cos_table, sin_table, rstd, gx, (float*)scratch, gweight, rows, T, H, st) \
    : gy_dtype == NLFA_DTYPE_F16 ? bwd_for_dim<TIn, __half>(D, gy, x, weight, cos_table, sin_table, rstd, gx, (float*)scratch, gweight, rows, T, H, st)       \
