@@ -246,7 +246,13 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (!(ok = mbar_wait(bar(Q_EMPTY + qb), qph ^ 1, wctx, 10))) return u;
         mbar_arrive_expect_tx(bar(Q_FULL + qb), w.n_valid * L::kTileBytes);
         for (int t = 0; t < NT; ++t) {
-          if (!w.valid[t]) continue;
+          if (!w.valid[t]) {
+            // nothing will be stored for this tile.  Its arrival comes from here, where the buffer's previous use is
+            // known to be over: the warpgroup without a tile runs through the published units ahead of the other
+            // one, and an arrival of its own for a later unit could complete the phase of this one.
+            mbar_arrive(bar(Q_EMPTY + qb));
+            continue;
+          }
           for (int x = 0; x < kBoxes; ++x)
             tma_load_4d(base + L::kQ + (qb * NT + t) * L::kTileBytes + x * kBoxBytes, &tm_q,
                         bar(Q_FULL + qb), 64 * x, w.h, (w.tile0 + t) * kTile, w.b);
@@ -508,16 +514,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       ok = __all_sync(0xffffffffu, ok);
       if (!ok || u < 0) break;
       if (!w.valid[t]) {
-        // Q_FULL first: it says that the buffer's previous use is over.  A warpgroup without a tile would
-        // otherwise run through the published units ahead of the other one, and its arrival for a later unit
-        // would complete the phase of this one -- the buffer reloaded under the other tile's output.
-        ok = mbar_wait(bar(Q_FULL + uc % QBUF), (uc / QBUF) & 1, wctx, 15);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        if (row == 0) {
-          release_pending();
-          mbar_arrive(bar(Q_EMPTY + (uc % QBUF)));                // nothing to store for this tile
-        }
+        if (row == 0) release_pending();                          // (the producer has arrived for this tile)
         continue;
       }
       const int tile = w.tile0 + t;
