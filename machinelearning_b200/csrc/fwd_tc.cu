@@ -533,7 +533,6 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         va = lo > 0 ? lo : 0;
         vsink = p.sinks < qpos + 1 ? p.sinks : qpos + 1;
       }
-      const unsigned vw = static_cast<unsigned>(qpos - va);
       for (int it = 0; it < w.n_iters; ++it) {
         const int j = w.block_at(it);
         if (!tile_sees_block(w.tr[t], j)) continue;
@@ -551,48 +550,23 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         tc_fence_before();
         mbar_arrive(bar(S_CONSUMED + t));
 
-        // Boundary blocks: a 32-column chunk that the whole warp sees entirely is left alone,
-        // the others pay per-element tests.  Masked scores
-        // become -inf and flow through the straight-line code below as zeros: skipping them
+        // Boundary blocks: a row's visible columns as bits, 32 at a time, whatever edges cut the block.  Masked
+        // scores become -inf and flow through the straight-line code below as zeros: skipping them
         // instead would put branches between the chunks, and the exponentials of a chunk on
         // its own are too few to cover the unit's latency (measured: 1760 clocks per row with
-        // per-chunk branches against 1130 without).
+        // per-chunk branches against 1130 without).  Comparing every column with the row's limits cost as much as the
+        // block's exponentials, and so did votes that spared chunks the whole warp sees: B=16 H=16 T=4096 window
+        // 256, where two of a tile's three blocks are cut, 257 -> 226 us (B=32 H=12 T=1024 123 -> 120 us).
         const int k0 = j * kTile;
-        const int edges = block_fully_visible(tile, j, p.window, p.sinks, p.block, p.T)
-                              ? -1 : block_edges(tile, j, p.window, p.sinks);
-        if (edges == EDGE_CAUSAL) {
-          // only the causal edge cuts the block: the row sees the columns up to its own
-          // position (block-causal: up to the end of its block) -- one compare per element
-          // against a per-thread limit
+        if (!block_fully_visible(tile, j, p.window, p.sinks, p.block, p.T)) {
+          // the row sees the columns [va, qlim] and, below the window, the sinks
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            const int last = qlim - (k0 + 32 * c);                       // last visible column of the chunk
-            if (__all_sync(0xffffffffu, last >= 31)) continue;
+            const int x0 = k0 + 32 * c;
+            const uint32_t keep = (bits_up_to(qlim - x0) & bits_from(va - x0)) | bits_up_to(vsink - 1 - x0);
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (i > last) sv[c][i] = __float_as_uint(-INFINITY);
-          }
-        } else if (edges == EDGE_WINDOW) {
-          // only the window's lower edge cuts the block: the row sees the columns from va on
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int first_vis = va - (k0 + 32 * c);                    // first visible column of the chunk
-            if (__all_sync(0xffffffffu, first_vis <= 0)) continue;
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (i < first_vis) sv[c][i] = __float_as_uint(-INFINITY);
-          }
-        } else if (edges == EDGE_BOTH) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int x0 = k0 + 32 * c, x1 = x0 + 31;
-            const bool in = (x0 >= va && x1 <= qpos) || x1 < vsink;
-            if (__all_sync(0xffffffffu, in)) continue;
-            const unsigned o = static_cast<unsigned>(x0 - va);            // wraps below va
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (!(o + static_cast<unsigned>(i) <= vw || x0 + i < vsink))
-                sv[c][i] = __float_as_uint(-INFINITY);
+              if (!(keep & (1u << i))) sv[c][i] = __float_as_uint(-INFINITY);
           }
         }
         // row maximum of the raw scores: two chains of 3-input max

@@ -473,6 +473,16 @@ struct Pack2<__half> {
   }
 };
 
+// Bit i of a 32-column chunk's mask: i <= last / i >= first.  A row's visible columns as bits cost a handful of
+// instructions per chunk, and testing bit i of a register takes about one predicate instruction per seven
+// elements, where comparing a limit with every column took one each.
+__device__ __forceinline__ uint32_t bits_up_to(int last) {
+  return last < 0 ? 0u : last >= 31 ? 0xffffffffu : (2u << last) - 1u;
+}
+__device__ __forceinline__ uint32_t bits_from(int first) {
+  return first <= 0 ? 0xffffffffu : first > 31 ? 0u : 0xffffffffu << first;
+}
+
 // three-input maximum (one instruction on sm_100)
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
   float d;
