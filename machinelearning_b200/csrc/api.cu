@@ -371,7 +371,7 @@ int nlfa_resolve_path(int dtype, int head_dim, int path) {
   if (dtype != NLFA_DTYPE_F32 && dtype != NLFA_DTYPE_F16 && dtype != NLFA_DTYPE_BF16)
     return -NLFA_ERR_BAD_DTYPE;
   if (head_dim != 32 && head_dim != 64 && head_dim != 128) return -NLFA_ERR_BAD_HEAD_DIM;
-  const bool tensor_ok = dtype != NLFA_DTYPE_F32;      // head dim 32 runs the 64-wide kernels, zero-padded by TMA
+  const bool tensor_ok = dtype != NLFA_DTYPE_F32;      // head dim 32 runs on 64-wide tiles, zero-padded by TMA
   if (path == NLFA_PATH_SIMT) return NLFA_PATH_SIMT;
   if (path == NLFA_PATH_TENSOR) return tensor_ok ? NLFA_PATH_TENSOR : -NLFA_ERR_UNSUPPORTED_PATH;
   if (path == NLFA_PATH_AUTO) return tensor_ok ? NLFA_PATH_TENSOR : NLFA_PATH_SIMT;
