@@ -691,14 +691,11 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
       BwdUnit<MODE> w;
       next_unit(uc, ok, w);                      // published by this warp: never waits
       if (!ok) break;
-      // The next unit's stationary tiles are requested once this unit's first streamed tiles
-      // are on their way (with one stationary buffer: only when this unit has released it).
-      int u_next = -2;
-      const int prefetch_at = XBUF > 1 ? (w.n_iters < STAGES ? w.n_iters : STAGES) : w.n_iters;
+      // The next unit is taken, and its stationary tiles requested, when this unit's last streamed tiles have been
+      // (the compute warps are then STAGES iterations behind).  Taken any earlier, a unit waits behind this
+      // one while other CTAs run out of work: B=3 H=2 T=5416 backward 123.6 -> 101.4 us.
       int inner = 0, g = 0;                       // it = g * n_inner + inner
       for (int it = 0; ok && it < w.n_iters; ++it, ++git, ++inner) {
-        if (it == prefetch_at) u_next = fetch_unit(uc + 1);
-        if (!ok) break;
         if (inner == w.n_inner) { inner = 0; ++g; }
         const int s = git % STAGES;
         const uint32_t ph = (git / STAGES) & 1;
@@ -734,8 +731,7 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
         }
         if (lane == 0) mbar_arrive(bar(Y_FULL + s));
       }
-      if (ok && u_next == -2) u_next = fetch_unit(uc + 1);
-      u = u_next;
+      if (ok) u = fetch_unit(uc + 1);
     }
   } else {
     // ================================ MMA issuer =============================

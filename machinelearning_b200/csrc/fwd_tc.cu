@@ -1,9 +1,10 @@
 // Tensor-core forward for sm_100a: S = Q K^T and O += P V on tcgen05 with the
 // accumulators in TMEM, tiles brought in by TMA, online softmax in registers.
 //
-// Persistent kernel: one CTA per SM takes work units from a global counter,
+// Persistent kernel: one CTA per SM (two at NT = 1, D <= 64) takes work units from a global counter,
 // heaviest first.  A unit is NT consecutive 128-row query tiles of one (batch,
-// head); the CTA visits the key blocks those tiles can see.  Warp roles:
+// head), NT = 1 or 2 (launch_fwd_tc has the rule); the CTA visits the key blocks those tiles can see.
+// Warp roles:
 //   warps [0, 4 NT)   softmax: warpgroup t owns query tile t, one thread per row
 //   warp  4 NT        scheduler + TMA producer (one lane): Q per unit, K / V ring
 //   warp  4 NT + 1    MMA issuer (one lane) and owner of the TMEM allocation
@@ -116,7 +117,7 @@ __device__ __forceinline__ Unit<NT> make_unit(int u, const FwdParams& p, int BH)
 // DR: the head dim; 32 runs on tiles 64 wide (D), with half the steps of the score product and an output product
 // half as wide (B=8 H=12/4 T=1024: 34.2 -> 32.4 us).
 template <typename T, int D, int DR, int NT, int STAGES, int QBUF>
-__global__ void __launch_bounds__(NT * 128 + 128, 1)
+__global__ void __launch_bounds__(NT * 128 + 128, NT == 1 && D == 64 ? 2 : 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
               const FwdParams p) {
@@ -128,7 +129,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   constexpr bool kSepP = NT * (128 + D + 64) <= 512;      // P has columns of its own
   constexpr uint32_t kPBase = NT * (128 + D);
   constexpr int kRing = L::kRing;
-  constexpr int kRegsLaunch = 168, kRegsCompute = 216, kRegsOther = 72;   // per thread
+  // registers per thread: at launch, of the softmax warps, of the others
+  constexpr int kRegsLaunch = NT == 1 ? 128 : 168, kRegsCompute = NT == 1 ? 200 : 216, kRegsOther = NT == 1 ? 56 : 72;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -209,14 +211,13 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     return a.x;
   };
 
-  // Register reallocation (NT = 2: 384 threads launch with 168 registers each): the
-  // warpgroup of the producer, the MMA issuer and two spare warps drops to 72, the softmax
-  // warpgroups take 216 each.
+  // Register reallocation: the warpgroup of the producer, the MMA issuer and two spare warps
+  // gives most of its registers to the softmax warpgroups.
   if (warp >= 4 * NT) {
-  if (NT == 2) setmaxnreg_dec<kRegsOther>();
+  setmaxnreg_dec<kRegsOther>();
   // setmaxnreg.inc blocks until the registers it asks for have been released, so the four
-  // warps that shrink must free at least what the eight that grow take.
-  static_assert((kRegsLaunch - kRegsOther) * 4 >= (kRegsCompute - kRegsLaunch) * 8,
+  // warps that shrink must free at least what those that grow take.
+  static_assert((kRegsLaunch - kRegsOther) * 4 >= (kRegsCompute - kRegsLaunch) * 4 * NT,
                 "register reallocation does not balance");
   if (dead || warp >= 4 * NT + 2) {
     // nothing to do (spare warps only complete the warpgroup)
@@ -266,13 +267,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         Unit<NT> w;
         next_unit(uc, ok, w);                    // published by this thread: never waits
         if (!ok) break;
-        // the next unit's Q is requested once this unit's first K/V blocks are on their way
-        // (with a single Q buffer: only when this unit has released it)
-        int u_next = -2;
-        const int prefetch_at = QBUF > 1 ? (w.n_iters < STAGES ? w.n_iters : STAGES) : w.n_iters;
+        // The next unit is taken, and its Q requested, when this unit's last K/V block has been: the softmax warps are
+        // then STAGES blocks behind, time enough for the loads.  Taken any earlier, a unit waits behind this one
+        // while other CTAs run out of work (B=2 H=8/2 T=4000: 78.6 -> 57.3 us; B=4 H=12 T=1024 25.0 -> 20.5).
         for (int it = 0; it < w.n_iters; ++it, ++git) {
-          if (it == prefetch_at) u_next = fetch_unit(uc + 1);
-          if (!ok) break;
           const int s = git % STAGES;
           const uint32_t ph = (git / STAGES) & 1;
           const int j = w.block_at(it);
@@ -287,8 +285,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             tma_load_4d(base + L::kV + s * L::kTileBytes + x * kBoxBytes, &tm_v, bar(V_FULL + s),
                         64 * x, w.hk, j * kTile, w.b);
         }
-        if (ok && u_next == -2) u_next = fetch_unit(uc + 1);
-        u = u_next;
+        if (ok) u = fetch_unit(uc + 1);
       }
     }
   } else if (warp == 4 * NT + 1) {
@@ -487,7 +484,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
   } else {
     // ================================= softmax ===============================
-    if (NT == 2) setmaxnreg_inc<kRegsCompute>();
+    setmaxnreg_inc<kRegsCompute>();
     if (!dead) {
     const int t = warp >> 2;                       // query tile of this warpgroup
     const int row = threadIdx.x - 128 * t;         // row inside the tile == TMEM lane
@@ -753,7 +750,8 @@ int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, con
   fp.status = status;
   const int sst = sched_counters(stream, &fp.sched);
   if (sst != NLFA_OK) return sst;
-  const int grid = fp.total_units < sm_count() ? fp.total_units : sm_count();
+  const int room = (NT == 1 && D == 64 ? 2 : 1) * sm_count();
+  const int grid = fp.total_units < room ? fp.total_units : room;
   if (launch_kernel(kern, dim3(grid), dim3(NT * 128 + 128), L::kDynamic, stream, overlap_launches(kOverlapFwd), mq, mk, mv, mo,
                     fp) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -778,8 +776,22 @@ int launch_fwd_tc(const Problem& p, const void* q, const void* k, const void* v,
   if (st == NLFA_OK) st = make_tile_map(&mo, o, p.dtype, p.B, p.T, p.H, p.D, kTile);
   if (st != NLFA_OK) return st;
   const bool bf16 = p.dtype == NLFA_DTYPE_BF16;
+  // One tile per unit or two?  Two share every K / V tile and keep the exponential unit fed from one CTA, which wins over
+  // long rows; one -- at D <= 64 with two CTAs per SM, four contexts' worth of unit starts and ends overlapping --
+  // balances better and wastes nothing on the second tile's longer row.  D <= 64: two tiles only where rows are
+  // long (one / two tiles per unit: T=1024 67.2 / 71.0 us, T=4096 202.6 / 204.6, T=8192 399 / 396, T=16384 810 / 792,
+  // all at 32K positions x 8 heads or more) and there are more tiles than SMs.  D = 128 (one CTA per SM either way):
+  // one tile while that makes at most two units per SM (B=1 H=8 T=4096: 42.6 / 65.9 us; 3.5 per SM: 45.2 / 41.9).
+  const long long tiles = static_cast<long long>(p.B) * p.H * ((p.T + kTile - 1) / kTile);
+  const int reach = p.window > 0 && p.window < p.T ? p.window : p.T;
+  const bool single = p.D == 128 ? tiles <= 2ll * sm_count() || p.T <= kTile : reach <= 4096 || tiles <= sm_count();
   auto go = [&](auto type) {
     using T = decltype(type);
+    if (single) {
+      if (p.D == 32) return launch_t<T, 64, 32, 1, 2, 2>(p, mq, mk, mv, mo, o, lse, status, stream);
+      if (p.D == 64) return launch_t<T, 64, 64, 1, 2, 2>(p, mq, mk, mv, mo, o, lse, status, stream);
+      return launch_t<T, 128, 128, 1, 2, 2>(p, mq, mk, mv, mo, o, lse, status, stream);
+    }
     if (p.D == 32) return launch_t<T, 64, 32, 2, 3, 2>(p, mq, mk, mv, mo, o, lse, status, stream);
     if (p.D == 64) return launch_t<T, 64, 64, 2, 3, 2>(p, mq, mk, mv, mo, o, lse, status, stream);
     return launch_t<T, 128, 128, 2, 2, 1>(p, mq, mk, mv, mo, o, lse, status, stream);

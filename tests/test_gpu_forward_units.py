@@ -1,0 +1,35 @@
+"""Both unit heights of the tensor-core forward -- one query tile, and two (long rows and more tiles than SMs at head dims
+up to 64; more than two tiles per SM at 128) -- against plain float32 attention on the GPU, at odd and even numbers of
+tiles, under every mask, and the logsumexp with them."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+#        B, T, H, Hkv, D, window, sinks, block, dtype
+CASES = [(1, 4200, 5, 1, 64, 0, 0, 0, torch.bfloat16), (1, 4353, 6, 2, 32, 0, 0, 0, torch.float16),   # two tiles
+         (1, 4300, 5, 5, 64, 4150, 70, 0, torch.bfloat16), (1, 4480, 5, 5, 64, 0, 0, 700, torch.bfloat16),
+         (25, 300, 4, 2, 128, 0, 0, 0, torch.bfloat16), (25, 385, 4, 4, 128, 150, 9, 0, torch.float16),
+         (25, 290, 4, 1, 128, 0, 0, 100, torch.bfloat16),
+         (1, 4096, 3, 1, 64, 0, 0, 0, torch.bfloat16), (1, 4200, 4, 2, 64, 0, 0, 0, torch.bfloat16),  # one tile
+         (1, 1100, 4, 2, 32, 200, 5, 0, torch.bfloat16), (3, 700, 6, 2, 128, 0, 0, 96, torch.float16)]
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,D,window,sinks,block,dtype", CASES)
+def test_forward_in_both_unit_heights(B, T, H, Hkv, D, window, sinks, block, dtype):
+    from machinelearning_b200 import flash_cuda as fc
+    assert fc.is_available(), fc.unavailable_reason()
+    g = torch.Generator(device="cuda").manual_seed(T + D)
+    q, k, v = (torch.randn(B, T, h, D, device="cuda", generator=g).to(dtype) for h in (H, Hkv, Hkv))
+    scale = D ** -0.5
+    o, lse = fc.fwd(q, k, v, scale, True, window, sinks, block)
+    i, j = torch.arange(T, device="cuda")[:, None], torch.arange(T, device="cuda")[None, :]
+    keep = (j // block <= i // block) if block else (j <= i)
+    if window:
+        keep = keep & ((j > i - (window - sinks)) | (j < sinks))
+    for b in range(0, B, 6):
+        s = torch.einsum("thd,shd->hts", q[b].float(), k[b].float().repeat_interleave(H // Hkv, 1)) * scale
+        s = s.masked_fill(~keep, float("-inf"))
+        want = torch.einsum("hts,shd->thd", s.softmax(-1), v[b].float().repeat_interleave(H // Hkv, 1))
+        assert (o[b].float() - want).abs().max().item() <= 2e-2 * want.abs().max().item()
+        assert (lse[b] - s.logsumexp(-1)).abs().max().item() <= 1e-3
