@@ -733,7 +733,7 @@ def run_whole_model_arm(args, rank, world, local_rank):
         return model, wm.DataParallelStep(model)
 
     # counts the library's launches: 1 forward + 3 backward kernels per flash_attn call, 1 forward +
-    # 2 backward kernels (gradient pass, fixed-order reduction) per qk_prologue and per value_blend
+    # 1 backward kernel per qk_prologue and per value_blend
     # call, 1 + 1 per head_gate call
     calls = {"n": 0, "prologue": 0, "blend": 0, "gate": 0}
     real_fwd, real_prologue = flash_cuda.fwd, qk_prologue.qk_prologue
@@ -834,7 +834,7 @@ def run_whole_model_arm(args, rank, world, local_rank):
                 "h2d_bytes_per_step": 2 * x_pin.numel() * x_pin.element_size(), "d2h_bytes_per_step": 4},
         # per flash_attn call: the forward and the backward's kernels for this per-GPU shape (three, or two
         # when the dQ pass forms Delta itself); the prologue, blend and gate calls launch 3, 3 and 2 each
-        "gpu_launches": (1 + attn_bwd_kernels) * n_calls["n"] + 3 * n_calls["prologue"] + 3 * n_calls["blend"]
+        "gpu_launches": (1 + attn_bwd_kernels) * n_calls["n"] + 2 * n_calls["prologue"] + 2 * n_calls["blend"]
                         + 2 * n_calls["gate"],
         "library_calls_per_step": {"flash_attn": n_calls["n"] // steps, "qk_prologue": n_calls["prologue"] // steps,
                                    "value_blend": n_calls["blend"] // steps, "head_gate": n_calls["gate"] // steps},

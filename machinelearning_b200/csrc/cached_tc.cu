@@ -16,8 +16,8 @@
 // out.  With few (batch, KV head) pairs the key blocks are split over the CTAs of a cluster (up to 16, as many as
 // can be resident), and the partial rows -- two per CTA -- are combined through distributed shared memory, in a
 // fixed order: no scratch, no second kernel.  Measured against one warpgroup, partial rows in global memory and a
-// merge kernel: B=1 H=16 D=128, 64 queries over 16,448 keys 72 -> 33 us (4.1 TB/s of K, V); B=1 H=12 D=64, 32 over
-// 1,056 17.5 -> 10 us.
+// merge kernel: B=1 H=16 D=128, 64 queries over 16,448 keys 72 -> 35 us (3.9 TB/s of K, V); B=1 H=12 D=64, 32 over
+// 1,056 17.5 -> 9 us.
 //
 // SPLIT_P: blocks so small that the fp32 kernel used to take them keep its precision: P goes in as the sum of two
 // 16-bit values (its rounding error is then below the accumulator's), at the price of a second P V product,
