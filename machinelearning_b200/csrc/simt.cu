@@ -8,9 +8,9 @@
 // The group's probabilities go through shared memory to become the other operand of the output product; only the
 // warp's own rows are involved, so that exchange needs no CTA-wide barrier.  No atomics: bit-reproducible.
 //
-// RM = 8 where there are enough row tiles to fill the GPU, RM = 4 (twice as many, half as long CTAs) otherwise.
-// Measured, a row per warp before -> tiles: B=4 H=4 T=256 D=64 forward 82 -> 19 us, backward 174 -> 53 us (one
-// CTA of four warps per SM there: latency); B=8 H=12/4 T=2048 D=64 forward 14.9 -> 1.41 ms (37 TFLOP/s, half of
+// RM = 8, 4 or 2 by the number of row tiles (rows_per_thread).  The dQ pass runs beside the dK/dV pass.
+// Measured, a row per warp before -> tiles: B=4 H=4 T=256 D=64 forward 82 -> 18 us, backward 174 -> 36 us
+// (latency); B=8 H=12/4 T=2048 D=64 forward 14.9 -> 1.41 ms (37 TFLOP/s, half of
 // what the FMA pipe can issue), backward 32.0 -> 4.98 ms.
 //
 // Algebra follows the reference's FMA kernels (nanolab/csrc/flash_attn_cuda.cu
@@ -148,7 +148,7 @@ template <typename T, int D, int RM, bool DKV, int NB>
 __global__ void __launch_bounds__(kThreads)
 bwd_tile_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q, const T* __restrict__ k,
                 const T* __restrict__ v, const float* __restrict__ lse, const float* __restrict__ delta,
-                T* __restrict__ out0, T* __restrict__ out1) {
+                T* __restrict__ out0, T* __restrict__ out1, int wait_first) {
   constexpr int BM = 8 * RM, kPitch = D + 4;
   extern __shared__ __align__(16) float smem[];
   float* x0 = smem;
@@ -206,6 +206,8 @@ bwd_tile_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q, 
     load_commit();
   };
 
+  if (wait_first) grid_dep_wait();
+  grid_dep_release();
   if (DKV) {
     load_rows<T, D>(x0, kb + r0 * k_stride, k_stride, BM, p.T - r0);
     load_rows<T, D>(x1, vb + r0 * k_stride, k_stride, BM, p.T - r0);
@@ -292,6 +294,8 @@ bwd_tile_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q, 
     store_row<T, D>(out0 + at, col, acc0[i], 1.f);
     if constexpr (DKV) store_row<T, D>(out1 + at, col, acc1[i], 1.f);
   }
+  // a pass that started beside its predecessor does not finish before it: what follows may rely on both
+  if (!wait_first) grid_dep_wait();
 }
 
 // Delta = rowsum(dO * O): pure streaming.  A lane moves 16 bytes of dO and of O per row and has two rows in flight;
@@ -340,13 +344,21 @@ delta_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ o, flo
   }
 }
 
-// Row tiles of 64 (RM = 8) when there are two per SM, else of 32.  At D = 128 always 32: the accumulators of both
-// gradients and the tiles of 64 rows would leave one CTA of four warps per SM.
-inline bool tall_tiles(const Problem& p, int heads) {
-  return p.D <= 64 && static_cast<long long>(p.B) * heads * ((p.T + 63) / 64) >= 2ll * sm_count();
+// Rows per group of a CTA's tile: 8 (64-row tiles) when there are two tiles per SM, else 4, or 2 where 32-row tiles
+// are fewer than `least` per SM: a CTA is four warps, so a lone one leaves its SM waiting on latency (B=4 H=4 T=256
+// forward 20.6 -> 18.5 us).  At D = 128 never 8: the accumulators of both gradients and the tiles of
+// 64 rows would leave one CTA of four warps per SM.
+inline int rows_per_thread(const Problem& p, int heads, int least) {
+  auto tiles = [&](int rows) { return static_cast<long long>(p.B) * heads * ((p.T + rows - 1) / rows); };
+  if (p.D <= 64 && tiles(64) >= 2ll * sm_count()) return 8;
+  return tiles(32) >= static_cast<long long>(least) * sm_count() ? 4 : 2;
 }
 
-int launched() { return cudaGetLastError() == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA; }
+int launched(cudaError_t e) {
+  if (e == cudaSuccess) return NLFA_OK;
+  (void)cudaGetLastError();
+  return NLFA_ERR_CUDA;
+}
 
 template <typename T, int D, int RM>
 int fwd_rm(const Problem& p, const T* q, const T* k, const T* v, T* o, float* lse, cudaStream_t s) {
@@ -355,15 +367,16 @@ int fwd_rm(const Problem& p, const T* q, const T* k, const T* v, T* o, float* ls
   auto kern = fwd_tile_kernel<T, D, RM>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != NLFA_OK) return NLFA_ERR_CUDA;
   const long long blocks = static_cast<long long>(p.B) * p.H * ((p.T + BM - 1) / BM);
-  kern<<<static_cast<unsigned>(blocks), kThreads, smem, s>>>(p, q, k, v, o, lse);
-  return launched();
+  return launched(launch_kernel(kern, dim3(static_cast<unsigned>(blocks)), dim3(kThreads), smem, s, false, p, q, k, v, o, lse));
 }
 
 template <typename T, int D>
 int fwd_t(const Problem& p, const void* q, const void* k, const void* v, void* o, float* lse, cudaStream_t s) {
   const T *q_ = static_cast<const T*>(q), *k_ = static_cast<const T*>(k), *v_ = static_cast<const T*>(v);
+  const int rm = rows_per_thread(p, p.H, 2);
   if constexpr (D <= 64)
-    if (tall_tiles(p, p.H)) return fwd_rm<T, D, 8>(p, q_, k_, v_, static_cast<T*>(o), lse, s);
+    if (rm == 8) return fwd_rm<T, D, 8>(p, q_, k_, v_, static_cast<T*>(o), lse, s);
+  if (rm == 2) return fwd_rm<T, D, 2>(p, q_, k_, v_, static_cast<T*>(o), lse, s);
   return fwd_rm<T, D, 4>(p, q_, k_, v_, static_cast<T*>(o), lse, s);
 }
 
@@ -382,26 +395,28 @@ int delta_t(const Problem& p, const void* dout, const void* o, float* delta, cud
 
 template <typename T, int D, int RM, bool DKV>
 int bwd_rm(const Problem& p, const T* dout, const T* q, const T* k, const T* v, const float* lse, const float* delta,
-           void* out0, void* out1, cudaStream_t s) {
+           void* out0, void* out1, bool beside_previous, cudaStream_t s) {
   constexpr int BM = 8 * RM;
-  constexpr int NB = RM == 4 && D <= 64 ? 2 : 1;       // a second streamed buffer where two CTAs still fit an SM
+  constexpr int NB = RM <= 4 && D <= 64 ? 2 : 1;       // a second streamed buffer where two CTAs still fit an SM
   constexpr int smem = ((2 * BM + NB * 2 * kBN) * (D + 4) + BM * kPPitch + NB * 2 * kBN) * 4;
   auto kern = bwd_tile_kernel<T, D, RM, DKV, NB>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem) != NLFA_OK) return NLFA_ERR_CUDA;
   const long long blocks = static_cast<long long>(p.B) * (DKV ? p.Hkv : p.H) * ((p.T + BM - 1) / BM);
-  kern<<<static_cast<unsigned>(blocks), kThreads, smem, s>>>(p, dout, q, k, v, lse, delta, static_cast<T*>(out0),
-                                                             static_cast<T*>(out1));
-  return launched();
+  const bool overlap = overlap_launches(DKV ? kOverlapDkv : kOverlapDq);
+  return launched(launch_kernel(kern, dim3(static_cast<unsigned>(blocks)), dim3(kThreads), smem, s, overlap, p, dout, q, k, v,
+                                lse, delta, static_cast<T*>(out0), static_cast<T*>(out1), overlap && beside_previous ? 0 : 1));
 }
 
 template <typename T, int D, bool DKV>
 int bwd_pass(const Problem& p, const void* dout, const void* q, const void* k, const void* v, const float* lse,
-             const float* delta, void* out0, void* out1, cudaStream_t s) {
+             const float* delta, void* out0, void* out1, bool beside_previous, cudaStream_t s) {
   const T *g = static_cast<const T*>(dout), *q_ = static_cast<const T*>(q), *k_ = static_cast<const T*>(k),
           *v_ = static_cast<const T*>(v);
+  const int rm = rows_per_thread(p, DKV ? p.Hkv : p.H, DKV ? 2 : 1);      // (the dQ pass has the dK/dV pass beside it)
   if constexpr (D <= 64)
-    if (tall_tiles(p, DKV ? p.Hkv : p.H)) return bwd_rm<T, D, 8, DKV>(p, g, q_, k_, v_, lse, delta, out0, out1, s);
-  return bwd_rm<T, D, 4, DKV>(p, g, q_, k_, v_, lse, delta, out0, out1, s);
+    if (rm == 8) return bwd_rm<T, D, 8, DKV>(p, g, q_, k_, v_, lse, delta, out0, out1, beside_previous, s);
+  if (rm == 2) return bwd_rm<T, D, 2, DKV>(p, g, q_, k_, v_, lse, delta, out0, out1, beside_previous, s);
+  return bwd_rm<T, D, 4, DKV>(p, g, q_, k_, v_, lse, delta, out0, out1, beside_previous, s);
 }
 
 template <typename T, int D>
@@ -409,8 +424,10 @@ int bwd_t(const Problem& p, const void* dout, const void* q, const void* k, cons
           const float* lse, void* dq, void* dk, void* dv, const float* delta, int passes,
           cudaStream_t s) {
   int st = NLFA_OK;
-  if (passes & NLFA_PASS_DQ) st = bwd_pass<T, D, false>(p, dout, q, k, v, lse, delta, dq, nullptr, s);
-  if (st == NLFA_OK && (passes & NLFA_PASS_DKV)) st = bwd_pass<T, D, true>(p, dout, q, k, v, lse, delta, dk, dv, s);
+  // The dQ pass reads nothing of the dK/dV pass right before it and starts beside it.
+  if (passes & NLFA_PASS_DKV) st = bwd_pass<T, D, true>(p, dout, q, k, v, lse, delta, dk, dv, false, s);
+  if (st == NLFA_OK && (passes & NLFA_PASS_DQ))
+    st = bwd_pass<T, D, false>(p, dout, q, k, v, lse, delta, dq, nullptr, (passes & NLFA_PASS_DKV) != 0, s);
   return st;
 }
 

@@ -1,5 +1,5 @@
 """The register-tiled fp32-arithmetic kernels (``use_mma=False``) against the float64 oracle at lengths around their
-32- and 64-row tiles, both tile heights (the tall one needs two row tiles per SM), every head dim and mask."""
+16-, 32- and 64-row tiles, each of those heights (chosen by the number of row tiles per SM), every head dim and mask."""
 import math
 
 import numpy as np
@@ -15,6 +15,7 @@ CASES = [(1, 1, 1, 1, 64, 0, 0, 0, torch.float32), (1, 31, 2, 1, 128, 0, 0, 0, t
          (2, 33, 2, 2, 32, 0, 0, 0, torch.float32), (1, 65, 4, 2, 64, 0, 0, 0, torch.float32),
          (1, 129, 2, 1, 128, 40, 0, 0, torch.float32), (1, 200, 2, 2, 64, 70, 65, 0, torch.float32),
          (1, 190, 4, 1, 32, 0, 0, 100, torch.float32), (1, 130, 2, 2, 64, 0, 0, 130, torch.bfloat16),
+         (3, 200, 16, 16, 64, 0, 0, 0, torch.float32), (6, 200, 16, 8, 128, 0, 0, 90, torch.float32),
          (13, 130, 12, 4, 64, 50, 3, 0, torch.float32), (13, 97, 16, 16, 32, 0, 0, 0, torch.float16)]
 
 
