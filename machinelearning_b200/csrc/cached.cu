@@ -30,6 +30,62 @@ using namespace tiles;
 using cached::CachedParams;
 using cached::KeyRange;
 
+// Combines the partial rows of a query tile, one part in the shared memory of each CTA of the cluster: rows of D
+// sums at a pitch of D + 4 (`rows`) and per row its (maximum, sum of exponentials) in base-2 units (`stats`).  CTA
+// `rank` finishes rows rank, rank + splits, ..: a warp turns a row's maxima and sums into weights at once (`weights`:
+// 32 floats per own row), then every thread adds up pieces of four columns with the loads of eight parts in flight,
+// its own CTA's first: in the same order everywhere, all CTAs would read one CTA's memory at a time, whose 38 bytes
+// per clock were the limit.
+template <typename T, int D, class RowOf>
+__device__ __forceinline__ void merge_rows(const CachedParams& p, int n, RowOf out_row, uint32_t rows, uint32_t stats,
+                                           float* weights, int rank) {
+  constexpr int kBatch = 8;
+  const int lane = threadIdx.x & 31, splits = p.splits;                          // at most 16
+  const int own = (n - rank + splits - 1) / splits;
+  const uint32_t stat_addr = cluster_addr(stats, lane < splits ? lane : 0);
+  for (int i = threadIdx.x >> 5; i < own; i += kThreads / 32) {
+    const int r = rank + i * splits;
+    float2 ml = ld_cluster_f2(stat_addr + 8u * r);
+    if (lane >= splits) ml = make_float2(-INFINITY, 0.f);
+    float mx = ml.x;
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    mx = __shfl_sync(0xffffffffu, mx, 0);
+    const float w = exp2f(ml.x - (mx == -INFINITY ? 0.f : mx));                  // a part that saw no key: 0
+    float sum = w * ml.y;
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    sum = __shfl_sync(0xffffffffu, sum, 0);
+    weights[32 * i + lane] = sum > 0.f ? w / sum : 0.f;                          // a row that sees no key gives zeros
+    if (p.lse && lane == 0) {
+      const long long row = out_row(r), t = (row / p.H) % p.Tq, h = row % p.H, b = row / (static_cast<long long>(p.H) * p.Tq);
+      p.lse[(b * p.H + h) * p.Tq + t] = sum > 0.f ? (mx + log2f(sum)) * kLn2 : -INFINITY;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < own * (D / 4); i += kThreads) {
+    const int k = i / (D / 4), c = 4 * (i % (D / 4)), r = rank + k * splits;
+    const uint32_t at = rows + (r * (D + 4) + c) * 4u;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < splits; s0 += kBatch) {
+      float4 y[kBatch];
+      float f[kBatch];
+#pragma unroll
+      for (int x = 0; x < kBatch; ++x) {
+        const bool is = s0 + x < splits;
+        int s = is ? s0 + x + rank : rank;
+        s = s < splits ? s : s - splits;
+        y[x] = ld_cluster_f4(cluster_addr(at, s));
+        f[x] = is ? weights[32 * k + s] : 0.f;
+      }
+#pragma unroll
+      for (int x = 0; x < kBatch; ++x)
+        acc = make_float4(fmaf(f[x], y[x].x, acc.x), fmaf(f[x], y[x].y, acc.y), fmaf(f[x], y[x].z, acc.z), fmaf(f[x], y[x].w, acc.w));
+    }
+    cached::store4(static_cast<T*>(p.o) + out_row(r) * D + c, acc);
+  }
+}
+
 template <typename T, int D, int RM>
 __global__ void __launch_bounds__(kThreads)
 fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v) {
@@ -163,8 +219,7 @@ fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__
   if (p.splits > 1) {
     cluster_arrive();
     cluster_wait();
-    cached::merge_rows<T, D, 1>(p, rows, out_row, smem_u32(ks), 0, smem_u32(vs), ps, static_cast<int>(blockIdx.y),
-                                [] { __syncthreads(); return true; }, threadIdx.x, kThreads);
+    merge_rows<T, D>(p, rows, out_row, smem_u32(ks), smem_u32(vs), ps, static_cast<int>(blockIdx.y));
     cluster_arrive();                                      // no CTA leaves while another reads its shared memory
     cluster_wait();
   }

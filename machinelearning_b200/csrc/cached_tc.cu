@@ -14,10 +14,12 @@
 // while one exponentiates, the products of the other's block run and K, V of the next blocks arrive (a
 // single one, strictly in order, spent twice the load time per block).  Warps without a query row sit the blocks
 // out.  With few (batch, KV head) pairs the key blocks are split over the CTAs of a cluster (up to 16, as many as
-// can be resident), and the partial rows -- two per CTA -- are combined through distributed shared memory, in a
-// fixed order: no scratch, no second kernel.  Measured against one warpgroup, partial rows in global memory and a
-// merge kernel: B=1 H=16 D=128, 64 queries over 16,448 keys 72 -> 35 us (3.9 TB/s of K, V); B=1 H=12 D=64, 32 over
-// 1,056 17.5 -> 9 us.
+// can be resident).  At the end the two warpgroups' sums of a row become one in shared memory, each CTA sends every other
+// one the rows that one finishes (a bulk copy per pair, counted by a barrier there), and a row's parts are added in the
+// order of the CTAs: no scratch, no second kernel, no wait for a remote read.  (Reading two parts per CTA from all the
+// others, the same one at the same time, took 4.5 of the 14.8 us of B=1 H=16 D=128, 64 queries over 2,048 keys; now
+// 12.1.  Through global memory with a ticket it was more still.)  B=1 H=16 D=128, 64 over 16,448: 35.7 -> 32.1 us
+// (4.2 TB/s of K, V; 72 with one softmax warpgroup and a merge kernel); B=1 H=12 D=64, 32 over 1,056: 9.9 -> 8.8.
 //
 // SPLIT_P: blocks so small that the fp32 kernel used to take them keep its precision: P goes in as the sum of two
 // 16-bit values (its rounding error is then below the accumulator's), at the price of a second P V product,
@@ -45,21 +47,24 @@ struct TileParams {
 template <int D, int STAGES>
 struct CachedSmem {
   static constexpr int kTileBytes = kTile * D * 2;
-  static constexpr int kK = 0;                                   // later: the two warpgroups' O, [2][128][D + 4] fp32
+  static constexpr int kK = 0;                                   // later: the rows to send, then those received
   static constexpr int kV = kK + STAGES * kTileBytes;
-  static constexpr int kQ = kV + STAGES * kTileBytes;            // later: the weights of the combination
+  static constexpr int kQ = kV + STAGES * kTileBytes;
   static constexpr int kPos = kQ + kTileBytes;                   // per K stage: 128 key positions
   static constexpr int kFull = kPos + STAGES * 512;              // per K stage: every key visible to every row
-  static constexpr int kPartBytes = 128 * (D + 4) * 4;
-  static constexpr int kStat = kK + 2 * kPartBytes;              // later: [2][128] (maximum, sum) per row
+  // A partial row: D sums, (maximum, sum of exponentials) of either warpgroup and of both, padding (12 floats, not 8:
+  // lanes a row apart hit different banks).  128 to send, then what the CTAs of the cluster send, one row each
+  // for every row this CTA finishes.
+  static constexpr int kPitch = 4 * (D + 12);
+  static constexpr int kReceived = kK + 128 * kPitch;
   static constexpr int kBar = kFull + (STAGES * 4 + 15) / 16 * 16;
-  // barriers: q_full, s_full[2], p_full[2], o_done, group, k_full[S], k_empty[S], v_full[S], v_empty[S]
-  static constexpr int kNumBars = 7 + 4 * STAGES;
+  // barriers: q_full, s_full[2], p_full[2], o_done, group, received, k_full[S], k_empty[S], v_full[S], v_empty[S]
+  static constexpr int kNumBars = 8 + 4 * STAGES;
   static constexpr int kTmemSlot = kBar + 8 * kNumBars;
   static constexpr int kAbort = kTmemSlot + 4;
   static constexpr int kTotal = kAbort + 4;
   static constexpr int kDynamic = kTotal + 1024;
-  static_assert(STAGES * 2 * kTileBytes >= 2 * kPartBytes + 2048 && kTileBytes >= 128 * 32 * 4, "the combination lies over dead tiles");
+  static_assert(STAGES * 2 * kTileBytes >= (128 + 128 + kMostCluster) * kPitch, "the combination lies over dead tiles");
 };
 
 template <typename T, int D, int STAGES, bool SPLIT_P>
@@ -80,7 +85,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   auto bar = [&](int i) -> uint32_t { return base + L::kBar + 8u * i; };
-  constexpr int Q_FULL = 0, S_FULL = 1, P_FULL = 3, O_DONE = 5, GROUP = 6, K_FULL = 7,
+  constexpr int Q_FULL = 0, S_FULL = 1, P_FULL = 3, O_DONE = 5, GROUP = 6, RECEIVED = 7, K_FULL = 8,
                 K_EMPTY = K_FULL + STAGES, V_FULL = K_EMPTY + STAGES, V_EMPTY = V_FULL + STAGES;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + L::kAbort);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L::kTmemSlot);
@@ -96,6 +101,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     mbar_init(bar(O_DONE), 1);
     mbar_init(bar(GROUP), 256);
+    mbar_init(bar(RECEIVED), 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(bar(K_FULL + s), 1);
       mbar_init(bar(K_EMPTY + s), 1);
@@ -131,6 +137,16 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   // the rows of other data they begin with end in lanes nobody reads).  B=8 H=12 D=64, 32 over 8,192: 69 -> 65 us.
   const int n_rows = tp.group * (t1 - t0 + 1);
   const int second_lane = kTile - (n_rows + 31) / 32 * 32;
+  // of these this CTA finishes rows_each, from own_first on (fewer at the end)
+  const int rank = static_cast<int>(blockIdx.y);
+  const int rows_each = (n_rows + p.splits - 1) / p.splits, own_first = rank * rows_each;
+  const int own = own_first >= n_rows ? 0 : own_first + rows_each < n_rows ? rows_each : n_rows - own_first;
+  if (threadIdx.x == 0 && p.splits > 1) mbar_arrive_expect_tx(bar(RECEIVED), p.splits * own * L::kPitch);
+  if (warp == 8 && lane == 0) {
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
 
   grid_dep_wait();
   grid_dep_release();
@@ -143,9 +159,6 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     } else if (warp == 8) {
       // =============================== TMA producer ============================
       if (lane == 0) {
-        tma_prefetch_desc(&tm_q);
-        tma_prefetch_desc(&tm_k);
-        tma_prefetch_desc(&tm_v);
         mbar_arrive_expect_tx(bar(Q_FULL), kBoxes * tp.group * tp.tq_tile * 128);
         for (int x = 0; x < kBoxes; ++x)
           tma_load_4d(base + L::kQ + x * kBoxBytes, &tm_q, bar(Q_FULL), 64 * x, hk * tp.group, t0, b);
@@ -389,45 +402,117 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       ok = __all_sync(0xffffffffu, ok);
       if (ok) tc_fence_after();
     }
-    // this warpgroup's partial rows go to shared memory (every product that read the tiles there is complete)
+    // Every product that read the tiles in shared memory is complete: the other CTAs may write there.
+    __syncwarp();
+    cluster_arrive();
+    // The two warpgroups' sums of a row become one: each hands over half of its columns and adds the other half.
+    float* dst = reinterpret_cast<float*>(gen + L::kK + row * L::kPitch);
+    const int theirs = w == 0 ? D / 2 : 0, mine = D / 2 - theirs;
+    const bool any = w < n_blocks;
     if (ok && warp_rows) {
-      const bool any = w < n_blocks;
-      reinterpret_cast<float2*>(gen + L::kStat)[128 * w + row] = any ? make_float2(m_ref, l) : make_float2(-INFINITY, 0.f);
-      float* dst = reinterpret_cast<float*>(gen + L::kK + w * L::kPartBytes) + row * (D + 4);
+      *reinterpret_cast<float2*>(dst + D + 2 * w) = any ? make_float2(m_ref, l) : make_float2(-INFINITY, 0.f);
       if (any) {
-#pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
+#pragma unroll
+        for (int c = 0; c < D / 2; c += 32) {
           uint32_t orr[32];
-          tmem_ld32(o_addr + 32 * c, orr);
+          tmem_ld32(o_addr + theirs + c, orr);
           tc_wait_ld();
 #pragma unroll
           for (int e = 0; e < 32; e += 4)
-            *reinterpret_cast<float4*>(dst + 32 * c + e) =
+            *reinterpret_cast<float4*>(dst + theirs + c + e) =
                 make_float4(__uint_as_float(orr[e]), __uint_as_float(orr[e + 1]), __uint_as_float(orr[e + 2]),
                             __uint_as_float(orr[e + 3]));
         }
       }
     }
+    auto group_sync = [&](uint32_t parity) {
+      mbar_arrive(bar(GROUP));
+      const bool met = mbar_wait(bar(GROUP), parity, wctx, 69);
+      ok = __all_sync(0xffffffffu, ok && met && *abort_flag == 0);
+    };
+    group_sync(0);
+    if (ok && warp_rows) {
+      const float4 ml = *reinterpret_cast<const float4*>(dst + D);           // m, l of the first, of the second
+      const float mx = fmaxf(ml.x, ml.z), ref = mx == -INFINITY ? 0.f : mx;
+      const float f0 = exp2f(ml.x - ref), f1 = exp2f(ml.z - ref);
+      const float f_mine = w == 0 ? f0 : f1, f_other = w == 0 ? f1 : f0;
+      if (w == 0) *reinterpret_cast<float2*>(dst + D + 4) = make_float2(mx, f0 * ml.y + f1 * ml.w);
+      const bool other = (w ^ 1) < n_blocks;                                 // (without a block, neither sums nor rows exist)
+#pragma unroll
+      for (int c = 0; c < D / 2; c += 32) {
+        uint32_t orr[32];
+        if (any) tmem_ld32(o_addr + mine + c, orr);
+        tc_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 32; e += 4) {
+          float4* at = reinterpret_cast<float4*>(dst + mine + c + e);
+          float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (other) {
+            y = *at;
+            y = make_float4(f_other * y.x, f_other * y.y, f_other * y.z, f_other * y.w);
+          }
+          if (any)
+            y = make_float4(fmaf(f_mine, __uint_as_float(orr[e]), y.x), fmaf(f_mine, __uint_as_float(orr[e + 1]), y.y),
+                            fmaf(f_mine, __uint_as_float(orr[e + 2]), y.z), fmaf(f_mine, __uint_as_float(orr[e + 3]), y.w));
+          *at = y;
+        }
+      }
+    }
+    fence_proxy_async_smem();
     __syncwarp();
-    cluster_arrive();
-    cluster_wait();
-    if (ok)
-      cached::merge_rows<T, D, 2>(p, n_rows, [&](int r) {
-        return (static_cast<long long>(b) * p.Tq + t0 + r / tp.group) * p.H + hk * tp.group + r % tp.group;
-      }, base + L::kK, L::kPartBytes, base + L::kStat, reinterpret_cast<float*>(gen + L::kQ), static_cast<int>(blockIdx.y),
-      [&]() -> bool {
-        mbar_arrive(bar(GROUP));
-        ok = mbar_wait(bar(GROUP), 0, wctx, 69);
-        ok = __all_sync(0xffffffffu, ok && *abort_flag == 0);
-        return ok;
-      }, threadIdx.x, 256);
+    cluster_wait();                                // every CTA's tiles are dead
+    group_sync(1);
+    // each CTA of the cluster gets the rows it finishes
+    if (ok && p.splits > 1) {
+      if (warp == 0 && lane < p.splits) {
+        const int first = lane * rows_each, count = first + rows_each < n_rows ? rows_each : n_rows - first;
+        if (count > 0)
+          bulk_copy_cluster(cluster_addr(base + L::kReceived + rank * rows_each * L::kPitch, lane),
+                            base + L::kK + first * L::kPitch, count * L::kPitch, cluster_addr(bar(RECEIVED), lane));
+      }
+      __syncwarp();
+      ok = mbar_wait(bar(RECEIVED), 0, wctx, 70);
+      ok = __all_sync(0xffffffffu, ok);
+    }
+    __syncwarp();
+    cluster_arrive();                              // what the others sent is here
+    if (ok) {
+      // one thread per four columns of a row, the parts in the order of the CTAs
+      const uint8_t* parts = gen + (p.splits > 1 ? L::kReceived : L::kK);
+      const int part_step = rows_each * L::kPitch;
+      for (int i = threadIdx.x; i < own * (D / 4); i += 256) {
+        const int k = i / (D / 4), c = 4 * (i % (D / 4));
+        const uint8_t* at = parts + k * L::kPitch;
+        float mx = -INFINITY;
+        for (int s = 0; s < p.splits; ++s) mx = fmaxf(mx, *reinterpret_cast<const float*>(at + s * part_step + 4 * (D + 4)));
+        const float ref = mx == -INFINITY ? 0.f : mx;
+        float sum = 0.f;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int s = 0; s < p.splits; ++s) {
+          const float2 ml = *reinterpret_cast<const float2*>(at + s * part_step + 4 * (D + 4));
+          const float4 y = *reinterpret_cast<const float4*>(at + s * part_step + 4 * c);
+          const float f = exp2f(ml.x - ref);                               // a part that saw no key: 0 (of zeros)
+          sum = fmaf(f, ml.y, sum);
+          acc = make_float4(fmaf(f, y.x, acc.x), fmaf(f, y.y, acc.y), fmaf(f, y.z, acc.z), fmaf(f, y.w, acc.w));
+        }
+        const int r = own_first + k, t = t0 + r / tp.group, h = hk * tp.group + r % tp.group;
+        if (c < p.D) {                                                       // head dim 32 on 64-wide tiles
+          const float inv = sum > 0.f ? 1.f / sum : 0.f;                     // a row that sees no key gives zeros
+          cached::store4(static_cast<T*>(p.o) + ((static_cast<long long>(b) * p.Tq + t) * p.H + h) * p.D + c,
+                         make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+        }
+        if (p.lse && c == 0)
+          p.lse[(static_cast<long long>(b) * p.H + h) * p.Tq + t] = sum > 0.f ? (mx + log2f(sum)) * kLn2 : -INFINITY;
+      }
+    }
     } else {
       cluster_arrive();
       cluster_wait();
+      cluster_arrive();
     }
     __syncwarp();
-    cluster_arrive();                              // no CTA leaves while another reads its shared memory
-    cluster_wait();
+    cluster_wait();                                // what this CTA sent has arrived
   }
 
   __syncwarp();

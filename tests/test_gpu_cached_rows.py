@@ -1,0 +1,35 @@
+"""The cached forward where its row combination can go wrong, against the float64 oracle: rows that do not divide
+by the CTAs a tile's keys are split over (or are fewer than those), one to four warps of rows, a second softmax
+warpgroup without a key block, CTAs that see no key; and the same split in fp32."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import cached_f64
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32], ids=["fp16", "fp32"])
+@pytest.mark.parametrize("T,H,Hkv,L,D,causal,window", [
+    (1, 1, 1, 130, 64, True, 0),            # one row; the first CTA's second warpgroup has no block
+    (1, 8, 2, 5000, 128, True, 0),          # four rows, more CTAs than rows
+    (33, 2, 2, 700, 32, False, 0),          # two warps of rows
+    (37, 4, 2, 2300, 64, True, 0),          # three
+    (128, 1, 1, 4100, 128, True, 0),        # four
+    (50, 6, 2, 1000, 128, True, 0),         # tiles of a ragged number of rows
+    (9, 4, 4, 3000, 64, True, 100),         # a window: most of the keys are not visited
+])
+def test_rows_of_a_split_cache_match_the_oracle(T, H, Hkv, L, D, causal, window, dtype):
+    from machinelearning_b200 import flash_cuda
+    assert flash_cuda.is_available(), flash_cuda.unavailable_reason()
+    g = torch.Generator().manual_seed(T + L)
+    q = torch.randn(1, T, H, D, generator=g).to("cuda", dtype)
+    k = torch.randn(1, Hkv, L, D, generator=g).to("cuda", dtype)
+    v = torch.randn(1, Hkv, L, D, generator=g).to("cuda", dtype)
+    y, lse = flash_cuda.flash_attn_cached(q, k, v, causal=causal, window=window, return_lse=True)
+    n = lambda x: x.double().cpu().numpy()
+    ref, lse_ref = cached_f64.forward(n(q), n(k), n(v), 1.0 / np.sqrt(D), np.arange(L - T, L), np.arange(L), causal,
+                                      window, 0)
+    tol = 1e-5 if dtype == torch.float32 else 5e-3 * np.abs(ref).max()
+    assert np.abs(n(y) - ref).max() <= tol
+    assert np.abs(n(lse) - lse_ref).max() <= (1e-5 if dtype == torch.float32 else 1e-3)
