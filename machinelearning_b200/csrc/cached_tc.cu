@@ -12,14 +12,20 @@
 // What bounds it is streaming K and V, so everything else has to hide behind the loads.  Two softmax
 // warpgroups take alternate key blocks, each with S / P and O columns and a running maximum of its own:
 // while one exponentiates, the products of the other's block run and K, V of the next blocks arrive (a
-// single one, strictly in order, spent twice the load time per block).  Warps without a query row sit the blocks
-// out.  With few (batch, KV head) pairs the key blocks are split over the CTAs of a cluster (up to 16, as many as
-// can be resident).  At the end the two warpgroups' sums of a row become one in shared memory, each CTA sends every other
-// one the rows that one finishes (a bulk copy per pair, counted by a barrier there), and a row's parts are added in the
-// order of the CTAs: no scratch, no second kernel, no wait for a remote read.  (Reading two parts per CTA from all the
-// others, the same one at the same time, took 4.5 of the 14.8 us of B=1 H=16 D=128, 64 queries over 2,048 keys; now
-// 12.1.  Through global memory with a ticket it was more still.)  B=1 H=16 D=128, 64 over 16,448: 35.7 -> 32.1 us
-// (4.2 TB/s of K, V; 72 with one softmax warpgroup and a merge kernel); B=1 H=12 D=64, 32 over 1,056: 9.9 -> 8.8.
+// single one, strictly in order, spent twice the load time per block).
+//
+// COPIES: up to 64 rows leave half or more of a tile's 128 lanes empty, and with them warps of either softmax
+// warpgroup.  The rows then stand in the tile two or four times, and each copy's warps exponentiate their share of a
+// block's columns (and put zeros where the other copies' probabilities stand): a block takes a half or a
+// quarter of the time, 1,900 -> 600 clocks, and the copies' sums are parts like the others.  B=8 H=12 D=64, 32 over 8,192:
+// 59 -> 41 us (4.9 TB/s); B=14 H=12 D=32, 8 over 3,000: 60 -> 39; B=1 H=12 D=64, 32 over 1,056: 8.8 -> 7.3.
+//
+// With few (batch, KV head) pairs the key blocks are split over the CTAs of a cluster (up to 16, as many as can be
+// resident).  At the end a CTA's parts of a row become one in shared memory, each CTA sends every other one the rows that
+// one finishes (a bulk copy per pair, counted by a barrier there), and a row's parts are added in the order of the
+// CTAs: no scratch, no second kernel, no wait for a remote read.  (Reading two parts per CTA from all the others, the
+// same one at the same time, took 4.5 of the 14.8 us of B=1 H=16 D=128, 64 queries over 2,048 keys, now 11.7; through
+// global memory with a ticket it was more still.)  B=1 H=16 D=128, 64 over 16,448: 35.7 -> 31.0 us (4.35 TB/s of K, V).
 //
 // SPLIT_P: blocks so small that the fp32 kernel used to take them keep its precision: P goes in as the sum of two
 // 16-bit values (its rounding error is then below the accumulator's), at the price of a second P V product,
@@ -44,7 +50,7 @@ struct TileParams {
   unsigned* status;
 };
 
-template <int D, int STAGES>
+template <int D, int STAGES, int COPIES>
 struct CachedSmem {
   static constexpr int kTileBytes = kTile * D * 2;
   static constexpr int kK = 0;                                   // later: the rows to send, then those received
@@ -52,11 +58,13 @@ struct CachedSmem {
   static constexpr int kQ = kV + STAGES * kTileBytes;
   static constexpr int kPos = kQ + kTileBytes;                   // per K stage: 128 key positions
   static constexpr int kFull = kPos + STAGES * 512;              // per K stage: every key visible to every row
-  // A partial row: D sums, (maximum, sum of exponentials) of either warpgroup and of both, padding (12 floats, not 8:
-  // lanes a row apart hit different banks).  128 to send, then what the CTAs of the cluster send, one row each
-  // for every row this CTA finishes.
+  // A partial row: D sums, (maximum, sum of exponentials) of its part (with one copy: of both), the same of the CTA's parts
+  // together, padding (12 floats, not 8: lanes a row apart hit different banks).  Of a split tile, what the CTAs of the
+  // cluster send comes behind them, one row each for every row this CTA finishes; with one copy, the two parts' rows
+  // are then the same (of any column, one of them is handed over), for room.
   static constexpr int kPitch = 4 * (D + 12);
-  static constexpr int kReceived = kK + 128 * kPitch;
+  static constexpr int kReceived = kK + (COPIES == 1 ? 128 : 256) * kPitch;
+  static constexpr int kPartStep = kTile / COPIES * kPitch, kSplitPartStep = COPIES == 1 ? 0 : kPartStep;
   static constexpr int kBar = kFull + (STAGES * 4 + 15) / 16 * 16;
   // barriers: q_full, s_full[2], p_full[2], o_done, group, received, k_full[S], k_empty[S], v_full[S], v_empty[S]
   static constexpr int kNumBars = 8 + 4 * STAGES;
@@ -64,14 +72,15 @@ struct CachedSmem {
   static constexpr int kAbort = kTmemSlot + 4;
   static constexpr int kTotal = kAbort + 4;
   static constexpr int kDynamic = kTotal + 1024;
-  static_assert(STAGES * 2 * kTileBytes >= (128 + 128 + kMostCluster) * kPitch, "the combination lies over dead tiles");
+  static_assert(STAGES * 2 * kTileBytes >= kReceived + (kTile / COPIES + kMostCluster) * kPitch && STAGES * 2 * kTileBytes >= 256 * kPitch, "the combination lies over dead tiles");
 };
 
-template <typename T, int D, int STAGES, bool SPLIT_P>
+template <typename T, int D, int STAGES, int COPIES, bool SPLIT_P>
 __global__ void __launch_bounds__(384, 1)
 cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const CachedParams p, const TileParams tp) {
-  using L = CachedSmem<D, STAGES>;
+  using L = CachedSmem<D, STAGES, COPIES>;
+  constexpr int kLanes = kTile / COPIES, kCols = kTile / COPIES;   // of a copy: its TMEM lanes, its columns of S
   constexpr int kBoxes = D / 64;
   constexpr int kBoxBytes = kTile * 128;
   constexpr bool kBf16 = Pack2<T>::kIsBf16;
@@ -132,11 +141,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const int n_begin = static_cast<int>(blockIdx.y) * per;
   const int n_stop = n_begin + per < range.count ? n_begin + per : range.count;
   const int n_blocks = n_stop > n_begin ? n_stop - n_begin : 0;            // block i of this CTA: range.at(n_begin + i)
-  // Query rows, and the TMEM lanes the second warpgroup has them in: the last ones, so that with few rows the two
-  // warpgroups' busy warps sit on different schedulers (its S products start that many rows before the Q tile;
-  // the rows of other data they begin with end in lanes nobody reads).  B=8 H=12 D=64, 32 over 8,192: 69 -> 65 us.
   const int n_rows = tp.group * (t1 - t0 + 1);
-  const int second_lane = kTile - (n_rows + 31) / 32 * 32;
   // of these this CTA finishes rows_each, from own_first on (fewer at the end)
   const int rank = static_cast<int>(blockIdx.y);
   const int rows_each = (n_rows + p.splits - 1) / p.splits, own_first = rank * rows_each;
@@ -159,9 +164,9 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     } else if (warp == 8) {
       // =============================== TMA producer ============================
       if (lane == 0) {
-        mbar_arrive_expect_tx(bar(Q_FULL), kBoxes * tp.group * tp.tq_tile * 128);
-        for (int x = 0; x < kBoxes; ++x)
-          tma_load_4d(base + L::kQ + x * kBoxBytes, &tm_q, bar(Q_FULL), 64 * x, hk * tp.group, t0, b);
+        mbar_arrive_expect_tx(bar(Q_FULL), COPIES * kBoxes * tp.group * tp.tq_tile * 128);
+        for (int x = 0; x < COPIES * kBoxes; ++x)
+          tma_load_4d(base + L::kQ + x / COPIES * kBoxBytes + x % COPIES * kLanes * 128, &tm_q, bar(Q_FULL), 64 * (x / COPIES), hk * tp.group, t0, b);
       }
       // the tile's query positions, as a range
       int qp_min = INT_MAX, qp_max = -INT_MAX;
@@ -235,7 +240,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const int s = i % STAGES;
         if (!(ok = wait_all(bar(K_FULL + s), (i / STAGES) & 1, 63))) return;
         tc_fence_after();
-        const uint32_t qa = base + L::kQ - ((i & 1) ? 128u * second_lane : 0u), ka = base + L::kK + s * L::kTileBytes;
+        const uint32_t qa = base + L::kQ, ka = base + L::kK + s * L::kTileBytes;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = (kk >> 2) * kBoxBytes + (kk & 3) * 32;
@@ -279,13 +284,13 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     setmaxnreg_inc<kRegsCompute>();
     if (!dead) {
     const int w = warp >> 2;                                     // warpgroup: blocks w, w + 2, ...
-    const int first_lane = w == 0 ? 0 : second_lane;             // TMEM lane of row 0
-    const int row = static_cast<int>(threadIdx.x & 127) - first_lane;
+    const int copy = (threadIdx.x & 127) / kLanes;               // the same for the whole warp
+    const int row = threadIdx.x % kLanes;                        // row of the tile; its TMEM lane is kLanes * copy + row
     const uint32_t lane_base = 32u * (warp & 3);
-    const uint32_t s_addr = tmem_addr(tmem, lane_base, 128 * w);
+    const uint32_t p_addr = tmem_addr(tmem, lane_base, 128 * w), s_addr = p_addr + kCols * copy;
     const uint32_t o_addr = tmem_addr(tmem, lane_base, 256 + D * w);
-    const bool valid = row >= 0 && row < n_rows;
-    const bool warp_rows = row - lane >= 0 && row - lane < n_rows;   // some row of this warp belongs to a query
+    const bool valid = row < n_rows;
+    const bool warp_rows = row - lane < n_rows;                  // some row of this warp belongs to a query
     const int qp = valid ? cached::query_position(p, t0 + row / tp.group) : 0;
     const int span = p.window - p.sinks;
     const uint64_t scale2 = pack_f2(p.scale_log2, p.scale_log2);
@@ -301,17 +306,17 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         continue;
       }
       tc_fence_after();
-      uint32_t sv[4][32];
+      uint32_t sv[kCols / 32][32];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(s_addr + 32 * c, sv[c]);
+      for (int c = 0; c < kCols / 32; ++c) tmem_ld32(s_addr + 32 * c, sv[c]);
       // (the stage's positions and flag stay: the producer rewrites them only once V_EMPTY says that this block's
       // P V product, which waits for this warpgroup, has completed)
       const bool full = full_flag[s] != 0;
       tc_wait_ld();
       if (!full) {
-        const int4* pos4 = reinterpret_cast<const int4*>(gen + L::kPos + s * 512);
+        const int4* pos4 = reinterpret_cast<const int4*>(gen + L::kPos + s * 512) + kCols / 4 * copy;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < kCols / 32; ++c) {
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {
             const int4 kp = pos4[8 * c + e / 4];
@@ -328,7 +333,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       float b0 = -INFINITY, b1 = -INFINITY;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < kCols / 32; ++c) {
 #pragma unroll
         for (int e = 0; e < 32; e += 4) {
           b0 = fmax3(b0, __uint_as_float(sv[c][e]), __uint_as_float(sv[c][e + 1]));
@@ -365,7 +370,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const uint64_t negm2 = pack_f2(-m_use, -m_use);
       uint64_t acc0 = 0ull, acc1 = 0ull;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
+      for (int c = 0; c < kCols / 32; ++c) {
         uint32_t pk[16], lo[16];
 #pragma unroll
         for (int e = 0; e < 32; e += 4) {
@@ -385,8 +390,18 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             lo[e / 2 + 1] = Pack2<T>::pack(e2 - static_cast<float>(r[2]), e3 - static_cast<float>(r[3]));
           }
         }
-        tmem_st16(s_addr + 16 * c, pk);
-        if constexpr (SPLIT_P) tmem_st16(s_addr + 64 + 16 * c, lo);
+        tmem_st16(p_addr + kCols / 2 * copy + 16 * c, pk);
+        if constexpr (SPLIT_P) tmem_st16(p_addr + 64 + kCols / 2 * copy + 16 * c, lo);
+      }
+      // the other copies' keys: nothing here
+      if constexpr (COPIES > 1) {
+        const uint32_t zero[16] = {};
+#pragma unroll
+        for (int c = 0; c < (COPIES - 1) * kCols / 32; ++c) {
+          const uint32_t at = p_addr + (kCols / 2 * (copy + 1) + 16 * c) % 64;
+          tmem_st16(at, zero);
+          if constexpr (SPLIT_P) tmem_st16(at + 64, zero);
+        }
       }
       {
         float x, y;
@@ -405,23 +420,30 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // Every product that read the tiles in shared memory is complete: the other CTAs may write there.
     __syncwarp();
     cluster_arrive();
-    // The two warpgroups' sums of a row become one: each hands over half of its columns and adds the other half.
-    float* dst = reinterpret_cast<float*>(gen + L::kK + row * L::kPitch);
-    const int theirs = w == 0 ? D / 2 : 0, mine = D / 2 - theirs;
+    // A row's sums -- of either warpgroup and every copy -- become one.  Of a split tile, each thread hands over all of
+    // its columns but one slice, in which it adds up what the others hand over; else all of them, to be finished at once.
+    constexpr int kParts = 2 * COPIES, kSlice = D / kParts, kStatStep = COPIES == 1 ? 2 : L::kPartStep / 4;
+    const bool split = p.splits > 1;
+    const int step = split ? L::kSplitPartStep / 4 : L::kPartStep / 4;
+    const int part = w * COPIES + copy;
+    float* first = reinterpret_cast<float*>(gen + L::kK + row * L::kPitch);  // the row of part 0: the result as well
     const bool any = w < n_blocks;
     if (ok && warp_rows) {
-      *reinterpret_cast<float2*>(dst + D + 2 * w) = any ? make_float2(m_ref, l) : make_float2(-INFINITY, 0.f);
+      float* dst = first + part * step;
+      const int keep = split ? part : -1;                                    // slice
+      *reinterpret_cast<float2*>(first + part * kStatStep + D) = any ? make_float2(m_ref, l) : make_float2(-INFINITY, 0.f);
       if (any) {
 #pragma unroll
-        for (int c = 0; c < D / 2; c += 32) {
+        for (int c = 0; c < D; c += 32) {
+          if (kSlice >= 32 && c / kSlice == keep) continue;
           uint32_t orr[32];
-          tmem_ld32(o_addr + theirs + c, orr);
+          tmem_ld32(o_addr + c, orr);
           tc_wait_ld();
 #pragma unroll
           for (int e = 0; e < 32; e += 4)
-            *reinterpret_cast<float4*>(dst + theirs + c + e) =
-                make_float4(__uint_as_float(orr[e]), __uint_as_float(orr[e + 1]), __uint_as_float(orr[e + 2]),
-                            __uint_as_float(orr[e + 3]));
+            if (kSlice >= 32 || (c + e) / kSlice != keep)
+              *reinterpret_cast<float4*>(dst + c + e) = make_float4(__uint_as_float(orr[e]), __uint_as_float(orr[e + 1]),
+                                                                    __uint_as_float(orr[e + 2]), __uint_as_float(orr[e + 3]));
         }
       }
     }
@@ -431,39 +453,50 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       ok = __all_sync(0xffffffffu, ok && met && *abort_flag == 0);
     };
     group_sync(0);
-    if (ok && warp_rows) {
-      const float4 ml = *reinterpret_cast<const float4*>(dst + D);           // m, l of the first, of the second
-      const float mx = fmaxf(ml.x, ml.z), ref = mx == -INFINITY ? 0.f : mx;
-      const float f0 = exp2f(ml.x - ref), f1 = exp2f(ml.z - ref);
-      const float f_mine = w == 0 ? f0 : f1, f_other = w == 0 ? f1 : f0;
-      if (w == 0) *reinterpret_cast<float2*>(dst + D + 4) = make_float2(mx, f0 * ml.y + f1 * ml.w);
-      const bool other = (w ^ 1) < n_blocks;                                 // (without a block, neither sums nor rows exist)
+    if (ok && split && warp_rows) {
+      float2 ml[kParts];
+      float mx = -INFINITY, sum = 0.f, f_mine = 0.f;
 #pragma unroll
-      for (int c = 0; c < D / 2; c += 32) {
-        uint32_t orr[32];
-        if (any) tmem_ld32(o_addr + mine + c, orr);
+      for (int x = 0; x < kParts; ++x) {
+        ml[x] = *reinterpret_cast<const float2*>(first + x * kStatStep + D);
+        mx = fmaxf(mx, ml[x].x);
+      }
+      const float ref = mx == -INFINITY ? 0.f : mx;
+#pragma unroll
+      for (int x = 0; x < kParts; ++x) {
+        ml[x].x = exp2f(ml[x].x - ref);                                      // a part that saw no key: 0
+        sum = fmaf(ml[x].x, ml[x].y, sum);
+        f_mine = x == part ? ml[x].x : f_mine;
+      }
+      if (part == 0) *reinterpret_cast<float2*>(first + D + 4) = make_float2(mx, sum);
+#pragma unroll
+      for (int c = 0; c < kSlice; c += 8) {
+        uint32_t orr[8];
+        if (any) tmem_ld8(o_addr + part * kSlice + c, orr);
         tc_wait_ld();
 #pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          float4* at = reinterpret_cast<float4*>(dst + mine + c + e);
-          float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (other) {
-            y = *at;
-            y = make_float4(f_other * y.x, f_other * y.y, f_other * y.z, f_other * y.w);
-          }
+        for (int e = 0; e < 8; e += 4) {
+          float* at = first + part * kSlice + c + e;
+          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
           if (any)
-            y = make_float4(fmaf(f_mine, __uint_as_float(orr[e]), y.x), fmaf(f_mine, __uint_as_float(orr[e + 1]), y.y),
-                            fmaf(f_mine, __uint_as_float(orr[e + 2]), y.z), fmaf(f_mine, __uint_as_float(orr[e + 3]), y.w));
-          *at = y;
+            acc = make_float4(f_mine * __uint_as_float(orr[e]), f_mine * __uint_as_float(orr[e + 1]),
+                              f_mine * __uint_as_float(orr[e + 2]), f_mine * __uint_as_float(orr[e + 3]));
+#pragma unroll
+          for (int x = 0; x < kParts; ++x) {
+            if (x == part || x / COPIES >= n_blocks) continue;               // (a warpgroup without a block handed nothing over)
+            const float4 y = *reinterpret_cast<const float4*>(at + x * step);
+            acc = make_float4(fmaf(ml[x].x, y.x, acc.x), fmaf(ml[x].x, y.y, acc.y), fmaf(ml[x].x, y.z, acc.z), fmaf(ml[x].x, y.w, acc.w));
+          }
+          *reinterpret_cast<float4*>(at) = acc;
         }
       }
     }
     fence_proxy_async_smem();
     __syncwarp();
     cluster_wait();                                // every CTA's tiles are dead
-    group_sync(1);
+    if (split) group_sync(1);
     // each CTA of the cluster gets the rows it finishes
-    if (ok && p.splits > 1) {
+    if (ok && split) {
       if (warp == 0 && lane < p.splits) {
         const int first = lane * rows_each, count = first + rows_each < n_rows ? rows_each : n_rows - first;
         if (count > 0)
@@ -476,34 +509,38 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     __syncwarp();
     cluster_arrive();                              // what the others sent is here
+    // four columns of a row of the tile, out of parts that lie `stride` floats apart, their statistics `stat_stride`
+    auto finish = [&](int r, int c, const float* at, int count, int stride, const float* stats, int stat_stride) {
+      float mx = -INFINITY;
+      for (int s = 0; s < count; ++s) mx = fmaxf(mx, stats[s * stat_stride]);
+      const float ref = mx == -INFINITY ? 0.f : mx;
+      float sum = 0.f;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int s = 0; s < count; ++s) {
+        const float2 ml = *reinterpret_cast<const float2*>(stats + s * stat_stride);
+        const float4 y = *reinterpret_cast<const float4*>(at + s * stride + c);
+        const float f = exp2f(ml.x - ref);                                   // a part that saw no key: 0 (of zeros)
+        sum = fmaf(f, ml.y, sum);
+        acc = make_float4(fmaf(f, y.x, acc.x), fmaf(f, y.y, acc.y), fmaf(f, y.z, acc.z), fmaf(f, y.w, acc.w));
+      }
+      const int t = t0 + r / tp.group, h = hk * tp.group + r % tp.group;
+      if (c < p.D) {                                                         // head dim 32 on 64-wide tiles
+        const float inv = sum > 0.f ? 1.f / sum : 0.f;                       // a row that sees no key gives zeros
+        cached::store4(static_cast<T*>(p.o) + ((static_cast<long long>(b) * p.Tq + t) * p.H + h) * p.D + c,
+                       make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+      }
+      if (p.lse && c == 0)
+        p.lse[(static_cast<long long>(b) * p.H + h) * p.Tq + t] = sum > 0.f ? (mx + log2f(sum)) * kLn2 : -INFINITY;
+    };
     if (ok) {
-      // one thread per four columns of a row, the parts in the order of the CTAs
-      const uint8_t* parts = gen + (p.splits > 1 ? L::kReceived : L::kK);
-      const int part_step = rows_each * L::kPitch;
+      // one thread per four columns: of the rows of the tile, or of those this CTA finishes, the parts in the order of the CTAs
+      const float* parts = reinterpret_cast<const float*>(gen + (split ? L::kReceived : L::kK));
       for (int i = threadIdx.x; i < own * (D / 4); i += 256) {
         const int k = i / (D / 4), c = 4 * (i % (D / 4));
-        const uint8_t* at = parts + k * L::kPitch;
-        float mx = -INFINITY;
-        for (int s = 0; s < p.splits; ++s) mx = fmaxf(mx, *reinterpret_cast<const float*>(at + s * part_step + 4 * (D + 4)));
-        const float ref = mx == -INFINITY ? 0.f : mx;
-        float sum = 0.f;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-        for (int s = 0; s < p.splits; ++s) {
-          const float2 ml = *reinterpret_cast<const float2*>(at + s * part_step + 4 * (D + 4));
-          const float4 y = *reinterpret_cast<const float4*>(at + s * part_step + 4 * c);
-          const float f = exp2f(ml.x - ref);                               // a part that saw no key: 0 (of zeros)
-          sum = fmaf(f, ml.y, sum);
-          acc = make_float4(fmaf(f, y.x, acc.x), fmaf(f, y.y, acc.y), fmaf(f, y.z, acc.z), fmaf(f, y.w, acc.w));
-        }
-        const int r = own_first + k, t = t0 + r / tp.group, h = hk * tp.group + r % tp.group;
-        if (c < p.D) {                                                       // head dim 32 on 64-wide tiles
-          const float inv = sum > 0.f ? 1.f / sum : 0.f;                     // a row that sees no key gives zeros
-          cached::store4(static_cast<T*>(p.o) + ((static_cast<long long>(b) * p.Tq + t) * p.H + h) * p.D + c,
-                         make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
-        }
-        if (p.lse && c == 0)
-          p.lse[(static_cast<long long>(b) * p.H + h) * p.Tq + t] = sum > 0.f ? (mx + log2f(sum)) * kLn2 : -INFINITY;
+        const float* at = parts + k * (L::kPitch / 4);
+        if (split) finish(own_first + k, c, at, p.splits, rows_each * (L::kPitch / 4), at + D + 4, rows_each * (L::kPitch / 4));
+        else finish(k, c, at, COPIES * (n_blocks < 2 ? n_blocks : 2), L::kPartStep / 4, at + D, kStatStep);
       }
     }
     } else {
@@ -524,12 +561,12 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   }
 }
 
-template <typename T, int D, int STAGES, bool SPLIT_P>
+template <typename T, int D, int STAGES, int COPIES, bool SPLIT_P>
 int launch_t(CachedParams p, const TileParams& tp, int n_blocks, const CUtensorMap& mq, const CUtensorMap& mk,
              const CUtensorMap& mv, cudaStream_t stream) {
-  using L = CachedSmem<D, STAGES>;
+  using L = CachedSmem<D, STAGES, COPIES>;
   static_assert(L::kDynamic <= 232448, "over the shared memory a CTA can have");
-  auto kern = cached_tc_kernel<T, D, STAGES, SPLIT_P>;
+  auto kern = cached_tc_kernel<T, D, STAGES, COPIES, SPLIT_P>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kDynamic) != NLFA_OK) return NLFA_ERR_CUDA;
   // As many CTAs per query tile as can be resident at once, with at least two key blocks (one per softmax
   // warpgroup) each.
@@ -544,14 +581,23 @@ int launch_t(CachedParams p, const TileParams& tp, int n_blocks, const CUtensorM
   return NLFA_OK;
 }
 
+template <typename T, int D, int STAGES, bool SPLIT_P>
+int launch_copies(const CachedParams& p, const TileParams& tp, int n_blocks, const CUtensorMap& mq, const CUtensorMap& mk,
+                  const CUtensorMap& mv, cudaStream_t stream) {
+  const int rows = tp.group * tp.tq_tile;
+  if (rows <= kTile / 4) return launch_t<T, D, STAGES, 4, SPLIT_P>(p, tp, n_blocks, mq, mk, mv, stream);
+  if (rows <= kTile / 2) return launch_t<T, D, STAGES, 2, SPLIT_P>(p, tp, n_blocks, mq, mk, mv, stream);
+  return launch_t<T, D, STAGES, 1, SPLIT_P>(p, tp, n_blocks, mq, mk, mv, stream);
+}
+
 template <typename T>
 int launch_for(const CachedParams& p, const TileParams& tp, int n_blocks, bool split_p, const CUtensorMap& mq,
                const CUtensorMap& mk, const CUtensorMap& mv, cudaStream_t stream) {
   if (p.D <= 64)
-    return split_p ? launch_t<T, 64, 5, true>(p, tp, n_blocks, mq, mk, mv, stream)
-                   : launch_t<T, 64, 5, false>(p, tp, n_blocks, mq, mk, mv, stream);
-  return split_p ? launch_t<T, 128, 3, true>(p, tp, n_blocks, mq, mk, mv, stream)
-                 : launch_t<T, 128, 3, false>(p, tp, n_blocks, mq, mk, mv, stream);
+    return split_p ? launch_copies<T, 64, 5, true>(p, tp, n_blocks, mq, mk, mv, stream)
+                   : launch_copies<T, 64, 5, false>(p, tp, n_blocks, mq, mk, mv, stream);
+  return split_p ? launch_copies<T, 128, 3, true>(p, tp, n_blocks, mq, mk, mv, stream)
+                 : launch_copies<T, 128, 3, false>(p, tp, n_blocks, mq, mk, mv, stream);
 }
 
 int positions_per_tile(int Tq, int group) { return Tq < kTile / group ? Tq : kTile / group; }

@@ -13,6 +13,9 @@ from oracle import cached_f64
 @pytest.mark.parametrize("T,H,Hkv,L,D,causal,window", [
     (1, 1, 1, 130, 64, True, 0),            # one row; the first CTA's second warpgroup has no block
     (1, 8, 2, 5000, 128, True, 0),          # four rows, more CTAs than rows
+    (20, 3, 3, 250, 128, False, 0),         # two blocks, one CTA: finished without a split
+    (40, 2, 2, 200, 128, True, 0),          # the same with two warps of rows
+    (100, 2, 2, 129, 64, True, 0),          # .. with four
     (33, 2, 2, 700, 32, False, 0),          # two warps of rows
     (37, 4, 2, 2300, 64, True, 0),          # three
     (128, 1, 1, 4100, 128, True, 0),        # four
