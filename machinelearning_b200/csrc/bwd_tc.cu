@@ -1257,6 +1257,21 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
   if (sst != NLFA_OK) return sst;
   const int grid = bp.total_units < sm_count() ? bp.total_units : sm_count();
   bp.sched_group = MODE == MODE_DQ ? bp.BH : grid;      // (the dQ pass gains nothing from groups)
+  if (MODE == MODE_DKV_DS) {
+    // This pass shares DRAM with the dS it writes: groups whose Q and dO stay in L2, where those of a head per CTA would
+    // not, as long as each gives every CTA two units (run long enough for the power cap to hold, the whole backward at
+    // B=8 H=16 T=3312 1,457 -> 1,327 us, B=55 H=6/2 T=1938 1,297 -> 1,208, B=4 H=16 T=8192 3,540 -> 3,425; a last group of
+    // fewer units cost 12% at B=2 H=16/4 T=7000).  Without the writes (D = 64) it gained nothing or lost up to 4%.
+    const long long rows = p.window > 0 && p.window + 2 * kTile < p.T ? p.window + 2 * kTile : p.T;
+    const long long bytes = rows * p.D * 4 * (p.H / p.Hkv);                     // of a pair's streamed tiles in use
+    const long long together = bp.BH < grid ? bp.BH : grid, most = bp.total_units / (2ll * grid);
+    if (bytes * together > (64ll << 20) && most > 1) {
+      const long long fits = bytes < (32ll << 20) ? (32ll << 20) / bytes : 1, want = (bp.BH + fits - 1) / fits;
+      const int groups = static_cast<int>(want < most ? want : most);
+      const int size = (bp.BH + groups - 1) / groups;
+      bp.sched_group = size < grid ? size : grid;
+    }
+  }
   // (the fused pass follows a memset, not a kernel: launched the plain way)
   const bool overlap = MODE != MODE_FUSED && !plain_launch && overlap_launches(MODE == MODE_DQ ? kOverlapDq : kOverlapDkv);
   bp.dep_wait_first = (overlap && beside_previous) ? 0 : 1;

@@ -59,3 +59,20 @@ def test_backward_with_room_for_ds(B, T, H, Hkv, window, sinks, block, dtype):
     for a, b, c, w in zip(recomputed, left, by_pair, want):
         assert torch.equal(a, b) and torch.equal(b, c)
         assert np.abs(b.double().cpu().numpy() - w).max() <= 2e-2 * max(np.abs(w).max(), 1e-2)
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,window", [(7, 1200, 16, 16, 0), (40, 1500, 6, 2, 0), (12, 1700, 16, 16, 700)])
+def test_heads_in_groups_change_nothing(B, T, H, Hkv, window):
+    """Streamed tiles beyond L2: the dK/dV pass takes its heads in (uneven) groups."""
+    from machinelearning_b200 import _lib as L, flash_cuda as fc
+    assert fc.is_available(), fc.unavailable_reason()
+    lib, D = fc._load(), 128
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q, k, v, do = (torch.randn(B, T, h, D, device="cuda", generator=g).bfloat16() for h in (H, Hkv, Hkv, H))
+    scale = 1.0 / math.sqrt(D)
+    o, lse = fc.fwd(q, k, v, scale, True, window, 0, 0)
+    whole = lib.nlfa_bwd_workspace_bytes(B, T, H, Hkv, D, window, 0, 0, L.DTYPE_BF16, L.PATH_TENSOR)
+    assert lib.nlfa_bwd_workspace_kernel_count(B, T, H, Hkv, D, window, 0, 0, L.DTYPE_BF16, L.PATH_TENSOR, whole) == 3
+    args = (lib, L, do, q, k, v, o, lse, scale, window, 0, 0)
+    for a, b in zip(_backward(*args, lib.nlfa_bwd_scratch_bytes(B, T, H)), _backward(*args, whole)):
+        assert torch.equal(a, b)

@@ -1,5 +1,5 @@
-"""Both unit heights of the tensor-core forward -- one query tile, and two (long rows and more tiles than SMs at head dims
-up to 64; more than two tiles per SM at 128) -- against plain float32 attention on the GPU, at odd and even numbers of
+"""Both unit heights of the tensor-core forward -- one query tile, and two (long rows and more tiles than SMs, or K and V beyond L2, at
+head dims up to 64; more than two tiles per SM at 128) -- against plain float32 attention on the GPU, at odd and even numbers of
 tiles, under every mask, and the logsumexp with them."""
 import pytest
 import torch
@@ -9,6 +9,7 @@ pytestmark = pytest.mark.gpu
 #        B, T, H, Hkv, D, window, sinks, block, dtype
 CASES = [(1, 4200, 5, 1, 64, 0, 0, 0, torch.bfloat16), (1, 4353, 6, 2, 32, 0, 0, 0, torch.float16),   # two tiles
          (1, 4300, 5, 5, 64, 4150, 70, 0, torch.bfloat16), (1, 4480, 5, 5, 64, 0, 0, 700, torch.bfloat16),
+         (16, 2100, 8, 8, 64, 0, 0, 0, torch.float16),                             # .. for K and V beyond L2
          (25, 300, 4, 2, 128, 0, 0, 0, torch.bfloat16), (25, 385, 4, 4, 128, 150, 9, 0, torch.float16),
          (25, 290, 4, 1, 128, 0, 0, 100, torch.bfloat16),
          (1, 4096, 3, 1, 64, 0, 0, 0, torch.bfloat16), (1, 4200, 4, 2, 64, 0, 0, 0, torch.bfloat16),  # one tile
