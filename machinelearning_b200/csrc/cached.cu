@@ -14,7 +14,7 @@
 // go to the tensor cores (cached_tc.cu).  The fp32 kernel: a CTA of 128 threads owns 8 RM query rows of one (batch, KV
 // head) -- the rows (t, g) of every query head of the group, so K and V are fetched once for all of them -- and
 // streams 64 keys at a time through shared memory, products in register tiles (tiles.cuh).  RM is the
-// largest of 4, 2, 1 that leaves two CTAs per SM: more rows per thread take fewer shared-memory reads per
+// largest of 4, 2, 1 that leaves enough CTAs (launch_dim): more rows per thread take fewer shared-memory reads per
 // multiply-add, but a block of a few rows needs CTAs.  Key blocks no row of the CTA can see (contiguous positions)
 // are skipped without being read; with few row tiles the key blocks are split over the CTAs of a cluster, which
 // combine the partial rows through distributed shared memory in a fixed order.  No atomics: bit-reproducible.
@@ -256,9 +256,12 @@ int launch_dim(const CachedParams& p, const void* q, const void* k, const void* 
     if (s > pairs) s = pairs;
     return static_cast<int>(s < 1 ? 1 : s);
   };
-  auto fills = [&](int rm) { return heads * ((head_rows + 8 * rm - 1) / (8 * rm)) * splits(rm) >= want; };
-  if (head_rows > 16 && fills(4)) return launch_rm<T, D, 4>(p, q, k, v, splits(4), st);
-  if (head_rows > 8 && fills(2)) return launch_rm<T, D, 2>(p, q, k, v, splits(2), st);
+  auto ctas = [&](int rm) { return heads * ((head_rows + 8 * rm - 1) / (8 * rm)) * splits(rm); };
+  // Half the height takes well over half the time: two rows a thread win over one as soon as they occupy most of the SMs (108
+  // to 216 CTAs, D = 32 / 64 / 128: H=12, 32 over 1,056 13.5 / 19.8 / 35.0 -> 12.5 / 16.5 / 25.3 us; H=8, 16 over 4,096 at
+  // D = 128 45.2 -> 41.0), not with a few dozen (H=4, 20 over 300: 10.4 / 12.4).
+  if (head_rows > 16 && ctas(4) >= want) return launch_rm<T, D, 4>(p, q, k, v, splits(4), st);
+  if (head_rows > 8 && 3 * ctas(2) >= want) return launch_rm<T, D, 2>(p, q, k, v, splits(2), st);
   return launch_rm<T, D, 1>(p, q, k, v, splits(1), st);
 }
 

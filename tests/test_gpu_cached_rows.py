@@ -20,6 +20,7 @@ from oracle import cached_f64
     (37, 4, 2, 2300, 64, True, 0),          # three
     (128, 1, 1, 4100, 128, True, 0),        # four
     (50, 6, 2, 1000, 128, True, 0),         # tiles of a ragged number of rows
+    (30, 12, 12, 1050, 64, True, 0),        # fp32: two rows a thread, fewer CTAs than two per SM
     (9, 4, 4, 3000, 64, True, 100),         # a window: most of the keys are not visited
 ])
 def test_rows_of_a_split_cache_match_the_oracle(T, H, Hkv, L, D, causal, window, dtype):
