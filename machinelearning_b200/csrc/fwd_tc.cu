@@ -781,14 +781,16 @@ int launch_fwd_tc(const Problem& p, const void* q, const void* k, const void* v,
   // second tile's longer row.  Run long enough for the power cap to hold, two tiles win at D <= 64 as soon as K and V no
   // longer fit in L2 (one / two tiles per unit, H=8: T=1024 B=32 72.9 / 73.4 us, B=128 317 / 295; T=4096 B=8 214 / 208,
   // B=32 1,013 / 896) except over rows of two tiles (T=256 B=512 139 / 151); below that one does (B=8 H=12 T=1024
-  // 28.8 / 30.8, B=2 T=4096 79.5 / 82.3) up to rows of 4,096, and where there are no more tiles than SMs.
+  // 28.8 / 30.8, B=2 T=4096 79.5 / 82.3) up to rows of 4,096, and where there are no more tiles than SMs.  Rows of up to
+  // 1,024 waste most on the second tile: there the line is all of L2, not the half next to an SM (H=12 T=1024 B=32, 100 MB,
+  // between backward passes: 101 / 107; alone level; B=64 T=512 H=8 48.8 / 50.7).
   // D = 128 (one CTA per SM either way): one tile while that makes at most two units per SM (B=1 H=8 T=4096:
   // 42.6 / 65.9 us; 3.5 per SM: 45.2 / 41.9).
   const long long tiles = static_cast<long long>(p.B) * p.H * ((p.T + kTile - 1) / kTile);
   const long long kv_bytes = static_cast<long long>(p.B) * p.Hkv * p.T * p.D * 4;
   const int reach = p.window > 0 && p.window < p.T ? p.window : p.T;
   const bool single = p.D == 128 ? tiles <= 2ll * sm_count() || p.T <= kTile
-                                 : (reach <= 4096 && kv_bytes < (64ll << 20)) || p.T <= 2 * kTile || tiles <= sm_count();
+                                 : (reach <= 4096 && kv_bytes < (reach <= 1024 ? 2 : 1) * (64ll << 20)) || p.T <= 2 * kTile || tiles <= sm_count();
   auto go = [&](auto type) {
     using T = decltype(type);
     if (single) {
