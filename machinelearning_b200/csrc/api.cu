@@ -111,9 +111,11 @@ int check_problem(const Problem& p) {
   return NLFA_OK;
 }
 
-// Masks that cut nothing become the plain causal one.
+// Masks that cut nothing become the plain causal one; extents end at T, so that index arithmetic on them (rounding up
+// to tiles, sums of them) stays far from 2^31 whatever the caller gave.
 void simplify_mask(Problem& p) {
-  if (p.window > 0 && p.window - p.sinks >= p.T) p.window = p.sinks = 0;      // the window never cuts anything
+  if (p.window > 0 && (p.window - p.sinks >= p.T || p.sinks >= p.T)) p.window = p.sinks = 0;   // it never cuts anything
+  if (p.block > p.T) p.block = p.T;                                          // one block: every key
   if (p.block == 1) p.block = 0;                                             // blocks of one position
 }
 
@@ -429,7 +431,7 @@ size_t round256(size_t n) { return (n + 255) / 256 * 256; }
 // Bytes of the dS tiles of one (batch, KV head) pair.
 size_t ds_pair_bytes(const Problem& p) {
   const DsLayout l = ds_layout(p.T, p.window, p.sinks, p.block);
-  return static_cast<size_t>(ds_tile_offset(l, l.n_tiles)) * kDsTileBytes * (p.H / p.Hkv);
+  return static_cast<size_t>(ds_tile_offset<long long>(l, l.n_tiles)) * kDsTileBytes * (p.H / p.Hkv);
 }
 
 constexpr size_t kDsMostBytes = size_t{4} << 30;        // dS of as many pairs at a time as fit here

@@ -137,16 +137,20 @@ __host__ __device__ inline int dq_turn_of_block(int block, int tile, int window,
 
 // Where the dK/dV pass leaves dS for the dQ pass (bwd_dq.cu): one 32 KB tile of 16-bit values per
 // (query head, query tile, key block the tile sees), a query tile's blocks side by side in the order
-// of dq_turn_of_block.  Tile `i`'s blocks start at slot ds_tile_offset(i) of its head.
+// of dq_turn_of_block.  Tile `i`'s blocks start at slot ds_tile_offset(i) of its head.  In 64 bits where the host sizes
+// the scratch (the square of the number of tiles leaves 32 bits at T = 5.9 million); a kernel addresses tiles that
+// exist, whose numbers fit an int.
 constexpr int kDsTileBytes = kTile * kTile * 2;
 struct DsLayout {
   int n_tiles;
   int stride;            // > 0 (windows): every query tile has this many slots
   int ahead;             // otherwise: tile i has min(n_tiles, i + 1 + ahead) of them (block-causal: ahead > 0)
 };
-__host__ __device__ inline int ds_tile_offset(const DsLayout& l, int i) {
+template <typename Int = int>
+__host__ __device__ inline Int ds_tile_offset(const DsLayout& l, int tile) {
+  const Int i = tile;
   if (l.stride > 0) return i * l.stride;
-  const int full = l.n_tiles - 1 - l.ahead > 0 ? l.n_tiles - 1 - l.ahead : 0;    // first tile that sees every block
+  const Int full = l.n_tiles - 1 - l.ahead > 0 ? l.n_tiles - 1 - l.ahead : 0;    // first tile that sees every block
   return i <= full ? i * (i + 1) / 2 + i * l.ahead : full * (full + 1) / 2 + full * l.ahead + (i - full) * l.n_tiles;
 }
 inline DsLayout ds_layout(int T, int window, int sinks, int block) {

@@ -146,3 +146,21 @@ def test_backward_kernel_count_follows_the_layout(lib):
     # the large-problem layout (needs the device's SM count on a GPU box; 4,096 x 12 x 8 tiles is large anywhere)
     assert count(4096, 1024, 12, 64, bf16, tensor, _lib.PASS_ALL) == 2
     assert count(4096, 1024, 12, 64, bf16, tensor, _lib.PASS_DELTA | _lib.PASS_DQ) == 1
+
+
+def test_workspace_sizes_of_extreme_extents(lib):
+    """Sizes whose tile arithmetic leaves 32 bits: one pair's dS is beyond the limit, so the tape alone is asked for; a block
+    length or a number of sinks next to 2^31 means what T does."""
+    from machinelearning_b200 import _lib as L
+    size = lambda T, window=0, sinks=0, block=0: lib.nlfa_bwd_workspace_bytes(
+        64, T, 4, 4, 128, window, sinks, block, L.DTYPE_BF16, L.PATH_TENSOR)
+    one = lambda T: lib.nlfa_bwd_workspace_bytes(1, T, 1, 1, 128, 0, 0, 0, L.DTYPE_BF16, L.PATH_TENSOR)
+    for T in (1 << 23, 46341 * 128, 65537 * 128):
+        assert one(T) == lib.nlfa_bwd_scratch_bytes(1, T, 1)
+        assert lib.nlfa_bwd_workspace_kernel_count(1, T, 1, 1, 128, 0, 0, 0, L.DTYPE_BF16, L.PATH_TENSOR, 64 << 30) == 3
+    big = (1 << 31) - 1
+    for T in (1, 300, 4096):
+        causal = size(T)
+        assert T == 1 or causal > lib.nlfa_bwd_scratch_bytes(64, T, 4)
+        assert size(T, block=big) == size(T, block=big - 126) == size(T, block=T)
+        assert size(T, window=big, sinks=big - 1) == size(T, window=big, sinks=T) == causal

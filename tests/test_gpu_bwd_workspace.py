@@ -76,3 +76,16 @@ def test_heads_in_groups_change_nothing(B, T, H, Hkv, window):
     args = (lib, L, do, q, k, v, o, lse, scale, window, 0, 0)
     for a, b in zip(_backward(*args, lib.nlfa_bwd_scratch_bytes(B, T, H)), _backward(*args, whole)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("extreme,same", [(dict(block=(1 << 31) - 1), dict(block=333)),
+                                          (dict(window=(1 << 31) - 1, sinks=(1 << 31) - 2), dict())])
+def test_extents_next_to_two_to_the_31(extreme, same):
+    from machinelearning_b200 import flash_cuda as fc
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, k, v, do = (torch.randn(40, 333, h, 128, device="cuda", generator=g).bfloat16() for h in (4, 2, 2, 4))
+    runs = []
+    for kw in (extreme, same):
+        o, lse = fc.fwd(q, k, v, 0.1, True, **kw)
+        runs.append((o, lse, *fc.bwd(do, q, k, v, o, lse, 0.1, True, **kw)))
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
