@@ -337,6 +337,8 @@ extern "C" int nlfa_fwd_cached_positions(const void* q, const void* k_cache, con
   if (rows == 0) return NLFA_OK;
   if (rows / 4 >= (1ll << 31)) return NLFA_ERR_BAD_SHAPE;
   if (!q || !o || (L > 0 && (!k_cache || !v_cache))) return NLFA_ERR_NULL_POINTER;
+  // a window that cuts nothing of a contiguous cache (and sinks next to 2^31 would overflow when rounded up to blocks)
+  if (window > 0 && qpos == nullptr && kpos == nullptr && (window - sinks >= L || sinks >= L)) window = sinks = 0;
   const CachedParams p{B, Tq, H, Hkv, L, D, causal ? 1 : 0, window, sinks, scale * kLog2e, qpos, kpos, position_bytes == 8,
                        1, o, lse};
   cudaStream_t st = (cudaStream_t)stream;

@@ -37,3 +37,14 @@ def test_rows_of_a_split_cache_match_the_oracle(T, H, Hkv, L, D, causal, window,
     tol = 1e-5 if dtype == torch.float32 else 5e-3 * np.abs(ref).max()
     assert np.abs(n(y) - ref).max() <= tol
     assert np.abs(n(lse) - lse_ref).max() <= (1e-5 if dtype == torch.float32 else 1e-3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32], ids=["fp16", "fp32"])
+def test_sinks_next_to_two_to_the_31(dtype):
+    from machinelearning_b200 import flash_cuda
+    g = torch.Generator().manual_seed(0)
+    q, k, v = (torch.randn(1, *s, 64, generator=g).to("cuda", dtype) for s in ((40, 4), (2, 900), (2, 900)))
+    want = flash_cuda.flash_attn_cached(q, k, v, causal=True)
+    for window, sinks in (((1 << 31) - 1, (1 << 31) - 2), ((1 << 31) - 1, 0), (901, 900)):
+        assert torch.equal(flash_cuda.flash_attn_cached(q, k, v, causal=True, window=window, sinks=sinks), want)
