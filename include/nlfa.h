@@ -290,7 +290,7 @@ int nlfa_fwd_cached(const void* q, const void* k_cache, const void* v_cache, voi
  * nlfa_fwd_cached does, takes the tensor-core kernel (TMA + tcgen05, keys in blocks of 128, the
  * query rows of a KV head's whole group in one tile) for 16-bit inputs with up to 128 query heads per KV
  * head, on a compute-capability 10.x device with 16-byte-aligned pointers and a positive scale;
- * otherwise the fp32 kernel.  Below 16 rows per KV head (Tq x group) or 256 keys the probabilities
+ * otherwise the fp32 kernel, for which K and V must be 16-byte aligned (NLFA_ERR_MISALIGNED) but q and o need not be.  Below 16 rows per KV head (Tq x group) or 256 keys the probabilities
  * enter the product as two 16-bit values each, so that such blocks get fp32-kernel precision.
  * TENSOR returns NLFA_ERR_UNSUPPORTED_PATH below those sizes or when those conditions do not hold. */
 int nlfa_fwd_cached_path(const void* q, const void* k_cache, const void* v_cache, void* o, float* lse,

@@ -82,7 +82,7 @@ __device__ __forceinline__ void merge_rows(const CachedParams& p, int n, RowOf o
       for (int x = 0; x < kBatch; ++x)
         acc = make_float4(fmaf(f[x], y[x].x, acc.x), fmaf(f[x], y[x].y, acc.y), fmaf(f[x], y[x].z, acc.z), fmaf(f[x], y[x].w, acc.w));
     }
-    cached::store4(static_cast<T*>(p.o) + out_row(r) * D + c, acc);
+    cached::store4(static_cast<T*>(p.o) + out_row(r) * D + c, acc, p.loose);
   }
 }
 
@@ -119,7 +119,7 @@ fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r < rows) {
       const T* src = q + out_row(r) * D + c;
-      if constexpr (sizeof(T) == 4) x = *reinterpret_cast<const float4*>(src);
+      if (sizeof(T) == 4 && !p.loose) x = *reinterpret_cast<const float4*>(src);
       else x = make_float4(to_f32(src[0]), to_f32(src[1]), to_f32(src[2]), to_f32(src[3]));
     }
     *reinterpret_cast<float4*>(qs + r * kPitch + c) = x;
@@ -210,7 +210,14 @@ fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__
     }
     const long long row = out_row(r);
     const float inv = sum > 0.f ? 1.f / sum : 0.f;         // a row that sees no key gives zeros
-    store_row<T, D>(static_cast<T*>(p.o) + row * D, col, acc[i], inv);
+    T* out = static_cast<T*>(p.o) + row * D;
+    if (!p.loose) {
+      store_row<T, D>(out, col, acc[i], inv);
+    } else {
+      constexpr int kRun = D == 32 ? 2 : 4;                // columns of a thread that stand together (store_row)
+#pragma unroll
+      for (int n = 0; n < D / 16; ++n) out[64 * (n / 4) + kRun * col + n % 4] = from_f32<T>(acc[i][n] * inv);
+    }
     if (p.lse && col == 0) {
       const long long t = (row / p.H) % p.Tq, h = row % p.H;
       p.lse[(static_cast<long long>(b) * p.H + h) * p.Tq + t] = sum > 0.f ? (m[i] + log2f(sum)) * kLn2 : -INFINITY;
@@ -339,16 +346,17 @@ extern "C" int nlfa_fwd_cached_positions(const void* q, const void* k_cache, con
   if (!q || !o || (L > 0 && (!k_cache || !v_cache))) return NLFA_ERR_NULL_POINTER;
   // a window that cuts nothing of a contiguous cache (and sinks next to 2^31 would overflow when rounded up to blocks)
   if (window > 0 && qpos == nullptr && kpos == nullptr && (window - sinks >= L || sinks >= L)) window = sinks = 0;
-  const CachedParams p{B, Tq, H, Hkv, L, D, causal ? 1 : 0, window, sinks, scale * kLog2e, qpos, kpos, position_bytes == 8,
-                       1, o, lse};
+  CachedParams p{B, Tq, H, Hkv, L, D, causal ? 1 : 0, window, sinks, scale * kLog2e, qpos, kpos, position_bytes == 8,
+                       1, o, lse, 0};
   cudaStream_t st = (cudaStream_t)stream;
-  const bool aligned = ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_cache) |
-                         reinterpret_cast<uintptr_t>(v_cache) | reinterpret_cast<uintptr_t>(o)) & 15u) == 0;
+  auto off = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15u) != 0; };
+  const bool kv_aligned = L == 0 || !(off(k_cache) || off(v_cache));
+  p.loose = off(q) || off(o);
   // 16-bit inputs: the products run on the tensor cores, whatever the block's size, because the cache's
   // bandwidth is what counts.  Blocks a caller cannot force onto them (fewer than 16 rows per KV head, or under
   // 256 keys) keep the fp32 kernel's precision there (SPLIT_P).
   const bool applies = cached_tc_applies(Tq, H, Hkv, L, D, dtype);
-  if (aligned && L > 0 && scale > 0.f && nlfa_device_supported() &&
+  if (kv_aligned && !p.loose && L > 0 && scale > 0.f && nlfa_device_supported() &&
       (path == NLFA_PATH_TENSOR ? applies : path == NLFA_PATH_AUTO && cached_tc_can(H, Hkv, D, dtype))) {
     if (nlfa_peek_status() != NLFA_OK) return NLFA_ERR_DEVICE_TIMEOUT;
     unsigned* status = status_block();
@@ -356,6 +364,7 @@ extern "C" int nlfa_fwd_cached_positions(const void* q, const void* k_cache, con
     return launch_fwd_cached_tc(p, q, k_cache, v_cache, dtype, !applies, status, st);
   }
   if (path == NLFA_PATH_TENSOR) return NLFA_ERR_UNSUPPORTED_PATH;
+  if (!kv_aligned) return NLFA_ERR_MISALIGNED;             // K and V come by 16-byte copies in this kernel, too
   if (dtype == NLFA_DTYPE_BF16) return launch_simt<__nv_bfloat16>(p, q, k_cache, v_cache, st);
   if (dtype == NLFA_DTYPE_F16) return launch_simt<__half>(p, q, k_cache, v_cache, st);
   return launch_simt<float>(p, q, k_cache, v_cache, st);

@@ -18,6 +18,7 @@ struct CachedParams {
   int splits;            // CTAs per query tile (blockIdx.y, one cluster): each takes a share of the key blocks
   void* o;
   float* lse;            // or nullptr
+  int loose;             // q or o is not 16-byte aligned (fp32 kernel only): one element at a time
 };
 
 // A position as the kernels use it; 64-bit ones are clamped into 32 bits (they are compared, and with a window
@@ -73,7 +74,13 @@ __device__ __forceinline__ bool all_visible(const CachedParams& p, int kp_min, i
 }
 
 template <typename T>
-__device__ __forceinline__ void store4(T* dst, float4 v) {
+__device__ __forceinline__ void store4(T* dst, float4 v, bool loose = false) {
+  if (loose) {
+    const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dst[i] = static_cast<T>(x[i]);
+    return;
+  }
   if constexpr (sizeof(T) == 4) {
     *reinterpret_cast<float4*>(dst) = v;
   } else {

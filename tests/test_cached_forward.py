@@ -54,6 +54,39 @@ def test_entry_point_refuses_bad_arguments_before_any_launch():
     assert sb(1, 64, 16, 16, 16448, 128) == 64 * 16 * 3 * 129 * 4      # three splits of a long cache
 
 
+def test_misaligned_keys_and_values_are_refused_before_any_launch():
+    """The fp32 kernel copies K and V 16 bytes at a time, so a base that is not 16-byte aligned is status 6, as in the
+    other entry points; forcing the tensor cores on any misaligned pointer stays status 7."""
+    from machinelearning_b200 import _build, _lib
+    _build.build()
+    f = _lib.load().nlfa_fwd_cached_path
+    call = lambda q=16, k=16, v=16, o=16, dtype=_lib.DTYPE_F32, path=_lib.PATH_AUTO: f(
+        q, k, v, o, None, None, None, 1, 4, 4, 2, 8, 64, 0.125, 1, 0, 0, dtype, path, None, 0, None)
+    for dtype in (_lib.DTYPE_F32, _lib.DTYPE_F16, _lib.DTYPE_BF16):
+        for path in (_lib.PATH_AUTO, _lib.PATH_SIMT):
+            assert call(k=24, dtype=dtype, path=path) == 6 and call(v=20, dtype=dtype, path=path) == 6
+        for pointer in ("q", "k", "v", "o"):
+            assert call(**{pointer: 24}, dtype=dtype, path=_lib.PATH_TENSOR) == 7
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["fp32", "bf16"])
+@pytest.mark.parametrize("T,L,D", [(3, 70, 32), (20, 900, 64), (40, 2100, 128)])       # unsplit, and split over a cluster
+def test_queries_and_outputs_off_the_16_byte_grid(T, L, D, dtype):
+    from machinelearning_b200 import _lib, flash_cuda
+    g = torch.Generator(device="cuda").manual_seed(T)
+    mk = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)
+    q, k, v = mk(1, T, 4, D), mk(1, 2, L, D), mk(1, 2, L, D)
+    want = flash_cuda.flash_attn_cached(q, k, v, causal=True, use_mma=False)
+    shifted = lambda t: torch.empty(t.numel() + 8, dtype=dtype, device="cuda")[1:1 + t.numel()].view(t.shape)
+    q1, o1 = shifted(q).copy_(q), shifted(q).zero_()
+    assert torch.equal(flash_cuda.flash_attn_cached(q1, k, v, causal=True, use_mma=False), want)
+    st = _lib.load().nlfa_fwd_cached_path(
+        q1.data_ptr(), k.data_ptr(), v.data_ptr(), o1.data_ptr(), None, None, None, 1, T, 4, 2, L, D, D ** -0.5, 1, 0, 0,
+        flash_cuda._DTYPE_CODE[dtype], _lib.PATH_AUTO, None, 0, torch.cuda.current_stream().cuda_stream)
+    assert st == 0 and torch.equal(o1, want)
+
+
 def test_python_wrapper_rejects_cpu_tensors_and_bidirectional_windows():
     from machinelearning_b200 import flash_cuda
     q, k = torch.zeros(1, 4, 2, 64), torch.zeros(1, 1, 8, 64)
