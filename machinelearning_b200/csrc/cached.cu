@@ -76,6 +76,7 @@ __device__ __forceinline__ void merge_rows(const CachedParams& p, int n, RowOf o
         int s = is ? s0 + x + rank : rank;
         s = s < splits ? s : s - splits;
         y[x] = ld_cluster_f4(cluster_addr(at, s));
+        if (!is) y[x] = make_float4(0.f, 0.f, 0.f, 0.f);                          // (0 times an infinity would be NaN)
         f[x] = is ? weights[32 * k + s] : 0.f;
       }
 #pragma unroll
@@ -168,10 +169,12 @@ fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__
 #pragma unroll
     for (int i = 0; i < RM; ++i) {
       float mx = m[i];
+      bool seen[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         s[i][j] *= p.scale_log2;
-        if (!full && !(in[j] && cached::position_visible(p, qp[i], kp[j]))) s[i][j] = -INFINITY;
+        seen[j] = full || (in[j] && cached::position_visible(p, qp[i], kp[j]));
+        if (!seen[j]) s[i][j] = -INFINITY;
         mx = fmaxf(mx, s[i][j]);
       }
 #pragma unroll
@@ -182,7 +185,7 @@ fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__
       l[i] *= alpha;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float e = exp2f(s[i][j] - ref);
+        const float e = seen[j] ? exp2f(s[i][j] - ref) : kHidden;
         l[i] += e;
         ps[(grp + 8 * i) * kPPitch + col + 16 * j] = e;
       }
@@ -190,8 +193,9 @@ fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__
       for (int x = 0; x < D / 16; ++x) acc[i][x] *= alpha;
     }
     load_wait<1>();
-    __syncthreads();                                       // V is there (and this warp's probabilities)
-    output_product<D, RM>(ps, vs, grp, col, acc);
+    // V is there (and this warp's probabilities)
+    const bool guard = __syncthreads_or(!full && !own_rows_finite<T, D>(vs, kBN)) != 0;
+    output_product<D, RM>(ps, vs, grp, col, acc, guard);
     __syncthreads();
     if (n + 1 < n_stop) load_kv(vs, vb, n + 1);
     else load_commit();

@@ -97,13 +97,14 @@ fwd_tile_kernel(Problem p, const T* __restrict__ q, const T* __restrict__ k, con
     for (int i = 0; i < RM; ++i) {
       const int qpos = q0 + grp + 8 * i;
       float mx = m[i];
+      bool seen[4] = {true, true, true, true};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         s[i][j] *= scale2;
         if (!full) {
           const int kp = k0 + col + 16 * j;
-          const bool vis = kp <= qlim[i] && (p.window == 0 || kp > qpos - (p.window - p.sinks) || kp < p.sinks);
-          s[i][j] = vis ? s[i][j] : -INFINITY;
+          seen[j] = kp <= qlim[i] && (p.window == 0 || kp > qpos - (p.window - p.sinks) || kp < p.sinks);
+          s[i][j] = seen[j] ? s[i][j] : -INFINITY;
         }
         mx = fmaxf(mx, s[i][j]);
       }
@@ -115,7 +116,7 @@ fwd_tile_kernel(Problem p, const T* __restrict__ q, const T* __restrict__ k, con
       l[i] *= alpha;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float e = exp2f(s[i][j] - ref);
+        const float e = seen[j] ? exp2f(s[i][j] - ref) : kHidden;
         l[i] += e;
         ps[(grp + 8 * i) * kPPitch + col + 16 * j] = e;
       }
@@ -123,8 +124,9 @@ fwd_tile_kernel(Problem p, const T* __restrict__ q, const T* __restrict__ k, con
       for (int n = 0; n < D / 16; ++n) acc[i][n] *= alpha;
     }
     load_wait<1>();
-    __syncthreads();                                   // V is there (and this warp's probabilities)
-    output_product<D, RM>(ps, vs, grp, col, acc);
+    // V is there (and this warp's probabilities)
+    const bool guard = __syncthreads_or(!full && !own_rows_finite<T, D>(vs, kBN)) != 0;
+    output_product<D, RM>(ps, vs, grp, col, acc, guard);
     __syncthreads();
     if (it + 1 < blocks.count) load_kv(vs, vb, blocks.at(it + 1));
     else load_commit();
@@ -241,15 +243,16 @@ bwd_tile_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q, 
       __syncthreads();
       load_y(it);
     }
-    load_wait<0>();
-    __syncthreads();
-    if (NB == 2 && it + 1 < n_iters) load_y(it + 1);             // its buffer was last read before the barrier
     const float* y0s = ys + (it % NB) * 2 * kBN * kPitch;
     const float* y1s = y0s + kBN * kPitch;
     const float* w = vec + (it % NB) * 2 * kBN;
     const int c0 = (DKV ? y_first + it % n_inner : blocks.at(it)) * kBN;
     const bool full = DKV ? c0 + kBN <= p.T && rect_fully_visible(c0, c0 + kBN - 1, r0, r0 + BM - 1, p.window, p.sinks, p.block, p.T)
                           : rect_fully_visible(r0, r0 + BM - 1, c0, c0 + kBN - 1, p.window, p.sinks, p.block, p.T);
+    load_wait<0>();
+    const bool guard = __syncthreads_or(!full && !(own_rows_finite<T, D>(y0s, kBN) &&
+                                                   (!DKV || own_rows_finite<T, D>(y1s, kBN)))) != 0;
+    if (NB == 2 && it + 1 < n_iters) load_y(it + 1);             // its buffer was last read before the barrier
     float s[RM][4], ds[RM][4];
     score_product<D, RM>(x0, y0s, grp, col, s);
     score_product<D, RM>(x1, y1s, grp, col, ds);
@@ -260,15 +263,16 @@ bwd_tile_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q, 
       for (int j = 0; j < 4; ++j) {
         const int c = c0 + col + 16 * j;
         const float ref = DKV ? w[col + 16 * j] : l2[i], dlt = DKV ? w[kBN + col + 16 * j] : dl[i];
-        float e = exp2f(fmaf(s[i][j], scale2, -ref));
+        float e = exp2f(fmaf(s[i][j], scale2, -ref)), de = e * (ds[i][j] - dlt) * p.scale;
         if (!full) {
           const int qp = DKV ? c : r, kp = DKV ? r : c;
           const bool vis = (DKV ? c >= edge[i] && c < p.T : c <= edge[i]) &&
                            (p.window == 0 || kp > qp - (p.window - p.sinks) || kp < p.sinks);
-          e = vis ? e : 0.f;
+          e = vis ? e : kHidden;
+          de = vis ? de + 0.f : kHidden;                         // (a visible -0 becomes +0)
         }
         s[i][j] = e;
-        ds[i][j] = e * (ds[i][j] - dlt) * p.scale;
+        ds[i][j] = de;
       }
     }
     auto hand_over = [&](const float (&x)[RM][4]) {              // within this warp's rows
@@ -281,10 +285,10 @@ bwd_tile_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q, 
     };
     if constexpr (DKV) {
       hand_over(s);
-      output_product<D, RM>(ws, y1s, grp, col, acc1);
+      output_product<D, RM>(ws, y1s, grp, col, acc1, guard);
     }
     hand_over(ds);
-    output_product<D, RM>(ws, y0s, grp, col, acc0);
+    output_product<D, RM>(ws, y0s, grp, col, acc0, guard);
   }
 #pragma unroll
   for (int i = 0; i < RM; ++i) {

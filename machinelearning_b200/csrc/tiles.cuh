@@ -72,6 +72,26 @@ __device__ __forceinline__ void load_commit() { asm volatile("cp.async.commit_gr
 template <int N>
 __device__ __forceinline__ void load_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// Pairs the mask hides must not touch an output, whatever stands in the hidden rows: a weight of zero does not do where
+// the other factor is infinite or NaN.  Hidden weights are therefore written as -0 (a visible one never is: kHidden),
+// and when a tile of a cut block holds such a value the output product leaves them out one by one (GUARD).  A
+// thread looks through what it loaded itself, so the check needs no barrier of its own: cut blocks only, a few per cent.
+constexpr float kHidden = -0.f;
+template <typename T, int D>
+__device__ __forceinline__ bool own_rows_finite(const float* tile, int rows) {
+  constexpr int kPitch = D + 4, V = sizeof(T) == 4 ? D / 4 : D / 8;                // as load_rows shares them out
+  float z = 0.f;
+  for (int i = threadIdx.x; i < rows * V; i += kThreads) {
+    const float* p = tile + (i / V) * kPitch + (D / V) * (i % V);
+#pragma unroll
+    for (int c = 0; c < D / V; c += 4) {
+      const float4 x = ld4(p + c);
+      z = fmaf(x.x, 0.f, fmaf(x.y, 0.f, fmaf(x.z, 0.f, fmaf(x.w, 0.f, z))));       // NaN once anything is not finite
+    }
+  }
+  return z == z;
+}
+
 // s[i][j] = row (grp + 8 i) of A . row (col + 16 j) of B
 template <int D, int RM>
 __device__ __forceinline__ void score_product(const float* a, const float* b, int grp, int col, float (&s)[RM][4]) {
@@ -98,8 +118,8 @@ __device__ __forceinline__ void score_product(const float* a, const float* b, in
 }
 
 // acc[i][.] += row (grp + 8 i) of the [rows][kBN] tile w times B [kBN][D]; a thread's D / 16 columns are 4 col ..
-// (per 64 columns), or 2 col .. at D = 32
-template <int D, int RM>
+// (per 64 columns), or 2 col .. at D = 32; `guard`: see kHidden
+template <int D, int RM, bool GUARD = false>
 __device__ __forceinline__ void output_product(const float* w, const float* b, int grp, int col, float (&acc)[RM][D / 16]) {
   constexpr int kPitch = D + 4;
   const float* wp = w + grp * kPPitch;
@@ -128,9 +148,17 @@ __device__ __forceinline__ void output_product(const float* w, const float* b, i
 #pragma unroll
       for (int i = 0; i < RM; ++i)
 #pragma unroll
-        for (int n = 0; n < D / 16; ++n) acc[i][n] = fmaf(wv[i][x], bv[n], acc[i][n]);
+        for (int n = 0; n < D / 16; ++n)
+          if (!GUARD || __float_as_uint(wv[i][x]) != __float_as_uint(kHidden)) acc[i][n] = fmaf(wv[i][x], bv[n], acc[i][n]);
     }
   }
+}
+
+template <int D, int RM>
+__device__ __forceinline__ void output_product(const float* w, const float* b, int grp, int col, float (&acc)[RM][D / 16],
+                                               bool guard) {
+  if (guard) output_product<D, RM, true>(w, b, grp, col, acc);
+  else output_product<D, RM, false>(w, b, grp, col, acc);
 }
 
 // one thread's D / 16 columns of an output row, times `mul`
