@@ -29,10 +29,15 @@
 //
 // SPLIT_P: blocks so small that the fp32 kernel used to take them keep its precision: P goes in as the sum of two
 // 16-bit values (its rounding error is then below the accumulator's), at the price of a second P V product,
-// which the loads hide.
+// which the loads hide.  It also keeps what that kernel does with infinities and NaN in V.  Of a key the mask hides they
+// reach no row: warps 10 and 11 go over the V tiles of blocks the mask cuts before the product reads them and put zeros for the
+// rows no query sees and for values that are not finite.  An infinity that a row does see stays one: what was replaced, and
+// what the product made NaN (zero times an infinity: the other copies' columns, a second part that is zero), is
+// put right at the end by a walk over the cache that only then happens.  Blocks the mask leaves whole cost nothing (going
+// over every tile: B=1 H=16 D=128, 1 query over 16,385, 30.5 -> 44.9 us).
 //
-// Warps 0-3 and 4-7 softmax, 8 TMA producer, 9 MMA issuer and TMEM owner, 10-11 idle (they complete the
-// warpgroup that gives its registers to the softmax warps).  Every wait bounded.
+// Warps 0-3 and 4-7 softmax, 8 TMA producer, 9 MMA issuer and TMEM owner, 10-11 idle or (SPLIT_P) looking through V; they
+// complete the warpgroup that gives its registers to the softmax warps.  Every wait bounded.
 #include <climits>
 
 #include "cached.cuh"
@@ -48,6 +53,7 @@ constexpr int kNoKey = INT_MAX;          // position written for keys past the e
 struct TileParams {
   int group, tq_tile, n_qtiles;          // query heads per KV head; block positions per CTA; tiles per (b, hk)
   unsigned* status;
+  const void* v;
 };
 
 template <int D, int STAGES, int COPIES>
@@ -66,11 +72,12 @@ struct CachedSmem {
   static constexpr int kReceived = kK + (COPIES == 1 ? 128 : 256) * kPitch;
   static constexpr int kPartStep = kTile / COPIES * kPitch, kSplitPartStep = COPIES == 1 ? 0 : kPartStep;
   static constexpr int kBar = kFull + (STAGES * 4 + 15) / 16 * 16;
-  // barriers: q_full, s_full[2], p_full[2], o_done, group, received, k_full[S], k_empty[S], v_full[S], v_empty[S]
-  static constexpr int kNumBars = 8 + 4 * STAGES;
+  // barriers: q_full, s_full[2], p_full[2], o_done, group, received, k_full[S], k_empty[S], v_full[S], v_empty[S], v_clean[S], scanned
+  static constexpr int kNumBars = 9 + 5 * STAGES;
   static constexpr int kTmemSlot = kBar + 8 * kNumBars;
   static constexpr int kAbort = kTmemSlot + 4;
-  static constexpr int kTotal = kAbort + 4;
+  static constexpr int kSpoilt = kAbort + 4;                     // V held a value that is not finite
+  static constexpr int kTotal = kSpoilt + 4;
   static constexpr int kDynamic = kTotal + 1024;
   static_assert(STAGES * 2 * kTileBytes >= kReceived + (kTile / COPIES + kMostCluster) * kPitch && STAGES * 2 * kTileBytes >= 256 * kPitch, "the combination lies over dead tiles");
 };
@@ -95,14 +102,17 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
   auto bar = [&](int i) -> uint32_t { return base + L::kBar + 8u * i; };
   constexpr int Q_FULL = 0, S_FULL = 1, P_FULL = 3, O_DONE = 5, GROUP = 6, RECEIVED = 7, K_FULL = 8,
-                K_EMPTY = K_FULL + STAGES, V_FULL = K_EMPTY + STAGES, V_EMPTY = V_FULL + STAGES;
+                K_EMPTY = K_FULL + STAGES, V_FULL = K_EMPTY + STAGES, V_EMPTY = V_FULL + STAGES, V_CLEAN = V_EMPTY + STAGES,
+                SCANNED = V_CLEAN + STAGES;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + L::kAbort);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L::kTmemSlot);
+  volatile int* spoilt_flag = reinterpret_cast<volatile int*>(gen + L::kSpoilt);
   volatile int* full_flag = reinterpret_cast<volatile int*>(gen + L::kFull);
   const WaitCtx wctx{abort_flag, tp.status};
 
   if (threadIdx.x == 0) {
     *abort_flag = (*reinterpret_cast<volatile unsigned*>(tp.status) != STATUS_OK) ? 1 : 0;
+    *spoilt_flag = 0;
     mbar_init(bar(Q_FULL), 1);
     for (int w = 0; w < 2; ++w) {
       mbar_init(bar(S_FULL + w), 1);
@@ -111,11 +121,13 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     mbar_init(bar(O_DONE), 1);
     mbar_init(bar(GROUP), 256);
     mbar_init(bar(RECEIVED), 1);
+    mbar_init(bar(SCANNED), 2);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(bar(K_FULL + s), 1);
       mbar_init(bar(K_EMPTY + s), 1);
       mbar_init(bar(V_FULL + s), 1);
       mbar_init(bar(V_EMPTY + s), 1);
+      mbar_init(bar(V_CLEAN + s), 2);
     }
     fence_mbar_init();
   }
@@ -153,14 +165,75 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tma_prefetch_desc(&tm_v);
   }
 
+  // the tile's query positions, as a range (every lane of a warp)
+  auto tile_positions = [&](int& qp_min, int& qp_max) {
+    if (!p.qpos) {
+      qp_min = p.L - p.Tq + t0;
+      qp_max = p.L - p.Tq + t1;
+      return;
+    }
+    qp_min = INT_MAX;
+    qp_max = -INT_MAX;
+    for (int t = t0 + lane; t <= t1; t += 32) {
+      const int x = cached::query_position(p, t);
+      qp_min = x < qp_min ? x : qp_min;
+      qp_max = x > qp_max ? x : qp_max;
+    }
+    qp_min = __reduce_min_sync(0xffffffffu, qp_min);
+    qp_max = __reduce_max_sync(0xffffffffu, qp_max);
+  };
+
   grid_dep_wait();
   grid_dep_release();
 
   if (warp >= 8) {
     setmaxnreg_dec<kRegsOther>();
     static_assert((kRegsLaunch - kRegsOther) * 4 >= (kRegsCompute - kRegsLaunch) * 8, "register reallocation does not balance");
-    if (dead || warp >= 10) {
+    if (dead || (!SPLIT_P && warp >= 10)) {
       // a give-up recorded earlier makes this launch a no-op; spare warps
+    } else if (warp >= 10) {
+      // ============ V of blocks the mask cuts: no hidden infinities and NaN ====
+      int qp_min, qp_max;
+      tile_positions(qp_min, qp_max);
+      for (int i = 0; i < n_blocks; ++i) {
+        const int s = i % STAGES;
+        const uint32_t ph = (i / STAGES) & 1;
+        if (!__all_sync(0xffffffffu, mbar_wait(bar(K_FULL + s), ph, wctx, 71))) break;      // the block's positions
+        if (full_flag[s] == 0) {
+          if (!__all_sync(0xffffffffu, mbar_wait(bar(V_FULL + s), ph, wctx, 72))) break;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const int r = 64 * (warp - 10) + 32 * half + lane;
+            const int kp = *reinterpret_cast<const int*>(gen + L::kPos + s * 512 + 4 * r);
+            if (kp == kNoKey) continue;                                      // past the end: zeros already
+            const bool shown = (!p.causal || kp <= qp_max) &&                // to some query, perhaps
+                               (p.window == 0 || kp > qp_min - (p.window - p.sinks) || kp < p.sinks);
+            uint4* tile_row = reinterpret_cast<uint4*>(gen + L::kV + s * L::kTileBytes + r * 128);
+#pragma unroll
+            for (int x = 0; x < kBoxes; ++x) {
+              uint4* piece = tile_row + x * (kBoxBytes / 16);                // [8], met in another order by each lane: banks
+              if (!shown) {
+#pragma unroll
+                for (int n = 0; n < 8; ++n) piece[n ^ (lane & 7)] = make_uint4(0u, 0u, 0u, 0u);
+                continue;
+              }
+              bool finite = true;
+#pragma unroll
+              for (int n = 0; n < 8; ++n) finite &= Pack2<T>::finite(piece[n ^ (lane & 7)]);
+              if (finite) continue;
+              *spoilt_flag = 1;
+              T* e = reinterpret_cast<T*>(piece);
+              for (int c = 0; c < 64; ++c)
+                if (!isfinite(static_cast<float>(e[c]))) e[c] = static_cast<T>(0.f);
+            }
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+        }
+        if (lane == 0) mbar_arrive(bar(V_CLEAN + s));
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(SCANNED));                  // the flag is final
     } else if (warp == 8) {
       // =============================== TMA producer ============================
       if (lane == 0) {
@@ -168,20 +241,8 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         for (int x = 0; x < COPIES * kBoxes; ++x)
           tma_load_4d(base + L::kQ + x / COPIES * kBoxBytes + x % COPIES * kLanes * 128, &tm_q, bar(Q_FULL), 64 * (x / COPIES), hk * tp.group, t0, b);
       }
-      // the tile's query positions, as a range
-      int qp_min = INT_MAX, qp_max = -INT_MAX;
-      if (p.qpos) {
-        for (int t = t0 + lane; t <= t1; t += 32) {
-          const int x = cached::query_position(p, t);
-          qp_min = x < qp_min ? x : qp_min;
-          qp_max = x > qp_max ? x : qp_max;
-        }
-        qp_min = __reduce_min_sync(0xffffffffu, qp_min);
-        qp_max = __reduce_max_sync(0xffffffffu, qp_max);
-      } else {
-        qp_min = p.L - p.Tq + t0;
-        qp_max = p.L - p.Tq + t1;
-      }
+      int qp_min, qp_max;
+      tile_positions(qp_min, qp_max);
       bool ok = true;
       for (int i = 0; ok && i < n_blocks; ++i) {
         const int j = range.at(n_begin + i);
@@ -254,6 +315,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const int s = i % STAGES, w = i & 1;
         if (!(ok = wait_all(bar(P_FULL + w), (i >> 1) & 1, 64))) return;
         if (!(ok = wait_all(bar(V_FULL + s), (i / STAGES) & 1, 65))) return;
+        if (SPLIT_P && !(ok = wait_all(bar(V_CLEAN + s), (i / STAGES) & 1, 68))) return;
         tc_fence_after();
         const uint32_t va = base + L::kV + s * L::kTileBytes;
 #pragma unroll
@@ -452,6 +514,10 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const bool met = mbar_wait(bar(GROUP), parity, wctx, 69);
       ok = __all_sync(0xffffffffu, ok && met && *abort_flag == 0);
     };
+    if constexpr (SPLIT_P) {
+      const bool met = mbar_wait(bar(SCANNED), 0, wctx, 72);
+      ok = __all_sync(0xffffffffu, ok && met);
+    }
     group_sync(0);
     if (ok && split && warp_rows) {
       float2 ml[kParts];
@@ -468,7 +534,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         sum = fmaf(ml[x].x, ml[x].y, sum);
         f_mine = x == part ? ml[x].x : f_mine;
       }
-      if (part == 0) *reinterpret_cast<float2*>(first + D + 4) = make_float2(mx, sum);
+      if (part == 0) *reinterpret_cast<float4*>(first + D + 4) = make_float4(mx, sum, *spoilt_flag ? 1.f : 0.f, 0.f);
 #pragma unroll
       for (int c = 0; c < kSlice; c += 8) {
         uint32_t orr[8];
@@ -516,8 +582,10 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const float ref = mx == -INFINITY ? 0.f : mx;
       float sum = 0.f;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      bool odd = SPLIT_P && !split && *spoilt_flag != 0;                     // values were taken out of V
 #pragma unroll 4
       for (int s = 0; s < count; ++s) {
+        if (SPLIT_P && split) odd |= stats[s * stat_stride + 2] != 0.f;
         const float2 ml = *reinterpret_cast<const float2*>(stats + s * stat_stride);
         const float4 y = *reinterpret_cast<const float4*>(at + s * stride + c);
         const float f = exp2f(ml.x - ref);                                   // a part that saw no key: 0 (of zeros)
@@ -527,8 +595,26 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const int t = t0 + r / tp.group, h = hk * tp.group + r % tp.group;
       if (c < p.D) {                                                         // head dim 32 on 64-wide tiles
         const float inv = sum > 0.f ? 1.f / sum : 0.f;                       // a row that sees no key gives zeros
-        cached::store4(static_cast<T*>(p.o) + ((static_cast<long long>(b) * p.Tq + t) * p.H + h) * p.D + c,
-                       make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+        acc = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+        if constexpr (SPLIT_P) {
+          // (a row whose own sum is NaN stays NaN)
+          if (sum > 0.f && (odd || isnan((acc.x + acc.y) + (acc.z + acc.w)))) {
+            const T* vr = static_cast<const T*>(tp.v) + (static_cast<long long>(b) * p.Hkv + hk) * p.L * p.D + c;
+            const int q_at = cached::query_position(p, t);
+            float x[4] = {0.f, 0.f, 0.f, 0.f};                               // what the row sees that is not finite
+            for (int key = 0; key < p.L; ++key, vr += p.D) {
+              if (!cached::position_visible(p, q_at, cached::key_position(p, key))) continue;
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float y = static_cast<float>(vr[e]);
+                if (!isfinite(y)) x[e] += y;
+              }
+            }
+            acc = make_float4(x[0] != 0.f ? x[0] : acc.x, x[1] != 0.f ? x[1] : acc.y, x[2] != 0.f ? x[2] : acc.z,
+                              x[3] != 0.f ? x[3] : acc.w);
+          }
+        }
+        cached::store4(static_cast<T*>(p.o) + ((static_cast<long long>(b) * p.Tq + t) * p.H + h) * p.D + c, acc);
       }
       if (p.lse && c == 0)
         p.lse[(static_cast<long long>(b) * p.H + h) * p.Tq + t] = sum > 0.f ? (mx + log2f(sum)) * kLn2 : -INFINITY;
@@ -623,6 +709,7 @@ int launch_fwd_cached_tc(CachedParams p, const void* q, const void* k_cache, con
   tp.tq_tile = positions_per_tile(p.Tq, tp.group);
   tp.n_qtiles = (p.Tq + tp.tq_tile - 1) / tp.tq_tile;
   tp.status = status;
+  tp.v = v_cache;
   int n_blocks = 0;                                         // key blocks of the tile that sees the most
   for (int qt = 0; qt < tp.n_qtiles; ++qt) {
     const int t0 = qt * tp.tq_tile, t1 = (t0 + tp.tq_tile < p.Tq ? t0 + tp.tq_tile : p.Tq) - 1;

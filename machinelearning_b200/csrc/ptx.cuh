@@ -477,6 +477,13 @@ struct Pack2<__nv_bfloat16> {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
   }
+  // none of the eight is infinite or NaN (0 times it would be NaN)
+  __device__ static __forceinline__ bool finite(const uint4& x) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&x);
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+    const __nv_bfloat162 z = __hfma2(h[0], zero, __hfma2(h[1], zero, __hfma2(h[2], zero, __hmul2(h[3], zero))));
+    return __hbeq2(z, z);
+  }
 };
 template <>
 struct Pack2<__half> {
@@ -484,6 +491,12 @@ struct Pack2<__half> {
   __device__ static __forceinline__ uint32_t pack(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
+  }
+  __device__ static __forceinline__ bool finite(const uint4& x) {
+    const __half2* h = reinterpret_cast<const __half2*>(&x);
+    const __half2 zero = __floats2half2_rn(0.f, 0.f);
+    const __half2 z = __hfma2(h[0], zero, __hfma2(h[1], zero, __hfma2(h[2], zero, __hmul2(h[3], zero))));
+    return __hbeq2(z, z);
   }
 };
 

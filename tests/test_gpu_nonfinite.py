@@ -1,5 +1,5 @@
 """What the mask hides does not reach a row, whatever stands there: infinities and NaN in hidden rows of K, V, Q and dO
-leave the visible pairs' results as they are, bit for bit, in the fp32 kernels."""
+leave the visible pairs' results as they are, bit for bit, in the fp32 kernels and the small cached blocks."""
 import pytest
 import torch
 
@@ -44,7 +44,7 @@ def test_hidden_rows_of_the_fp32_kernels(B, T, H, Hkv, D, window, sinks, block, 
         assert torch.equal(a[:, m:], b[:, m:]) and not torch.isfinite(b[:, :m].float()).all()
 
 
-@pytest.mark.parametrize("dtype", [torch.float32], ids=["fp32"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16], ids=["fp32", "fp16", "bf16"])
 @pytest.mark.parametrize("B,T,H,Hkv,L,D", [(1, 1, 4, 2, 300, 64), (2, 5, 2, 2, 90, 128), (1, 12, 4, 4, 2100, 64),
                                            (1, 60, 4, 2, 200, 32), (1, 9, 2, 2, 1500, 128), (1, 100, 2, 2, 250, 128)])
 def test_hidden_rows_of_a_cache(B, T, H, Hkv, L, D, dtype):
