@@ -161,7 +161,7 @@ fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__
                       cached::all_visible(p, k0, k0 + kBN - 1, p.L - p.Tq + t0, p.L - p.Tq + t1);
     load_wait<1>();
     __syncthreads();                                       // K (and Q) are there; V may be on its way
-    float s[RM][4];
+    float s[RM][4], alpha[RM];
     score_product<D, RM>(qs, ks, grp, col, s);
     __syncthreads();
     if (n + 1 < n_stop) load_kv(ks, kb, n + 1);
@@ -172,30 +172,26 @@ fwd_cached_kernel(CachedParams p, const T* __restrict__ q, const T* __restrict__
       bool seen[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        s[i][j] *= p.scale_log2;
         seen[j] = full || (in[j] && cached::position_visible(p, qp[i], kp[j]));
-        if (!seen[j]) s[i][j] = -INFINITY;
-        mx = fmaxf(mx, s[i][j]);
+        mx = fmaxf(mx, seen[j] ? s[i][j] * p.scale_log2 : -INFINITY);
       }
 #pragma unroll
       for (int off = 8; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
       const float ref = mx == -INFINITY ? 0.f : mx;        // nothing seen yet
-      const float alpha = exp2f(m[i] - ref);
+      alpha[i] = exp2f(m[i] - ref);
       m[i] = mx;
-      l[i] *= alpha;
+      float e[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float e = seen[j] ? exp2f(s[i][j] - ref) : kHidden;
-        l[i] += e;
-        ps[(grp + 8 * i) * kPPitch + col + 16 * j] = e;
+        e[j] = seen[j] ? exp2f(fmaf(s[i][j], p.scale_log2, -ref)) : kHidden;
+        ps[(grp + 8 * i) * kPPitch + col + 16 * j] = e[j];
       }
-#pragma unroll
-      for (int x = 0; x < D / 16; ++x) acc[i][x] *= alpha;
+      l[i] = fmaf(l[i], alpha[i], (e[0] + e[1]) + (e[2] + e[3]));
     }
     load_wait<1>();
     // V is there (and this warp's probabilities)
     const bool guard = __syncthreads_or(!full && !own_rows_finite<T, D>(vs, kBN)) != 0;
-    output_product<D, RM>(ps, vs, grp, col, acc, guard);
+    output_product<D, RM>(ps, vs, grp, col, acc, alpha, guard);
     __syncthreads();
     if (n + 1 < n_stop) load_kv(vs, vb, n + 1);
     else load_commit();

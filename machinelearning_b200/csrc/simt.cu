@@ -45,7 +45,7 @@ __device__ __forceinline__ KeyBlocks key_blocks(const Problem& p, int q_lo, int 
 }
 
 template <typename T, int D, int RM>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, RM == 8 ? 3 : RM == 4 && D == 64 ? 4 : 1)
 fwd_tile_kernel(Problem p, const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                 T* __restrict__ o, float* __restrict__ lse) {
   constexpr int BM = 8 * RM, kPitch = D + 4;
@@ -92,6 +92,7 @@ fwd_tile_kernel(Problem p, const T* __restrict__ q, const T* __restrict__ k, con
     __syncthreads();
     if (it + 1 < blocks.count) load_kv(ks, kb, blocks.at(it + 1));
     else load_commit();
+    float alpha[RM];
     const bool full = rect_fully_visible(q0, q0 + BM - 1, k0, k0 + kBN - 1, p.window, p.sinks, p.block, p.T);
 #pragma unroll
     for (int i = 0; i < RM; ++i) {
@@ -100,33 +101,29 @@ fwd_tile_kernel(Problem p, const T* __restrict__ q, const T* __restrict__ k, con
       bool seen[4] = {true, true, true, true};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        s[i][j] *= scale2;
         if (!full) {
           const int kp = k0 + col + 16 * j;
           seen[j] = kp <= qlim[i] && (p.window == 0 || kp > qpos - (p.window - p.sinks) || kp < p.sinks);
-          s[i][j] = seen[j] ? s[i][j] : -INFINITY;
         }
-        mx = fmaxf(mx, s[i][j]);
+        mx = fmaxf(mx, seen[j] ? s[i][j] * scale2 : -INFINITY);
       }
 #pragma unroll
       for (int off = 8; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
       const float ref = mx == -INFINITY ? 0.f : mx;    // nothing seen yet
-      const float alpha = exp2f(m[i] - ref);
+      alpha[i] = exp2f(m[i] - ref);
       m[i] = mx;
-      l[i] *= alpha;
+      float e[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float e = seen[j] ? exp2f(s[i][j] - ref) : kHidden;
-        l[i] += e;
-        ps[(grp + 8 * i) * kPPitch + col + 16 * j] = e;
+        e[j] = seen[j] ? exp2f(fmaf(s[i][j], scale2, -ref)) : kHidden;
+        ps[(grp + 8 * i) * kPPitch + col + 16 * j] = e[j];
       }
-#pragma unroll
-      for (int n = 0; n < D / 16; ++n) acc[i][n] *= alpha;
+      l[i] = fmaf(l[i], alpha[i], (e[0] + e[1]) + (e[2] + e[3]));
     }
     load_wait<1>();
     // V is there (and this warp's probabilities)
     const bool guard = __syncthreads_or(!full && !own_rows_finite<T, D>(vs, kBN)) != 0;
-    output_product<D, RM>(ps, vs, grp, col, acc, guard);
+    output_product<D, RM>(ps, vs, grp, col, acc, alpha, guard);
     __syncthreads();
     if (it + 1 < blocks.count) load_kv(vs, vb, blocks.at(it + 1));
     else load_commit();
@@ -147,7 +144,7 @@ fwd_tile_kernel(Problem p, const T* __restrict__ q, const T* __restrict__ k, con
 // head of the group.  T0 = X0 Y0^T, T1 = X1 Y1^T; P from T0 and the taped logsumexp, dS = P (T1 - Delta) scale;
 // dV += P dO, dQ or dK += dS Y0.  NB: buffers of streamed tiles.
 template <typename T, int D, int RM, bool DKV, int NB>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, RM == 8 && D == 32 ? 3 : 1)
 bwd_tile_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q, const T* __restrict__ k,
                 const T* __restrict__ v, const float* __restrict__ lse, const float* __restrict__ delta,
                 T* __restrict__ out0, T* __restrict__ out1, int wait_first) {
@@ -238,6 +235,9 @@ bwd_tile_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q, 
       if (DKV) acc1[i][n] = 0.f;
     }
   }
+  float one[RM];
+#pragma unroll
+  for (int i = 0; i < RM; ++i) one[i] = 1.f;
   for (int it = 0; it < n_iters; ++it) {
     if (NB == 1 && it > 0) {
       __syncthreads();
@@ -285,10 +285,10 @@ bwd_tile_kernel(Problem p, const T* __restrict__ dout, const T* __restrict__ q, 
     };
     if constexpr (DKV) {
       hand_over(s);
-      output_product<D, RM>(ws, y1s, grp, col, acc1, guard);
+      output_product<D, RM>(ws, y1s, grp, col, acc1, one, guard);
     }
     hand_over(ds);
-    output_product<D, RM>(ws, y0s, grp, col, acc0, guard);
+    output_product<D, RM>(ws, y0s, grp, col, acc0, one, guard);
   }
 #pragma unroll
   for (int i = 0; i < RM; ++i) {

@@ -5,6 +5,8 @@
 // D + 4.
 #pragma once
 
+#include <type_traits>
+
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -92,73 +94,152 @@ __device__ __forceinline__ bool own_rows_finite(const float* tile, int rows) {
   return z == z;
 }
 
-// s[i][j] = row (grp + 8 i) of A . row (col + 16 j) of B
+// Sums are taken in short runs whose totals are added (eight products, the runs of a block, the blocks): the rounding error
+// of one chain grows with the square root of half its length.  With chains of D products and of all keys the relative error
+// against 64 bits was up to 1.35 times (attention) and 3.4 times (cached) that of the kernels with one warp lane per key;
+// as it is, o of B=2 H=6/2 T=700 D=128: lanes 2.9e-7, chains 3.6e-7, runs 1.4e-7; of 64 queries over 16,448 keys at D = 128
+// 3.7e-7, 9.3e-7, 2.2e-7.  RM = 8, where sums of runs would take the registers of a CTA per SM, keeps one chain over the
+// keys, as the lanes had (B=8 H=12/4 T=1024 D=64: 3.3e-7, 3.3e-7, 2.7e-7).
+
+// s[i][j] = row (grp + 8 i) of A . row (col + 16 j) of B.  Packed: even and odd elements in the two halves, D = 128 as two
+// sums of 64.  At RM = 8 packed sums would take the registers of a CTA per SM: runs of eight, their halves added to one sum.
 template <int D, int RM>
 __device__ __forceinline__ void score_product(const float* a, const float* b, int grp, int col, float (&s)[RM][4]) {
-  constexpr int kPitch = D + 4;
-#pragma unroll
-  for (int i = 0; i < RM; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+  constexpr int kPitch = D + 4, kSpan = D < 64 ? D : 64;
   const float* ap = a + grp * kPitch;
   const float* bp = b + col * kPitch;
-#pragma unroll 2
-  for (int d = 0; d < D; d += 4) {
-    float4 bv[4];
+  auto ld2 = [](const float* p) { return *reinterpret_cast<const ulonglong2*>(p); };
+  if constexpr (RM == 8) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) bv[j] = ld4(bp + 16 * j * kPitch + d);
+    for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int i = 0; i < RM; ++i) {
-      const float4 av = ld4(ap + 8 * i * kPitch + d);
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 1
+    for (int d = 0; d < D; d += 8) {
+      ulonglong2 b0[4], b1[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        s[i][j] = fmaf(av.w, bv[j].w, fmaf(av.z, bv[j].z, fmaf(av.y, bv[j].y, fmaf(av.x, bv[j].x, s[i][j]))));
-    }
-  }
-}
-
-// acc[i][.] += row (grp + 8 i) of the [rows][kBN] tile w times B [kBN][D]; a thread's D / 16 columns are 4 col ..
-// (per 64 columns), or 2 col .. at D = 32; `guard`: see kHidden
-template <int D, int RM, bool GUARD = false>
-__device__ __forceinline__ void output_product(const float* w, const float* b, int grp, int col, float (&acc)[RM][D / 16]) {
-  constexpr int kPitch = D + 4;
-  const float* wp = w + grp * kPPitch;
-#pragma unroll 2
-  for (int k = 0; k < kBN; k += 4) {
-    float wv[RM][4];
-#pragma unroll
-    for (int i = 0; i < RM; ++i) {
-      const float4 t = ld4(wp + 8 * i * kPPitch + k);
-      wv[i][0] = t.x; wv[i][1] = t.y; wv[i][2] = t.z; wv[i][3] = t.w;
-    }
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      float bv[D / 16];
-      const float* row = b + (k + x) * kPitch;
-      if constexpr (D == 32) {
-        const float2 t = *reinterpret_cast<const float2*>(row + 2 * col);
-        bv[0] = t.x; bv[1] = t.y;
-      } else {
-#pragma unroll
-        for (int h = 0; h < D / 64; ++h) {
-          const float4 t = ld4(row + 64 * h + 4 * col);
-          bv[4 * h] = t.x; bv[4 * h + 1] = t.y; bv[4 * h + 2] = t.z; bv[4 * h + 3] = t.w;
-        }
+      for (int j = 0; j < 4; ++j) {
+        b0[j] = ld2(bp + 16 * j * kPitch + d);
+        b1[j] = ld2(bp + 16 * j * kPitch + d + 4);
       }
 #pragma unroll
-      for (int i = 0; i < RM; ++i)
+      for (int i = 0; i < RM; ++i) {
+        const ulonglong2 a0 = ld2(ap + 8 * i * kPitch + d), a1 = ld2(ap + 8 * i * kPitch + d + 4);
 #pragma unroll
-        for (int n = 0; n < D / 16; ++n)
-          if (!GUARD || __float_as_uint(wv[i][x]) != __float_as_uint(kHidden)) acc[i][n] = fmaf(wv[i][x], bv[n], acc[i][n]);
+        for (int j = 0; j < 4; ++j) {
+          float x, y;
+          unpack_f2(ffma2(a1.y, b1[j].y, ffma2(a1.x, b1[j].x, ffma2(a0.y, b0[j].y, fmul2(a0.x, b0[j].x)))), x, y);
+          s[i][j] += x + y;
+        }
+      }
     }
+    return;
+  }
+#pragma unroll
+  for (int d0 = 0; d0 < D; d0 += kSpan) {
+    uint64_t sum[RM][4];
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum[i][j] = 0ull;
+#pragma unroll(RM <= 2 ? 2 : 1)
+    for (int d = d0; d < d0 + kSpan; d += 8) {
+      ulonglong2 b0[4], b1[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        b0[j] = ld2(bp + 16 * j * kPitch + d);
+        b1[j] = ld2(bp + 16 * j * kPitch + d + 4);
+      }
+#pragma unroll
+      for (int i = 0; i < RM; ++i) {
+        const ulonglong2 a0 = ld2(ap + 8 * i * kPitch + d), a1 = ld2(ap + 8 * i * kPitch + d + 4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          sum[i][j] = fadd2(sum[i][j], ffma2(a1.y, b1[j].y, ffma2(a1.x, b1[j].x, ffma2(a0.y, b0[j].y, fmul2(a0.x, b0[j].x)))));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float x, y;
+        unpack_f2(sum[i][j], x, y);
+        s[i][j] = d0 == 0 ? x + y : s[i][j] + (x + y);
+      }
   }
 }
 
+// acc[i][.] = acc[i][.] mul[i] + row (grp + 8 i) of the [rows][kBN] tile w times B [kBN][D]; a thread's D / 16 columns are
+// 4 col .. (per 64 columns), or 2 col .. at D = 32; `guard`: see kHidden
 template <int D, int RM>
 __device__ __forceinline__ void output_product(const float* w, const float* b, int grp, int col, float (&acc)[RM][D / 16],
-                                               bool guard) {
-  if (guard) output_product<D, RM, true>(w, b, grp, col, acc);
-  else output_product<D, RM, false>(w, b, grp, col, acc);
+                                               const float (&mul)[RM], bool guard) {
+  constexpr int kPitch = D + 4, N = D / 16, kRun = RM == 8 ? 4 : 8;
+  const float* wp = w + grp * kPPitch;
+  auto columns = [&](const float* row, float (&v)[N]) {
+    if constexpr (D == 32) {
+      const float2 t = *reinterpret_cast<const float2*>(row + 2 * col);
+      v[0] = t.x; v[1] = t.y;
+    } else {
+#pragma unroll
+      for (int h = 0; h < D / 64; ++h) {
+        const float4 t = ld4(row + 64 * h + 4 * col);
+        v[4 * h] = t.x; v[4 * h + 1] = t.y; v[4 * h + 2] = t.z; v[4 * h + 3] = t.w;
+      }
+    }
+  };
+  auto product = [&](auto guarded, float (&sum)[RM][N]) {
+#pragma unroll(RM <= 2 || RM == 8 ? 2 : 1)
+    for (int k = 0; k < kBN; k += kRun) {
+      float bv[kRun][N];
+#pragma unroll
+      for (int x = 0; x < kRun; ++x) columns(b + (k + x) * kPitch, bv[x]);
+#pragma unroll
+      for (int i = 0; i < RM; ++i) {
+        float wv[kRun];
+#pragma unroll
+        for (int x = 0; x < kRun; x += 4) *reinterpret_cast<float4*>(wv + x) = ld4(wp + 8 * i * kPPitch + k + x);
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+          constexpr int kPer = RM == 1 ? 2 : kRun;         // products in a chain; RM = 1 is all latency: pairs, as a tree
+          float t[kRun / kPer];
+#pragma unroll
+          for (int x = 0; x < kRun; ++x) {
+            const bool hidden = decltype(guarded)::value && __float_as_uint(wv[x]) == __float_as_uint(kHidden);
+            float& c = t[x / kPer];
+            if (x % kPer == 0 && RM < 8) c = hidden ? 0.f : wv[x] * bv[x][n];
+            else if (x == 0) c = hidden ? sum[i][n] : fmaf(wv[0], bv[0][n], sum[i][n]);
+            else c = hidden ? c : fmaf(wv[x], bv[x][n], c);
+          }
+          if constexpr (RM == 8) sum[i][n] = t[0];
+          else if constexpr (RM == 1) sum[i][n] += (t[0] + t[1]) + (t[2] + t[3]);
+          else sum[i][n] += t[0];
+        }
+      }
+    }
+  };
+  auto add = [&](float (&sum)[RM][N]) {
+    if (guard) product(std::true_type{}, sum);
+    else product(std::false_type{}, sum);
+  };
+  if constexpr (RM == 8) {                                 // (sums of runs and blocks would take another CTA's registers: a chain)
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+      for (int n = 0; n < N; ++n) acc[i][n] *= mul[i];
+    add(acc);
+  } else {
+    float sum[RM][N];
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+      for (int n = 0; n < N; ++n) sum[i][n] = 0.f;
+    add(sum);
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+      for (int n = 0; n < N; ++n) acc[i][n] = fmaf(acc[i][n], mul[i], sum[i][n]);
+  }
 }
 
 // one thread's D / 16 columns of an output row, times `mul`
