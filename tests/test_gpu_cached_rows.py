@@ -48,3 +48,44 @@ def test_sinks_next_to_two_to_the_31(dtype):
     want = flash_cuda.flash_attn_cached(q, k, v, causal=True)
     for window, sinks in (((1 << 31) - 1, (1 << 31) - 2), ((1 << 31) - 1, 0), (901, 900)):
         assert torch.equal(flash_cuda.flash_attn_cached(q, k, v, causal=True, window=window, sinks=sinks), want)
+
+
+def _sparse(T, L, dtype=torch.float32):
+    """A window of 256 with 4 sinks over a cache that was not compacted, its keys in an order of their own."""
+    g = torch.Generator().manual_seed(L)
+    q, k, v = (torch.randn(1, *s, 64, generator=g).to("cuda", dtype) for s in ((T, 4), (2, L), (2, L)))
+    kpos = torch.arange(L).reshape(-1, 8).flip(1).reshape(-1) if L % 8 == 0 else torch.arange(L)
+    return q, k, v, torch.arange(L - T, L), kpos
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,L", [(1, 16384), (5, 9000), (40, 20001), (17, 130), (3, 70000)])
+def test_hidden_stretches_of_a_cache_with_positions(T, L):
+    from machinelearning_b200 import flash_cuda
+    q, k, v, qpos, kpos = _sparse(T, L)
+    y, lse = flash_cuda.flash_attn_cached(q, k, v, qpos=qpos, kpos=kpos, causal=True, window=256, sinks=4, return_lse=True)
+    n = lambda x: x.double().cpu().numpy()
+    ref, lse_ref = cached_f64.forward(n(q), n(k), n(v), 0.125, qpos.numpy(), kpos.numpy(), True, 256, 4)
+    assert np.abs(n(y) - ref).max() <= 1e-5 and np.abs(n(lse) - lse_ref).max() <= 1e-5
+
+
+@pytest.mark.gpu
+def test_hidden_stretches_of_a_cache_are_not_read():
+    """Of 262,144 keys a window shows 256: a fraction of the time of a causal call, which reads them all."""
+    from machinelearning_b200 import flash_cuda
+    q, k, v, qpos, kpos = _sparse(1, 262144)
+    qpos, kpos = qpos.cuda(), kpos.cuda()
+
+    def microseconds(**kw):
+        times = []
+        for _ in range(12):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            for _ in range(4):
+                flash_cuda.flash_attn_cached(q, k, v, qpos=qpos, kpos=kpos, causal=True, **kw)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return sorted(times)[6]
+
+    assert microseconds(window=256, sinks=4) < 0.5 * microseconds()
