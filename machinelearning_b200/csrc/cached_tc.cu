@@ -275,7 +275,8 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int c = 4 * lane + e, key = j * kTile + c;
-            const int x = key < p.L ? cached::key_position(p, key) : kNoKey;
+            // (without a mask by positions they may be anything, the mark for "no key" among them)
+            const int x = key >= p.L ? kNoKey : p.causal ? cached::key_position(p, key) : 0;
             pos[c] = x;
             kp_min = x < kp_min ? x : kp_min;
             kp_max = x > kp_max ? x : kp_max;

@@ -89,3 +89,15 @@ def test_hidden_stretches_of_a_cache_are_not_read():
         return sorted(times)[6]
 
     assert microseconds(window=256, sinks=4) < 0.5 * microseconds()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [4, 40])
+def test_positions_of_an_unmasked_block_may_be_anything(T):
+    from machinelearning_b200 import flash_cuda
+    g = torch.Generator().manual_seed(T)
+    q, k, v = (torch.randn(1, *s, 64, generator=g).to("cuda", torch.bfloat16) for s in ((T, 4), (2, 300), (2, 300)))
+    kpos = torch.full((300,), 2147483647, dtype=torch.int32, device="cuda")
+    kpos[::3] = -5
+    y = flash_cuda.flash_attn_cached(q, k, v, qpos=torch.zeros(T, dtype=torch.int32, device="cuda"), kpos=kpos)
+    assert torch.equal(y, flash_cuda.flash_attn_cached(q, k, v))
