@@ -101,12 +101,13 @@ int nlfa_fwd_masked(const void* q, const void* k, const void* v, void* o, float*
 size_t nlfa_bwd_scratch_bytes(int B, int T, int H);
 
 /* Bytes of scratch with which the backward runs fastest: the tape, and behind it (rounded up to 256
- * bytes) room for dS of as many (batch, KV head) pairs as fit 4 GiB -- 32 KB per query head, 128-row
+ * bytes) room for dS of as many (batch, KV head) pairs as fit 4 GiB (or the environment's
+ * NLFA_BWD_WORKSPACE_MB, read once; 0: the tape alone) -- 32 KB per query head, 128-row
  * query tile and 128-key block the tile sees.  Given at least one pair's worth, the entry points below
  * (every pass asked for, tensor-core path) let the dK/dV kernel leave dS there and form dQ as one product
  * over it, that many pairs per launch; given less they recompute dS in the dQ kernel.  Same bits either way.
  * Equals nlfa_bwd_scratch_bytes where there is nothing to gain (head dims below 128, fp32 path, a pair larger
- * than 4 GiB, launches too small to fill the GPU). */
+ * than that, launches too small to fill the GPU). */
 size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
                                 int path);
 

@@ -434,7 +434,15 @@ size_t ds_pair_bytes(const Problem& p) {
   return static_cast<size_t>(ds_tile_offset<long long>(l, l.n_tiles)) * kDsTileBytes * (p.H / p.Hkv);
 }
 
-constexpr size_t kDsMostBytes = size_t{4} << 30;        // dS of as many pairs at a time as fit here
+// dS of as many pairs at a time as fit here: 4 GiB, or NLFA_BWD_WORKSPACE_MB (0: the tape alone).
+size_t ds_most_bytes() {
+  static const size_t most = [] {
+    const char* v = std::getenv("NLFA_BWD_WORKSPACE_MB");
+    const long long mb = v != nullptr ? std::atoll(v) : 4096;
+    return static_cast<size_t>(mb < 0 ? 0 : mb > (1ll << 20) ? 1ll << 20 : mb) << 20;
+  }();
+  return most;
+}
 }  // namespace
 
 size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
@@ -446,7 +454,7 @@ size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window,
     return tape;
   simplify_mask(p);
   const size_t pair = ds_pair_bytes(p), all = static_cast<size_t>(B) * Hkv;
-  const size_t most = kDsMostBytes / pair;
+  const size_t most = ds_most_bytes() / pair;
   if (most == 0) return tape;
   // The dQ pass that recomputes dS starts beside the dK/dV pass and takes the SMs it leaves idle; one that reads
   // dS cannot.  So every launch has to keep the GPU busy by itself: half as many units (key blocks) again as SMs,

@@ -135,7 +135,15 @@ variable_list attn_backward(const Tensor& dout, const Tensor& q, const Tensor& k
   const size_t bytes = fused ? nlfa_bwd_fused_scratch_bytes(s.B, s.T, s.H, s.D)
                              : nlfa_bwd_workspace_bytes(s.B, s.T, s.H, s.Hkv, s.D, m.window, m.sinks, m.block, s.dtype, path);
   Tensor dq = empty_as(q), dk = empty_as(k), dv = empty_as(v);
-  Tensor scratch = empty({static_cast<int64_t>(bytes > 16 ? bytes : 16)}, at::kByte, q);
+  Tensor scratch;
+  try {
+    scratch = empty({static_cast<int64_t>(bytes > 16 ? bytes : 16)}, at::kByte, q);
+  } catch (const c10::OutOfMemoryError&) {
+    // room for dS is a matter of speed: with the tape alone the backward recomputes it, to the same bits
+    const size_t least = nlfa_bwd_scratch_bytes(s.B, s.T, s.H);
+    if (fused || bytes <= least) throw;
+    scratch = empty({static_cast<int64_t>(least > 16 ? least : 16)}, at::kByte, q);
+  }
   check("nlfa_bwd_masked",
         nlfa_bwd_masked(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(),
                         static_cast<const float*>(lse.data_ptr()), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),

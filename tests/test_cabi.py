@@ -164,3 +164,22 @@ def test_workspace_sizes_of_extreme_extents(lib):
         assert T == 1 or causal > lib.nlfa_bwd_scratch_bytes(64, T, 4)
         assert size(T, block=big) == size(T, block=big - 126) == size(T, block=T)
         assert size(T, window=big, sinks=big - 1) == size(T, window=big, sinks=T) == causal
+
+
+@pytest.mark.parametrize("megabytes,most", [("0", 0), ("512", 512 << 20), ("100000", None), (None, 4 << 30)])
+def test_workspace_limit_from_the_environment(lib, megabytes, most):
+    """``NLFA_BWD_WORKSPACE_MB`` limits the room for dS; it is read once per process."""
+    import os
+    import subprocess
+    import sys
+    from machinelearning_b200 import _lib as L
+    args = (32, 4096, 16, 16, 128, 0, 0, 0, L.DTYPE_BF16, L.PATH_TENSOR)
+    env = {k: v for k, v in os.environ.items() if k != "NLFA_BWD_WORKSPACE_MB"}
+    if megabytes is not None:
+        env["NLFA_BWD_WORKSPACE_MB"] = megabytes
+    code = f"from machinelearning_b200 import _lib; print(_lib.load().nlfa_bwd_workspace_bytes{args})"
+    size = int(subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env, capture_output=True, text=True,
+                              check=True).stdout.split()[-1])
+    tape, pair = 32 * 16 * 4096 * 4, 32 * 33 // 2 * 32768
+    pairs = 32 * 16 if most is None else min(32 * 16, most // pair)
+    assert size == tape + pairs * pair

@@ -89,3 +89,27 @@ def test_extents_next_to_two_to_the_31(extreme, same):
         o, lse = fc.fwd(q, k, v, 0.1, True, **kw)
         runs.append((o, lse, *fc.bwd(do, q, k, v, o, lse, 0.1, True, **kw)))
     assert all(torch.equal(a, b) for a, b in zip(*runs))
+
+
+def test_backward_without_memory_for_the_workspace():
+    """When the allocator has no room for dS the backward goes on with the tape, to the same bits."""
+    from machinelearning_b200 import _lib as L, flash_cuda as fc
+    assert fc.is_available(), fc.unavailable_reason()
+    B, T, H, D = 4, 4096, 16, 128
+    g = torch.Generator(device="cuda").manual_seed(0)
+    q, k, v = (torch.randn(B, T, H, D, device="cuda", generator=g).bfloat16().requires_grad_() for _ in range(3))
+    do = torch.randn(B, T, H, D, device="cuda", generator=g).bfloat16()
+    y = fc.flash_attn(q, k, v)
+    want = torch.autograd.grad(y, (q, k, v), do, retain_graph=True)
+    size = fc._load().nlfa_bwd_workspace_bytes(B, T, H, H, D, 0, 0, 0, L.DTYPE_BF16, L.PATH_TENSOR)
+    assert size > 1 << 30
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:                                             # what is in use, the three gradients, and half of the workspace
+        room = torch.cuda.memory_reserved() + 3 * do.nbytes + size // 2
+        torch.cuda.set_per_process_memory_fraction(room / total)
+        got = torch.autograd.grad(y, (q, k, v), do)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
