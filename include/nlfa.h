@@ -230,7 +230,7 @@ size_t nlfa_qk_prologue_scratch_bytes(int D);
  * i.e. dq or dk of the attention backward) -> gx [B,T,H,D] of x_dtype and
  * gweight [D] float32 (overwritten).  Stands where autograd's backward of the
  * same nanolab lines stands.  The weight gradient is reduced in a fixed order
- * (per-CTA partial sums in `scratch`, then one small kernel): bit-reproducible. */
+ * (per-CTA partial sums in `scratch`, added by the CTA that finishes last): bit-reproducible. */
 int nlfa_qk_prologue_bwd(const void* gy, int gy_dtype, const void* x, int x_dtype,
                          const float* weight, const float* cos_table, const float* sin_table,
                          const float* rstd, void* gx, float* gweight, void* scratch,
@@ -244,7 +244,7 @@ int nlfa_qk_prologue_bwd(const void* gy, int gy_dtype, const void* x, int x_dtyp
 int nlfa_value_blend_fwd(const void* v, const void* v0, int v_dtype, const float* lambda, void* out,
                          int out_dtype, long long n, void* stream);
 
-/* Bytes of device scratch `nlfa_value_blend_bwd` needs (per-CTA partial sums). */
+/* Bytes of device scratch `nlfa_value_blend_bwd` needs (per-CTA partial sums and a ticket). */
 size_t nlfa_value_blend_scratch_bytes(void);
 
 /* Backward of nlfa_value_blend_fwd: g (gradient of out, g_dtype) -> dv = (1 - s) g and

@@ -26,6 +26,10 @@ constexpr unsigned kEagerSlots = 1024;       // ring for ordinary launches
 constexpr unsigned kGraphSlots = 15360;      // handed out once each to launches under capture
 __device__ unsigned g_sched[kEagerSlots + kGraphSlots][2];
 
+// Tickets on which the CTAs of an ordinary launch count themselves off (rowwise.cuh): a ring.
+constexpr unsigned kTickets = 1024;
+__device__ unsigned g_tickets[kTickets];
+
 namespace {
 
 constexpr int kMaxDevices = 64;
@@ -33,9 +37,11 @@ std::mutex g_host_mutex;                     // guards the per-device tables bel
 unsigned* g_status_ptr[kMaxDevices];
 unsigned* g_status_mirror[kMaxDevices];      // host address of the registered copy, or null
 unsigned* g_sched_ptr[kMaxDevices];
+unsigned* g_ticket_ptr[kMaxDevices];
 int g_sm_count[kMaxDevices];
 std::atomic<unsigned> g_next_eager{0};
 std::atomic<unsigned> g_next_graph{0};
+std::atomic<unsigned> g_next_ticket{0};
 
 int current_device() {
   int dev = 0;
@@ -262,6 +268,26 @@ int sched_counters(cudaStream_t stream, unsigned** out) {
   const unsigned slot = g_next_graph.fetch_add(1u, std::memory_order_relaxed);
   if (slot >= kGraphSlots) return NLFA_ERR_GRAPH_SLOTS;   // every slot is bound into some captured graph
   *out = base + 2 * (kEagerSlots + slot);
+  return NLFA_OK;
+}
+
+int launch_ticket(cudaStream_t stream, unsigned* own, unsigned** out, bool* captured) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) return NLFA_ERR_CUDA;
+  *captured = cap != cudaStreamCaptureStatusNone;
+  if (*captured) {
+    *out = own;
+    return cudaMemsetAsync(own, 0, sizeof(unsigned), stream) == cudaSuccess ? NLFA_OK : NLFA_ERR_CUDA;
+  }
+  const int dev = current_device();
+  if (dev < 0) return NLFA_ERR_CUDA;
+  std::lock_guard<std::mutex> lock(g_host_mutex);
+  if (g_ticket_ptr[dev] == nullptr) {
+    void* ptr = nullptr;
+    if (cudaGetSymbolAddress(&ptr, g_tickets) != cudaSuccess) return NLFA_ERR_CUDA;
+    g_ticket_ptr[dev] = static_cast<unsigned*>(ptr);
+  }
+  *out = g_ticket_ptr[dev] + g_next_ticket.fetch_add(1u, std::memory_order_relaxed) % kTickets;
   return NLFA_OK;
 }
 

@@ -337,8 +337,6 @@ int launch_t(const CUtensorMap& mk, const CUtensorMap& mdq, DqParams dp, cudaStr
   static_assert(L::kDynamic <= 232448, "over the shared memory a CTA can have");
   auto kern = dq_from_ds_kernel<T>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kDynamic) != NLFA_OK) return NLFA_ERR_CUDA;
-  const int sst = sched_counters(stream, &dp.sched);
-  if (sst != NLFA_OK) return sst;
   const int grid = dp.total_units < sm_count() ? dp.total_units : sm_count();
   dp.sched_group = dp.heads < grid ? dp.heads : grid;
   if (launch_kernel(kern, dim3(grid), dim3(256), L::kDynamic, stream, overlap_launches(kOverlapDq), mk, mdq, dp) !=
@@ -352,7 +350,7 @@ int launch_t(const CUtensorMap& mk, const CUtensorMap& mdq, DqParams dp, cudaStr
 }  // namespace
 
 int launch_dq_from_ds(const Problem& p, const void* k, const void* ds, const DsLayout& layout, int first_pair, int pairs,
-                      void* dq, unsigned* status, cudaStream_t stream) {
+                      void* dq, unsigned* sched, unsigned* status, cudaStream_t stream) {
   CUtensorMap mk, mdq;
   int st = make_tile_map(&mk, k, p.dtype, p.B, p.T, p.Hkv, p.D, 64);
   if (st == NLFA_OK) st = make_tile_map(&mdq, dq, p.dtype, p.B, p.T, p.H, p.D, kTile);
@@ -370,6 +368,7 @@ int launch_dq_from_ds(const Problem& p, const void* k, const void* ds, const DsL
   dp.per_head = ds_tile_offset(layout, layout.n_tiles);
   dp.ds = static_cast<const uint8_t*>(ds);
   dp.scale = p.scale;
+  dp.sched = sched;
   dp.status = status;
   return p.dtype == NLFA_DTYPE_BF16 ? launch_t<__nv_bfloat16>(mk, mdq, dp, stream) : launch_t<__half>(mk, mdq, dp, stream);
 }

@@ -1190,7 +1190,7 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
                 const float* lse, const float* delta, void* out0, void* out1, unsigned* status,
                 cudaStream_t stream, void* dq = nullptr, const FusedScratch* fused = nullptr,
                 bool beside_previous = false, const void* o_for_delta = nullptr, float* delta_out = nullptr,
-                bool plain_launch = false, void* ds = nullptr, int first_pair = 0, int pairs = 0) {
+                bool plain_launch = false, void* ds = nullptr, int first_pair = 0, int pairs = 0, unsigned* sched = nullptr) {
   // stationary tensors in boxes of 128 rows, streamed tensors in boxes of YR rows; output tiles
   // leave through TMA stores: dQ is [B,T,H,D], dK and dV are [B,T,Hkv,D]
   const void* x0 = MODE == MODE_DQ ? q : k;
@@ -1253,8 +1253,11 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
                         stream) != cudaSuccess)
       return NLFA_ERR_CUDA;
   }
-  const int sst = sched_counters(stream, &bp.sched);
-  if (sst != NLFA_OK) return sst;
+  bp.sched = sched;
+  if (sched == nullptr) {
+    const int sst = sched_counters(stream, &bp.sched);
+    if (sst != NLFA_OK) return sst;
+  }
   const int grid = bp.total_units < sm_count() ? bp.total_units : sm_count();
   bp.sched_group = MODE == MODE_DQ ? bp.BH : grid;      // (the dQ pass gains nothing from groups)
   if (MODE == MODE_DKV_DS) {
@@ -1322,12 +1325,18 @@ int launch_both(const Problem& p, const void* dout, const void* q, const void* k
     // tile pair has half the products for the same bytes and the staging tile costs a streamed stage
     // (B=32 H=12 T=1024: 274 -> 300 us), so there the dQ pass recomputes dS.
     const DsLayout layout = ds_layout(p.T, p.window, p.sinks, p.block);
+    // Each kernel's launches follow one another (a part's dQ pass has waited for its dK/dV pass, the next part waits for
+    // that before it touches anything), so they share their counters.
+    unsigned *sched_dkv = nullptr, *sched_dq = nullptr;
+    st = sched_counters(stream, &sched_dkv);
+    if (st == NLFA_OK) st = sched_counters(stream, &sched_dq);
+    if (st != NLFA_OK) return st;
     const int all = p.B * p.Hkv, chunks = (all + ds->pairs - 1) / ds->pairs, per = (all + chunks - 1) / chunks;
     for (int first = 0; first < all; first += per) {
       const int pairs = all - first < per ? all - first : per;
       st = launch_mode<T, D, DR, MODE_DKV_DS, STAGES, XBUF, YR>(p, dout, q, k, v, lse, delta, dk, dv, status, stream, nullptr,
-                                                           nullptr, false, nullptr, nullptr, false, ds->tiles, first, pairs);
-      if (st == NLFA_OK) st = launch_dq_from_ds(p, k, ds->tiles, layout, first, pairs, dq, status, stream);
+                                                           nullptr, false, nullptr, nullptr, false, ds->tiles, first, pairs, sched_dkv);
+      if (st == NLFA_OK) st = launch_dq_from_ds(p, k, ds->tiles, layout, first, pairs, dq, sched_dq, status, stream);
       if (st != NLFA_OK) return st;
     }
     return NLFA_OK;

@@ -202,7 +202,7 @@ int launch_bwd_tc(const Problem& p, const void* dout, const void* q, const void*
                   const DsScratch* ds);
 // dQ of the query heads of (batch, KV head) pairs [first_pair, first_pair + pairs) from their dS tiles.
 int launch_dq_from_ds(const Problem& p, const void* k, const void* ds, const DsLayout& layout, int first_pair, int pairs,
-                      void* dq, unsigned* status, cudaStream_t stream);
+                      void* dq, unsigned* sched, unsigned* status, cudaStream_t stream);
 int launch_selftest_tiles(int dtype, int head_dim, const void* q, const void* k, const void* v,
                           float* s_out, float* o_out, unsigned* status, cudaStream_t stream);
 
@@ -223,6 +223,11 @@ int make_map(CUtensorMap* map, const void* base, int dtype, const unsigned long 
 // the address for as long as it is replayed; eager launches take turns on a ring.  Returns an
 // NLFA_* status (NLFA_ERR_GRAPH_SLOTS when the graph range is used up).
 int sched_counters(cudaStream_t stream, unsigned** out);
+
+// A ticket for one launch whose CTAs count themselves off and leave it at zero (rowwise.cuh, last_cta): of a ring for
+// ordinary launches; under capture `own`, in the caller's scratch, zeroed by a node of the graph in front of the launch,
+// so that captures are not limited (the launch then follows a memset: not overlapped).
+int launch_ticket(cudaStream_t stream, unsigned* own, unsigned** out, bool* captured);
 
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize), once per kernel and device.
 int ensure_dynamic_smem(const void* kernel, int bytes);

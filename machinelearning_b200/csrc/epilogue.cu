@@ -225,10 +225,11 @@ int blend_bwd_go(const void* g, const void* v, const void* v0, const float* lam,
                  float* dlam, unsigned nvec, cudaStream_t st) {
   const int grid = cta_count(nvec, kThreads, kMaxPartials);
   unsigned* ticket = nullptr;
-  const int rc = sched_counters(st, &ticket);
+  bool captured = false;
+  const int rc = launch_ticket(st, reinterpret_cast<unsigned*>(partial + kMaxPartials), &ticket, &captured);
   if (rc != NLFA_OK) return rc;
   return launched(launch_kernel(value_blend_bwd_kernel<TV, TG>, dim3(grid), dim3(kThreads), 0, st,
-                                overlap_launches(kOverlapRowwise), (const TG*)g, (const TV*)v, (const TV*)v0, lam, (TV*)dv,
+                                !captured && overlap_launches(kOverlapRowwise), (const TG*)g, (const TV*)v, (const TV*)v0, lam, (TV*)dv,
                                 (TV*)dv0, partial, dlam, ticket, nvec));
 }
 template <typename TV>
@@ -278,7 +279,9 @@ int gate_dispatch(bool backward, int y_dtype, int gate_dtype, int D, const void*
 
 extern "C" {
 
-size_t nlfa_value_blend_scratch_bytes(void) { return (size_t)nlfa::rowwise::kMaxPartials * sizeof(float); }
+size_t nlfa_value_blend_scratch_bytes(void) {              // partial sums, and the ticket
+  return (size_t)nlfa::rowwise::kMaxPartials * sizeof(float) + 16;
+}
 
 int nlfa_value_blend_fwd(const void* v, const void* v0, int v_dtype, const float* lambda, void* out, int out_dtype,
                          long long n, void* stream) {

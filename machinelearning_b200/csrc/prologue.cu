@@ -253,16 +253,18 @@ template <typename TIn, typename TG>
 int bwd_for_dim(int D, const void* gy, const void* x, const float* w, const float* c, const float* s,
                 const float* rstd, void* gx, float* partial, float* gweight, long long rows, int T, int H,
                 cudaStream_t st) {
-  const int grid = grid_for(rows, D, 2 * sm_count() < kMaxPartials ? 2 * sm_count() : kMaxPartials, Elem<TIn>::kInFlight);
+  // (the scratch's last row is the ticket's)
+  const int grid = grid_for(rows, D, 2 * sm_count() < kMaxPartials - 1 ? 2 * sm_count() : kMaxPartials - 1, Elem<TIn>::kInFlight);
   unsigned* ticket = nullptr;
+  bool captured = false;
   if (w != nullptr) {
-    const int rc = sched_counters(st, &ticket);
+    const int rc = launch_ticket(st, reinterpret_cast<unsigned*>(partial + (size_t)(kMaxPartials - 1) * D), &ticket, &captured);
     if (rc != NLFA_OK) return rc;
   }
   cudaError_t e;
 #define NLFA_GO(DD)                                                                                               \
   e = launch_kernel(qk_prologue_bwd_kernel<TIn, TG, DD>, dim3(grid), dim3(kThreads), 0, st,                       \
-                    overlap_launches(kOverlapRowwise), (const TG*)gy, (const TIn*)x, w, c, s, rstd, (TIn*)gx,     \
+                    !captured && overlap_launches(kOverlapRowwise), (const TG*)gy, (const TIn*)x, w, c, s, rstd, (TIn*)gx,     \
                     partial, gweight, ticket, (unsigned)rows, (unsigned)T, (unsigned)H)
   if (D == 32) NLFA_GO(32); else if (D == 64) NLFA_GO(64); else NLFA_GO(128);
 #undef NLFA_GO
@@ -324,7 +326,7 @@ int nlfa_qk_prologue_bwd(const void* gy, int gy_dtype, const void* x, int x_dtyp
   if (weight && scratch_bytes < nlfa_qk_prologue_scratch_bytes(D)) return NLFA_ERR_SCRATCH_TOO_SMALL;
   if (!aligned16(gy) || !aligned16(gx) || !aligned16(x) || !aligned16(cos_table) || !aligned16(sin_table))
     return NLFA_ERR_MISALIGNED;
-  // (the kernel reads the partial sums 16 bytes at a time; the scratch has room to spare)
+  // (the kernel reads the partial sums 16 bytes at a time; the scratch's last row, the ticket's, has room to spare)
   scratch = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(scratch) + 15u) & ~static_cast<uintptr_t>(15u));
 #define NLFA_G(TIn)                                                                                               \
   (gy_dtype == NLFA_DTYPE_BF16 ? bwd_for_dim<TIn, __nv_bfloat16>(D, gy, x, weight, cos_table, sin_table, rstd, gx, (float*)scratch, gweight, rows, T, H, st) \

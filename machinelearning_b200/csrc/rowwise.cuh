@@ -107,7 +107,7 @@ template <int LPR> __device__ inline float row_sum(float v) {
 }
 
 
-// The CTAs of a launch count themselves off on a ticket that wraps to zero (sched_counters); true in every thread of
+// The CTAs of a launch count themselves off on a ticket that wraps to zero (launch_ticket); true in every thread of
 // the last one, which then sees what all of them wrote before this call.  `flag` is in shared memory.
 __device__ inline bool last_cta(unsigned* ticket, unsigned ctas, int* flag) {
   __threadfence();

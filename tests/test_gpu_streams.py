@@ -129,3 +129,59 @@ print("digest", h.hexdigest())
         assert r.returncode == 0, r.stderr[-2000:]
         digests.append(r.stdout.strip().splitlines()[-1])
     assert digests[0] == digests[1]
+
+
+def test_captures_of_the_elementwise_steps_and_of_parts_are_not_limited():
+    """Scheduler counters are handed out once to captured launches, 15,360 per process.  The elementwise backward kernels
+    take none, however often they are captured, and a D = 128 backward in parts takes two, as one without parts does."""
+    from machinelearning_b200 import _lib as L, flash_cuda as fc, qk_prologue, value_gate
+    assert fc.is_available(), fc.unavailable_reason()
+    lib = fc._load()
+    g = torch.Generator(device="cuda").manual_seed(0)
+    x, gy, v0 = (torch.randn(2, 40, 2, 64, device="cuda", generator=g).bfloat16() for _ in range(3))
+    w, lam = torch.randn(64, device="cuda", generator=g), torch.tensor([0.3], device="cuda")
+    _, rstd = qk_prologue.fwd(x, w, None, None, 1e-6, torch.bfloat16)
+    want = (*qk_prologue.bwd(gy, x, w, None, None, rstd), *value_gate.blend_bwd(gy, x, v0, lam))
+    out = [torch.empty_like(t) for t in want]
+    s1 = torch.full((lib.nlfa_qk_prologue_scratch_bytes(64),), 0xff, dtype=torch.uint8, device="cuda")
+    s2 = torch.full((lib.nlfa_value_blend_scratch_bytes(),), 0xff, dtype=torch.uint8, device="cuda")
+    # one (batch, KV head) pair's dS at a time: 1,024 parts
+    B, T, H, D = 256, 8, 4, 128
+    q, k, v, do = (torch.randn(B, T, H, D, device="cuda", generator=g).bfloat16() for _ in range(4))
+    o, lse = fc.fwd(q, k, v, 0.1, True)
+    grads = fc.bwd(do, q, k, v, o, lse, 0.1, True)
+    parts = [torch.empty_like(t) for t in grads]
+    tape = (lib.nlfa_bwd_scratch_bytes(B, T, H) + 255) // 256 * 256
+    s3 = torch.empty(tape + 32768, dtype=torch.uint8, device="cuda")
+    assert lib.nlfa_bwd_workspace_kernel_count(B, T, H, H, D, 0, 0, 0, L.DTYPE_BF16, L.PATH_TENSOR, s3.numel()) == 2049
+    bf16 = L.DTYPE_BF16
+
+    def steps(stream, n):
+        for _ in range(n):
+            L.check("prologue", lib.nlfa_qk_prologue_bwd(
+                gy.data_ptr(), bf16, x.data_ptr(), bf16, w.data_ptr(), None, None, rstd.data_ptr(), out[0].data_ptr(),
+                out[1].data_ptr(), s1.data_ptr(), s1.numel(), 2, 40, 2, 64, stream))
+            L.check("blend", lib.nlfa_value_blend_bwd(
+                gy.data_ptr(), bf16, x.data_ptr(), v0.data_ptr(), bf16, lam.data_ptr(), out[2].data_ptr(), out[3].data_ptr(),
+                out[4].data_ptr(), s2.data_ptr(), s2.numel(), x.numel(), stream))
+
+    def in_parts(stream):
+        L.check("parts", lib.nlfa_bwd_masked(
+            *(t.data_ptr() for t in (do, q, k, v, o, lse, *parts, s3)), s3.numel(), B, T, H, H, D, 0.1, 0, 0, 0, bf16,
+            L.PATH_TENSOR, L.PASS_ALL, stream))
+
+    steps(torch.cuda.current_stream().cuda_stream, 1)
+    in_parts(torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    for run, count in ((lambda s: steps(s, 500), 17), (in_parts, 8)):            # 17,000 launches, 16,384 in parts
+        for _ in range(count):
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                run(torch.cuda.current_stream().cuda_stream)
+        for t in (*out, *parts):
+            t.fill_(float("nan"))
+        graph.replay()
+        graph.replay()
+        torch.cuda.synchronize()
+        got, ref = (out, want) if count == 17 else (parts, grads)
+        assert all(torch.equal(a, b) for a, b in zip(got, ref))
