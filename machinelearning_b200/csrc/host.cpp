@@ -345,17 +345,27 @@ bool is_tensor(PyObject* o) { return THPVariable_Check(o); }
 bool tensor_or_none(PyObject* o) { return o == Py_None || THPVariable_Check(o); }
 const Tensor& tensor(PyObject* o) { return THPVariable_Unpack(o); }
 Tensor maybe(PyObject* o) { return o == Py_None ? Tensor() : THPVariable_Unpack(o); }
+// What int(o), float(o) and bool(o) give, as the general path takes these arguments (a window of 4.0, a scale tensor).
 int integer(PyObject* o) {
-  const long v = PyLong_AsLong(o);
+  const THPObjectPtr i(PyLong_Check(o) ? Py_NewRef(o) : PyNumber_Long(o));
+  const long v = i ? PyLong_AsLong(i.get()) : -1;
   if (v == -1 && PyErr_Occurred()) throw python_error();
   return static_cast<int>(v);
 }
 double number(PyObject* o) {
-  const double v = PyFloat_AsDouble(o);
-  if (v == -1.0 && PyErr_Occurred()) throw python_error();
-  return v;
+  const THPObjectPtr f(PyFloat_Check(o) ? Py_NewRef(o) : PyNumber_Float(o));
+  if (!f) throw python_error();
+  return PyFloat_AsDouble(f.get());
 }
-bool truth(PyObject* o) { return PyObject_IsTrue(o) == 1; }
+bool truth(PyObject* o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw python_error();
+  return v == 1;
+}
+void require_tensors(const char* fn, PyObject* const* a, int n) {
+  for (int i = 0; i < n; ++i)
+    TORCH_CHECK_TYPE(is_tensor(a[i]), fn, ": argument ", i + 1, " must be a tensor, not ", Py_TYPE(a[i])->tp_name);
+}
 PyObject* decline() { Py_RETURN_NONE; }
 
 bool head_dim(int64_t D) { return D == 32 || D == 64 || D == 128; }
@@ -423,6 +433,7 @@ PyObject* py_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 8, "attn_fwd takes 8 arguments");
+  require_tensors("attn_fwd", a, 3);
   const Mask m{integer(a[5]), integer(a[6]), integer(a[7])};
   const double scale = number(a[3]);
   const bool tc = truth(a[4]);
@@ -440,6 +451,7 @@ PyObject* py_attn_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_attn_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 12, "attn_bwd takes 12 arguments");
+  require_tensors("attn_bwd", a, 6);
   const Mask m{integer(a[9]), integer(a[10]), integer(a[11])};
   const double scale = number(a[6]);
   const bool tc = truth(a[7]), fused = truth(a[8]);

@@ -57,3 +57,26 @@ def test_refusals_and_the_autograd_contract():
     y.backward(do)
     with pytest.raises(RuntimeError, match="second time"):
         y.backward(do)
+
+
+def test_arguments_as_the_python_path_takes_them():
+    """Numbers of any kind, as int() and float() read them; what is no tensor raises instead of being read as one."""
+    import numpy as np
+    from machinelearning_b200 import flash_cuda as fc
+    q = torch.randn(1, 40, 2, 64, device="cuda", dtype=torch.bfloat16)
+    want = fc.flash_attn(q, q, q, 0.25, window=8, sinks=2)
+    for window, sinks, scale in ((8.0, 2.0, np.float32(0.25)), (np.int64(8), True + 1, torch.tensor(0.25)),
+                                 (torch.tensor(8), torch.tensor(2, device="cuda"), "0.25")):
+        assert torch.equal(fc.flash_attn(q, q, q, scale, window=window, sinks=sinks), want)
+        assert torch.equal(fc.fwd(q, q, q, scale, 1, window, sinks)[0], want)
+    k = q.transpose(1, 2).contiguous()
+    want = fc.flash_attn_cached(q, k, k, 0.25, causal=True, window=8, sinks=2)
+    assert torch.equal(fc.flash_attn_cached(q, k, k, np.float64(0.25), causal=np.bool_(True), window=8.0, sinks=2.0), want)
+    for bad in ({"window": None}, {"window": "x"}, {"use_mma": np.ones(2)}):
+        with pytest.raises((TypeError, ValueError)):
+            fc.flash_attn(q, q, q, **bad)
+    with pytest.raises(TypeError):
+        fc.fwd(q, None, q, 0.25, True)
+    o, lse = fc.fwd(q, q, q, 0.25, True)
+    with pytest.raises(TypeError):
+        fc.bwd(None, q, q, q, o, lse, 0.25, True)
