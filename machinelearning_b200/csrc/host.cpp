@@ -22,6 +22,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <cmath>
@@ -347,13 +348,13 @@ const Tensor& tensor(PyObject* o) { return THPVariable_Unpack(o); }
 Tensor maybe(PyObject* o) { return o == Py_None ? Tensor() : THPVariable_Unpack(o); }
 // What int(o), float(o) and bool(o) give, as the general path takes these arguments (a window of 4.0, a scale tensor).
 int integer(PyObject* o) {
-  const THPObjectPtr i(PyLong_Check(o) ? Py_NewRef(o) : PyNumber_Long(o));
+  THPObjectPtr i(PyLong_Check(o) ? Py_NewRef(o) : PyNumber_Long(o));
   const long v = i ? PyLong_AsLong(i.get()) : -1;
   if (v == -1 && PyErr_Occurred()) throw python_error();
   return static_cast<int>(v);
 }
 double number(PyObject* o) {
-  const THPObjectPtr f(PyFloat_Check(o) ? Py_NewRef(o) : PyNumber_Float(o));
+  THPObjectPtr f(PyFloat_Check(o) ? Py_NewRef(o) : PyNumber_Float(o));
   if (!f) throw python_error();
   return PyFloat_AsDouble(f.get());
 }
