@@ -76,19 +76,43 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
                     print(f"== {name}\n{log}")
     objs = [OBJ / (s.stem + ".o") for s in sources()]
     if force or jobs or _stale(LIB, objs):
-        cmd = [nvcc, "-shared", "-o", str(LIB), *map(str, objs),
-               "-gencode", "arch=compute_100a,code=sm_100a"]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+        def link(out):
+            cmd = [nvcc, "-shared", "-o", str(out), *map(str, objs), "-gencode", "arch=compute_100a,code=sm_100a"]
+            r = subprocess.run(cmd, capture_output=True, text=True)
+            if r.returncode != 0:
+                raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+        _into_place(LIB, link)
     build_host(force)
     return LIB
+
+
+def _into_place(target: pathlib.Path, make) -> None:
+    """``make(path)`` under a name of this process's own, then one rename: another process that starts at the same time
+    loads the whole file or none."""
+    part = target.with_name(f"{target.name}.{os.getpid()}.part")
+    try:
+        make(part)
+        os.replace(part, target)
+    finally:
+        part.unlink(missing_ok=True)
+
+
+def _host_stamp() -> str:
+    """What ``_host.so`` was compiled against; ``host.cpp`` carries it as a string."""
+    import torch
+    return f"nlfa host module for torch {torch.__version__}, python {sys.version_info[0]}.{sys.version_info[1]};"
+
+
+def host_fits() -> bool:
+    """Whether ``_host.so`` is there and was compiled against this torch and this Python (it uses torch's C++ interface,
+    which no other build shares)."""
+    return HOST.exists() and _host_stamp().encode() in HOST.read_bytes()
 
 
 def build_host(force: bool = False) -> pathlib.Path:
     """Compile ``csrc/host.cpp``; it finds ``libnlfa.so`` next to itself."""
     src = CSRC / "host.cpp"
-    if not force and not _stale(HOST, [src, PKG.parent / "include" / "nlfa.h"]):
+    if not force and not _stale(HOST, [src, PKG.parent / "include" / "nlfa.h"]) and host_fits():
         return HOST
     import sysconfig
 
@@ -97,14 +121,17 @@ def build_host(force: bool = False) -> pathlib.Path:
     cuda = pathlib.Path(_nvcc()).resolve().parent.parent
     include = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], str(cuda / "include")]
     libs = pathlib.Path(torch.__file__).parent / "lib"
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
-           *(f"-isystem{p}" for p in include), str(src), "-o", str(HOST),
-           f"-L{libs}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
-           f"-L{PKG}", "-l:libnlfa.so", "-Wl,-rpath,$ORIGIN"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"g++ failed on host.cpp:\n{r.stdout}\n{r.stderr}")
+
+    def compile_to(out):
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", f'-DNLFA_HOST_STAMP="{_host_stamp()}"',
+               *(f"-isystem{p}" for p in include), str(src), "-o", str(out),
+               f"-L{libs}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
+               f"-L{PKG}", "-l:libnlfa.so", "-Wl,-rpath,$ORIGIN"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed on host.cpp:\n{r.stdout}\n{r.stderr}")
+    _into_place(HOST, compile_to)
     return HOST
 
 

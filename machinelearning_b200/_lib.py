@@ -101,10 +101,11 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
 
 
 def load_host():
-    """The extension module of ``csrc/host.cpp`` (torch-facing call path); built in-tree when it is absent."""
+    """The extension module of ``csrc/host.cpp`` (torch-facing call path); built in-tree when it is absent or was compiled
+    against another torch or Python."""
     lib = load()
-    if not (PKG / "_host.so").exists():
-        from . import _build
+    from . import _build
+    if not _build.host_fits():
         _build.build_host()
     from . import _host
     return lib, _host

@@ -621,4 +621,13 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_host", "torch-facing call path 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&g_module); }
+#ifndef NLFA_HOST_STAMP
+#define NLFA_HOST_STAMP ""
+#endif
+
+// What this was compiled against (_build.py looks for the text in the file before it is loaded).
+PyMODINIT_FUNC PyInit__host(void) {
+  PyObject* m = PyModule_Create(&g_module);
+  if (m != nullptr) PyModule_AddStringConstant(m, "built_for", NLFA_HOST_STAMP);
+  return m;
+}

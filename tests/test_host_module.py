@@ -78,3 +78,24 @@ def test_window_accepts_valid(fc):
     fc.check_window(0, 0)
     fc.check_window(64, 4)
     fc.check_window(1, 0)
+
+
+def test_host_module_is_rebuilt_for_another_torch_and_put_in_place_whole(tmp_path, monkeypatch):
+    from machinelearning_b200 import _build
+    _build.build()
+    assert _build.host_fits()
+    monkeypatch.setattr(torch, "__version__", "9.9.9")
+    assert not _build.host_fits()                          # up to date by its times, but compiled against another torch
+    target = tmp_path / "x.so"
+    target.write_text("old")
+
+    def interrupted(path):
+        path.write_text("half")
+        assert target.read_text() == "old"                 # nobody loads a file that is being written
+        raise RuntimeError("stopped")
+
+    with pytest.raises(RuntimeError):
+        _build._into_place(target, interrupted)
+    assert target.read_text() == "old" and list(tmp_path.iterdir()) == [target]
+    _build._into_place(target, lambda path: path.write_text("new"))
+    assert target.read_text() == "new" and list(tmp_path.iterdir()) == [target]
