@@ -660,11 +660,6 @@ int nlfa_check_mask_geometry_masked(int T, int window, int sinks, int block, int
           const int qt = orient == 0 ? t : y, kb = orient == 0 ? y : t;
           if (block_fully_visible(qt, kb, window, sinks, block, T) && !all) return 1 + check;
           ++check;
-          if (!all) {
-            const int be = block_edges(qt, kb, window, sinks);
-            if ((be == EDGE_CAUSAL && !causal_only) || (be == EDGE_WINDOW && !window_only)) return 1 + check;
-          }
-          ++check;
         }
       }
   // (4) fused backward: the key blocks that stream query tile t take the turns 0 .. count - 1

@@ -80,23 +80,11 @@ __host__ __device__ inline bool block_fully_visible(int tile, int j, int window,
   return true;
 }
 
-// Which edges of the mask cut through query tile `tile` x key block `j` (for blocks that are
-// not fully visible): only the causal edge k <= q (plain causal, or windows whose lower edge
-// stays below the block), only the window's lower edge k > q - (window - sinks) (blocks below
-// the diagonal that hold no sink keys), or both / sinks involved.  One-edge blocks need a
-// single compare per element against a per-thread limit.
+// The same question for a rectangle of query positions [q_lo, q_hi] x key positions [k_lo, k_hi] (tiles of unequal
+// height), and which edges of the mask cut through one that is not fully visible: only the causal edge k <= q (plain
+// causal, or windows whose lower edge stays below it), only the window's lower edge k > q - (window - sinks) (below the
+// diagonal, no sink keys), or both / sinks involved.  With one edge a compare per element against a per-thread limit does.
 enum { EDGE_CAUSAL = 0, EDGE_WINDOW = 1, EDGE_BOTH = 2 };
-__host__ __device__ inline int block_edges(int tile, int j, int window, int sinks) {
-  if (window == 0) return EDGE_CAUSAL;
-  const int span = window - sinks;
-  const int last_row = tile * kTile + kTile - 1;
-  if (j * kTile > last_row - span) return EDGE_CAUSAL;           // lower edge below the block
-  if (j < tile && j * kTile >= sinks) return EDGE_WINDOW;        // causal edge above, no sink keys
-  return EDGE_BOTH;
-}
-
-// The same two questions for a rectangle of query positions [q_lo, q_hi] x key positions
-// [k_lo, k_hi] (tiles of unequal height).
 __host__ __device__ inline bool rect_fully_visible(int q_lo, int q_hi, int k_lo, int k_hi,
                                                    int window, int sinks, int block = 0, int t_len = 1 << 30) {
   if (k_hi > last_key_of_query(q_lo, block, t_len)) return false;          // causal edge cuts in
