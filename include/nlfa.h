@@ -279,8 +279,7 @@ int nlfa_head_gate_bwd(const void* g, const void* y, int y_dtype, const void* ga
  * zeros and lse = -inf.
  * With few query rows (long caches, small batches) the keys are split over the CTAs of a cluster, which
  * combine their partial rows in a fixed order through distributed shared memory.  Nothing is kept in
- * `scratch`, which may be NULL; it and nlfa_fwd_cached_scratch_bytes (what a split through global memory
- * would take) remain for existing callers. */
+ * `scratch`, which may be NULL; it and nlfa_fwd_cached_scratch_bytes (0) remain for existing callers. */
 size_t nlfa_fwd_cached_scratch_bytes(int B, int Tq, int H, int Hkv, int L, int D);
 int nlfa_fwd_cached(const void* q, const void* k_cache, const void* v_cache, void* o, float* lse,
                     const int* qpos, const int* kpos, int B, int Tq, int H, int Hkv, int L, int D,

@@ -331,18 +331,6 @@ int launch_simt(const CachedParams& p, const void* q, const void* k, const void*
   return launch_dim<T, 128>(p, q, k, v, st);
 }
 
-// How many ways the keys would be split through global memory (nlfa_fwd_cached_scratch_bytes).
-int choose_splits(int B, int Tq, int H, int Hkv, int L, int D) {
-  const long long rpc = D <= 64 ? 8 : 4;
-  const long long base = static_cast<long long>(B) * Hkv * ((static_cast<long long>(Tq) * (H / Hkv) + rpc - 1) / rpc);
-  const long long tiles = (L + 31) / 32;
-  if (base <= 0 || base >= 296 || tiles < 8) return 1;
-  long long s = (592 + base - 1) / base;
-  if (s > tiles / 4) s = tiles / 4;
-  if (s > 32) s = 32;
-  return s < 1 ? 1 : static_cast<int>(s);
-}
-
 }  // namespace
 
 // tensor-core form (cached_tc.cu)
@@ -354,11 +342,8 @@ unsigned* status_block();      // api.cu
 
 }  // namespace nlfa
 
-extern "C" size_t nlfa_fwd_cached_scratch_bytes(int B, int Tq, int H, int Hkv, int L, int D) {
-  if (B <= 0 || Tq <= 0 || H <= 0 || Hkv <= 0 || L <= 0 || H % Hkv != 0) return 0;
-  const int s = nlfa::choose_splits(B, Tq, H, Hkv, L, D);
-  return s <= 1 ? 0 : static_cast<size_t>(B) * Tq * H * s * (static_cast<size_t>(D) + 1) * sizeof(float);
-}
+// Nothing is kept in scratch: the partial rows of a split stay in the cluster's shared memory.
+extern "C" size_t nlfa_fwd_cached_scratch_bytes(int, int, int, int, int, int) { return 0; }
 
 extern "C" int nlfa_fwd_cached(const void* q, const void* k_cache, const void* v_cache, void* o, float* lse,
                                const int* qpos, const int* kpos, int B, int Tq, int H, int Hkv, int L, int D,
@@ -381,7 +366,7 @@ extern "C" int nlfa_fwd_cached_positions(const void* q, const void* k_cache, con
                                          int Hkv, int L, int D, float scale, int causal, int window, int sinks, int dtype,
                                          int path, void* scratch, size_t scratch_bytes, void* stream) {
   using namespace nlfa;
-  (void)scratch;                 // the split's partial rows stay in shared memory
+  (void)scratch;
   (void)scratch_bytes;
   if (path != NLFA_PATH_AUTO && path != NLFA_PATH_SIMT && path != NLFA_PATH_TENSOR) return NLFA_ERR_UNSUPPORTED_PATH;
   if (position_bytes != 4 && position_bytes != 8) return NLFA_ERR_BAD_ARGUMENT;

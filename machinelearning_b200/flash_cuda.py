@@ -391,8 +391,9 @@ def flash_attn_cached(q: torch.Tensor, k_full: torch.Tensor, v_full: torch.Tenso
     Forward only (nanolab runs this path under ``no_grad``); returns ``[B,T,H,D]`` (and the
     logsumexp ``[B,H,T]`` with ``return_lse``).  Raises ``ValueError`` for unsupported inputs.
     ``use_mma`` as in ``flash_attn``: ``None`` lets the library take its tensor-core kernel where it
-    applies (16-bit inputs, a block of at least 16 rows per KV head over at least 256 keys) and the fp32
-    kernel elsewhere; ``False`` / ``True`` force one (``True`` raises where it does not apply).
+    can run the call (16-bit inputs, up to 128 query heads per KV head, a positive scale) and the fp32 kernel
+    elsewhere; ``False`` / ``True`` force one (``True`` raises below 16 rows per KV head or 256 keys, where the
+    tensor-core kernel takes each probability as two 16-bit values to come out at fp32 precision).
     """
     if _load() is not None:
         out = _host.attn_cached(q, k_full, v_full, scale, qpos, kpos, causal, window, sinks, return_lse, use_mma)
