@@ -39,6 +39,7 @@ unsigned* g_status_mirror[kMaxDevices];      // host address of the registered c
 unsigned* g_sched_ptr[kMaxDevices];
 unsigned* g_ticket_ptr[kMaxDevices];
 int g_sm_count[kMaxDevices];
+long long g_l2_bytes[kMaxDevices];
 std::atomic<unsigned> g_next_eager{0};
 std::atomic<unsigned> g_next_graph{0};
 std::atomic<unsigned> g_next_ticket{0};
@@ -341,6 +342,18 @@ bool overlap_launches(int kernel) {
     return v != nullptr ? std::atoi(v) : kOverlapDefault;
   }();
   return (mask & kernel) != 0;
+}
+
+long long l2_bytes() {
+  const int dev = current_device();
+  if (dev < 0) return 0;
+  std::lock_guard<std::mutex> lock(g_host_mutex);
+  if (g_l2_bytes[dev] == 0) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrL2CacheSize, dev) != cudaSuccess || n <= 0) n = 1;
+    g_l2_bytes[dev] = n;
+  }
+  return g_l2_bytes[dev];
 }
 
 int sm_count() {

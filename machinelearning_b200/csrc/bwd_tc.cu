@@ -1268,8 +1268,9 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
     const long long rows = p.window > 0 && p.window + 2 * kTile < p.T ? p.window + 2 * kTile : p.T;
     const long long bytes = rows * p.D * 4 * (p.H / p.Hkv);                     // of a pair's streamed tiles in use
     const long long together = bp.BH < grid ? bp.BH : grid, most = bp.total_units / (2ll * grid);
-    if (bytes * together > (64ll << 20) && most > 1) {
-      const long long fits = bytes < (32ll << 20) ? (32ll << 20) / bytes : 1, want = (bp.BH + fits - 1) / fits;
+    const long long l2 = l2_bytes();
+    if (bytes * together > l2 / 2 && most > 1) {
+      const long long fits = bytes < l2 / 4 ? l2 / 4 / bytes : 1, want = (bp.BH + fits - 1) / fits;
       const int groups = static_cast<int>(want < most ? want : most);
       const int size = (bp.BH + groups - 1) / groups;
       bp.sched_group = size < grid ? size : grid;

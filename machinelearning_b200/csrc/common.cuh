@@ -221,6 +221,7 @@ int launch_ticket(cudaStream_t stream, unsigned* own, unsigned** out, bool* capt
 int ensure_dynamic_smem(const void* kernel, int bytes);
 
 int sm_count();
+long long l2_bytes();
 
 // How many clusters of `size` CTAs (up to kMostCluster, along y) of a kernel can be resident at once; asked of the
 // driver once per kernel and device.

@@ -780,19 +780,22 @@ int launch_fwd_tc(const Problem& p, const void* q, const void* k, const void* v,
   const bool bf16 = p.dtype == NLFA_DTYPE_BF16;
   // One tile per unit or two?  Two share every K / V tile, which is less traffic and power; one -- at D <= 64 with two
   // CTAs per SM, four contexts' worth of unit starts and ends overlapping -- balances better and wastes nothing on the
-  // second tile's longer row.  Run long enough for the power cap to hold, two tiles win at D <= 64 as soon as K and V no
-  // longer fit in L2 (one / two tiles per unit, H=8: T=1024 B=32 72.9 / 73.4 us, B=128 317 / 295; T=4096 B=8 214 / 208,
-  // B=32 1,013 / 896) except over rows of two tiles (T=256 B=512 139 / 151); below that one does (B=8 H=12 T=1024
-  // 28.8 / 30.8, B=2 T=4096 79.5 / 82.3) up to rows of 4,096, and where there are no more tiles than SMs.  Rows of up to
-  // 1,024 waste most on the second tile: there the line is all of L2, not the half next to an SM (H=12 T=1024 B=32, 100 MB,
-  // between backward passes: 101 / 107; alone level; B=64 T=512 H=8 48.8 / 50.7).
+  // second tile's longer row.  One wins where there are no more tiles than SMs, over rows of up to two tiles (one / two
+  // tiles per unit, us: T=256 B=512 H=8 139 / 151), and up to a reach (the row, or its window) of 4,096 while K and V take
+  // half of L2 (B=8 H=12 T=1024 28.8 / 30.8, B=2 T=4096 79.5 / 82.3; T=4096 H=8 B=8, 67 MB, 214 / 208, B=32 1,013 / 896).
+  // Rows that reach no more than 1,024 waste most on the second tile: there the line is all of L2.  After 0.3 s of load,
+  // of 27 shapes with 64 to 128 MiB of K and V one tile won 26: T=1024 B=24 H=16 109 / 117, B=48 H=8 109 / 118, B=90
+  // H=12/4 298 / 310, D=32 B=64 H=12 183 / 192; T=512 B=64 H=12 70 / 81; T=300 B=40 H=32 72 / 100; window 256 T=4096 B=8
+  // H=12 82 / 84, T=16384 B=3 H=8 82 / 84; window 512 T=2048 B=16 H=12 109 / 112; the other, window 1,000 T=8192 B=4 H=12,
+  // 186 / 183 with 7 between its runs.  Further on it depends on the chip: T=1024 H=8 B=128, 268 MB, 317 / 295 on one, B=100
+  // 239 / 249 on another.
   // D = 128 (one CTA per SM either way): one tile while that makes at most two units per SM (B=1 H=8 T=4096:
   // 42.6 / 65.9 us; 3.5 per SM: 45.2 / 41.9).
   const long long tiles = static_cast<long long>(p.B) * p.H * ((p.T + kTile - 1) / kTile);
   const long long kv_bytes = static_cast<long long>(p.B) * p.Hkv * p.T * p.D * 4;
   const int reach = p.window > 0 && p.window < p.T ? p.window : p.T;
   const bool single = p.D == 128 ? tiles <= 2ll * sm_count() || p.T <= kTile
-                                 : (reach <= 4096 && kv_bytes < (reach <= 1024 ? 2 : 1) * (64ll << 20)) || p.T <= 2 * kTile || tiles <= sm_count();
+                                 : (reach <= 4096 && kv_bytes < (reach <= 1024 ? l2_bytes() : l2_bytes() / 2)) || p.T <= 2 * kTile || tiles <= sm_count();
   auto go = [&](auto type) {
     using T = decltype(type);
     if (single) {
