@@ -129,9 +129,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   constexpr bool kSepP = NT * (128 + D + 64) <= 512;      // P has columns of its own
   constexpr uint32_t kPBase = NT * (128 + D);
   constexpr int kRing = L::kRing;
-  // Registers per thread: at launch, of the softmax warps, of the others.  (NT = 1 at D = 128 has the SM to itself and as
-  // many as it can use from the start.)
-  constexpr bool kMoveRegs = NT == 2 || D == 64;
+  // registers per thread: at launch, of the softmax warps, of the others
   constexpr int kRegsLaunch = NT == 1 ? 128 : 168, kRegsCompute = NT == 1 ? 200 : 216, kRegsOther = NT == 1 ? 56 : 72;
 
   extern __shared__ uint8_t smem_raw[];
@@ -216,10 +214,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   // Register reallocation: the warpgroup of the producer, the MMA issuer and two spare warps
   // gives most of its registers to the softmax warpgroups.
   if (warp >= 4 * NT) {
-  if constexpr (kMoveRegs) setmaxnreg_dec<kRegsOther>();
+  setmaxnreg_dec<kRegsOther>();
   // setmaxnreg.inc blocks until the registers it asks for have been released, so the four
   // warps that shrink must free at least what those that grow take.
-  static_assert(!kMoveRegs || (kRegsLaunch - kRegsOther) * 4 >= (kRegsCompute - kRegsLaunch) * 4 * NT,
+  static_assert((kRegsLaunch - kRegsOther) * 4 >= (kRegsCompute - kRegsLaunch) * 4 * NT,
                 "register reallocation does not balance");
   if (dead || warp >= 4 * NT + 2) {
     // nothing to do (spare warps only complete the warpgroup)
@@ -486,7 +484,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
   } else {
     // ================================= softmax ===============================
-    if constexpr (kMoveRegs) setmaxnreg_inc<kRegsCompute>();
+    setmaxnreg_inc<kRegsCompute>();
     if (!dead) {
     const int t = warp >> 2;                       // query tile of this warpgroup
     const int row = threadIdx.x - 128 * t;         // row inside the tile == TMEM lane
