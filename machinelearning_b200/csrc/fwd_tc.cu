@@ -129,8 +129,11 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   constexpr bool kSepP = NT * (128 + D + 64) <= 512;      // P has columns of its own
   constexpr uint32_t kPBase = NT * (128 + D);
   constexpr int kRing = L::kRing;
-  // registers per thread: at launch, of the softmax warps, of the others
-  constexpr int kRegsLaunch = NT == 1 ? 128 : 168, kRegsCompute = NT == 1 ? 200 : 216, kRegsOther = NT == 1 ? 56 : 72;
+  // Registers per thread: at launch, of the softmax warps, of the others.  NT = 1 at D = 128 has the SM to itself, and the
+  // compiler lets it start with as many as the softmax warps ask for: there the request raises nothing.
+  constexpr bool kOwnSm = NT == 1 && D == 128;
+  constexpr int kRegsCompute = kOwnSm ? 208 : NT == 1 ? 200 : 216, kRegsOther = NT == 1 ? 56 : 72;
+  constexpr int kRegsLaunch = kOwnSm ? kRegsCompute : NT == 1 ? 128 : 168;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
