@@ -833,7 +833,7 @@ def run_whole_model_arm(args, rank, world, local_rank):
         "e2e": {"value": tokens / (e2e_ms * 1e-3), "unit": "tokens/s", "ms_per_step": e2e_ms,
                 "h2d_bytes_per_step": 2 * x_pin.numel() * x_pin.element_size(), "d2h_bytes_per_step": 4},
         # per flash_attn call: the forward and the backward's kernels for this per-GPU shape (three, or two
-        # when the dQ pass forms Delta itself); the prologue, blend and gate calls launch 3, 3 and 2 each
+        # when the dQ pass forms Delta itself); the prologue, blend and gate calls launch 2 each
         "gpu_launches": (1 + attn_bwd_kernels) * n_calls["n"] + 2 * n_calls["prologue"] + 2 * n_calls["blend"]
                         + 2 * n_calls["gate"],
         "library_calls_per_step": {"flash_attn": n_calls["n"] // steps, "qk_prologue": n_calls["prologue"] // steps,

@@ -498,7 +498,7 @@ size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window,
   // The dQ pass that recomputes dS starts beside the dK/dV pass and takes the SMs it leaves idle; one that reads
   // dS cannot.  So every launch has to keep the GPU busy by itself: half as many units (key blocks) again as SMs,
   // three per SM where the problem goes in parts.  Measured recomputing / reading: B=2 H=8/2 T=3000 (96 units)
-  // 200 / 264 us, B=4 H=12/4 T=2048 (256) 198 / 182, B=22 H=12 T=60 (264) 32 / 29, two parts of 218 units each
+  // 200 / 264 us, B=4 H=12/4 T=2048 (256) 204 / 190, B=22 H=12 T=60 (264) 31 / 25, two parts of 218 units each
   // (B=4 H=4/1 T=13866) 3.26 / 3.42 ms for the whole step.
   const size_t parts = (all + most - 1) / most, per = (all + parts - 1) / parts;
   const size_t units = per * ((T + kTile - 1) / kTile), sms = static_cast<size_t>(sm_count());

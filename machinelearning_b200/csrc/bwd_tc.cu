@@ -1322,7 +1322,7 @@ int launch_both(const Problem& p, const void* dout, const void* q, const void* k
     // exponent phase per tile pair instead of seven and two.  As many (batch, KV head) pairs at a time as
     // the scratch holds, shared out evenly.  At D = 128 the dS traffic (32 KB written and read per pair of
     // 128 x 128) hides behind the pass's products and the dQ pass runs at DRAM speed: B=1 H=16 T=16384
-    // backward 3.70 -> 3.08 ms, B=2 T=8192 1.82 -> 1.64 ms, B=4 H=12/4 T=2048 190 -> 172 us.  At D = 64 a
+    // backward 3.63 -> 3.25 ms, B=2 T=8192 1.94 -> 1.72 ms, B=4 H=12/4 T=2048 204 -> 190 us.  At D = 64 a
     // tile pair has half the products for the same bytes and the staging tile costs a streamed stage
     // (B=32 H=12 T=1024: 274 -> 300 us), so there the dQ pass recomputes dS.
     const DsLayout layout = ds_layout(p.T, p.window, p.sinks, p.block);

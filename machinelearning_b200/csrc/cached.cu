@@ -18,8 +18,8 @@
 // multiply-add, but a block of a few rows needs CTAs.  Key blocks no row of the CTA can see (contiguous positions)
 // are skipped without being read; with few row tiles the key blocks are split over the CTAs of a cluster, which
 // combine the partial rows through distributed shared memory in a fixed order.  No atomics: bit-reproducible.
-// A warp of lanes over the keys of 8 rows before -> tiles: B=2 H=8 T=32 L=2048 D=64 in fp32 56 -> 28 us,
-// B=4 H=16/4 T=100 L=4096 848 -> 353 us.
+// A warp of lanes over the keys of 8 rows before -> tiles: B=2 H=8 T=32 L=2048 D=64 in fp32 56 -> 25 us,
+// B=4 H=16/4 T=100 L=4096 848 -> 367 us.
 #include "cached.cuh"
 #include "tiles.cuh"
 

@@ -9,9 +9,9 @@
 // warp's own rows are involved, so that exchange needs no CTA-wide barrier.  No atomics: bit-reproducible.
 //
 // RM = 8, 4 or 2 by the number of row tiles (rows_per_thread).  The dQ pass runs beside the dK/dV pass.
-// Measured, a row per warp before -> tiles: B=4 H=4 T=256 D=64 forward 82 -> 18 us, backward 174 -> 36 us
-// (latency); B=8 H=12/4 T=2048 D=64 forward 14.9 -> 1.41 ms (37 TFLOP/s, half of
-// what the FMA pipe can issue), backward 32.0 -> 4.98 ms.
+// Measured, a row per warp before -> tiles: B=4 H=4 T=256 D=64 forward 82 -> 16 us, backward 174 -> 34 us
+// (latency); B=8 H=12/4 T=2048 D=64 forward 14.9 -> 1.49 ms (35 TFLOP/s, half of
+// what the FMA pipe can issue), backward 32.0 -> 4.63 ms.
 //
 // Algebra follows the reference's FMA kernels (nanolab/csrc/flash_attn_cuda.cu
 // :147-281 forward, :1234-1262 Delta, :1265-1366 dQ, :1371-1482 dK/dV): softmax
