@@ -21,11 +21,18 @@
 // 59 -> 41 us (4.9 TB/s); B=14 H=12 D=32, 8 over 3,000: 60 -> 39; B=1 H=12 D=64, 32 over 1,056: 8.8 -> 7.3.
 //
 // With few (batch, KV head) pairs the key blocks are split over the CTAs of a cluster (up to 16, as many as can be
-// resident).  At the end a CTA's parts of a row become one in shared memory, each CTA sends every other one the rows that
-// one finishes (a bulk copy per pair, counted by a barrier there), and a row's parts are added in the order of the
-// CTAs: no scratch, no second kernel, no wait for a remote read.  (Reading two parts per CTA from all the others, the
-// same one at the same time, took 4.5 of the 14.8 us of B=1 H=16 D=128, 64 queries over 2,048 keys, now 11.7; through
-// global memory with a ticket it was more still.)  B=1 H=16 D=128, 64 over 16,448: 35.7 -> 31.0 us (4.35 TB/s of K, V).
+// resident).  At the end a CTA's parts of a row become one, each CTA sends every other one the rows that one finishes (a bulk
+// copy per pair, counted by a barrier there), and a row's parts are added in the order of the CTAs: no scratch, no second
+// kernel, no wait for a remote read.  (Remote reads took 4.5 of 14.8 us of B=1 H=16 D=128, 64 queries over 2,048 keys; through
+// global memory with a ticket it was more still; 16-byte remote stores, 2,800 clocks where the copies take 1,100.)
+//
+// Of a small block this end is half of the time, and it is a chain of short steps by few warps, so what counts is its length:
+// the parts' statistics are exchanged, and their weights formed, while the last products run; the two warpgroups' sums of a
+// row stand in one TMEM lane, so each warpgroup adds up half of the columns in registers and only copies go through shared
+// memory; no element has a branch of its own (a condition on the number of blocks inside the loop over columns cost 34 clocks
+// a column); a thread finishing a row loads all of its parts at once.  Before / after (us): B=1 H=12 D=64, 32 over 1,056
+// 6.3 / 5.7; B=1 H=16 D=128, 64 over 2,048 10.5 / 9.5, 64 over 16,448 31.0 / 28.0 (4.8 TB/s of K, V), 128 over 4,096 17.6 / 15.1;
+// B=1 H=2 D=64, 100 over 129 13.4 / 9.7; one query over 1,057 (SPLIT_P) 6.8 / 6.1.
 //
 // SPLIT_P: blocks so small that the fp32 kernel used to take them keep its precision: P goes in as the sum of two
 // 16-bit values (its rounding error is then below the accumulator's), at the price of a second P V product,
@@ -39,6 +46,7 @@
 // Warps 0-3 and 4-7 softmax, 8 TMA producer, 9 MMA issuer and TMEM owner, 10-11 idle or (SPLIT_P) looking through V; they
 // complete the warpgroup that gives its registers to the softmax warps.  Every wait bounded.
 #include <climits>
+#include <type_traits>
 
 #include "cached.cuh"
 
@@ -52,6 +60,7 @@ constexpr int kNoKey = INT_MAX;          // position written for keys past the e
 
 struct TileParams {
   int group, tq_tile, n_qtiles;          // query heads per KV head; block positions per CTA; tiles per (b, hk)
+  FastDiv by_group, by_qtiles, by_heads, by_splits;
   unsigned* status;
   const void* v;
 };
@@ -64,13 +73,12 @@ struct CachedSmem {
   static constexpr int kQ = kV + STAGES * kTileBytes;
   static constexpr int kPos = kQ + kTileBytes;                   // per K stage: 128 key positions
   static constexpr int kFull = kPos + STAGES * 512;              // per K stage: every key visible to every row
-  // A partial row: D sums, (maximum, sum of exponentials) of its part (with one copy: of both), the same of the CTA's parts
-  // together, padding (12 floats, not 8: lanes a row apart hit different banks).  Of a split tile, what the CTAs of the
-  // cluster send comes behind them, one row each for every row this CTA finishes; with one copy, the two parts' rows
-  // are then the same (of any column, one of them is handed over), for room.
-  static constexpr int kPitch = 4 * (D + 12);
-  static constexpr int kReceived = kK + (COPIES == 1 ? 128 : 256) * kPitch;
-  static constexpr int kPartStep = kTile / COPIES * kPitch, kSplitPartStep = COPIES == 1 ? 0 : kPartStep;
+  // Rows of sums on their way together, four floats of padding apart (lanes a row apart hit different banks) in which the
+  // maximum, the sum of exponentials and whether V held a value that is not finite travel: what the copies hand over, the
+  // tile's rows, and what the CTAs of a split tile send, one row each for every row this CTA finishes.
+  static constexpr int kPitch = 4 * (D + 4);
+  static constexpr int kRows = kK + (COPIES > 1 ? kTile * kPitch : 0);
+  static constexpr int kReceived = kRows + kTile / COPIES * kPitch;
   static constexpr int kBar = kFull + (STAGES * 4 + 15) / 16 * 16;
   // barriers: q_full, s_full[2], p_full[2], o_done, group, received, k_full[S], k_empty[S], v_full[S], v_empty[S], v_clean[S], scanned
   static constexpr int kNumBars = 9 + 5 * STAGES;
@@ -79,13 +87,34 @@ struct CachedSmem {
   static constexpr int kSpoilt = kAbort + 4;                     // V held a value that is not finite
   static constexpr int kTotal = kSpoilt + 4;
   static constexpr int kDynamic = kTotal + 1024;
-  static_assert(STAGES * 2 * kTileBytes >= kReceived + (kTile / COPIES + kMostCluster) * kPitch && STAGES * 2 * kTileBytes >= 256 * kPitch, "the combination lies over dead tiles");
+  static_assert(STAGES * 2 * kTileBytes >= kReceived + (kTile / COPIES + kMostCluster) * kPitch && kTileBytes >= 256 * 8,
+                "the combination lies over dead tiles");
 };
+
+// N columns of a row whose V held values that are not finite: what the row sees of them, as it is (`vr`: the columns of
+// the first key).  A call: rare, and long.
+template <typename T, int N>
+__device__ __noinline__ void put_right(const CachedParams& p, const T* vr, int t, float (&x)[N]) {
+  const int q_at = cached::query_position(p, t);
+  float odd[N] = {};
+  for (int key = 0; key < p.L; ++key, vr += p.D) {
+    if (!cached::position_visible(p, q_at, cached::key_position(p, key))) continue;
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+      const float y = static_cast<float>(vr[e]);
+      if (!isfinite(y)) odd[e] += y;
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < N; ++e)
+    if (odd[e] != 0.f) x[e] = odd[e];
+}
 
 template <typename T, int D, int STAGES, int COPIES, bool SPLIT_P>
 __global__ void __launch_bounds__(384, 1)
 cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                 const __grid_constant__ CUtensorMap tm_v, const CachedParams p, const TileParams tp) {
+                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CachedParams p,
+                 const __grid_constant__ TileParams tp) {
   using L = CachedSmem<D, STAGES, COPIES>;
   constexpr int kLanes = kTile / COPIES, kCols = kTile / COPIES;   // of a copy: its TMEM lanes, its columns of S
   constexpr int kBoxes = D / 64;
@@ -110,26 +139,60 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   volatile int* full_flag = reinterpret_cast<volatile int*>(gen + L::kFull);
   const WaitCtx wctx{abort_flag, tp.status};
 
-  if (threadIdx.x == 0) {
-    *abort_flag = (*reinterpret_cast<volatile unsigned*>(tp.status) != STATUS_OK) ? 1 : 0;
-    *spoilt_flag = 0;
-    mbar_init(bar(Q_FULL), 1);
-    for (int w = 0; w < 2; ++w) {
-      mbar_init(bar(S_FULL + w), 1);
-      mbar_init(bar(P_FULL + w), 128);
-    }
-    mbar_init(bar(O_DONE), 1);
-    mbar_init(bar(GROUP), 256);
-    mbar_init(bar(RECEIVED), 1);
-    mbar_init(bar(SCANNED), 2);
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(bar(K_FULL + s), 1);
-      mbar_init(bar(K_EMPTY + s), 1);
-      mbar_init(bar(V_FULL + s), 1);
-      mbar_init(bar(V_EMPTY + s), 1);
-      mbar_init(bar(V_CLEAN + s), 2);
-    }
+  // this CTA's tile and its share of the key blocks the tile sees
+  const int unit = blockIdx.x, bh = tp.by_qtiles.div(unit), qt = unit - bh * tp.n_qtiles;
+  const int b = tp.by_heads.div(bh), hk = bh - b * p.Hkv;
+  const int t0 = qt * tp.tq_tile;
+  const int t1 = (t0 + tp.tq_tile < p.Tq ? t0 + tp.tq_tile : p.Tq) - 1;
+  const KeyRange range = cached::key_range(p.Tq, p.L, p.qpos != nullptr || p.kpos != nullptr, p.causal, p.window, p.sinks,
+                                           t0, t1, kTile);
+  const int per = tp.by_splits.div(range.count + p.splits - 1);
+  const int n_begin = static_cast<int>(blockIdx.y) * per;
+  const int n_stop = n_begin + per < range.count ? n_begin + per : range.count;
+  const int n_blocks = n_stop > n_begin ? n_stop - n_begin : 0;            // block i of this CTA: range.at(n_begin + i)
+  const int n_rows = tp.group * (t1 - t0 + 1);
+  // of these this CTA finishes rows_each, from own_first on (fewer at the end)
+  const int rank = static_cast<int>(blockIdx.y);
+  const int rows_each = tp.by_splits.div(n_rows + p.splits - 1), own_first = rank * rows_each;
+  const int own = own_first >= n_rows ? 0 : own_first + rows_each < n_rows ? rows_each : n_rows - own_first;
+  // Set-up by different warps at once: the barriers, and behind them the loads of Q and of the first block, whose latency then
+  // passes under the rest of it (B=1 H=16 D=128, 64 over 16,448: 31.5 -> 29.6 us; every stage's loads there would hold up the
+  // others: B=14 H=12 D=32, 8 over 3,000, 39.9 -> 43 us).
+  const int ahead = n_blocks < 1 ? 0 : 1;
+  auto load_k = [&](int i) {
+    const int s = i % STAGES, j = range.at(n_begin + i);
+    mbar_expect_tx(bar(K_FULL + s), L::kTileBytes);
+    for (int x = 0; x < kBoxes; ++x)
+      tma_load_4d(base + L::kK + s * L::kTileBytes + x * kBoxBytes, &tm_k, bar(K_FULL + s), 64 * x, j * kTile, hk, b);
+  };
+  auto load_v = [&](int i) {
+    const int s = i % STAGES, j = range.at(n_begin + i);
+    mbar_arrive_expect_tx(bar(V_FULL + s), L::kTileBytes);
+    for (int x = 0; x < kBoxes; ++x)
+      tma_load_4d(base + L::kV + s * L::kTileBytes + x * kBoxBytes, &tm_v, bar(V_FULL + s), 64 * x, j * kTile, hk, b);
+  };
+  if (warp == 8) {
+    if (lane < 3) tma_prefetch_desc(lane == 0 ? &tm_q : lane == 1 ? &tm_k : &tm_v);
+    for (int i = lane; i < L::kNumBars; i += 32)
+      mbar_init(bar(i), i >= P_FULL && i < P_FULL + 2 ? 128u : i == GROUP ? 256u : i >= V_CLEAN ? 2u : 1u);
     fence_mbar_init();
+    __syncwarp();
+    grid_dep_wait();
+    if (lane == 0) {
+      if (p.splits > 1) mbar_arrive_expect_tx(bar(RECEIVED), p.splits * own * L::kPitch);
+      mbar_arrive_expect_tx(bar(Q_FULL), COPIES * kBoxes * tp.group * tp.tq_tile * 128);
+      for (int x = 0; x < COPIES * kBoxes; ++x)
+        tma_load_4d(base + L::kQ + x / COPIES * kBoxBytes + x % COPIES * kLanes * 128, &tm_q, bar(Q_FULL), 64 * (x / COPIES), hk * tp.group, t0, b);
+      for (int i = 0; i < ahead; ++i) {
+        load_k(i);
+        load_v(i);
+      }
+    }
+    __syncwarp();
+  }
+  if (threadIdx.x == 0) {
+    *spoilt_flag = 0;
+    *abort_flag = (*reinterpret_cast<volatile unsigned*>(tp.status) != STATUS_OK) ? 1 : 0;
   }
   if (warp == 9) {
     tmem_alloc(base + L::kTmemSlot, kTmemCols);
@@ -140,31 +203,6 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const bool dead = *abort_flag != 0;
-  // this CTA's tile and its share of the key blocks the tile sees
-  const int unit = blockIdx.x;
-  const int qt = unit % tp.n_qtiles;
-  const int bh = unit / tp.n_qtiles;
-  const int hk = bh % p.Hkv, b = bh / p.Hkv;
-  const int t0 = qt * tp.tq_tile;
-  const int t1 = (t0 + tp.tq_tile < p.Tq ? t0 + tp.tq_tile : p.Tq) - 1;
-  const KeyRange range = cached::key_range(p.Tq, p.L, p.qpos != nullptr || p.kpos != nullptr, p.causal, p.window, p.sinks,
-                                           t0, t1, kTile);
-  const int per = (range.count + p.splits - 1) / p.splits;
-  const int n_begin = static_cast<int>(blockIdx.y) * per;
-  const int n_stop = n_begin + per < range.count ? n_begin + per : range.count;
-  const int n_blocks = n_stop > n_begin ? n_stop - n_begin : 0;            // block i of this CTA: range.at(n_begin + i)
-  const int n_rows = tp.group * (t1 - t0 + 1);
-  // of these this CTA finishes rows_each, from own_first on (fewer at the end)
-  const int rank = static_cast<int>(blockIdx.y);
-  const int rows_each = (n_rows + p.splits - 1) / p.splits, own_first = rank * rows_each;
-  const int own = own_first >= n_rows ? 0 : own_first + rows_each < n_rows ? rows_each : n_rows - own_first;
-  if (threadIdx.x == 0 && p.splits > 1) mbar_arrive_expect_tx(bar(RECEIVED), p.splits * own * L::kPitch);
-  if (warp == 8 && lane == 0) {
-    tma_prefetch_desc(&tm_q);
-    tma_prefetch_desc(&tm_k);
-    tma_prefetch_desc(&tm_v);
-  }
-
   // the tile's query positions, as a range (every lane of a warp)
   auto tile_positions = [&](int& qp_min, int& qp_max) {
     if (!p.qpos) {
@@ -189,8 +227,23 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (warp >= 8) {
     setmaxnreg_dec<kRegsOther>();
     static_assert((kRegsLaunch - kRegsOther) * 4 >= (kRegsCompute - kRegsLaunch) * 8, "register reallocation does not balance");
-    if (dead || (!SPLIT_P && warp >= 10)) {
-      // a give-up recorded earlier makes this launch a no-op; spare warps
+    if (dead) {
+      // A give-up recorded earlier makes this launch a no-op.  Its loads are in flight: they land before the CTA leaves.
+      if (warp == 8 && lane == 0) {
+        const unsigned long long t0 = globaltimer_ns();
+        auto landed = [&](uint32_t bb) {
+          while (!mbar_try_wait(bb, 0))
+            if (globaltimer_ns() - t0 > wctx.limit()) break;
+        };
+        landed(bar(Q_FULL));
+        for (int i = 0; i < ahead; ++i) {
+          mbar_arrive(bar(K_FULL + i));                          // (the arrival that brings the block's positions)
+          landed(bar(K_FULL + i));
+          landed(bar(V_FULL + i));
+        }
+      }
+    } else if (!SPLIT_P && warp >= 10) {
+      // spare warps
     } else if (warp >= 10) {
       // ============ V of blocks the mask cuts: no hidden infinities and NaN ====
       int qp_min, qp_max;
@@ -236,11 +289,6 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (lane == 0) mbar_arrive(bar(SCANNED));                  // the flag is final
     } else if (warp == 8) {
       // =============================== TMA producer ============================
-      if (lane == 0) {
-        mbar_arrive_expect_tx(bar(Q_FULL), COPIES * kBoxes * tp.group * tp.tq_tile * 128);
-        for (int x = 0; x < COPIES * kBoxes; ++x)
-          tma_load_4d(base + L::kQ + x / COPIES * kBoxBytes + x % COPIES * kLanes * 128, &tm_q, bar(Q_FULL), 64 * (x / COPIES), hk * tp.group, t0, b);
-      }
       int qp_min, qp_max;
       tile_positions(qp_min, qp_max);
       bool ok = true;
@@ -248,22 +296,18 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const int j = range.at(n_begin + i);
         const int s = i % STAGES;
         const uint32_t ph = (i / STAGES) & 1;
-        if (lane == 0) ok = mbar_wait(bar(K_EMPTY + s), ph ^ 1, wctx, 60);
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        if (!ok) break;
-        if (lane == 0) {
-          mbar_expect_tx(bar(K_FULL + s), L::kTileBytes);
-          for (int x = 0; x < kBoxes; ++x)
-            tma_load_4d(base + L::kK + s * L::kTileBytes + x * kBoxBytes, &tm_k, bar(K_FULL + s), 64 * x, j * kTile, hk, b);
-          ok = mbar_wait(bar(V_EMPTY + s), ph ^ 1, wctx, 61);
-          if (ok) {
-            mbar_arrive_expect_tx(bar(V_FULL + s), L::kTileBytes);
-            for (int x = 0; x < kBoxes; ++x)
-              tma_load_4d(base + L::kV + s * L::kTileBytes + x * kBoxBytes, &tm_v, bar(V_FULL + s), 64 * x, j * kTile, hk, b);
+        if (i >= ahead) {
+          if (lane == 0) {
+            ok = mbar_wait(bar(K_EMPTY + s), ph ^ 1, wctx, 60);
+            if (ok) {
+              load_k(i);
+              ok = mbar_wait(bar(V_EMPTY + s), ph ^ 1, wctx, 61);
+            }
+            if (ok) load_v(i);
           }
+          ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+          if (!ok) break;
         }
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        if (!ok) break;
         // positions of the block's keys (a key past the end of the cache gets the "no key" mark), and whether
         // the mask cuts the block at all
         int kp_min = j * kTile, kp_max = j * kTile + kTile - 1;
@@ -339,7 +383,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     __syncwarp();
     for (int i = 0; i < 2; ++i) {
-      cluster_arrive();
+      cluster_arrive_relaxed();
       cluster_wait();
     }
   } else {
@@ -354,7 +398,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const uint32_t o_addr = tmem_addr(tmem, lane_base, 256 + D * w);
     const bool valid = row < n_rows;
     const bool warp_rows = row - lane < n_rows;                  // some row of this warp belongs to a query
-    const int qp = valid ? cached::query_position(p, t0 + row / tp.group) : 0;
+    const int qp = valid ? cached::query_position(p, t0 + tp.by_group.div(row)) : 0;
     const int span = p.window - p.sinks;
     const uint64_t scale2 = pack_f2(p.scale_log2, p.scale_log2);
     float m_ref = -INFINITY, l = 0.f;
@@ -475,165 +519,188 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       tc_fence_before();
       mbar_arrive(bar(P_FULL + w));
     }
-    if (ok) {
-      ok = mbar_wait(bar(O_DONE), 0, wctx, 67);
-      ok = __all_sync(0xffffffffu, ok);
-      if (ok) tc_fence_after();
-    }
-    // Every product that read the tiles in shared memory is complete: the other CTAs may write there.
-    __syncwarp();
-    cluster_arrive();
-    // A row's sums -- of either warpgroup and every copy -- become one.  Of a split tile, each thread hands over all of
-    // its columns but one slice, in which it adds up what the others hand over; else all of them, to be finished at once.
-    constexpr int kParts = 2 * COPIES, kSlice = D / kParts, kStatStep = COPIES == 1 ? 2 : L::kPartStep / 4;
+    // A row's parts -- of either warpgroup and every copy -- become one.  Their statistics are exchanged first, over Q, while the
+    // last products run: Q is dead when both warpgroups' last score products have completed.
+    constexpr int kParts = 2 * COPIES, kSlice = D / kParts;
     const bool split = p.splits > 1;
-    const int step = split ? L::kSplitPartStep / 4 : L::kPartStep / 4;
     const int part = w * COPIES + copy;
-    float* first = reinterpret_cast<float*>(gen + L::kK + row * L::kPitch);  // the row of part 0: the result as well
     const bool any = w < n_blocks;
-    if (ok && warp_rows) {
-      float* dst = first + part * step;
-      const int keep = split ? part : -1;                                    // slice
-      *reinterpret_cast<float2*>(first + part * kStatStep + D) = any ? make_float2(m_ref, l) : make_float2(-INFINITY, 0.f);
-      if (any) {
-#pragma unroll
-        for (int c = 0; c < D; c += 32) {
-          if (kSlice >= 32 && c / kSlice == keep) continue;
-          uint32_t orr[32];
-          tmem_ld32(o_addr + c, orr);
-          tc_wait_ld();
-#pragma unroll
-          for (int e = 0; e < 32; e += 4)
-            if (kSlice >= 32 || (c + e) / kSlice != keep)
-              *reinterpret_cast<float4*>(dst + c + e) = make_float4(__uint_as_float(orr[e]), __uint_as_float(orr[e + 1]),
-                                                                    __uint_as_float(orr[e + 2]), __uint_as_float(orr[e + 3]));
-        }
-      }
-    }
     auto group_sync = [&](uint32_t parity) {
       mbar_arrive(bar(GROUP));
       const bool met = mbar_wait(bar(GROUP), parity, wctx, 69);
       ok = __all_sync(0xffffffffu, ok && met && *abort_flag == 0);
     };
+    ok = ok && mbar_wait(bar(Q_FULL), 0, wctx, 73);
+    if (ok && (w ^ 1) < n_blocks) {
+      const int last = n_blocks - 1 - ((n_blocks - 1 - (w ^ 1)) & 1);        // the other warpgroup's
+      ok = mbar_wait(bar(S_FULL + (w ^ 1)), (last >> 1) & 1, wctx, 74);
+    }
+    float2* stats = reinterpret_cast<float2*>(gen + L::kQ) + row;            // [kParts][kLanes]
+    if (warp_rows) stats[part * kLanes] = any ? make_float2(m_ref, l) : make_float2(-INFINITY, 0.f);
+    group_sync(0);
+    float mx = -INFINITY, sum = 0.f;
+#pragma unroll
+    for (int x = 0; x < kParts; ++x) mx = fmaxf(mx, stats[x * kLanes].x);
+    const float ref = mx == -INFINITY ? 0.f : mx;
+#pragma unroll
+    for (int x = 0; x < kParts; ++x) {
+      const float2 ml = stats[x * kLanes];
+      sum = fmaf(exp2f(ml.x - ref), ml.y, sum);                              // a part that saw no key: 0
+    }
+    const float f_first = exp2f(stats[copy * kLanes].x - ref), f_second = exp2f(stats[(COPIES + copy) * kLanes].x - ref);
+    if (ok) ok = mbar_wait(bar(O_DONE), 0, wctx, 67);
     if constexpr (SPLIT_P) {
       const bool met = mbar_wait(bar(SCANNED), 0, wctx, 72);
-      ok = __all_sync(0xffffffffu, ok && met);
+      ok = ok && met;
     }
-    group_sync(0);
-    if (ok && split && warp_rows) {
-      float2 ml[kParts];
-      float mx = -INFINITY, sum = 0.f, f_mine = 0.f;
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) tc_fence_after();
+    // Every product that read the tiles in shared memory is complete: the other CTAs may write there.
+    __syncwarp();
+    cluster_arrive_relaxed();
+    // Both warpgroups' sums of a row stand in the same TMEM lane: each warpgroup adds up its half of the columns.  With
+    // copies, each thread hands its sums over and adds up one slice of the half.
+    constexpr int kHalf = D / 2;
+    float sums[kHalf];
 #pragma unroll
-      for (int x = 0; x < kParts; ++x) {
-        ml[x] = *reinterpret_cast<const float2*>(first + x * kStatStep + D);
-        mx = fmaxf(mx, ml[x].x);
-      }
-      const float ref = mx == -INFINITY ? 0.f : mx;
+    for (int c = 0; c < kHalf; ++c) sums[c] = 0.f;
+    const bool has_columns = warp_rows && kHalf * w < p.D;                   // (head dim 32 on 64-wide tiles: the first half)
+    if (ok && has_columns) {
+      const uint32_t at = tmem_addr(tmem, lane_base, 256 + kHalf * w);
+      auto add = [&](uint32_t from, float weight) {
 #pragma unroll
-      for (int x = 0; x < kParts; ++x) {
-        ml[x].x = exp2f(ml[x].x - ref);                                      // a part that saw no key: 0
-        sum = fmaf(ml[x].x, ml[x].y, sum);
-        f_mine = x == part ? ml[x].x : f_mine;
-      }
-      if (part == 0) *reinterpret_cast<float4*>(first + D + 4) = make_float4(mx, sum, *spoilt_flag ? 1.f : 0.f, 0.f);
+        for (int c = 0; c < kHalf; c += 32) {
+          uint32_t x[32];
+          tmem_ld32(from + c, x);
+          tc_wait_ld();
 #pragma unroll
-      for (int c = 0; c < kSlice; c += 8) {
-        uint32_t orr[8];
-        if (any) tmem_ld8(o_addr + part * kSlice + c, orr);
-        tc_wait_ld();
+          for (int e = 0; e < 32; ++e) sums[c + e] = fmaf(weight, __uint_as_float(x[e]), sums[c + e]);
+        }
+      };
+      if (n_blocks > 0) add(at, f_first);
+      if (n_blocks > 1) add(at + D, f_second);                               // (what no product wrote may be anything)
+    }
+    auto put = [&](uint8_t* to, const float* v, int n) {
 #pragma unroll
-        for (int e = 0; e < 8; e += 4) {
-          float* at = first + part * kSlice + c + e;
-          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (any)
-            acc = make_float4(f_mine * __uint_as_float(orr[e]), f_mine * __uint_as_float(orr[e + 1]),
-                              f_mine * __uint_as_float(orr[e + 2]), f_mine * __uint_as_float(orr[e + 3]));
+      for (int c = 0; c < n; c += 4) *reinterpret_cast<float4*>(to + 4 * c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+    };
+    const int col = kHalf * w + kSlice * copy;                               // first column of this thread's slice
+    if constexpr (COPIES > 1) {
+      if (ok && has_columns) put(gen + L::kK + (kLanes * copy + row) * L::kPitch + 4 * kHalf * w, sums, kHalf);
+      group_sync(1);
+      if (ok && has_columns) {
+        const uint8_t* from = gen + L::kK + row * L::kPitch + 4 * col;
 #pragma unroll
-          for (int x = 0; x < kParts; ++x) {
-            if (x == part || x / COPIES >= n_blocks) continue;               // (a warpgroup without a block handed nothing over)
-            const float4 y = *reinterpret_cast<const float4*>(at + x * step);
-            acc = make_float4(fmaf(ml[x].x, y.x, acc.x), fmaf(ml[x].x, y.y, acc.y), fmaf(ml[x].x, y.z, acc.z), fmaf(ml[x].x, y.w, acc.w));
+        for (int c = 0; c < kSlice; c += 4) {
+          float4 acc = *reinterpret_cast<const float4*>(from + 4 * c);
+#pragma unroll
+          for (int x = 1; x < COPIES; ++x) {
+            const float4 y = *reinterpret_cast<const float4*>(from + x * kLanes * L::kPitch + 4 * c);
+            acc = make_float4(acc.x + y.x, acc.y + y.y, acc.z + y.z, acc.w + y.w);
           }
-          *reinterpret_cast<float4*>(at) = acc;
+          sums[c] = acc.x; sums[c + 1] = acc.y; sums[c + 2] = acc.z; sums[c + 3] = acc.w;
         }
       }
     }
-    fence_proxy_async_smem();
-    __syncwarp();
-    cluster_wait();                                // every CTA's tiles are dead
-    if (split) group_sync(1);
-    // each CTA of the cluster gets the rows it finishes
-    if (ok && split) {
-      if (warp == 0 && lane < p.splits) {
-        const int first = lane * rows_each, count = first + rows_each < n_rows ? rows_each : n_rows - first;
-        if (count > 0)
-          bulk_copy_cluster(cluster_addr(base + L::kReceived + rank * rows_each * L::kPitch, lane),
-                            base + L::kK + first * L::kPitch, count * L::kPitch, cluster_addr(bar(RECEIVED), lane));
-      }
-      __syncwarp();
-      ok = mbar_wait(bar(RECEIVED), 0, wctx, 70);
-      ok = __all_sync(0xffffffffu, ok);
-    }
-    __syncwarp();
-    cluster_arrive();                              // what the others sent is here
-    // four columns of a row of the tile, out of parts that lie `stride` floats apart, their statistics `stat_stride`
-    auto finish = [&](int r, int c, const float* at, int count, int stride, const float* stats, int stat_stride) {
-      float mx = -INFINITY;
-      for (int s = 0; s < count; ++s) mx = fmaxf(mx, stats[s * stat_stride]);
-      const float ref = mx == -INFINITY ? 0.f : mx;
-      float sum = 0.f;
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      bool odd = SPLIT_P && !split && *spoilt_flag != 0;                     // values were taken out of V
-#pragma unroll 4
-      for (int s = 0; s < count; ++s) {
-        if (SPLIT_P && split) odd |= stats[s * stat_stride + 2] != 0.f;
-        const float2 ml = *reinterpret_cast<const float2*>(stats + s * stat_stride);
-        const float4 y = *reinterpret_cast<const float4*>(at + s * stride + c);
-        const float f = exp2f(ml.x - ref);                                   // a part that saw no key: 0 (of zeros)
-        sum = fmaf(f, ml.y, sum);
-        acc = make_float4(fmaf(f, y.x, acc.x), fmaf(f, y.y, acc.y), fmaf(f, y.z, acc.z), fmaf(f, y.w, acc.w));
-      }
-      const int t = t0 + r / tp.group, h = hk * tp.group + r % tp.group;
-      if (c < p.D) {                                                         // head dim 32 on 64-wide tiles
-        const float inv = sum > 0.f ? 1.f / sum : 0.f;                       // a row that sees no key gives zeros
-        acc = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+    const float spoilt = SPLIT_P && *spoilt_flag != 0 ? 1.f : 0.f;           // values were taken out of V
+    // `n` columns (a multiple of four) of a row of the tile, from its sums, its maximum and its sum of exponentials
+    auto finish = [&](int r, int c, const float* v, auto n, float mx, float sum, bool odd) {
+      constexpr int N = decltype(n)::value < 8 ? 4 : 8;
+      const int at = tp.by_group.div(r), t = t0 + at, h = hk * tp.group + (r - at * tp.group);
+      const float inv = sum > 0.f ? 1.f / sum : 0.f;                         // a row that sees no key gives zeros
+      T* out = static_cast<T*>(p.o) + ((static_cast<long long>(b) * p.Tq + t) * p.H + h) * p.D + c;
+#pragma unroll
+      for (int e = 0; e < decltype(n)::value; e += N) {
+        if (c + e >= p.D) break;                                             // head dim 32 on 64-wide tiles
+        float x[N], total = 0.f;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          x[i] = v[e + i] * inv;
+          total += x[i];
+        }
         if constexpr (SPLIT_P) {
           // (a row whose own sum is NaN stays NaN)
-          if (sum > 0.f && (odd || isnan((acc.x + acc.y) + (acc.z + acc.w)))) {
-            const T* vr = static_cast<const T*>(tp.v) + (static_cast<long long>(b) * p.Hkv + hk) * p.L * p.D + c;
-            const int q_at = cached::query_position(p, t);
-            float x[4] = {0.f, 0.f, 0.f, 0.f};                               // what the row sees that is not finite
-            for (int key = 0; key < p.L; ++key, vr += p.D) {
-              if (!cached::position_visible(p, q_at, cached::key_position(p, key))) continue;
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float y = static_cast<float>(vr[e]);
-                if (!isfinite(y)) x[e] += y;
-              }
-            }
-            acc = make_float4(x[0] != 0.f ? x[0] : acc.x, x[1] != 0.f ? x[1] : acc.y, x[2] != 0.f ? x[2] : acc.z,
-                              x[3] != 0.f ? x[3] : acc.w);
-          }
+          if (sum > 0.f && (odd || isnan(total)))
+            put_right<T, N>(p, static_cast<const T*>(tp.v) + (static_cast<long long>(b) * p.Hkv + hk) * p.L * p.D + c + e, t, x);
         }
-        cached::store4(static_cast<T*>(p.o) + ((static_cast<long long>(b) * p.Tq + t) * p.H + h) * p.D + c, acc);
+        uint32_t packed[N / 2];
+#pragma unroll
+        for (int i = 0; i < N; i += 2) packed[i / 2] = Pack2<T>::pack(x[i], x[i + 1]);
+        if constexpr (N == 8) *reinterpret_cast<uint4*>(out + e) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        else *reinterpret_cast<uint2*>(out + e) = make_uint2(packed[0], packed[1]);
       }
       if (p.lse && c == 0)
         p.lse[(static_cast<long long>(b) * p.H + h) * p.Tq + t] = sum > 0.f ? (mx + log2f(sum)) * kLn2 : -INFINITY;
     };
-    if (ok) {
-      // one thread per four columns: of the rows of the tile, or of those this CTA finishes, the parts in the order of the CTAs
-      const float* parts = reinterpret_cast<const float*>(gen + (split ? L::kReceived : L::kK));
-      for (int i = threadIdx.x; i < own * (D / 4); i += 256) {
-        const int k = i / (D / 4), c = 4 * (i % (D / 4));
-        const float* at = parts + k * (L::kPitch / 4);
-        if (split) finish(own_first + k, c, at, p.splits, rows_each * (L::kPitch / 4), at + D + 4, rows_each * (L::kPitch / 4));
-        else finish(k, c, at, COPIES * (n_blocks < 2 ? n_blocks : 2), L::kPartStep / 4, at + D, kStatStep);
+    if (split) {
+      if (ok && warp_rows) {
+        uint8_t* to = gen + L::kRows + row * L::kPitch;
+        if (has_columns) put(to + 4 * col, sums, kSlice);
+        if (part == 0) *reinterpret_cast<float4*>(to + 4 * D) = make_float4(mx, 0.f, sum, spoilt);
       }
+      fence_proxy_async_smem();
+      group_sync(COPIES > 1 ? 0 : 1);
+      cluster_wait();                              // every CTA's tiles are dead
+      // each CTA of the cluster gets the rows it finishes
+      if (ok && warp == 0 && lane < p.splits) {
+        const int first = lane * rows_each, count = first + rows_each < n_rows ? rows_each : n_rows - first;
+        if (count > 0)
+          bulk_copy_cluster(cluster_addr(base + L::kReceived + rank * rows_each * L::kPitch, lane),
+                            base + L::kRows + first * L::kPitch, count * L::kPitch, cluster_addr(bar(RECEIVED), lane));
+      }
+      __syncwarp();
+      if (ok) ok = mbar_wait(bar(RECEIVED), 0, wctx, 70);
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) {
+        // one thread per eight columns of the rows this CTA finishes, or where that leaves threads enough per four; the parts
+        // in the order of the CTAs
+        auto rows = [&](auto n) {
+          constexpr int N = decltype(n)::value;
+          for (int i = threadIdx.x; i < own * (D / N); i += 256) {
+            const int k = i / (D / N), c = N * (i % (D / N));
+            if (c >= p.D) continue;                                          // head dim 32 on 64-wide tiles
+            const uint8_t* at = gen + L::kReceived + k * L::kPitch;
+            const int step = rows_each * L::kPitch;
+            // (all loads of a kind at once: one after another their latency was most of this)
+            float m[kMostCluster], mx = -INFINITY, sum = 0.f;
+#pragma unroll
+            for (int s = 0; s < kMostCluster; ++s) m[s] = s < p.splits ? *reinterpret_cast<const float*>(at + s * step + 4 * D) : -INFINITY;
+#pragma unroll
+            for (int s = 0; s < kMostCluster; ++s) mx = fmaxf(mx, m[s]);
+            const float ref = mx == -INFINITY ? 0.f : mx;
+            float v[N] = {};
+            bool odd = false;
+#pragma unroll
+            for (int s = 0; s < kMostCluster; ++s) {
+              if (s >= p.splits) break;
+              const float2 l = *reinterpret_cast<const float2*>(at + s * step + 4 * D + 8);
+              const float f = exp2f(m[s] - ref);
+              sum = fmaf(f, l.x, sum);
+#pragma unroll
+              for (int e = 0; e < N; e += 4) {
+                const float4 y = *reinterpret_cast<const float4*>(at + s * step + 4 * (c + e));
+                v[e] = fmaf(f, y.x, v[e]); v[e + 1] = fmaf(f, y.y, v[e + 1]);
+                v[e + 2] = fmaf(f, y.z, v[e + 2]); v[e + 3] = fmaf(f, y.w, v[e + 3]);
+              }
+              if (SPLIT_P) odd |= l.y != 0.f;
+            }
+            finish(own_first + k, c, v, n, mx, sum, odd);
+          }
+        };
+        if (own * (D / 4) > 256) rows(std::integral_constant<int, 8>{});
+        else rows(std::integral_constant<int, 4>{});
+      }
+      __syncwarp();
+      cluster_arrive_relaxed();                    // what the others sent is here
+    } else {
+      cluster_wait();
+      cluster_arrive_relaxed();
+      if (ok && valid) finish(row, col, sums, std::integral_constant<int, kSlice>{}, mx, sum, spoilt != 0.f);
     }
     } else {
-      cluster_arrive();
+      cluster_arrive_relaxed();
       cluster_wait();
-      cluster_arrive();
+      cluster_arrive_relaxed();
     }
     __syncwarp();
     cluster_wait();                                // what this CTA sent has arrived
@@ -649,7 +716,7 @@ cached_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 }
 
 template <typename T, int D, int STAGES, int COPIES, bool SPLIT_P>
-int launch_t(CachedParams p, const TileParams& tp, int n_blocks, const CUtensorMap& mq, const CUtensorMap& mk,
+int launch_t(CachedParams p, TileParams tp, int n_blocks, const CUtensorMap& mq, const CUtensorMap& mk,
              const CUtensorMap& mv, cudaStream_t stream) {
   using L = CachedSmem<D, STAGES, COPIES>;
   static_assert(L::kDynamic <= 232448, "over the shared memory a CTA can have");
@@ -659,6 +726,7 @@ int launch_t(CachedParams p, const TileParams& tp, int n_blocks, const CUtensorM
   // warpgroup) each.
   const int tiles = p.B * p.Hkv * tp.n_qtiles;
   p.splits = cached::cluster_splits(reinterpret_cast<const void*>(kern), 384, L::kDynamic, tiles, (n_blocks + 1) / 2);
+  tp.by_splits = FastDiv(p.splits);
   const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(p.splits));
   if (launch_cluster(kern, grid, dim3(384), L::kDynamic, stream, overlap_launches(kOverlapFwd), p.splits, mq, mk, mv, p, tp) !=
       cudaSuccess) {
@@ -707,8 +775,11 @@ int launch_fwd_cached_tc(CachedParams p, const void* q, const void* k_cache, con
                          unsigned* status, cudaStream_t stream) {
   TileParams tp;
   tp.group = p.H / p.Hkv;
+  tp.by_group = FastDiv(tp.group);
   tp.tq_tile = positions_per_tile(p.Tq, tp.group);
   tp.n_qtiles = (p.Tq + tp.tq_tile - 1) / tp.tq_tile;
+  tp.by_qtiles = FastDiv(tp.n_qtiles);
+  tp.by_heads = FastDiv(p.Hkv);
   tp.status = status;
   tp.v = v_cache;
   int n_blocks = 0;                                         // key blocks of the tile that sees the most

@@ -40,6 +40,25 @@ __host__ __device__ inline int first_query_of_key(int k, int block) {
   return block > 1 ? (k / block) * block : k;
 }
 
+// Division of a non-negative int by a divisor the host knows: q = (mulhi(n, mul) + n) >> shift with 2^shift >= d and
+// mul = floor(2^32 (2^shift - d) / d) + 1, the usual round-up method, exact for every n < 2^31.
+struct FastDiv {
+  unsigned mul, shift;
+  int d;
+  FastDiv() = default;
+  explicit FastDiv(int divisor) : mul(0), shift(0), d(divisor) {
+    while ((1ull << shift) < static_cast<unsigned long long>(divisor)) ++shift;
+    mul = static_cast<unsigned>(((1ull << 32) * ((1ull << shift) - divisor)) / divisor + 1);
+  }
+  __host__ __device__ __forceinline__ int div(int n) const {
+#ifdef __CUDA_ARCH__
+    return static_cast<int>((__umulhi(static_cast<unsigned>(n), mul) + static_cast<unsigned>(n)) >> shift);
+#else
+    return static_cast<int>(((static_cast<unsigned long long>(n) * mul >> 32) + n) >> shift);
+#endif
+  }
+};
+
 // Which key blocks a 128-row query tile must visit.  Block j covers keys
 // [128 j, 128 j + 127].  The mask is the reference's sliding_window_mask
 // (nanolab/mixers.py:125-132): keep k <= q and (k > q - (window - sinks) or

@@ -40,6 +40,28 @@ def test_rows_of_a_split_cache_match_the_oracle(T, H, Hkv, L, D, causal, window,
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("T,H,Hkv,L,D", [
+    (64, 16, 16, 2048, 128),                # finished eight columns a thread: more than 256 pieces of four
+    (128, 3, 3, 1500, 64),                  # .. one copy, rows that do not divide by the CTAs
+    (32, 12, 12, 1056, 64),                 # .. four columns a thread
+    (70, 2, 2, 1300, 32),                   # head dim 32: the second warpgroup's half of the columns is none
+    (9, 160, 160, 400, 32),                 # .. whole tiles, finished where their sums are
+    (100, 150, 150, 300, 128),              # whole tiles, one copy: 64 columns a thread
+    (5, 150, 150, 90, 128),                 # whole tiles of one key block
+])
+def test_pieces_of_finished_rows_match_the_oracle(T, H, Hkv, L, D):
+    from machinelearning_b200 import flash_cuda
+    g = torch.Generator().manual_seed(T * L)
+    q, k, v = (torch.randn(1, *s, D, generator=g).to("cuda", torch.bfloat16) for s in ((T, H), (Hkv, L), (Hkv, L)))
+    y, lse = flash_cuda.flash_attn_cached(q, k, v, causal=True, return_lse=True)
+    n = lambda x: x.double().cpu().numpy()
+    ref, lse_ref = cached_f64.forward(n(q), n(k), n(v), 1.0 / np.sqrt(D), np.arange(L - T, L), np.arange(L), True, 0, 0)
+    # P and the result rounded to 8 bits of mantissa, errors of a row's keys independent: 2^-9 of the largest value each
+    assert np.abs(n(y) - ref).max() <= 8e-3 * np.abs(ref).max()
+    assert np.abs(n(lse) - lse_ref).max() <= 1e-3
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32], ids=["fp16", "fp32"])
 def test_sinks_next_to_two_to_the_31(dtype):
     from machinelearning_b200 import flash_cuda
