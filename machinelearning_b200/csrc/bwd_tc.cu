@@ -686,11 +686,28 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       return __shfl_sync(0xffffffffu, u, 0);
     };
+    // dK/dV over 64-row tiles: the row statistics of the next tile are requested as soon as this one's are in shared memory,
+    // so that their latency (900 of 1,300 clocks per tile, against 1,850 of an iteration) passes while this warp waits for a
+    // free stage.  B=2 H=16/8 T=8192 window 512, D = 128: backward 428 -> 397 us; B=4 H=12/4 T=2048 191.6 -> 189.8.  At
+    // D <= 64 an iteration has time for it, and the kernel came out slower (B=16 H=16 T=4096 window 256 dK/dV 278 -> 291 us).
+    constexpr bool kStatsAhead = kKeyStat && YR == 64;
+    float stat_lse[YR / 32], stat_delta[YR / 32];
+    auto load_stats = [&](const BwdUnit<MODE>& w, int idx, int h) {
+      const long long row0 = (static_cast<long long>(w.b) * p.H + h) * p.T;
+#pragma unroll
+      for (int i = 0; i < YR / 32; ++i) {
+        const int qpos = idx * YR + lane * (YR / 32) + i;
+        const bool in = qpos < p.T;
+        stat_lse[i] = in ? p.lse[row0 + qpos] : INFINITY;
+        stat_delta[i] = in ? p.delta[row0 + qpos] : 0.f;
+      }
+    };
     int u = fetch_unit(0);
     for (int uc = 0; ok && u >= 0; ++uc) {
       BwdUnit<MODE> w;
       next_unit(uc, ok, w);                      // published by this warp: never waits
       if (!ok) break;
+      if constexpr (kStatsAhead) load_stats(w, w.streamed_index(0), w.h);
       // The next unit is taken, and its stationary tiles requested, when this unit's last streamed tiles have been
       // (the compute warps are then STAGES iterations behind).  Taken any earlier, a unit waits behind this
       // one while other CTAs run out of work: B=3 H=2 T=5416 backward 123.6 -> 101.4 us.
@@ -722,6 +739,11 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
 #pragma unroll
           for (int i = 0; i < YR / 32; ++i) {
             const int c = lane * (YR / 32) + i;
+            if constexpr (kStatsAhead) {
+              vec[c] = -stat_lse[i] * kLog2e;
+              vec[YR + c] = -stat_delta[i];
+              continue;
+            }
             const int qpos = idx * YR + c;
             const bool in = qpos < p.T;
             vec[c] = in ? -p.lse[row0 + qpos] * kLog2e : -INFINITY;
@@ -730,6 +752,12 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
           __syncwarp();
         }
         if (lane == 0) mbar_arrive(bar(Y_FULL + s));
+        if constexpr (kStatsAhead) {
+          if (it + 1 < w.n_iters) {
+            const bool next_head = inner + 1 == w.n_inner;
+            load_stats(w, w.streamed_index(next_head ? 0 : inner + 1), next_head ? yh + 1 : yh);
+          }
+        }
       }
       if (ok) u = fetch_unit(uc + 1);
     }
