@@ -634,13 +634,13 @@ int nlfa_check_mask_geometry_masked(int T, int window, int sinks, int block, int
   const int n128 = (T + kTile - 1) / kTile;
   const int nys = (T + stream_rows - 1) / stream_rows;
   int check = 0;
-  // (1) key blocks given to a query tile cover every block with a visible pair
+  // (1) key blocks (of stream_rows keys) given to a query tile cover every block with a visible pair
   for (int t = 0; t < n128; ++t) {
-    const TileRange r = tile_range(t, window, sinks, block, n128);
-    for (int j = 0; j < n128; ++j, ++check) {
+    const TileRange r = tile_range(t, window, sinks, block, nys, stream_rows);
+    for (int j = 0; j < nys; ++j, ++check) {
       bool any = false;
       for (int q = t * kTile; q < (t + 1) * kTile && !any; ++q)
-        for (int k = j * kTile; k < (j + 1) * kTile && !any; ++k) any = key_visible(q, k, window, sinks, block, T);
+        for (int k = j * stream_rows; k < (j + 1) * stream_rows && !any; ++k) any = key_visible(q, k, window, sinks, block, T);
       const bool given = (j >= r.lo && j <= r.hi) || j < r.sink_blocks;
       if (any && !given) return 1 + check;
     }
@@ -669,11 +669,6 @@ int nlfa_check_mask_geometry_masked(int T, int window, int sinks, int block, int
         ++check;
         if (e == EDGE_WINDOW && !window_only) return 1 + check;
         ++check;
-        if (stream_rows == kTile) {
-          const int qt = orient == 0 ? t : y, kb = orient == 0 ? y : t;
-          if (block_fully_visible(qt, kb, window, sinks, block, T) && !all) return 1 + check;
-          ++check;
-        }
       }
   // (4) fused backward: the key blocks that stream query tile t take the turns 0 .. count - 1
   //     exactly once each, in ascending block order

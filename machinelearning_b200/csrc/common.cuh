@@ -60,7 +60,7 @@ struct FastDiv {
 };
 
 // Which key blocks a 128-row query tile must visit.  Block j covers keys
-// [128 j, 128 j + 127].  The mask is the reference's sliding_window_mask
+// [w j, w j + w - 1], w = `width`.  The mask is the reference's sliding_window_mask
 // (nanolab/mixers.py:125-132): keep k <= q and (k > q - (window - sinks) or
 // k < sinks).
 struct TileRange {
@@ -69,38 +69,25 @@ struct TileRange {
 };
 
 // `block` > 0 (block-causal; window must be 0) lets a tile see past the diagonal, up to the end
-// of its last row's block; `n_tiles` bounds that.
+// of its last row's block; `n_blocks` key blocks bound that.
 __host__ __device__ inline TileRange tile_range(int tile, int window, int sinks, int block = 0,
-                                                int n_tiles = 1 << 30) {
+                                                int n_blocks = 1 << 30, int width = kTile) {
   TileRange r;
-  r.hi = last_key_of_query(tile * kTile + kTile - 1, block) / kTile;
-  r.hi = r.hi < n_tiles - 1 ? r.hi : n_tiles - 1;
+  r.hi = last_key_of_query(tile * kTile + kTile - 1, block) / width;
+  r.hi = r.hi < n_blocks - 1 ? r.hi : n_blocks - 1;
   r.lo = 0;
   r.sink_blocks = 0;
   if (window > 0) {
     const int span = window - sinks;
     const int first_key = tile * kTile - span + 1;     // lowest recent key of the tile's first row
-    r.lo = first_key > 0 ? first_key / kTile : 0;
-    r.sink_blocks = (sinks + kTile - 1) / kTile;
+    r.lo = first_key > 0 ? first_key / width : 0;
+    r.sink_blocks = (sinks + width - 1) / width;
   }
   return r;
 }
 
-// True when every (row, key) of query tile `tile` x key block `j` survives the
-// mask, so the element-wise predicate can be skipped.
-__host__ __device__ inline bool block_fully_visible(int tile, int j, int window, int sinks, int block = 0,
-                                                    int t_len = 1 << 30) {
-  if (j * kTile + kTile - 1 > last_key_of_query(tile * kTile, block, t_len)) return false;   // the causal edge cuts in
-  if (window > 0) {
-    const int span = window - sinks;
-    const int last_row = tile * kTile + kTile - 1;
-    if (j * kTile <= last_row - span) return false;              // lower window edge cuts in
-  }
-  return true;
-}
-
-// The same question for a rectangle of query positions [q_lo, q_hi] x key positions [k_lo, k_hi] (tiles of unequal
-// height), and which edges of the mask cut through one that is not fully visible: only the causal edge k <= q (plain
+// Whether every (query, key) of a rectangle of query positions [q_lo, q_hi] x key positions [k_lo, k_hi] survives the mask,
+// so that the element-wise predicate can be skipped, and which edges of the mask cut through one that is not fully visible: only the causal edge k <= q (plain
 // causal, or windows whose lower edge stays below it), only the window's lower edge k > q - (window - sinks) (below the
 // diagonal, no sink keys), or both / sinks involved.  With one edge a compare per element against a per-thread limit does.
 enum { EDGE_CAUSAL = 0, EDGE_WINDOW = 1, EDGE_BOTH = 2 };

@@ -1,9 +1,9 @@
 // Tensor-core forward for sm_100a: S = Q K^T and O += P V on tcgen05 with the
 // accumulators in TMEM, tiles brought in by TMA, online softmax in registers.
 //
-// Persistent kernel: one CTA per SM (two at NT = 1, D <= 64) takes work units from a global counter,
-// heaviest first.  A unit is NT consecutive 128-row query tiles of one (batch,
-// head), NT = 1 or 2 (launch_fwd_tc has the rule); the CTA visits the key blocks those tiles can see.
+// Persistent kernel: one CTA per SM (at NT = 1, D <= 64 two, or three with key blocks of 64) takes work units from a global
+// counter, heaviest first.  A unit is NT consecutive 128-row query tiles of one (batch, head), NT = 1 or 2; the CTA visits
+// the key blocks, BN = 128 or 64 keys each, that those tiles can see (launch_fwd_tc has the rules).
 // Warp roles:
 //   warps [0, 4 NT)   softmax: warpgroup t owns query tile t, one thread per row
 //   warp  4 NT        scheduler + TMA producer (one lane): Q per unit, K / V ring
@@ -13,11 +13,11 @@
 // ready.  While the softmax warps finish a unit (normalise and store O) the
 // producer and the MMA issuer are already on the next one.
 //
-// TMEM columns: S_t at 128 t (fp32, 128 columns), O_t at 128 NT + D t.  P_t (16
-// bit, the A operand of the PV product) has its own 64 columns after the O tiles
-// when they fit (D = 64); the next S product is then issued as soon as the softmax
+// TMEM columns: S_t at BN t (fp32, BN columns), O_t at BN NT + D t.  P_t (16
+// bit, the A operand of the PV product) has its own BN / 2 columns after the O tiles
+// when they fit (D = 64; key blocks of 64: head dim 32); the next S product is then issued as soon as the softmax
 // warps have pulled S into registers, so the tensor pipe runs under the
-// exponentials.  Otherwise (D = 128) P_t overwrites the first 64 columns of S_t.
+// exponentials.  Otherwise P_t overwrites the first BN / 2 columns of S_t.
 //
 // Computes what nanolab/csrc/flash_attn_cuda.cu:583-797 computes (softmax in
 // base 2, L = m ln2 + log l at :279), with the sliding-window mask of
@@ -34,7 +34,7 @@ struct FwdParams {
   int T, H, Hkv;
   int window, sinks;
   int block;              // > 0: block-causal mask of this many positions (window == 0)
-  int n_tiles;            // ceil(T / 128)
+  int n_tiles, n_blocks;  // ceil(T / 128), ceil(T / BN)
   int n_units;            // ceil(n_tiles / NT)
   int total_units;        // n_units * B * H
   float scale_log2;       // scale * log2(e), > 0
@@ -44,13 +44,14 @@ struct FwdParams {
   unsigned* sched;        // this launch's two counters
 };
 
-template <int D, int NT, int STAGES, int QBUF>
+template <int D, int NT, int STAGES, int QBUF, int BN>
 struct FwdSmem {
   static constexpr int kTileBytes = kTile * D * 2;          // one 128 x D 16-bit tile
+  static constexpr int kKvBytes = BN * D * 2;               // one block of K or V
   static constexpr int kQ = 0;                              // [QBUF][NT] tiles
   static constexpr int kK = kQ + QBUF * NT * kTileBytes;
-  static constexpr int kV = kK + STAGES * kTileBytes;
-  static constexpr int kBar = kV + STAGES * kTileBytes;
+  static constexpr int kV = kK + STAGES * kKvBytes;
+  static constexpr int kBar = kV + STAGES * kKvBytes;
   // barriers (8 bytes each): q_full[QBUF], q_empty[QBUF], s_full[NT], s_consumed[NT],
   // p_full[NT], o_ready[NT], k_full[S], k_empty[S], v_full[S], v_empty[S], sched_full[kRing]
   static constexpr int kRing = 8;
@@ -85,7 +86,7 @@ struct Unit {
   }
 };
 
-template <int NT>
+template <int NT, int BN>
 __device__ __forceinline__ Unit<NT> make_unit(int u, const FwdParams& p, int BH) {
   Unit<NT> w;
   const int rank = u / BH;                    // heavy (late) query tiles first
@@ -101,7 +102,7 @@ __device__ __forceinline__ Unit<NT> make_unit(int u, const FwdParams& p, int BH)
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
     w.valid[t] = (w.tile0 + t) < p.n_tiles;
-    w.tr[t] = tile_range(w.tile0 + t, p.window, p.sinks, p.block, p.n_tiles);
+    w.tr[t] = tile_range(w.tile0 + t, p.window, p.sinks, p.block, p.n_blocks, BN);
     if (w.valid[t]) {
       w.lo = w.tr[t].lo < w.lo ? w.tr[t].lo : w.lo;
       hi = w.tr[t].hi > hi ? w.tr[t].hi : hi;
@@ -116,24 +117,27 @@ __device__ __forceinline__ Unit<NT> make_unit(int u, const FwdParams& p, int BH)
 
 // DR: the head dim; 32 runs on tiles 64 wide (D), with half the steps of the score product and an output product
 // half as wide (B=8 H=12/4 T=1024: 34.2 -> 32.4 us).
-template <typename T, int D, int DR, int NT, int STAGES, int QBUF>
-__global__ void __launch_bounds__(NT * 128 + 128, NT == 1 && D == 64 ? 2 : 1)
+template <typename T, int D, int DR, int NT, int STAGES, int QBUF, int BN>
+__global__ void __launch_bounds__(NT * 128 + 128, BN == 64 ? 3 : NT == 1 && D == 64 ? 2 : 1)
 fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
               const FwdParams p) {
-  using L = FwdSmem<D, NT, STAGES, QBUF>;
+  using L = FwdSmem<D, NT, STAGES, QBUF, BN>;
+  static_assert(BN == 128 || (BN == 64 && NT == 1 && D == 64), "key blocks of 64: one tile per unit, head dims up to 64");
   constexpr int kBoxes = D / 64;                 // 64-element column boxes per tile
   constexpr int kBoxBytes = kTile * 128;         // 128 rows x 128 bytes
-  constexpr uint32_t kTmemCols = (NT * (128 + D) <= 256) ? 256u : 512u;
+  constexpr int kKvBoxBytes = BN * 128;          // ... of a block of K or V
+  constexpr uint32_t kTmemCols = BN == 64 ? 128u : (NT * (128 + D) <= 256) ? 256u : 512u;
   constexpr bool kBf16 = Pack2<T>::kIsBf16;
-  constexpr bool kSepP = NT * (128 + D + 64) <= 512;      // P has columns of its own
-  constexpr uint32_t kPBase = NT * (128 + D);
+  constexpr bool kSepP = BN == 64 ? DR == 32 : NT * (128 + D + 64) <= 512;      // P has columns of its own
+  constexpr uint32_t kPBase = BN == 64 ? BN + DR : NT * (128 + D);
   constexpr int kRing = L::kRing;
   // Registers per thread: at launch, of the softmax warps, of the others.  NT = 1 at D = 128 has the SM to itself, and the
   // compiler lets it start with as many as the softmax warps ask for: there the request raises nothing.
   constexpr bool kOwnSm = NT == 1 && D == 128;
-  constexpr int kRegsCompute = kOwnSm ? 208 : NT == 1 ? 200 : 216, kRegsOther = NT == 1 ? 56 : 72;
-  constexpr int kRegsLaunch = kOwnSm ? kRegsCompute : NT == 1 ? 128 : 168;
+  constexpr int kRegsCompute = BN == 64 ? 120 : kOwnSm ? 208 : NT == 1 ? 200 : 216;
+  constexpr int kRegsOther = BN == 64 ? 40 : NT == 1 ? 56 : 72;
+  constexpr int kRegsLaunch = BN == 64 ? 80 : kOwnSm ? kRegsCompute : NT == 1 ? 128 : 168;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -238,7 +242,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         int u = static_cast<int>(atomicAdd(&p.sched[0], 1u));
         if (u >= p.total_units) u = -1;
         Unit<NT> w{};
-        if (u >= 0) w = make_unit<NT>(u, p, BH);
+        if (u >= 0) w = make_unit<NT, BN>(u, p, BH);
         volatile int* e = sched_ring + 16 * (uc % kRing);
         e[0] = u; e[1] = w.b; e[2] = w.h; e[3] = w.hk;
         e[4] = w.tile0; e[5] = w.lo; e[6] = w.extra_sinks; e[7] = w.n_iters;
@@ -278,15 +282,15 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           const uint32_t ph = (git / STAGES) & 1;
           const int j = w.block_at(it);
           if (!(ok = mbar_wait(bar(K_EMPTY + s), ph ^ 1, wctx, 1))) break;
-          mbar_arrive_expect_tx(bar(K_FULL + s), L::kTileBytes);
+          mbar_arrive_expect_tx(bar(K_FULL + s), L::kKvBytes);
           for (int x = 0; x < kBoxes; ++x)
-            tma_load_4d(base + L::kK + s * L::kTileBytes + x * kBoxBytes, &tm_k, bar(K_FULL + s),
-                        64 * x, w.hk, j * kTile, w.b);
+            tma_load_4d(base + L::kK + s * L::kKvBytes + x * kKvBoxBytes, &tm_k, bar(K_FULL + s),
+                        64 * x, w.hk, j * BN, w.b);
           if (!(ok = mbar_wait(bar(V_EMPTY + s), ph ^ 1, wctx, 2))) break;
-          mbar_arrive_expect_tx(bar(V_FULL + s), L::kTileBytes);
+          mbar_arrive_expect_tx(bar(V_FULL + s), L::kKvBytes);
           for (int x = 0; x < kBoxes; ++x)
-            tma_load_4d(base + L::kV + s * L::kTileBytes + x * kBoxBytes, &tm_v, bar(V_FULL + s),
-                        64 * x, w.hk, j * kTile, w.b);
+            tma_load_4d(base + L::kV + s * L::kKvBytes + x * kKvBoxBytes, &tm_v, bar(V_FULL + s),
+                        64 * x, w.hk, j * BN, w.b);
         }
         if (ok) u = fetch_unit(uc + 1);
       }
@@ -301,27 +305,27 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       auto wait_all = [&](uint32_t b, uint32_t parity, unsigned where) -> bool {
         return __all_sync(0xffffffffu, mbar_wait(b, parity, wctx, where));
       };
-      constexpr uint32_t idesc_qk = make_idesc(kBf16, 128, 128, false, false);
+      constexpr uint32_t idesc_qk = make_idesc(kBf16, 128, BN, false, false);
       constexpr uint32_t idesc_pv = make_idesc(kBf16, 128, DR, false, true);
 
       auto issue_s = [&](int qb, int t, int s) {
         const uint32_t qa = base + L::kQ + (qb * NT + t) * L::kTileBytes;
-        const uint32_t ka = base + L::kK + s * L::kTileBytes;
+        const uint32_t ka = base + L::kK + s * L::kKvBytes;
 #pragma unroll
         for (int kk = 0; kk < DR / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * kBoxBytes + (kk & 3) * 32;
-          umma_ss(leader, tmem + 128 * t, make_smem_desc(qa + off, 16, 1024),
-                 make_smem_desc(ka + off, 16, 1024), idesc_qk, kk > 0 ? 1u : 0u);
+          const uint32_t off = (kk >> 2) * kBoxBytes + (kk & 3) * 32, k_off = (kk >> 2) * kKvBoxBytes + (kk & 3) * 32;
+          umma_ss(leader, tmem + BN * t, make_smem_desc(qa + off, 16, 1024),
+                 make_smem_desc(ka + k_off, 16, 1024), idesc_qk, kk > 0 ? 1u : 0u);
         }
       };
       auto issue_pv = [&](int t, int s, bool accumulate) {
-        const uint32_t va = base + L::kV + s * L::kTileBytes;
-        const uint32_t pa = kSepP ? kPBase + 64 * t : 128 * t;
+        const uint32_t va = base + L::kV + s * L::kKvBytes;
+        const uint32_t pa = kSepP ? kPBase + 64 * t : BN * t;
 #pragma unroll
-        for (int kk = 0; kk < kTile / 16; ++kk) {
+        for (int kk = 0; kk < BN / 16; ++kk) {
           // 16 keys per step: 8 packed TMEM columns of P, 16 rows (2048 bytes) of V
-          umma_ts(leader, tmem + 128 * NT + D * t, tmem + pa + 8 * kk,
-                 make_smem_desc(va + kk * 2048, kBoxBytes, 1024), idesc_pv,
+          umma_ts(leader, tmem + BN * NT + D * t, tmem + pa + 8 * kk,
+                 make_smem_desc(va + kk * 2048, kKvBoxBytes, 1024), idesc_pv,
                  (accumulate || kk > 0) ? 1u : 0u);
         }
       };
@@ -492,9 +496,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const int t = warp >> 2;                       // query tile of this warpgroup
     const int row = threadIdx.x - 128 * t;         // row inside the tile == TMEM lane
     const uint32_t lane_base = 32u * (warp & 3);
-    const uint32_t s_addr = tmem_addr(tmem, lane_base, 128 * t);
-    const uint32_t o_addr = tmem_addr(tmem, lane_base, 128 * NT + D * t);
-    const uint32_t p_addr = tmem_addr(tmem, lane_base, kSepP ? kPBase + 64 * t : 128 * t);
+    const uint32_t s_addr = tmem_addr(tmem, lane_base, BN * t);
+    const uint32_t o_addr = tmem_addr(tmem, lane_base, BN * NT + D * t);
+    const uint32_t p_addr = tmem_addr(tmem, lane_base, kSepP ? kPBase + 64 * t : BN * t);
+    constexpr int kC = BN / 32;                    // 32-column chunks of a row
     const uint64_t scale2 = pack_f2(p.scale_log2, p.scale_log2);
     int s_count = 0, o_count = 0;      // S_FULL / O_READY phases this thread has observed
     uint32_t group_phase = 0;          // uses of this warpgroup's barrier (GROUP + t)
@@ -528,6 +533,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // which keeps P within 16-bit range and makes the TMEM round trip of O rare.
       float m_ref = -INFINITY, l = 0.f;
       bool first = true;
+      // With key blocks of 64 the second block raises it by any amount, as if the two were one of 128: a row's largest
+      // P is exact more often then (error of O to 64 bits with blocks of 128 / 64 / 64 and this: B=8 H=16 T=2048 D=32 window
+      // 700, bf16, 2.118e-3 / 2.132e-3 / 2.113e-3).
+      float slack = BN == 64 ? 0.f : 8.f;
       // keys this row can see: [va, qpos] plus the sink prefix [0, vsink)
       int va = 0, vsink = 0;
       if (p.window > 0) {
@@ -545,9 +554,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         tc_fence_after();
 
         // the whole row of S into registers; from then on S_t belongs to the MMA issuer again
-        uint32_t sv[4][32];
+        uint32_t sv[kC][32];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld32(s_addr + 32 * c, sv[c]);
+        for (int c = 0; c < kC; ++c) tmem_ld32(s_addr + 32 * c, sv[c]);
         tc_wait_ld();
         tc_fence_before();
         mbar_arrive(bar(S_CONSUMED + t));
@@ -559,11 +568,11 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         // per-chunk branches against 1130 without).  Comparing every column with the row's limits cost as much as the
         // block's exponentials, and so did votes that spared chunks the whole warp sees: B=16 H=16 T=4096 window
         // 256, where two of a tile's three blocks are cut, 257 -> 226 us (B=32 H=12 T=1024 123 -> 120 us).
-        const int k0 = j * kTile;
-        if (!block_fully_visible(tile, j, p.window, p.sinks, p.block, p.T)) {
+        const int k0 = j * BN;
+        if (!rect_fully_visible(tile * kTile, tile * kTile + kTile - 1, k0, k0 + BN - 1, p.window, p.sinks, p.block, p.T)) {
           // the row sees the columns [va, qlim] and, below the window, the sinks
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < kC; ++c) {
             const int x0 = k0 + 32 * c;
             const uint32_t keep = (bits_up_to(qlim - x0) & bits_from(va - x0)) | bits_up_to(vsink - 1 - x0);
 #pragma unroll
@@ -574,7 +583,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         // row maximum of the raw scores: two chains of 3-input max
         float b0 = -INFINITY, b1 = -INFINITY;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < kC; ++c) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             b0 = fmax3(b0, __uint_as_float(sv[c][i]), __uint_as_float(sv[c][i + 1]));
@@ -587,20 +596,21 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         bool rescale = false;
         if (first) {
           m_ref = mx;
-        } else if (mx > m_ref + 8.f) {
+        } else if (mx > m_ref + slack) {
           alpha = fast_exp2(m_ref - mx);       // m_ref == -inf gives 0
           m_ref = mx;
           rescale = true;
           l *= alpha;
         }
+        if (BN == 64 && !first) slack = 8.f;
 
         // all exponentials of the row first (P stays in registers) ...
         const float m_use = (m_ref == -INFINITY) ? 0.f : m_ref;
         const uint64_t negm2 = pack_f2(-m_use, -m_use);
         uint64_t acc0 = 0ull, acc1 = 0ull;              // packed (0.f, 0.f)
-        uint32_t pk[4][16];
+        uint32_t pk[kC][16];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < kC; ++c) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             float e0, e1, e2, e3;
@@ -643,7 +653,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         first = false;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_st16(p_addr + 16 * c, pk[c]);
+        for (int c = 0; c < kC; ++c) tmem_st16(p_addr + 16 * c, pk[c]);
         tc_wait_st();
         tc_fence_before();
         mbar_arrive(bar(P_FULL + t));
@@ -730,11 +740,11 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
 }
 
-template <typename T, int D, int DR, int NT, int STAGES, int QBUF>
+template <typename T, int D, int DR, int NT, int STAGES, int QBUF, int BN = kTile>
 int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
              const CUtensorMap& mo, void* o, float* lse, unsigned* status, cudaStream_t stream) {
-  using L = FwdSmem<D, NT, STAGES, QBUF>;
-  auto kern = fwd_tc_kernel<T, D, DR, NT, STAGES, QBUF>;
+  using L = FwdSmem<D, NT, STAGES, QBUF, BN>;
+  auto kern = fwd_tc_kernel<T, D, DR, NT, STAGES, QBUF, BN>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::kDynamic) != NLFA_OK)
     return NLFA_ERR_CUDA;
   FwdParams fp;
@@ -745,6 +755,7 @@ int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, con
   fp.sinks = p.sinks;
   fp.block = p.block;
   fp.n_tiles = (p.T + kTile - 1) / kTile;
+  fp.n_blocks = (p.T + BN - 1) / BN;
   fp.n_units = (fp.n_tiles + NT - 1) / NT;
   fp.total_units = fp.n_units * p.B * p.H;
   fp.scale_log2 = p.scale * kLog2e;
@@ -753,7 +764,7 @@ int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, con
   fp.status = status;
   const int sst = sched_counters(stream, &fp.sched);
   if (sst != NLFA_OK) return sst;
-  const int room = (NT == 1 && D == 64 ? 2 : 1) * sm_count();
+  const int room = (BN == 64 ? 3 : NT == 1 && D == 64 ? 2 : 1) * sm_count();
   const int grid = fp.total_units < room ? fp.total_units : room;
   if (launch_kernel(kern, dim3(grid), dim3(NT * 128 + 128), L::kDynamic, stream, overlap_launches(kOverlapFwd), mq, mk, mv, mo,
                     fp) != cudaSuccess) {
@@ -761,6 +772,33 @@ int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, con
     return NLFA_ERR_CUDA;
   }
   return NLFA_OK;
+}
+
+// Head dims up to 64: key blocks of 64 instead of 128, and three CTAs per SM instead of two (each with 128 TMEM columns and 64
+// KB).  A block costs more for its width, but a window's edges cut less off: a tile of a window of 64 visits 192 keys, not
+// 256, one of 300 visits 448, not 512.  And a third context fills more of the others' waits at the ends of short rows.
+// Measured, blocks of 128 / 64, us (columns to visit in blocks of 64 over those in blocks of 128):
+//   few columns: whatever the number of tiles.  T=3000 window 64 with 4 sinks, D = 64 (0.5): 1 tile per SM 10.9 / 10.4, 2.6
+//     per SM 16.7 / 12.2, 8 per SM 33.4 / 25.1; B=4 H=16 T=16384 window 64 (0.75) 173 / 125
+//   up to 0.9 of them: from 4.5 tiles per SM on.  T=4096 window 300, D = 64 (0.88): 1.5 per SM 14.0 / 15.7, 3.2 20.9 / 23.0, 4.5
+//     27.1 / 25.7, 8 40.4 / 37.2; B=8 H=16 T=8192 window 400 with 4 sinks (0.83) 347 / 301
+//   as many: with eight tiles per SM, for head dim 32 (whose P has columns of its own) up to a reach of 4,096: B=64 H=16 T=1024
+//     243 / 222, 8 per SM 38.9 / 37.8, B=4 H=16 T=4096 190.6 / 188, but T=8192 1,366 / 1,410 and 4.5 per SM 25.1 / 26.4; for head
+//     dim 64 rows of up to three blocks of a window: B=32 H=16 T=2048 window 200 215 / 210, B=16 H=16 T=4096 window 256
+//     211 / 208, but window 1,000 59.7 / 64.4 and causal T=1024 41.6 / 41.9.
+bool narrow_blocks(const Problem& p, long long tiles) {
+  if (p.D > 64) return false;
+  const long long sms = sm_count();
+  const int reach = p.window > 0 && p.window < p.T ? p.window : p.T;
+  if (p.window == 0) return p.D == 32 && reach <= 4096 && tiles >= 8 * sms;
+  auto blocks = [&](int width) {                 // of the last tile: one that sees a whole window, if any does
+    const TileRange r = tile_range((p.T - 1) / kTile, p.window, p.sinks, 0, (p.T + width - 1) / width, width);
+    return static_cast<long long>(r.hi - r.lo + 1) + (r.sink_blocks < r.lo ? r.sink_blocks : r.lo);
+  };
+  const long long wide = blocks(kTile), narrow = blocks(64);
+  return 5 * narrow <= 6 * wide ||                                           // 0.6 of the columns or fewer
+         (10 * narrow <= 18 * wide && 2 * tiles >= 9 * sms) ||               // 0.9
+         (tiles >= 8 * sms && (p.D == 32 ? reach <= 4096 : wide <= 3));
 }
 
 }  // namespace
@@ -797,8 +835,18 @@ int launch_fwd_tc(const Problem& p, const void* q, const void* k, const void* v,
   const int reach = p.window > 0 && p.window < p.T ? p.window : p.T;
   const bool single = p.D == 128 ? tiles <= 2ll * sm_count() || p.T <= kTile
                                  : (reach <= 4096 && kv_bytes < (reach <= 1024 ? l2_bytes() : l2_bytes() / 2)) || p.T <= 2 * kTile || tiles <= sm_count();
+  const bool narrow = narrow_blocks(p, tiles);
+  if (narrow) {
+    st = make_tile_map(&mk, k, p.dtype, p.B, p.T, p.Hkv, p.D, 64);
+    if (st == NLFA_OK) st = make_tile_map(&mv, v, p.dtype, p.B, p.T, p.Hkv, p.D, 64);
+    if (st != NLFA_OK) return st;
+  }
   auto go = [&](auto type) {
     using T = decltype(type);
+    if (narrow) {
+      if (p.D == 32) return launch_t<T, 64, 32, 1, 2, 2, 64>(p, mq, mk, mv, mo, o, lse, status, stream);
+      return launch_t<T, 64, 64, 1, 2, 2, 64>(p, mq, mk, mv, mo, o, lse, status, stream);
+    }
     if (single) {
       if (p.D == 32) return launch_t<T, 64, 32, 1, 2, 2>(p, mq, mk, mv, mo, o, lse, status, stream);
       if (p.D == 64) return launch_t<T, 64, 64, 1, 2, 2>(p, mq, mk, mv, mo, o, lse, status, stream);

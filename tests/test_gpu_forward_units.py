@@ -1,6 +1,6 @@
-"""Both unit heights of the tensor-core forward -- one query tile, and two (long rows and more tiles than SMs, or K and V beyond L2, at
-head dims up to 64; more than two tiles per SM at 128) -- against plain float32 attention on the GPU, at odd and even numbers of
-tiles, under every mask, and the logsumexp with them."""
+"""Both unit heights of the tensor-core forward -- one query tile, and two (long rows and more tiles than SMs, or K and V beyond
+L2, at head dims up to 64; more than two tiles per SM at 128) -- and both widths of its key blocks, against plain float32
+attention on the GPU, at odd and even numbers of tiles, under every mask, and the logsumexp with them."""
 import pytest
 import torch
 
@@ -16,7 +16,17 @@ CASES = [(1, 4200, 5, 1, 64, 0, 0, 0, torch.bfloat16), (1, 4353, 6, 2, 32, 0, 0,
          (1, 1100, 4, 2, 32, 200, 5, 0, torch.bfloat16), (3, 700, 6, 2, 128, 0, 0, 96, torch.float16)]
 
 
-@pytest.mark.parametrize("B,T,H,Hkv,D,window,sinks,block,dtype", CASES)
+# key blocks of 64: few columns for any number of tiles, fewer from 4.5 tiles per SM on, as many from eight on; the edges of a
+# window at, before and behind a block's, sinks of one block and of two, ragged rows; T = 63 .. 65 into a block, rows inside one
+NARROW = [(1, 3000, 2, 1, 64, 64, 4, 0, torch.bfloat16), (1, 1089, 4, 2, 32, 50, 0, 0, torch.float16),
+          (1, 2111, 3, 3, 64, 128, 64, 0, torch.float16), (1, 191, 2, 2, 32, 65, 1, 0, torch.bfloat16),
+          (8, 1500, 9, 3, 64, 300, 4, 0, torch.bfloat16), (8, 1473, 9, 9, 32, 333, 70, 0, torch.float16),
+          (12, 1100, 12, 4, 64, 200, 0, 0, torch.bfloat16), (12, 1025, 12, 12, 64, 256, 0, 0, torch.float16),
+          (12, 1000, 12, 4, 32, 0, 0, 0, torch.bfloat16), (12, 1088, 12, 12, 32, 0, 0, 100, torch.float16),
+          (30, 450, 12, 6, 32, 0, 0, 0, torch.bfloat16), (60, 63, 20, 4, 32, 0, 0, 16, torch.bfloat16)]
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,D,window,sinks,block,dtype", CASES + NARROW)
 def test_forward_in_both_unit_heights(B, T, H, Hkv, D, window, sinks, block, dtype):
     from machinelearning_b200 import flash_cuda as fc
     assert fc.is_available(), fc.unavailable_reason()
