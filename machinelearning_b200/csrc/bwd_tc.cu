@@ -1213,6 +1213,18 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
   }
 }
 
+// (batch, KV head) pairs whose dK/dV units are handed out together: one per CTA -- unless that left a last group of less
+// than half as many, whose first and longest units would start when most CTAs have nothing left; then all groups get the
+// same size.  Backward, H=2 T=1024 D=64: B=150 (300 pairs: 148 + 148 + 4) 252.5 -> 243.7 us, B=225 (450) 375.8 -> 365.3;
+// H=6/2 T=1000 block 32 B=75 (150) 366 -> 342; H=2 T=2048 window 256, 4 sinks, B=80 (160) 240 -> 228.  With a last
+// group of more than half (384 pairs at 148 CTAs) both orders measure the same.
+inline int group_of_pairs(int pairs, int ctas) {
+  const int last = pairs % ctas;
+  if (pairs < ctas || last == 0 || 2 * last >= ctas) return ctas;
+  const int groups = pairs / ctas + 1;
+  return (pairs + groups - 1) / groups;
+}
+
 template <typename T, int D, int DR, int MODE, int STAGES, int XBUF, int YR>
 int launch_mode(const Problem& p, const void* dout, const void* q, const void* k, const void* v,
                 const float* lse, const float* delta, void* out0, void* out1, unsigned* status,
@@ -1288,6 +1300,7 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
   }
   const int grid = bp.total_units < sm_count() ? bp.total_units : sm_count();
   bp.sched_group = MODE == MODE_DQ ? bp.BH : grid;      // (the dQ pass gains nothing from groups)
+  if (MODE == MODE_DKV || MODE == MODE_DKV_DS) bp.sched_group = group_of_pairs(bp.BH, grid);
   if (MODE == MODE_DKV_DS) {
     // This pass shares DRAM with the dS it writes: groups whose Q and dO stay in L2, where those of a head per CTA would
     // not, as long as each gives every CTA two units (run long enough for the power cap to hold, the whole backward at

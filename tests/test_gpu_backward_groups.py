@@ -1,0 +1,29 @@
+"""The dK/dV pass hands its units out in groups of (batch, KV head) pairs, one pair per SM, or in groups of equal size where the
+last would have less than half as many: gradients against plain float32 autograd at both edges of that rule."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (32, torch.float16), (128, torch.bfloat16)])
+@pytest.mark.parametrize("extra,groups", [(0, 1), (1, 1), (0.5, 1), (0.49, 1), (1, 2), (-1, 1)])
+def test_gradients_for_any_number_of_pairs(D, dtype, extra, groups):
+    from machinelearning_b200 import flash_cuda as fc
+    assert fc.is_available(), fc.unavailable_reason()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B, T, H, window, sinks = groups * sms + (int(extra * sms) if isinstance(extra, float) else extra), 300, 2, 140, 3
+    g = torch.Generator(device="cuda").manual_seed(B + D)
+    q, k, v, do = (torch.randn(B, T, h, D, device="cuda", generator=g).to(dtype) for h in (H, 1, 1, H))
+    scale = D ** -0.5
+    o, lse = fc.fwd(q, k, v, scale, True, window, sinks)
+    got = fc.bwd(do, q, k, v, o, lse, scale, True, window, sinks)
+    i, j = torch.arange(T, device="cuda")[:, None], torch.arange(T, device="cuda")[None, :]
+    keep = (j <= i) & ((j > i - (window - sinks)) | (j < sinks))
+    qf, kf, vf = (t.float().requires_grad_() for t in (q, k, v))
+    s = torch.einsum("bthd,bsd->bhts", qf, kf[:, :, 0]) * scale
+    p = s.masked_fill(~keep, float("-inf")).softmax(-1)
+    torch.einsum("bhts,bsd->bthd", p, vf[:, :, 0]).backward(do.float())
+    # o, P, dS and the results are rounded to 16 bits: four errors of at most 2^-8 of the largest terms
+    for a, want in zip(got, (qf.grad, kf.grad, vf.grad)):
+        assert (a.float() - want).abs().max().item() <= 4 * 2.0 ** -8 * want.abs().max().item()
