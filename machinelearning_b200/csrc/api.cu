@@ -482,6 +482,21 @@ size_t ds_most_bytes() {
   }();
   return most;
 }
+// Kernels of these passes with no more scratch than the tape (0: refused).
+int passes_kernel_count(const Problem& p, int path, int passes) {
+  if (passes <= 0 || passes > (NLFA_PASS_ALL | NLFA_PASS_FUSED) || p.B <= 0 || p.T <= 0 || p.H <= 0) return 0;
+  const int resolved = nlfa_resolve_path(p.dtype, p.D, path);
+  if (resolved < 0) return 0;
+  const int delta = (passes & NLFA_PASS_DELTA) ? 1 : 0;
+  if (passes & NLFA_PASS_FUSED) {
+    if ((passes & (NLFA_PASS_DKV | NLFA_PASS_DQ)) || resolved != NLFA_PATH_TENSOR || p.D > 64) return 0;
+    return delta + 2;                                          // the pass and the convert kernel
+  }
+  const int two = ((passes & NLFA_PASS_DKV) ? 1 : 0) + ((passes & NLFA_PASS_DQ) ? 1 : 0);
+  if (resolved == NLFA_PATH_TENSOR && bwd_delta_in_dq(p, passes)) return two;
+  return delta + two;
+}
+
 }  // namespace
 
 size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
@@ -526,20 +541,7 @@ int nlfa_bwd_fused(const void* dout, const void* q, const void* k, const void* v
 }
 
 int nlfa_bwd_kernel_count(int B, int T, int H, int D, int dtype, int path, int passes) {
-  if (passes <= 0 || passes > (NLFA_PASS_ALL | NLFA_PASS_FUSED) || B <= 0 || T <= 0 || H <= 0) return 0;
-  const int resolved = nlfa_resolve_path(dtype, D, path);
-  if (resolved < 0) return 0;
-  const int delta = (passes & NLFA_PASS_DELTA) ? 1 : 0;
-  if (passes & NLFA_PASS_FUSED) {
-    if ((passes & (NLFA_PASS_DKV | NLFA_PASS_DQ)) || resolved != NLFA_PATH_TENSOR || D > 64) return 0;
-    return delta + 2;                                          // the pass and the convert kernel
-  }
-  const int two = ((passes & NLFA_PASS_DKV) ? 1 : 0) + ((passes & NLFA_PASS_DQ) ? 1 : 0);
-  if (resolved == NLFA_PATH_TENSOR) {
-    Problem p{B, T, H, H, D, 0, 0, 1.f, dtype, 0};
-    if (bwd_delta_in_dq(p, passes)) return two;
-  }
-  return delta + two;
+  return passes_kernel_count(Problem{B, T, H, H, D, 0, 0, 1.f, dtype, 0}, path, passes);
 }
 
 int nlfa_bwd_workspace_kernel_count(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
@@ -549,7 +551,7 @@ int nlfa_bwd_workspace_kernel_count(int B, int T, int H, int Hkv, int D, int win
   simplify_mask(p);
   const size_t tape = round256(nlfa_bwd_scratch_bytes(B, T, H)), pair = ds_pair_bytes(p);
   if (D != 128 || nlfa_resolve_path(dtype, D, path) != NLFA_PATH_TENSOR || scratch_bytes < tape + pair)
-    return nlfa_bwd_kernel_count(B, T, H, D, dtype, path, NLFA_PASS_ALL);
+    return passes_kernel_count(p, path, NLFA_PASS_ALL);
   const size_t pairs = (scratch_bytes - tape) / pair, all = static_cast<size_t>(B) * Hkv;
   return 1 + 2 * static_cast<int>((all + pairs - 1) / pairs);
 }

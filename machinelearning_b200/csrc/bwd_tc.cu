@@ -1340,7 +1340,13 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
 // delta_kernel's bit for bit) -- and a problem large enough for it to pay.  With fewer than
 // sixteen query tiles per SM the backward is faster the other way round (measured at B = 4, 8, 16
 // of H = 12, T = 1024: the dQ pass can then start beside the dK/dV pass, and a short Delta kernel
-// costs less than the later start of the first unit).  NLFA_DELTA_IN_DQ=0 / 1 forces either.
+// costs less than the later start of the first unit); with sixteen or more it gains 1-6% (B=130 H=12 T=256 204 -> 193 us,
+// B=32 T=1024 320 -> 313, B=12 H=8 T=8192 window 600 748 -> 722).  Two kinds of windows stay with the three kernels at
+// any size.  Up to a tile wide, the units are too short to hide the next one's Delta (H=16 T=4096 window 64 B=5 172.3 against
+// 175.0 us, B=12 406 / 410, with 4 sinks 485 / 495; H=12/4 window 200 B=8 220 against 211 the other way).  And with sinks
+// the first key block is seen by every query, one unit as long as a whole head group: where that is most of the dK/dV
+// pass, the dQ pass has to run beside it (B=5 H=12/4 T=4096 window 500, 16 sinks, 1.07 of a CTA's share: 212 against
+// 242 us; 0.67 of it, B=8: 345 / 340).  NLFA_DELTA_IN_DQ=0 / 1 forces either.
 inline bool delta_in_dq_pass(const Problem& p, int passes) {
   static const int forced = [] {
     const char* v = std::getenv("NLFA_DELTA_IN_DQ");
@@ -1350,7 +1356,14 @@ inline bool delta_in_dq_pass(const Problem& p, int passes) {
   if (p.D != 64 || (passes & NLFA_PASS_FUSED) != 0 || (passes & both) != both || forced == 0) return false;
   if (forced == 1) return true;
   const long long tiles = static_cast<long long>(p.B) * p.H * ((p.T + kTile - 1) / kTile);
-  return tiles >= 16ll * sm_count();
+  if (tiles < 16ll * sm_count()) return false;
+  if (p.window <= 0) return true;
+  if (p.window <= kTile) return false;
+  if (p.sinks <= 0) return true;
+  // iterations, in multiples of T / kTile times the group: the longest unit 1, a CTA's share (B Hkv / SMs) times a key
+  // block's mean of window / kTile + 1.5 and the sink block's 1
+  const long long share_x256 = static_cast<long long>(p.B) * p.Hkv * (2ll * p.window + 5 * kTile);    // * 2 kTile
+  return 4 * share_x256 >= 5ll * 2 * kTile * sm_count();                                           // longest <= 0.8 share
 }
 
 template <typename T, int D, int DR, int STAGES, int XBUF, int YR>
@@ -1391,7 +1404,8 @@ int launch_both(const Problem& p, const void* dout, const void* q, const void* k
     // The whole backward in two launches: the dQ pass forms Delta on its way and runs first, the
     // dK/dV pass reads it.
     if constexpr (DR == 64) if (delta_in_dq_pass(p, passes)) {
-      // (plain launches: between these two long kernels the overlapped set-up measured slower)
+      // (plain launches: back to back the overlapped set-up is 0.5% faster, in a training step -- B=32 H=12 T=1024 forward and
+      // backward 429.3 us -- 0.4% slower with the second overlapped, 1.1% with both)
       st = launch_mode<T, D, DR, MODE_DQ, STAGES, XBUF, YR>(p, dout, q, k, v, lse, delta, dq, nullptr, status, stream,
                                                        nullptr, nullptr, false, o, delta, true);
       if (st != NLFA_OK || (passes & NLFA_PASS_DKV) == 0) return st;

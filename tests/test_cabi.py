@@ -148,6 +148,16 @@ def test_backward_kernel_count_follows_the_layout(lib):
     assert count(4096, 1024, 12, 64, bf16, tensor, _lib.PASS_DELTA | _lib.PASS_DQ) == 1
 
 
+@pytest.mark.parametrize("window,sinks,block,kernels", [(0, 0, 0, 2), (0, 0, 700, 2), (128, 0, 0, 3), (1, 0, 0, 3), (129, 0, 0, 2),
+                                                        (129, 4, 0, 2), (128, 4, 0, 3), (4096, 0, 0, 2), (5000, 7, 0, 2)])
+def test_backward_kernel_count_of_a_window(lib, window, sinks, block, kernels):
+    """Windows of up to a tile keep the Delta kernel at any size; one that hides nothing means no window."""
+    from machinelearning_b200 import _lib as L
+    count = lambda D: lib.nlfa_bwd_workspace_kernel_count(1024, 4096, 16, 16, D, window, sinks, block, L.DTYPE_BF16, L.PATH_TENSOR, 0)
+    assert count(64) == kernels
+    assert count(32) == 3
+
+
 def test_workspace_sizes_of_extreme_extents(lib):
     """Sizes whose tile arithmetic leaves 32 bits: one pair's dS is beyond the limit, so the tape alone is asked for; a block
     length or a number of sinks next to 2^31 means what T does."""

@@ -1,5 +1,6 @@
 """The dK/dV pass hands its units out in groups of (batch, KV head) pairs, one pair per SM, or in groups of equal size where the
-last would have less than half as many: gradients against plain float32 autograd at both edges of that rule."""
+last would have less than half as many: gradients against plain float32 autograd at both edges of that rule, and which
+of its two layouts a window with sinks gets."""
 import pytest
 import torch
 
@@ -27,3 +28,13 @@ def test_gradients_for_any_number_of_pairs(D, dtype, extra, groups):
     # o, P, dS and the results are rounded to 16 bits: four errors of at most 2^-8 of the largest terms
     for a, want in zip(got, (qf.grad, kf.grad, vf.grad)):
         assert (a.float() - want).abs().max().item() <= 4 * 2.0 ** -8 * want.abs().max().item()
+
+
+def test_long_sink_blocks_keep_the_delta_kernel():
+    """One sink block's unit is group * T / 128 iterations; dQ runs beside it unless it is at most 0.8 of a CTA's share."""
+    from machinelearning_b200 import _lib as L, flash_cuda as fc
+    count = lambda B, T: fc._load().nlfa_bwd_workspace_kernel_count(B, T, 12, 4, 64, 500, 16, 0, L.DTYPE_BF16, L.PATH_TENSOR, 0)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    enough = -(-5 * 256 * sms // (4 * 4 * (2 * 500 + 640)))           # pairs * (2 w + 640) * 4 >= 5 * 256 * SMs, four pairs each
+    assert count(enough, 16384) == 2
+    assert count(enough - 1, 16384) == 3
