@@ -107,7 +107,7 @@ size_t nlfa_bwd_scratch_bytes(int B, int T, int H);
  * (every pass asked for, tensor-core path) let the dK/dV kernel leave dS there and form dQ as one product
  * over it, that many pairs per launch; given less they recompute dS in the dQ kernel.  Same bits either way.
  * Equals nlfa_bwd_scratch_bytes where there is nothing to gain (head dims below 128, fp32 path, a pair larger
- * than that, launches too small to fill the GPU). */
+ * than that, launches too small to fill the GPU, windows whose sink block is most of the dK/dV pass). */
 size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
                                 int path);
 

@@ -518,6 +518,12 @@ size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window,
   const size_t parts = (all + most - 1) / most, per = (all + parts - 1) / parts;
   const size_t units = per * ((T + kTile - 1) / kTile), sms = static_cast<size_t>(sm_count());
   if (2 * units < 3 * sms || (parts > 1 && units < 3 * sms)) return tape;
+  // With sinks the first key block's unit is as long as a whole head group: beyond one and a half of a CTA's share of the dK/dV
+  // pass (per key block window / kTile + 1.5 iterations, about one more to start it, and 1 of the sink block's) the dQ pass has to run
+  // beside it.  Reading / recomputing, us: B=2 H=12/4 T=16384 window 500, 16 sinks (2.5 shares) 926 / 720, B=2 H=12/4 T=8192 window
+  // 1,000, 4 sinks (1.6) 535 / 410, B=1 H=8 T=16384 (1.6) 371 / 311, B=1 H=12/4 T=8192 window 2,000 (1.9) 484 / 353; B=3 H=8 T=8192
+  // window 128 (1.4) 208 / 217, B=2 H=12/4 T=8192 window 2,000 (1.0) 653 / 721, T=4096 313 / 297, B=8 (0.2) 1,050 / 1,252.
+  if (p.window > 0 && p.sinks > 0 && 3 * all * (2 * static_cast<size_t>(p.window) + 7 * kTile) < 2 * 2 * kTile * sms) return tape;
   return round256(tape) + pair * (all < most ? all : most);
 }
 
