@@ -775,30 +775,17 @@ int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, con
 }
 
 // Head dims up to 64: key blocks of 64 instead of 128, and three CTAs per SM instead of two (each with 128 TMEM columns and 64
-// KB).  A block costs more for its width, but a window's edges cut less off: a tile of a window of 64 visits 192 keys, not
-// 256, one of 300 visits 448, not 512.  And a third context fills more of the others' waits at the ends of short rows.
-// Measured, blocks of 128 / 64, us (columns to visit in blocks of 64 over those in blocks of 128):
-//   few columns: whatever the number of tiles.  T=3000 window 64 with 4 sinks, D = 64 (0.5): 1 tile per SM 10.9 / 10.4, 2.6
-//     per SM 16.7 / 12.2, 8 per SM 33.4 / 25.1; B=4 H=16 T=16384 window 64 (0.75) 173 / 125
-//   up to 0.9 of them: from 4.5 tiles per SM on.  T=4096 window 300, D = 64 (0.88): 1.5 per SM 14.0 / 15.7, 3.2 20.9 / 23.0, 4.5
-//     27.1 / 25.7, 8 40.4 / 37.2; B=8 H=16 T=8192 window 400 with 4 sinks (0.83) 347 / 301
-//   as many: with eight tiles per SM, for head dim 32 (whose P has columns of its own) up to a reach of 4,096: B=64 H=16 T=1024
-//     243 / 222, 8 per SM 38.9 / 37.8, B=4 H=16 T=4096 190.6 / 188, but T=8192 1,366 / 1,410 and 4.5 per SM 25.1 / 26.4; for head
-//     dim 64 rows of up to three blocks of a window: B=32 H=16 T=2048 window 200 215 / 210, B=16 H=16 T=4096 window 256
-//     211 / 208, but window 1,000 59.7 / 64.4 and causal T=1024 41.6 / 41.9.
-bool narrow_blocks(const Problem& p, long long tiles) {
-  if (p.D > 64) return false;
-  const long long sms = sm_count();
-  const int reach = p.window > 0 && p.window < p.T ? p.window : p.T;
-  if (p.window == 0) return p.D == 32 && reach <= 4096 && tiles >= 8 * sms;
+// KB).  A block costs more for its width, but a short window's edges cut less off: a tile of a window of 64 visits 192 keys, not 256.
+// The two widths round P at different references, so the width follows from the mask and the row's length alone: any slice of
+// the batch or of the heads has the bits of the whole call.  (With eight tiles per SM blocks of 64 are 2-20% faster for most
+// windows and for short rows of head dim 32; with two they are as much slower.)  Hence few columns, 0.6 of those in blocks of 128.
+bool narrow_blocks(const Problem& p) {
+  if (p.D > 64 || p.window == 0) return false;
   auto blocks = [&](int width) {                 // of the last tile: one that sees a whole window, if any does
     const TileRange r = tile_range((p.T - 1) / kTile, p.window, p.sinks, 0, (p.T + width - 1) / width, width);
     return static_cast<long long>(r.hi - r.lo + 1) + (r.sink_blocks < r.lo ? r.sink_blocks : r.lo);
   };
-  const long long wide = blocks(kTile), narrow = blocks(64);
-  return 5 * narrow <= 6 * wide ||                                           // 0.6 of the columns or fewer
-         (10 * narrow <= 18 * wide && 2 * tiles >= 9 * sms) ||               // 0.9
-         (tiles >= 8 * sms && (p.D == 32 ? reach <= 4096 : wide <= 3));
+  return 5 * blocks(64) <= 6 * blocks(kTile);
 }
 
 }  // namespace
@@ -835,7 +822,7 @@ int launch_fwd_tc(const Problem& p, const void* q, const void* k, const void* v,
   const int reach = p.window > 0 && p.window < p.T ? p.window : p.T;
   const bool single = p.D == 128 ? tiles <= 2ll * sm_count() || p.T <= kTile
                                  : (reach <= 4096 && kv_bytes < (reach <= 1024 ? l2_bytes() : l2_bytes() / 2)) || p.T <= 2 * kTile || tiles <= sm_count();
-  const bool narrow = narrow_blocks(p, tiles);
+  const bool narrow = narrow_blocks(p);
   if (narrow) {
     st = make_tile_map(&mk, k, p.dtype, p.B, p.T, p.Hkv, p.D, 64);
     if (st == NLFA_OK) st = make_tile_map(&mv, v, p.dtype, p.B, p.T, p.Hkv, p.D, 64);

@@ -17,6 +17,9 @@ def _pinned(shape, seed, dtype):
     (8, 256, 4, 4, 64, 0, 0, 4),
     (5, 200, 4, 2, 64, 64, 4, 3),      # ragged slices, GQA, window with sinks, odd T
     (2, 384, 2, 2, 128, 0, 0, 8),      # more slices asked for than batch elements
+    # the whole batch has more tiles than eight, sixteen or 4.5 per SM, a slice fewer
+    (16, 1024, 12, 12, 32, 0, 0, 2), (8, 2048, 12, 4, 64, 256, 0, 2), (4, 2048, 12, 4, 64, 400, 4, 2),
+    (6, 4160, 12, 4, 64, 150, 0, 6), (4, 2500, 12, 4, 32, 64, 4, 4), (20, 1000, 12, 12, 64, 0, 0, 2),
 ])
 def test_pipeline_matches_whole_batch(B, T, H, Hkv, D, window, sinks, slices):
     from machinelearning_b200 import flash_cuda, host_pipeline
