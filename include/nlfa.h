@@ -96,6 +96,11 @@ int nlfa_fwd_masked(const void* q, const void* k, const void* v, void* o, float*
                     int H, int Hkv, int D, float scale, int window, int sinks, int block, int dtype,
                     int path, void* stream);
 
+/* Keys per block in which the tensor-core forward walks a row under this mask: 128, or 64 for short windows at head
+ * dims up to 64 (0: arguments it refuses, or the fp32 path).  The block sets where P is rounded, so it depends on no
+ * extent but T: a slice of the batch or of the heads gives the bits of the whole call. */
+int nlfa_fwd_key_block(int T, int D, int window, int sinks, int block, int dtype, int path);
+
 /* Bytes of device scratch `nlfa_bwd` needs (the Delta tape, [B,H,T] float32).
  * The reference allocates the same tensor itself (flash_attn_cuda.cu:1770-1773). */
 size_t nlfa_bwd_scratch_bytes(int B, int T, int H);

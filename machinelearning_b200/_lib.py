@@ -29,6 +29,7 @@ SIGNATURES = {
     "nlfa_resolve_path": (_c_int, [_c_int, _c_int, _c_int]),
     "nlfa_fwd": (_c_int, [_c_void_p] * 5 + [_c_int] * 5 + [_c_float] + [_c_int] * 4 + [_c_void_p]),
     "nlfa_fwd_masked": (_c_int, [_c_void_p] * 5 + [_c_int] * 5 + [_c_float] + [_c_int] * 5 + [_c_void_p]),
+    "nlfa_fwd_key_block": (_c_int, [_c_int] * 7),
     "nlfa_bwd_masked": (_c_int, [_c_void_p] * 10 + [_c_size_t] + [_c_int] * 5 + [_c_float]
                         + [_c_int] * 6 + [_c_void_p]),
     "nlfa_bwd_scratch_bytes": (_c_size_t, [_c_int, _c_int, _c_int]),

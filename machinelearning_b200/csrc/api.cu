@@ -499,6 +499,13 @@ int passes_kernel_count(const Problem& p, int path, int passes) {
 
 }  // namespace
 
+int nlfa_fwd_key_block(int T, int D, int window, int sinks, int block, int dtype, int path) {
+  Problem p{1, T, 1, 1, D, window, sinks, 1.f, dtype, block};
+  if (T <= 0 || check_problem(p) != NLFA_OK || nlfa_resolve_path(dtype, D, path) != NLFA_PATH_TENSOR) return 0;
+  simplify_mask(p);
+  return fwd_key_block(p);
+}
+
 size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
                                 int path) {
   const size_t tape = nlfa_bwd_scratch_bytes(B, T, H);

@@ -177,6 +177,7 @@ int launch_bwd_simt(const Problem& p, const void* dout, const void* q, const voi
                     float* delta, int passes, cudaStream_t stream);
 int launch_delta(const Problem& p, const void* dout, const void* o, float* delta,
                  cudaStream_t stream);
+int fwd_key_block(const Problem& p);            // keys per block of the tensor-core forward
 int launch_fwd_tc(const Problem& p, const void* q, const void* k, const void* v, void* o,
                   float* lse, unsigned* status, cudaStream_t stream);
 // Scratch of the fused backward pass (head dim <= 64), behind the Delta tape in the caller's

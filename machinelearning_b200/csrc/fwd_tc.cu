@@ -775,20 +775,24 @@ int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, con
 }
 
 // Head dims up to 64: key blocks of 64 instead of 128, and three CTAs per SM instead of two (each with 128 TMEM columns and 64
-// KB).  A block costs more for its width, but a short window's edges cut less off: a tile of a window of 64 visits 192 keys, not 256.
-// The two widths round P at different references, so the width follows from the mask and the row's length alone: any slice of
-// the batch or of the heads has the bits of the whole call.  (With eight tiles per SM blocks of 64 are 2-20% faster for most
-// windows and for short rows of head dim 32; with two they are as much slower.)  Hence few columns, 0.6 of those in blocks of 128.
+// KB).  A block costs more for its width, but a short window's edges cut less off: with 2 to 65 recent keys and sinks in one
+// block of 64, a full tile visits 192 + 64 columns in blocks of 64 and 256 + 128 in blocks of 128 (a cut tile at the end of the
+// row does not count, nor do rows of up to two tiles, which have no full one).  The two widths round P at different references,
+// so the choice follows from the mask and the row's length alone: any slice of the batch or of the heads has the bits of the
+// whole call.  Blocks of 128 / 64, us, at about 0.5, 1, 2, 2.6, 4 and 8 tiles per SM:
+//   T=4096 D=64 window 64             8.9/8.5 9.5/9.5 10.1/10.4 13.0/9.9 17.3/15.2 25.1/21.1   (long rows, 16 per SM: 46.5/38.5)
+//   T=4096 D=64 window 64, 4 sinks    9.5/9.3 11.3/10.6 11.6/11.6 .. 22.0/17.3 33.2/25.0        D=32 .. 21.2/15.9 32.0/22.7
+// of 36 such masks and lengths (300 to 16,384) the worst is 0.96 of the speed, below two tiles per SM, the best 1.42.  Every
+// other mask loses somewhere: 66 to 129 recent keys 0.84 to 1.1, 130 to 193 0.88 to 1.25, 300 0.81 to 1.17, sinks in two
+// blocks of 64 0.85 to 1.18, one or two tiles per row 0.84 to 1.3.
 bool narrow_blocks(const Problem& p) {
-  if (p.D > 64 || p.window == 0) return false;
-  auto blocks = [&](int width) {                 // of the last tile: one that sees a whole window, if any does
-    const TileRange r = tile_range((p.T - 1) / kTile, p.window, p.sinks, 0, (p.T + width - 1) / width, width);
-    return static_cast<long long>(r.hi - r.lo + 1) + (r.sink_blocks < r.lo ? r.sink_blocks : r.lo);
-  };
-  return 5 * blocks(64) <= 6 * blocks(kTile);
+  const int recent = p.window - p.sinks;
+  return p.D <= 64 && p.window > 0 && p.T > 2 * kTile && p.sinks <= 64 && recent >= 2 && recent <= 65;
 }
 
 }  // namespace
+
+int fwd_key_block(const Problem& p) { return narrow_blocks(p) ? 64 : kTile; }
 
 int launch_fwd_tc(const Problem& p, const void* q, const void* k, const void* v, void* o,
                   float* lse, unsigned* status, cudaStream_t stream) {

@@ -123,6 +123,23 @@ def test_mask_geometry_rejects_bad_arguments(lib):
     assert lib.nlfa_check_mask_geometry(256, 0, 0, 96) < 0
 
 
+@pytest.mark.parametrize("window,sinks,width", [(0, 0, 128), (1, 0, 128), (2, 0, 64), (65, 0, 64), (66, 0, 128), (66, 1, 64), (6, 4, 64),
+                                                (5, 4, 128), (69, 4, 64), (70, 4, 128), (128, 64, 64), (129, 64, 64), (130, 64, 128),
+                                                (128, 65, 128), (256, 0, 128)])
+def test_forward_key_block_of_a_full_tile(lib, window, sinks, width):
+    """The width of the forward's key blocks is that of a tile inside the row, whatever is left of the last one."""
+    from machinelearning_b200 import _lib as L
+    for D in (32, 64):
+        for T in (257, 320, 384, 1000, 3000, 4095, 4096, 4097, 4160, 4161, 16384):
+            assert lib.nlfa_fwd_key_block(T, D, window, sinks, 0, L.DTYPE_BF16, L.PATH_TENSOR) == width
+        assert lib.nlfa_fwd_key_block(256, D, window, sinks, 0, L.DTYPE_F16, L.PATH_AUTO) == 128
+    assert lib.nlfa_fwd_key_block(4096, 128, window, sinks, 0, L.DTYPE_BF16, L.PATH_TENSOR) == 128
+    assert lib.nlfa_fwd_key_block(4096, 64, window, sinks, 0, L.DTYPE_F32, L.PATH_AUTO) == 0
+    if 0 < window and 0 < sinks:
+        assert lib.nlfa_fwd_key_block(4096, 64, sinks, window, 0, L.DTYPE_BF16, L.PATH_TENSOR) == 0
+    assert lib.nlfa_fwd_key_block(0, 64, window, sinks, 0, L.DTYPE_BF16, L.PATH_TENSOR) == 0
+
+
 def test_backward_kernel_count_follows_the_layout(lib):
     """``nlfa_bwd_kernel_count``: Delta + dK/dV + dQ; two kernels where the dQ pass forms Delta (head dim
     64, tensor-core path, a large problem -- every problem is large next to the one SM a machine

@@ -44,3 +44,15 @@ def test_forward_in_both_unit_heights(B, T, H, Hkv, D, window, sinks, block, dty
         want = torch.einsum("hts,shd->thd", s.softmax(-1), v[b].float().repeat_interleave(H // Hkv, 1))
         assert (o[b].float() - want).abs().max().item() <= 2e-2 * want.abs().max().item()
         assert (lse[b] - s.logsumexp(-1)).abs().max().item() <= 1e-3
+
+
+@pytest.mark.parametrize("D,window,sinks", [(64, 64, 0), (32, 64, 4), (64, 128, 0), (64, 256, 0), (32, 400, 4), (64, 66, 0)])
+def test_the_end_of_a_row_changes_nothing_before_it(D, window, sinks):
+    """Causal rows see nothing behind them: the first rows of a longer call have the bits of the shorter one, also where the last
+    tile is cut."""
+    from machinelearning_b200 import flash_cuda as fc
+    q, k, v = (torch.randn(1, 1152, 6, D, device="cuda", generator=torch.Generator(device="cuda").manual_seed(D)).half() for _ in range(3))
+    o, lse = fc.fwd(q, k, v, D ** -0.5, True, window, sinks)
+    for T in (1024, 1025, 1060, 1088, 1090):
+        o1, lse1 = fc.fwd(*(t[:, :T].contiguous() for t in (q, k, v)), D ** -0.5, True, window, sinks)
+        assert torch.equal(o1, o[:, :T]) and torch.equal(lse1, lse[:, :, :T])
