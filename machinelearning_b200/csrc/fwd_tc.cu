@@ -533,9 +533,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // which keeps P within 16-bit range and makes the TMEM round trip of O rare.
       float m_ref = -INFINITY, l = 0.f;
       bool first = true;
-      // With key blocks of 64 the second block raises it by any amount, as if the two were one of 128: a row's largest
-      // P is exact more often then (error of O to 64 bits with blocks of 128 / 64 / 64 and this: B=8 H=16 T=2048 D=32 window
-      // 700, bf16, 2.118e-3 / 2.132e-3 / 2.113e-3).
+      // With key blocks of 64 the tile's second block raises it by any amount, so that a row's largest P is exact about as often as
+      // with blocks of 128.  Error of o to 64 bits against those, bf16 / fp16, under the windows that get blocks of 64: 2
+      // -0.03 / -0.02%, 16 -0.15 / -0.15%, 40 -0.40 / -0.41%, 64 -0.53 / -0.64%, with 4 sinks -2.4%.  (Where a tile visits
+      // more of them, rows that see nothing of its first block come out worse: windows of 96 +0.6%, 160 +0.5%, 200 +0.9%.)
       float slack = BN == 64 ? 0.f : 8.f;
       // keys this row can see: [va, qpos] plus the sink prefix [0, vsink)
       int va = 0, vsink = 0;

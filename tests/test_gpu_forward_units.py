@@ -56,3 +56,31 @@ def test_the_end_of_a_row_changes_nothing_before_it(D, window, sinks):
     for T in (1024, 1025, 1060, 1088, 1090):
         o1, lse1 = fc.fwd(*(t[:, :T].contiguous() for t in (q, k, v)), D ** -0.5, True, window, sinks)
         assert torch.equal(o1, o[:, :T]) and torch.equal(lse1, lse[:, :, :T])
+
+
+@pytest.mark.parametrize("D,window,sinks", [(64, 2, 0), (64, 16, 0), (32, 65, 0), (64, 69, 4), (32, 129, 64), (64, 96, 0), (64, 200, 0),
+                                            (32, 160, 0)])
+def test_windows_lose_no_precision_to_the_width_of_key_blocks(D, window, sinks):
+    """Error to 64 bits against that of a float64 walk in blocks of 128 that rounds only P and o: the two share their roundings but
+    for the last bits of the scores, so a quarter of a percent is far above their difference and far below what a row's
+    reference taken from fewer keys costs (0.5 to 0.9%)."""
+    from machinelearning_b200 import flash_cuda as fc
+    T, H, dtype, scale = 4096, 40, torch.bfloat16, D ** -0.5
+    g = torch.Generator(device="cuda").manual_seed(window)
+    q, k, v = (torch.randn(1, T, H, D, device="cuda", generator=g).to(dtype) for _ in range(3))
+    o, _ = fc.fwd(q, k, v, scale, True, window, sinks)
+    i, j = torch.arange(T, device="cuda")[:, None], torch.arange(T, device="cuda")[None, :]
+    keep = (j <= i) & ((j > i - (window - sinks)) | (j < sinks))
+    got = walk = 0.0
+    for h in range(H):
+        s = (q[0, :, h].double() @ k[0, :, h].double().T * scale).masked_fill(~keep, float("-inf"))
+        exact = s.softmax(-1) @ v[0, :, h].double()
+        # the reference of a row is the maximum of the first block its tile visits, the first visible one's if that hides from it
+        # (a later block would have to exceed it by a factor of 256)
+        by_block = s.view(T, T // 128, 128).amax(-1)
+        first = (by_block > float("-inf")).int().argmax(-1)
+        p = (s - by_block.gather(1, first[:, None])).exp()
+        mean = (p.to(dtype).double() @ v[0, :, h].double()) / p.sum(-1, keepdim=True)
+        got += (o[0, :, h].double() - exact).square().sum()
+        walk += (mean.to(dtype).double() - exact).square().sum()
+    assert got.sqrt().item() <= 1.0025 * walk.sqrt().item(), (got.sqrt() / walk.sqrt()).item()
