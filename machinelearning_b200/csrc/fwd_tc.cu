@@ -802,10 +802,11 @@ int launch_fwd_tc(const Problem& p, const void* q, const void* k, const void* v,
   // Head dim 32: the tensor maps describe the real 32 columns, the TMA boxes are 64 wide, so loads fill columns
   // 32-63 with zeros, which no product reads, and stores drop them.
   if (!(p.scale > 0.f)) return NLFA_ERR_UNSUPPORTED_PATH;     // row max is taken before scaling
+  const int width = fwd_key_block(p);
   CUtensorMap mq, mk, mv, mo;
   int st = make_tile_map(&mq, q, p.dtype, p.B, p.T, p.H, p.D, kTile);
-  if (st == NLFA_OK) st = make_tile_map(&mk, k, p.dtype, p.B, p.T, p.Hkv, p.D, kTile);
-  if (st == NLFA_OK) st = make_tile_map(&mv, v, p.dtype, p.B, p.T, p.Hkv, p.D, kTile);
+  if (st == NLFA_OK) st = make_tile_map(&mk, k, p.dtype, p.B, p.T, p.Hkv, p.D, width);
+  if (st == NLFA_OK) st = make_tile_map(&mv, v, p.dtype, p.B, p.T, p.Hkv, p.D, width);
   if (st == NLFA_OK) st = make_tile_map(&mo, o, p.dtype, p.B, p.T, p.H, p.D, kTile);
   if (st != NLFA_OK) return st;
   const bool bf16 = p.dtype == NLFA_DTYPE_BF16;
@@ -827,15 +828,9 @@ int launch_fwd_tc(const Problem& p, const void* q, const void* k, const void* v,
   const int reach = p.window > 0 && p.window < p.T ? p.window : p.T;
   const bool single = p.D == 128 ? tiles <= 2ll * sm_count() || p.T <= kTile
                                  : (reach <= 4096 && kv_bytes < (reach <= 1024 ? l2_bytes() : l2_bytes() / 2)) || p.T <= 2 * kTile || tiles <= sm_count();
-  const bool narrow = narrow_blocks(p);
-  if (narrow) {
-    st = make_tile_map(&mk, k, p.dtype, p.B, p.T, p.Hkv, p.D, 64);
-    if (st == NLFA_OK) st = make_tile_map(&mv, v, p.dtype, p.B, p.T, p.Hkv, p.D, 64);
-    if (st != NLFA_OK) return st;
-  }
   auto go = [&](auto type) {
     using T = decltype(type);
-    if (narrow) {
+    if (width == 64) {
       if (p.D == 32) return launch_t<T, 64, 32, 1, 2, 2, 64>(p, mq, mk, mv, mo, o, lse, status, stream);
       return launch_t<T, 64, 64, 1, 2, 2, 64>(p, mq, mk, mv, mo, o, lse, status, stream);
     }
