@@ -112,7 +112,8 @@ size_t nlfa_bwd_scratch_bytes(int B, int T, int H);
  * (every pass asked for, tensor-core path) let the dK/dV kernel leave dS there and form dQ as one product
  * over it, that many pairs per launch; given less they recompute dS in the dQ kernel.  Same bits either way.
  * Equals nlfa_bwd_scratch_bytes where there is nothing to gain (head dims below 128, fp32 path, a pair larger
- * than that, launches too small to fill the GPU, windows whose sink block is most of the dK/dV pass). */
+ * than that, launches too small to fill the GPU, windows under which a key block with sinks is more than 1.4 of
+ * an SM's share of a launch of the dK/dV pass). */
 size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
                                 int path);
 
@@ -151,7 +152,7 @@ int nlfa_bwd_passes(const void* dout, const void* q, const void* k, const void* 
  * current device (0 for inputs it would refuse; for any mask, and all passes:
  * nlfa_bwd_workspace_kernel_count).  On the tensor-core path at
  * D = 64 a large problem (at least sixteen 128-row query tiles per SM; not under windows of up
- * to 128, nor where one sink block is most of the dK/dV pass) takes two:
+ * to 128, nor where one key block with sinks is more than an SM's share of the dK/dV pass) takes two:
  * the dQ pass forms Delta itself -- the row sums of dO * O, added in the order of
  * the Delta kernel, so the gradients are bit-identical either way -- and runs
  * before the dK/dV pass; smaller problems and other head dims take the three

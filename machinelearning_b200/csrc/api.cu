@@ -525,12 +525,16 @@ size_t nlfa_bwd_workspace_bytes(int B, int T, int H, int Hkv, int D, int window,
   const size_t parts = (all + most - 1) / most, per = (all + parts - 1) / parts;
   const size_t units = per * ((T + kTile - 1) / kTile), sms = static_cast<size_t>(sm_count());
   if (2 * units < 3 * sms || (parts > 1 && units < 3 * sms)) return tape;
-  // With sinks the first key block's unit is as long as a whole head group: beyond one and a half of a CTA's share of the dK/dV
-  // pass (per key block window / kTile + 1.5 iterations, about one more to start it, and 1 of the sink block's) the dQ pass has to run
-  // beside it.  Reading / recomputing, us: B=2 H=12/4 T=16384 window 500, 16 sinks (2.5 shares) 926 / 720, B=2 H=12/4 T=8192 window
-  // 1,000, 4 sinks (1.6) 535 / 410, B=1 H=8 T=16384 (1.6) 371 / 311, B=1 H=12/4 T=8192 window 2,000 (1.9) 484 / 353; B=3 H=8 T=8192
-  // window 128 (1.4) 208 / 217, B=2 H=12/4 T=8192 window 2,000 (1.0) 653 / 721, T=4096 313 / 297, B=8 (0.2) 1,050 / 1,252.
-  if (p.window > 0 && p.sinks > 0 && 3 * all * (2 * static_cast<size_t>(p.window) + 7 * kTile) < 2 * 2 * kTile * sms) return tape;
+  // Blocks with sinks are seen by every query behind them, units of up to a whole head group's iterations: where one of those is
+  // longer than 1.4 of a CTA's share of a launch, the dQ pass has to run beside it.  Of 120 random shapes reading was 1.0 to 1.3x
+  // faster below that line and recomputing up to 1.4x beyond it, but for up to 8% within 0.05 of it; reading / recomputing, us: 1.09
+  // shares (B=23 H=2/1 T=16384 window 500, 16 sinks) 1,004 / 1,264, 1.34 (B=5 H=16/4 T=4096 window 500, 130 sinks) 462 / 506, 1.46 (B=28
+  // H=16/1 T=2048 window 150, 130 sinks) 891 / 915, 1.47 (B=6 H=2/1 T=16384 window 2,000, 300 sinks) 786 / 720, 1.76 (B=3 H=2/1
+  // T=12000 window 4,000, 4 sinks) 546 / 419, in two parts 1.99 (B=16 H=16/1 T=8192 window 1,000, 100 sinks) 5,386 / 4,228.
+  if (p.window > 0 && p.sinks > 0) {
+    const DkvWork w = dkv_work(T, p.window, p.sinks);
+    if (5 * w.longest * static_cast<long long>(sms) > 7 * w.total * static_cast<long long>(per)) return tape;
+  }
   return round256(tape) + pair * (all < most ? all : most);
 }
 
@@ -702,6 +706,17 @@ int nlfa_check_mask_geometry_masked(int T, int window, int sinks, int block, int
       if (expect != count) return 1 + check;
       ++check;
     }
+  // (5) dkv_work under a window: the query tiles of every key block, counted one by one
+  if (stream_rows == kTile && window > 0) {
+    long long longest = 0, total = 0;
+    for (int j = 0; j < n128; ++j) {
+      const long long tiles = last_query_tile_of_block(j, n128, kTile, window, sinks) - j + 1;
+      longest = tiles > longest ? tiles : longest;
+      total += tiles;
+    }
+    const DkvWork w = dkv_work(T, window, sinks);
+    if (w.longest != longest || w.total != total) return 1 + check;
+  }
   return 0;
 }
 

@@ -1343,10 +1343,14 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
 // costs less than the later start of the first unit); with sixteen or more it gains 1-6% (B=130 H=12 T=256 204 -> 193 us,
 // B=32 T=1024 320 -> 313, B=12 H=8 T=8192 window 600 748 -> 722).  Two kinds of windows stay with the three kernels at
 // any size.  Up to a tile wide, the units are too short to hide the next one's Delta (H=16 T=4096 window 64 B=5 172.3 against
-// 175.0 us, B=12 406 / 410, with 4 sinks 485 / 495; H=12/4 window 200 B=8 220 against 211 the other way).  And with sinks
-// the first key block is seen by every query, one unit as long as a whole head group: where that is most of the dK/dV
-// pass, the dQ pass has to run beside it (B=5 H=12/4 T=4096 window 500, 16 sinks, 1.07 of a CTA's share: 212 against
-// 242 us; 0.67 of it, B=8: 345 / 340).  NLFA_DELTA_IN_DQ=0 / 1 forces either.
+// 175.0 us, B=12 406 / 410, with 4 sinks 485 / 495; H=12/4 window 200 B=8 220 against 211 the other way).  And blocks with
+// sinks are seen by every query behind them, units of up to a whole head group's iterations: where one of those is longer than
+// a CTA's share of the dK/dV pass, the dQ pass has to run beside it.  Of 120 random shapes two kernels were up to 5% faster below
+// that line and at most 4% slower, three up to 1.4x beyond it; two / three kernels, us: longest unit of 0.80 shares (B=12
+// H=12/4 T=6000 window 150, 16 sinks) 552 / 576, 0.86 (B=15 H=8/2 T=8192 window 500, 300 sinks) 863 / 902, 1.05 (B=12 H=12/4 T=6000
+// window 150, 100 sinks) 485 / 472, 1.28 (B=3 H=16/4 T=16384 window 1,000, 600 sinks) 1,167 / 1,057, 1.45 (B=12 H=16/1 T=2048
+// window 2,000, 130 sinks) 541 / 450, 1.9 (B=2 H=12/4 T=16384 window 1,000, 130 sinks) 735 / 516.  NLFA_DELTA_IN_DQ=0 / 1
+// forces either.
 inline bool delta_in_dq_pass(const Problem& p, int passes) {
   static const int forced = [] {
     const char* v = std::getenv("NLFA_DELTA_IN_DQ");
@@ -1360,10 +1364,8 @@ inline bool delta_in_dq_pass(const Problem& p, int passes) {
   if (p.window <= 0) return true;
   if (p.window <= kTile) return false;
   if (p.sinks <= 0) return true;
-  // iterations, in multiples of T / kTile times the group: the longest unit 1, a CTA's share (B Hkv / SMs) times a key
-  // block's mean of window / kTile + 1.5 and the sink block's 1
-  const long long share_x256 = static_cast<long long>(p.B) * p.Hkv * (2ll * p.window + 5 * kTile);    // * 2 kTile
-  return 4 * share_x256 >= 5ll * 2 * kTile * sm_count();                                           // longest <= 0.8 share
+  const DkvWork w = dkv_work(p.T, p.window, p.sinks);
+  return w.longest * sm_count() <= w.total * p.B * p.Hkv;                    // longest <= a CTA's share
 }
 
 template <typename T, int D, int DR, int STAGES, int XBUF, int YR>

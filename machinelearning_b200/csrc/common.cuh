@@ -117,6 +117,20 @@ __host__ __device__ inline int last_query_tile_of_block(int block, int n_ytiles,
   return hi;
 }
 
+// Iterations (128-row query tiles, of one query head) of the dK/dV pass over one (batch, KV head) pair under a window: of its
+// longest unit, and of all.  A block with sink keys is streamed past by every tile from its own on, one behind the sinks by
+// those a window further.
+struct DkvWork {
+  long long longest, total;
+};
+inline DkvWork dkv_work(int T, int window, int sinks) {
+  const long long n = (static_cast<long long>(T) + kTile - 1) / kTile, span = static_cast<long long>(window) - sinks;
+  const long long with_sinks = (static_cast<long long>(sinks) + kTile - 1) / kTile, ns = with_sinks < n ? with_sinks : n;
+  const long long reach = (span + kTile - 2) / kTile + 1, rest = n - ns;               // of a block without sinks, inside the row
+  const long long behind = rest <= reach ? rest * (rest + 1) / 2 : reach * (reach + 1) / 2 + (rest - reach) * reach;
+  return {ns > 0 ? n : rest < reach ? rest : reach, ns * n - ns * (ns - 1) / 2 + behind};
+}
+
 // Fused backward: key block `block`'s place in the fixed order in which the blocks that see
 // 128-row query tile `tile` add their dQ shares (ascending block index: sink blocks below the
 // window first, then the window's blocks up to the last one the tile sees -- the diagonal, or

@@ -99,7 +99,7 @@ def test_argument_checks_answer_without_a_gpu(lib):
 @pytest.mark.parametrize("T,window,sinks", [
     (1024, 0, 0), (300, 0, 0), (129, 0, 0),
     (1024, 256, 0), (1024, 64, 4), (900, 300, 130), (700, 256, 0), (2048, 512, 4),
-    (300, 400, 4), (511, 64, 0), (640, 129, 128), (384, 128, 0), (385, 1, 0),
+    (300, 400, 4), (511, 64, 0), (640, 129, 128), (384, 128, 0), (385, 1, 0), (1500, 1400, 4), (1300, 900, 600), (300, 290, 280),
 ])
 @pytest.mark.parametrize("stream_rows", [64, 128])
 def test_mask_geometry_matches_the_elementwise_predicate(lib, T, window, sinks, stream_rows):

@@ -30,27 +30,68 @@ def test_gradients_for_any_number_of_pairs(D, dtype, extra, groups):
         assert (a.float() - want).abs().max().item() <= 4 * 2.0 ** -8 * want.abs().max().item()
 
 
-def test_long_sink_blocks_keep_the_delta_kernel():
-    """One sink block's unit is group * T / 128 iterations; dQ runs beside it unless it is at most 0.8 of a CTA's share."""
+def _shares(T, window, sinks, pairs):
+    """The dK/dV pass's longest unit (a key block's query tiles, for each head of the group) over what falls to one SM, counted
+    from the visible pairs themselves."""
+    n = -(-T // 128)
+    units = []
+    for j in range(n):
+        k0, k1 = 128 * j, min(T, 128 * j + 128) - 1
+        last = lambda k: T - 1 if k < sinks else min(T - 1, k + window - sinks - 1)          # last query that sees key k
+        reach = max(last(k0), last(k1), last(min(k1, sinks - 1)) if k0 < sinks else 0)
+        units.append(reach // 128 - j + 1)
+    return max(units) * torch.cuda.get_device_properties(0).multi_processor_count / (pairs * sum(units))
+
+
+# several sink blocks, windows as long as the row, pairs for either side of the lines
+SINKS = [(16384, 500, 16), (6000, 150, 16), (4096, 2000, 1000), (4096, 4000, 600), (2048, 2000, 130), (3000, 1000, 300), (8192, 300, 100)]
+
+
+@pytest.mark.parametrize("T,window,sinks", SINKS)
+def test_long_sink_blocks_keep_the_delta_kernel(T, window, sinks):
+    """dQ runs beside the dK/dV pass, and so behind a Delta kernel, where a key block with sinks is longer than an SM's share."""
     from machinelearning_b200 import _lib as L, flash_cuda as fc
-    count = lambda B, T: fc._load().nlfa_bwd_workspace_kernel_count(B, T, 12, 4, 64, 500, 16, 0, L.DTYPE_BF16, L.PATH_TENSOR, 0)
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    enough = -(-5 * 256 * sms // (4 * 4 * (2 * 500 + 640)))           # pairs * (2 w + 640) * 4 >= 5 * 256 * SMs, four pairs each
-    assert count(enough, 16384) == 2
-    assert count(enough - 1, 16384) == 3
+    kernels = {}
+    for B in range(1, 40):
+        if B * 64 * -(-T // 128) < 16 * torch.cuda.get_device_properties(0).multi_processor_count:
+            continue
+        shares = _shares(T, window, sinks, 4 * B)
+        kernels[shares <= 1] = fc._load().nlfa_bwd_workspace_kernel_count(B, T, 64, 4, 64, window, sinks, 0, L.DTYPE_BF16, L.PATH_TENSOR, 0)
+        assert kernels[shares <= 1] == (2 if shares <= 1 else 3), (B, shares)
+    assert kernels[True] == 2
 
 
-def test_long_sink_blocks_leave_no_ds():
-    """At head dim 128 dS is left behind for the dQ pass unless one sink block is more than 1.5 of a CTA's share of the dK/dV
-    pass; with either amount of scratch the gradients have the same bits."""
+@pytest.mark.parametrize("T,window,sinks", SINKS)
+def test_long_sink_blocks_get_no_ds_scratch(T, window, sinks):
+    """At head dim 128 there is room for dS unless a key block with sinks is more than 1.4 of an SM's share of one launch."""
+    from machinelearning_b200 import _lib as L, flash_cuda as fc
+    lib, sms = fc._load(), torch.cuda.get_device_properties(0).multi_processor_count
+    seen = set()
+    for H, Hkv in ((4, 4), (64, 4)):
+        for B in range(1, 30):
+            tape = (lib.nlfa_bwd_scratch_bytes(B, T, H) + 255) // 256 * 256
+            size = lib.nlfa_bwd_workspace_bytes(B, T, H, Hkv, 128, window, sinks, 0, L.DTYPE_BF16, L.PATH_TENSOR)
+            tiles = -(-T // 128)
+            widest = max(min(t, -(-sinks // 128)) + t - max(min(t, -(-sinks // 128)), max(0, 128 * t - (window - sinks) + 1) // 128) + 1
+                         for t in range(tiles))                                    # key blocks of a query tile
+            most = (4 << 30) // (widest * tiles * 32768 * (H // Hkv))             # pairs of one launch
+            if most == 0:
+                assert size <= tape
+                continue
+            parts = -(-B * Hkv // most)
+            per = -(-B * Hkv // parts)
+            full = 2 * per * tiles >= 3 * sms and (parts == 1 or per * tiles >= 3 * sms)
+            wanted = full and _shares(T, window, sinks, per) <= 1.4
+            assert (size > tape) == wanted, (B, H, parts, _shares(T, window, sinks, per))
+            seen.add((full, wanted))
+    assert (True, True) in seen
+
+
+def test_either_amount_of_scratch_gives_the_same_bits_under_sinks():
     from machinelearning_b200 import _lib as L, flash_cuda as fc
     lib = fc._load()
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
     T, window, sinks = 9000, 260, 5
-    enough = -(-2 * 256 * sms // (3 * (2 * window + 896)))                   # 3 * pairs * (2 w + 896) >= 2 * 256 * SMs
     tape = lambda B: (lib.nlfa_bwd_scratch_bytes(B, T, 2) + 255) // 256 * 256
-    size = lambda B: lib.nlfa_bwd_workspace_bytes(B, T, 2, 1, 128, window, sinks, 0, L.DTYPE_BF16, L.PATH_TENSOR)
-    assert size(enough) > tape(enough) and size(enough - 1) <= tape(enough - 1)
     B = 3
     g = torch.Generator(device="cuda").manual_seed(2)
     q, k, v, do = (torch.randn(B, T, h, 128, device="cuda", generator=g).bfloat16() for h in (2, 1, 1, 2))
