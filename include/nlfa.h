@@ -151,8 +151,8 @@ int nlfa_bwd_passes(const void* dout, const void* q, const void* k, const void* 
 /* How many kernels nlfa_bwd_passes launches for this problem without a window on the
  * current device (0 for inputs it would refuse; for any mask, and all passes:
  * nlfa_bwd_workspace_kernel_count).  On the tensor-core path at
- * D = 64 a large problem (at least sixteen 128-row query tiles per SM; not under windows of up
- * to 128, nor where one key block with sinks is more than an SM's share of the dK/dV pass) takes two:
+ * D = 64 a large problem (at least sixteen 128-row query tiles per SM; not under windows of fewer
+ * than 128 recent keys, nor where one key block with sinks is more than an SM's share of the dK/dV pass) takes two:
  * the dQ pass forms Delta itself -- the row sums of dO * O, added in the order of
  * the Delta kernel, so the gradients are bit-identical either way -- and runs
  * before the dK/dV pass; smaller problems and other head dims take the three

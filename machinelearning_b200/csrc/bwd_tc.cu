@@ -1342,8 +1342,10 @@ int launch_mode(const Problem& p, const void* dout, const void* q, const void* k
 // of H = 12, T = 1024: the dQ pass can then start beside the dK/dV pass, and a short Delta kernel
 // costs less than the later start of the first unit); with sixteen or more it gains 1-6% (B=130 H=12 T=256 204 -> 193 us,
 // B=32 T=1024 320 -> 313, B=12 H=8 T=8192 window 600 748 -> 722).  Two kinds of windows stay with the three kernels at
-// any size.  Up to a tile wide, the units are too short to hide the next one's Delta (H=16 T=4096 window 64 B=5 172.3 against
-// 175.0 us, B=12 406 / 410, with 4 sinks 485 / 495; H=12/4 window 200 B=8 220 against 211 the other way).  And blocks with
+// any size.  With fewer recent keys than a tile's rows, the units are too short to hide the next one's Delta, and both edges of the mask
+// cut the diagonal blocks (110 shapes; 120 to 127 recent keys: two kernels 5% slower to 2% faster, most 1-2% slower; 128 and 129
+// 2-8% faster, in groups of 16 equal or slower, with sinks equal; two / three, us: B=12 H=16/4 T=3000 window 127 248 / 244, B=11 H=12
+// T=8192 window 140, 20 sinks 664 / 652; B=30 H=8 T=4096 window 128 458 / 490, B=15 H=16/4 T=4096 window 129 374 / 393).  And blocks with
 // sinks are seen by every query behind them, units of up to a whole head group's iterations: where one of those is longer than
 // a CTA's share of the dK/dV pass, the dQ pass has to run beside it.  Of 120 random shapes two kernels were up to 5% faster below
 // that line and at most 4% slower, three up to 1.4x beyond it; two / three kernels, us: longest unit of 0.80 shares (B=12
@@ -1362,7 +1364,7 @@ inline bool delta_in_dq_pass(const Problem& p, int passes) {
   const long long tiles = static_cast<long long>(p.B) * p.H * ((p.T + kTile - 1) / kTile);
   if (tiles < 16ll * sm_count()) return false;
   if (p.window <= 0) return true;
-  if (p.window <= kTile) return false;
+  if (p.window - p.sinks < kTile) return false;
   if (p.sinks <= 0) return true;
   const DkvWork w = dkv_work(p.T, p.window, p.sinks);
   return w.longest * sm_count() <= w.total * p.B * p.Hkv;                    // longest <= a CTA's share
