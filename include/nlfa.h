@@ -125,7 +125,7 @@ int nlfa_bwd_workspace_kernel_count(int B, int T, int H, int Hkv, int D, int win
  * taped lse.  Replaces `flash_attn_bwd` (nanolab/csrc/flash_attn_cuda.cu:1744-1813)
  * and its launch sequence (:1518-1587): Delta kernel, dK/dV kernel, dQ kernel on
  * one stream (two kernels for large problems at D = 64, see
- * nlfa_bwd_kernel_count), no atomics, bit-reproducible.  `scratch` must hold
+ * nlfa_bwd_masked_kernel_count), no atomics, bit-reproducible.  `scratch` must hold
  * nlfa_bwd_scratch_bytes(B, T, H) bytes; Delta is left in it. */
 int nlfa_bwd(const void* dout, const void* q, const void* k, const void* v, const void* o,
              const float* lse, void* dq, void* dk, void* dv, void* scratch, size_t scratch_bytes,
@@ -148,8 +148,8 @@ int nlfa_bwd_passes(const void* dout, const void* q, const void* k, const void* 
                     size_t scratch_bytes, int B, int T, int H, int Hkv, int D, float scale,
                     int window, int sinks, int dtype, int path, int passes, void* stream);
 
-/* How many kernels nlfa_bwd_passes launches for this problem without a window on the
- * current device (0 for inputs it would refuse; for any mask, and all passes:
+/* How many kernels nlfa_bwd_masked launches on the current device for this problem, mask and choice of passes
+ * with a scratch that holds the tape alone (0 for inputs it would refuse; with more scratch, and every pass:
  * nlfa_bwd_workspace_kernel_count).  On the tensor-core path at
  * D = 64 a large problem (at least sixteen 128-row query tiles per SM; not under windows of fewer
  * than 128 recent keys, nor where one key block with sinks is more than an SM's share of the dK/dV pass) takes two:
@@ -157,6 +157,10 @@ int nlfa_bwd_passes(const void* dout, const void* q, const void* k, const void* 
  * the Delta kernel, so the gradients are bit-identical either way -- and runs
  * before the dK/dV pass; smaller problems and other head dims take the three
  * kernels named above.  For launch accounting (bench.py's `gpu_launches`). */
+int nlfa_bwd_masked_kernel_count(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
+                                 int path, int passes);
+
+/* The same without a window: what nlfa_bwd_passes launches with window == 0. */
 int nlfa_bwd_kernel_count(int B, int T, int H, int D, int dtype, int path, int passes);
 
 /* nlfa_bwd_passes with the mask given in full (`block` as in nlfa_fwd_masked). */

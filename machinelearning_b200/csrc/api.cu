@@ -557,6 +557,14 @@ int nlfa_bwd_fused(const void* dout, const void* q, const void* k, const void* v
                          fused ? (NLFA_PASS_DELTA | NLFA_PASS_FUSED) : NLFA_PASS_ALL, stream);
 }
 
+int nlfa_bwd_masked_kernel_count(int B, int T, int H, int Hkv, int D, int window, int sinks, int block, int dtype,
+                                 int path, int passes) {
+  Problem p{B, T, H, Hkv, D, window, sinks, 1.f, dtype, block};
+  if (check_problem(p) != NLFA_OK) return 0;
+  simplify_mask(p);
+  return passes_kernel_count(p, path, passes);
+}
+
 int nlfa_bwd_kernel_count(int B, int T, int H, int D, int dtype, int path, int passes) {
   return passes_kernel_count(Problem{B, T, H, H, D, 0, 0, 1.f, dtype, 0}, path, passes);
 }

@@ -175,6 +175,23 @@ def test_backward_kernel_count_of_a_window(lib, window, sinks, block, kernels):
     assert count(32) == 3
 
 
+def test_backward_kernel_count_of_any_passes_under_a_mask(lib):
+    from machinelearning_b200 import _lib as L
+    bf16, tensor = L.DTYPE_BF16, L.PATH_TENSOR
+    count = lambda passes, window=0, sinks=0, block=0, D=64, B=1024, Hkv=16, dtype=bf16: lib.nlfa_bwd_masked_kernel_count(
+        B, 4096, 16, Hkv, D, window, sinks, block, dtype, tensor, passes)
+    for mask in ((0, 0, 0), (256, 0, 0), (64, 0, 0), (64, 4, 0), (300, 4, 0), (0, 0, 96), (9000, 5, 0)):
+        kernels = count(L.PASS_ALL, *mask)
+        assert kernels == lib.nlfa_bwd_workspace_kernel_count(1024, 4096, 16, 16, 64, *mask, bf16, tensor, 0)
+        assert count(L.PASS_DELTA | L.PASS_DQ, *mask) == kernels - 1 and count(L.PASS_DKV, *mask) == 1
+        assert count(L.PASS_DELTA | L.PASS_FUSED, *mask) == 3 and count(L.PASS_ALL, *mask, D=128) == 3
+    for passes in range(16):
+        assert count(passes) == lib.nlfa_bwd_kernel_count(1024, 4096, 16, 64, bf16, tensor, passes)
+    assert count(L.PASS_ALL, 64) == 3 and count(L.PASS_ALL, 256) == 2
+    for bad in (dict(window=4, sinks=4), dict(window=64, block=8), dict(Hkv=3), dict(Hkv=0), dict(D=48), dict(B=0), dict(dtype=L.DTYPE_F32)):
+        assert count(L.PASS_ALL, **bad) == 0
+
+
 def test_workspace_sizes_of_extreme_extents(lib):
     """Sizes whose tile arithmetic leaves 32 bits: one pair's dS is beyond the limit, so the tape alone is asked for; a block
     length or a number of sinks next to 2^31 means what T does."""
