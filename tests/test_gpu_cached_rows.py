@@ -41,9 +41,14 @@ def test_rows_of_a_split_cache_match_the_oracle(T, H, Hkv, L, D, causal, window,
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("T,H,Hkv,L,D", [
-    (64, 16, 16, 2048, 128),                # finished eight columns a thread: more than 256 pieces of four
-    (128, 3, 3, 1500, 64),                  # .. one copy, rows that do not divide by the CTAs
-    (32, 12, 12, 1056, 64),                 # .. four columns a thread
+    # the rows a CTA finishes, eight columns a thread: at most two CTAs share four key blocks, so more than 256 pieces of four
+    (64, 16, 16, 500, 128),                 # .. two copies of the rows
+    (30, 16, 16, 500, 128),                 # .. four
+    (101, 3, 3, 300, 128),                  # .. one, rows that do not divide by the CTAs
+    (77, 4, 4, 500, 64),
+    (64, 16, 16, 2048, 128),                # split over eight CTAs: just 256 pieces of four
+    (128, 3, 3, 1500, 64),                  # one copy, up to six CTAs, which the rows do not divide by
+    (32, 12, 12, 1056, 64),                 # four columns a thread: at most 256 pieces of four however it is split
     (70, 2, 2, 1300, 32),                   # head dim 32: the second warpgroup's half of the columns is none
     (9, 160, 160, 400, 32),                 # .. whole tiles, finished where their sums are
     (100, 150, 150, 300, 128),              # whole tiles, one copy: 64 columns a thread

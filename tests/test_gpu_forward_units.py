@@ -16,20 +16,29 @@ CASES = [(1, 4200, 5, 1, 64, 0, 0, 0, torch.bfloat16), (1, 4353, 6, 2, 32, 0, 0,
          (1, 1100, 4, 2, 32, 200, 5, 0, torch.bfloat16), (3, 700, 6, 2, 128, 0, 0, 96, torch.float16)]
 
 
-# key blocks of 64: few columns for any number of tiles, fewer from 4.5 tiles per SM on, as many from eight on; the edges of a
-# window at, before and behind a block's, sinks of one block and of two, ragged rows; T = 63 .. 65 into a block, rows inside one
-NARROW = [(1, 3000, 2, 1, 64, 64, 4, 0, torch.bfloat16), (1, 1089, 4, 2, 32, 50, 0, 0, torch.float16),
-          (1, 2111, 3, 3, 64, 128, 64, 0, torch.float16), (1, 191, 2, 2, 32, 65, 1, 0, torch.bfloat16),
-          (8, 1500, 9, 3, 64, 300, 4, 0, torch.bfloat16), (8, 1473, 9, 9, 32, 333, 70, 0, torch.float16),
+# one tile of each kind of mask next to the line between the widths of key blocks, and masks with many tiles
+CASES += [(8, 1500, 9, 3, 64, 300, 4, 0, torch.bfloat16), (8, 1473, 9, 9, 32, 333, 70, 0, torch.float16),
           (12, 1100, 12, 4, 64, 200, 0, 0, torch.bfloat16), (12, 1025, 12, 12, 64, 256, 0, 0, torch.float16),
           (12, 1000, 12, 4, 32, 0, 0, 0, torch.bfloat16), (12, 1088, 12, 12, 32, 0, 0, 100, torch.float16),
-          (30, 450, 12, 6, 32, 0, 0, 0, torch.bfloat16), (60, 63, 20, 4, 32, 0, 0, 16, torch.bfloat16)]
+          (30, 450, 12, 6, 32, 0, 0, 0, torch.bfloat16), (60, 63, 20, 4, 32, 0, 0, 16, torch.bfloat16),
+          (1, 191, 2, 2, 32, 65, 1, 0, torch.bfloat16), (2, 256, 3, 3, 64, 30, 0, 0, torch.float16),
+          (2, 1000, 3, 3, 64, 66, 0, 0, torch.bfloat16), (2, 1000, 3, 1, 32, 120, 65, 0, torch.bfloat16)]
+
+# key blocks of 64: the edges of a window at, before and behind a block's, sinks of part of a block and of a whole one, ragged rows;
+# the shortest row that gets them, its last tile one row high; T = 63 .. 65 into a block, few tiles and many
+NARROW = [(1, 3000, 2, 1, 64, 64, 4, 0, torch.bfloat16), (1, 1089, 4, 2, 32, 50, 0, 0, torch.float16),
+          (1, 2111, 3, 3, 64, 128, 64, 0, torch.float16), (2, 257, 2, 2, 32, 66, 1, 0, torch.bfloat16),
+          (8, 1500, 9, 3, 64, 69, 4, 0, torch.bfloat16), (8, 1473, 9, 9, 32, 2, 0, 0, torch.float16),
+          (12, 1024, 12, 4, 64, 65, 0, 0, torch.bfloat16), (12, 1025, 12, 12, 64, 33, 20, 0, torch.float16),
+          (1, 4096, 3, 1, 64, 64, 0, 0, torch.float16), (30, 448, 12, 6, 32, 129, 64, 0, torch.bfloat16)]
 
 
-@pytest.mark.parametrize("B,T,H,Hkv,D,window,sinks,block,dtype", CASES + NARROW)
-def test_forward_in_both_unit_heights(B, T, H, Hkv, D, window, sinks, block, dtype):
+@pytest.mark.parametrize("B,T,H,Hkv,D,window,sinks,block,dtype,width", [(*c, 128) for c in CASES] + [(*c, 64) for c in NARROW])
+def test_forward_in_both_unit_heights(B, T, H, Hkv, D, window, sinks, block, dtype, width):
     from machinelearning_b200 import flash_cuda as fc
     assert fc.is_available(), fc.unavailable_reason()
+    from machinelearning_b200 import _lib
+    assert fc._load().nlfa_fwd_key_block(T, D, window, sinks, block, _lib.DTYPE_BF16, _lib.PATH_TENSOR) == width
     g = torch.Generator(device="cuda").manual_seed(T + D)
     q, k, v = (torch.randn(B, T, h, D, device="cuda", generator=g).to(dtype) for h in (H, Hkv, Hkv))
     scale = D ** -0.5
