@@ -115,11 +115,11 @@ template <int MODE, int YR>
 __device__ __forceinline__ BwdUnit<MODE> make_bwd_unit(int u, const BwdParams& p) {
   BwdUnit<MODE> w;
   // Heaviest units first (rank = stationary tile), all (batch, head) pairs of one rank together.
-  // The key-block-stationary passes do this in groups of `sched_group` (batch, KV head) pairs (one
-  // per CTA of the launch), so that a head's tiles -- and in the fused pass its fp32 dQ sums -- are
-  // still in L2 when its next key block comes round (dK/dV pass at B=32, H=12, T=1024: 0.145 ->
-  // 0.139 ms), while a key block still starts a whole wave of units after the block below it,
-  // whose dQ turns the fused pass waits for.
+  // The key-block-stationary passes do this in groups of `sched_group` (batch, KV head) pairs, so that a head's tiles --
+  // and in the fused pass its fp32 dQ sums -- are still in L2 when its next key block comes round (dK/dV pass at B=32, H=12,
+  // T=1024: 0.145 -> 0.139 ms).  The fused pass keeps one pair per CTA of the launch: a key block then starts a whole wave
+  // of units after the block below it, whose dQ turns it waits for.  The dK/dV pass has no turns, and its groups may be smaller
+  // (group_of_pairs, and the rule on L2 beside it).
   int rank, bh;
   if (MODE == MODE_FUSED || p.sched_group < p.BH) {
     const int per_group = p.sched_group * p.n_tiles;
@@ -688,8 +688,10 @@ bwd_tc_kernel(const __grid_constant__ CUtensorMap tm_x0, const __grid_constant__
     };
     // dK/dV over 64-row tiles: the row statistics of the next tile are requested as soon as this one's are in shared memory,
     // so that their latency (900 of 1,300 clocks per tile, against 1,850 of an iteration) passes while this warp waits for a
-    // free stage.  B=2 H=16/8 T=8192 window 512, D = 128: backward 428 -> 397 us; B=4 H=12/4 T=2048 191.6 -> 189.8.  At
-    // D <= 64 an iteration has time for it, and the kernel came out slower (B=16 H=16 T=4096 window 256 dK/dV 278 -> 291 us).
+    // free stage.  Backward under load, D = 128: B=16 H=12/4 T=512 84.1 -> 82.6 us, B=4 H=12/4 T=2048 196.1 -> 195.2, B=1 H=16/4 T=8191
+    // 875 -> 867, B=2 H=16/8 T=8192 window 512 with 4 sinks 427 -> 424, without 329 / 329; all but the first within the spread of
+    // one side.  At D <= 64 an iteration has time for it, and the kernel came out slower (B=16 H=16 T=4096 window 256 dK/dV 278 ->
+    // 291 us).
     constexpr bool kStatsAhead = kKeyStat && YR == 64;
     float stat_lse[YR / 32], stat_delta[YR / 32];
     auto load_stats = [&](const BwdUnit<MODE>& w, int idx, int h) {

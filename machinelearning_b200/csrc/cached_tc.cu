@@ -32,7 +32,9 @@
 // memory; no element has a branch of its own (a condition on the number of blocks inside the loop over columns cost 34 clocks
 // a column); a thread finishing a row loads all of its parts at once.  Before / after (us): B=1 H=12 D=64, 32 over 1,056
 // 6.3 / 5.7; B=1 H=16 D=128, 64 over 2,048 10.5 / 9.5, 64 over 16,448 31.0 / 28.0 (4.8 TB/s of K, V), 128 over 4,096 17.6 / 15.1;
-// B=1 H=2 D=64, 100 over 129 13.4 / 9.7; one query over 1,057 (SPLIT_P) 6.8 / 6.1.
+// B=1 H=2 D=64, 100 over 129 13.4 / 9.7; one query over 1,057 (SPLIT_P) 6.8 / 6.1.  It costs registers: every variant spills (12 to
+// 84 bytes stored and 96 to 480 loaded a thread; 0 to 68 and 0 to 252 with the former end), since a thread is compiled for the 168
+// that 384 threads start with, and the softmax warps' 216 come later.
 //
 // SPLIT_P: blocks so small that the fp32 kernel used to take them keep its precision: P goes in as the sum of two
 // 16-bit values (its rounding error is then below the accumulator's), at the price of a second P V product,

@@ -41,7 +41,8 @@ __host__ __device__ inline int first_query_of_key(int k, int block) {
 }
 
 // Division of a non-negative int by a divisor the host knows: q = (mulhi(n, mul) + n) >> shift with 2^shift >= d and
-// mul = floor(2^32 (2^shift - d) / d) + 1, the usual round-up method, exact for every n < 2^31.
+// mul = floor(2^32 (2^shift - d) / d) + 1 (Granlund and Montgomery, "Division by Invariant Integers using Multiplication",
+// PLDI 1994, figure 4.1), exact for every n < 2^31.
 struct FastDiv {
   unsigned mul, shift;
   int d;
