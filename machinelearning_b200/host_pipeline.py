@@ -11,8 +11,11 @@ PCIe is full duplex, so a step costs about the larger of the two copy times
 instead of the sum of both copies and the kernels.
 
 There is no counterpart in the reference: its callers hold device tensors
-(``nanolab/mixers.py:347-370``).  Results are bit-identical to one whole-batch
-call, because every kernel treats batch elements independently.
+(``nanolab/mixers.py:347-370``).  Every kernel treats batch elements independently,
+and on the tensor-core path no choice that reaches the bits looks at how many there
+are: float16 and bfloat16 results are bit-identical to one whole-batch call.  The
+float32 kernels take rows in registers, eight a thread at head dims up to 64 where
+there are enough tiles, and sum in another order then: equal up to rounding.
 """
 from __future__ import annotations
 
