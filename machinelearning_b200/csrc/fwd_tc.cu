@@ -780,12 +780,14 @@ int launch_t(const Problem& p, const CUtensorMap& mq, const CUtensorMap& mk, con
 // block of 64, a full tile visits 192 + 64 columns in blocks of 64 and 256 + 128 in blocks of 128 (a cut tile at the end of the
 // row does not count, nor do rows of up to two tiles, which have no full one).  The two widths round P at different references,
 // so the choice follows from the mask and the row's length alone: any slice of the batch or of the heads has the bits of the
-// whole call.  Blocks of 128 / 64, us, at about 0.5, 1, 2, 2.6, 4 and 8 tiles per SM:
-//   T=4096 D=64 window 64             8.9/8.5 9.5/9.5 10.1/10.4 13.0/9.9 17.3/15.2 25.1/21.1   (long rows, 16 per SM: 46.5/38.5)
-//   T=4096 D=64 window 64, 4 sinks    9.5/9.3 11.3/10.6 11.6/11.6 .. 22.0/17.3 33.2/25.0        D=32 .. 21.2/15.9 32.0/22.7
-// of 36 such masks and lengths (300 to 16,384) the worst is 0.96 of the speed, below two tiles per SM, the best 1.42.  Every
-// other mask loses somewhere: 66 to 129 recent keys 0.84 to 1.1, 130 to 193 0.88 to 1.25, 300 0.81 to 1.17, sinks in two
-// blocks of 64 0.85 to 1.18, one or two tiles per row 0.84 to 1.3.
+// whole call.  T=4096, blocks of 128 / 64, us, at 0.4, 1.1, 1.9, 2.6, 4.5, 8 and 16 tiles per SM:
+//   D=64 window 64             8.4/8.5   9.5/9.2  10.1/10.1  13.9/10.4  17.3/14.6  25.5/21.1  46.6/38.4
+//   D=64 window 64, 4 sinks    9.7/9.5  11.1/10.5 11.6/11.5  15.6/11.8  22.1/17.0  33.4/24.8  59.6/44.7
+//   D=32 window 64, 4 sinks    9.5/8.8  10.8/8.9  11.3/11.3  15.2/11.5  21.3/16.2  32.0/22.7  56.6/40.4
+// Over windows of 2 to 65 recent keys, with and without sinks, rows of 258 to 16,384 and 0.4 to 16 tiles per SM 0.95 to 1.44 of
+// the speed, at two tiles per SM and beyond never below 0.96.  Every other mask loses somewhere: 66 to 129 recent keys 0.82 to
+// 1.2, 130 to 193 0.86 to 1.3, 258 to 321 0.81 to 1.2, sinks in two blocks of 64 0.85 to 1.2, rows of one tile 0.86 to 1.1, of two
+// 0.83 to 1.36.
 bool narrow_blocks(const Problem& p) {
   const int recent = p.window - p.sinks;
   return p.D <= 64 && p.window > 0 && p.T > 2 * kTile && p.sinks <= 64 && recent >= 2 && recent <= 65;
